@@ -27,8 +27,8 @@ EPS = 1e-6
 
 def listed():
     return [
-        # the smallest call of all: one 4096 x 4096 matvec, latency and launch cost count as much as bytes
-        {"name": "matvec_q8_0", "kind": "mul_mat", "dtype": "q8_0", "k": 4096, "n": 4096, "m": 1},
+        # the smallest call: one matvec over the joined Q, K and V rows of a layer, launch cost and latency count as much as bytes
+        {"name": "matvec_q8_0", "kind": "mul_mat", "dtype": "q8_0", "k": 4096, "n": 6144, "m": 1},
         # the vocabulary head of a Q4_K_M model: one activation column over the largest matrix there is
         {"name": "head_q6_k", "kind": "mul_mat", "dtype": "q6_k", "k": 4096, "n": 151936, "m": 1},
         # the projections of decode, one column, as a program replays them: one graph over four layers' matrices
