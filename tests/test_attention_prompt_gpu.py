@@ -1,0 +1,74 @@
+"""GPU parity of the many-query attention kernel (head dimension 128, enough row tiles to occupy the GPU) against the CPU oracle.
+
+Tolerance: f32 throughout; sums of up to a few hundred rounded terms in chains of 32, so about 3e-7 relative: NMSE 1e-12 (ten times
+that squared)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import sgref
+from tests import util as U
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+SCALE = float(1.0 / np.sqrt(128))
+
+
+def _run(sm100, stream, q, k, v, causal, offset, mask=None, mask_heads=1, positions=None):
+    hq, nq, d = q.shape
+    hkv, nk, _ = k.shape
+    qb, kb, vb = (U.to_device(sm100, stream, a) for a in (q, k, v))
+    mb = U.to_device(sm100, stream, mask) if mask is not None else None
+    pb = U.to_device(sm100, stream, np.array(positions, np.int32)) if positions is not None else None
+    ob, optr = U.guarded_output(sm100, stream, hq * nq * d)
+    before = sm100.lib().sm100_launch_count()
+    sm100.check(sm100.lib().sm100_attention(stream.handle, qb.at(), kb.at(), vb.at(), mb.at() if mb else None, mask_heads, C.c_void_p(optr), d, d, nq, nk, hq, hkv,
+                                            int(causal), offset, pb.at() if pb else None, SCALE), "attention")
+    assert sm100.lib().sm100_launch_count() - before == 1
+    stream.sync()
+    return U.read_guarded(sm100, stream, ob, hq * nq * d).reshape(hq, nq, d).copy()
+
+
+def _inputs(hq, hkv, nq, nk, seed=0):
+    rng = np.random.default_rng(hq * 100 + nq + nk + seed)
+    return tuple(rng.standard_normal(s).astype(np.float32) for s in ((hq, nq, 128), (hkv, nk, 128), (hkv, nk, 128)))
+
+
+# whole and ragged row tiles, heads per group 1, 3, 4, 8; one key tile, a partial one, several; the first query sees one key or many
+@pytest.mark.parametrize("hq,hkv,nq,nk", [(32, 8, 128, 128), (32, 8, 131, 200), (48, 16, 70, 97), (64, 64, 65, 65), (64, 8, 64, 33), (32, 8, 128, 31)], ids=lambda v: str(v))
+def test_causal_full_and_masked(sm100, stream, hq, hkv, nq, nk):
+    q, k, v = _inputs(hq, hkv, nq, nk)
+    off = max(nk - nq, 0)
+    want = sgref.attention(q, k, v, True, off, SCALE)
+    assert sgref.nmse(_run(sm100, stream, q, k, v, True, off), want) <= TOL
+    assert sgref.nmse(_run(sm100, stream, q, k, v, True, 0, positions=[off]), want) <= TOL
+    assert sgref.nmse(_run(sm100, stream, q, k, v, False, 0), sgref.attention(q, k, v, False, 0, SCALE)) <= TOL
+    for low in (-np.inf, np.finfo(np.float32).min):
+        mask = np.zeros((1, nq, nk), np.float32)
+        mask[0, :, nk // 3:] = low
+        got = _run(sm100, stream, q, k, v, False, 0, mask=mask)
+        assert sgref.nmse(got, sgref.attention(q, k[:, :nk // 3], v[:, :nk // 3], False, 0, SCALE)) <= TOL
+    per_head = (0.5 * np.random.default_rng(3).standard_normal((hq, nq, nk))).astype(np.float32)
+    got = _run(sm100, stream, q, k, v, True, off, mask=per_head, mask_heads=hq)
+    g = hq // hkv
+    s = np.einsum("hqd,hkd->hqk", q.astype(np.float64), np.repeat(k, g, 0).astype(np.float64)) * SCALE + per_head
+    s[:, np.arange(nk)[None] > off + np.arange(nq)[:, None]] = -np.inf
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = np.einsum("hqk,hkd->hqd", p / p.sum(-1, keepdims=True), np.repeat(v, g, 0).astype(np.float64))
+    assert sgref.nmse(got.astype(np.float64), want) <= TOL
+
+
+def test_rows_without_keys_and_hidden_values(sm100, stream):
+    """Queries before the first key give zeros; a value row holding NaN or infinity reaches the queries that see it and no other."""
+    hq, hkv, nq, nk = 32, 8, 140, 120
+    q, k, v = _inputs(hq, hkv, nq, nk)
+    got = _run(sm100, stream, q, k, v, True, -20)
+    want = sgref.attention(q[:, 20:], k, v, True, 0, SCALE)
+    assert np.all(got[:, :20] == 0.0) and sgref.nmse(got[:, 20:], want) <= TOL
+    bad = v.copy()
+    bad[:, 100, 5] = np.nan
+    bad[:, 110, 9] = np.inf
+    got2 = _run(sm100, stream, q, k, bad, True, -20)
+    assert np.array_equal(got2[:, :120], got[:, :120])
+    assert np.isnan(got2[:, 120:, 5]).all() and not np.isfinite(got2[:, 130:, 9]).any()
