@@ -1,0 +1,547 @@
+// MUL_MAT of packed quantized weights on the fifth-generation tensor cores at the precision of the integer matvecs:
+// batches of up to 32 activation columns, and prompts of any length over Q6_K weights.
+//
+//   y[N, M] = W[K, N] . x[K, M]      values of src/core/ref/quant.cpp:30-108 and src/core/ref/ops.cpp:891-984
+//
+// The f16 GEMM (sm100_gemm.cu) rounds both operands to 11 bits (relative error 3e-4).  Here both are split into two
+// bf16 numbers, w = wh + wl and x = xh + xl (16 bits of each, any magnitude a float has: no scaling, no overflow), and
+//   w x = wh xh + (wh xl + wl xh)
+// is three bf16 products with f32 accumulation (wl xl, below 2^-17, is taken along where it costs nothing).  The large and the small products have
+// accumulators of their own (the tensor core truncates when it adds, so the long chain holds the large products only).
+//
+// One CTA takes 128 weight rows x TN tokens.  Warp 0 owns tensor memory and issues the MMAs; two or three groups of eight warps from warp 4 on dequantize
+// the weights chunk by chunk (64 weights of each row) in packed bf16 arithmetic and store wh and wl to tensor memory, the A
+// operand of the MMA.  Two ways for the activations:
+//   PREP = false  (up to 32 tokens)  warps 1-3 and 20-24 read the f32 rows, split them and store the stage themselves: no launch
+//                                     and no memory for it.  The padding tokens of a stage are zeroed once.
+//   PREP = true   (prompts)          split_prep_x writes the stage images once per call, warps 1-3 fetch them by bulk copy.
+// Few tiles, or a last wave of few, leave SMs idle: such tiles have their K range cut over several CTAs (plan_tiles), whose partial
+// tiles go to scratch memory of the call; split_reduce adds them in a fixed order.
+//
+// What bounds it: up to 32 tokens the hand-over from chunk to chunk and the dequantizing warps (about 900 cycles a chunk of 64
+// weights x 128 rows), with prompts the tensor core (12 MMAs of 64 cycles in a chunk's 1090).  Measured, us, before / now: Q4_0
+// 4096 x 12288, 8 columns 64 / 30; Q4_K 12288 x 4096, 24 columns 63 / 37; Q6_K 12288 x 4096, 512 columns 3740 / 168 (before: one
+// launch per 8 or 4 columns).  Tried: K over a cluster with the exchange in distributed shared memory (wrong sums; taken out),
+// three converting warps with their loads in registers (Q4_K, 24 columns: 41).
+//
+// Every wait is bounded; a CTA that gives up raises the fault flag (reported by the next stream synchronisation), drains its copies,
+// frees its TMEM and returns.
+#include "sm100_common.cuh"
+#include "sm100_gemm_src.cuh"
+#include "sm100_tc.cuh"
+
+#include <atomic>
+
+namespace sm100 {
+
+int call_scratch_alloc(cudaStream_t s, size_t bytes, void ** out);
+int call_scratch_free(cudaStream_t s, void * p);
+
+namespace {
+
+constexpr int SP_TM = 128;             // weight rows per CTA = TMEM lanes
+constexpr int SP_KC = 64;              // weights of a row per chunk
+constexpr int SP_FIRST_PRODUCER = 4;
+// Groups of 8 producer warps, a chunk each in turn, and the warps that bring the activations: three issue bulk copies, or eight
+// convert (a lane per 8 weights of a token: with three such warps they bounded 32 columns, 1320 cycles a chunk).
+template <bool PREP> constexpr int sp_groups = PREP ? 3 : 2;
+template <bool PREP> constexpr int sp_threads = 32 * (SP_FIRST_PRODUCER + 8 * sp_groups<PREP> + (PREP ? 0 : 5));
+constexpr int SP_BULK_WARPS = 3, SP_CONVERT_WARPS = 8;
+constexpr int SP_A_COLS = 64;          // TMEM columns of a weight stage: wh (32), wl (32)
+
+__device__ int g_split_fault;   // 0, or 1 + the wait site that gave up
+
+struct SplitArgs {
+    WeightRef w;
+    const float * x;           // PREP = false: activations, column stride ldx
+    int64_t ldx;
+    const uint8_t * image;     // PREP = true: prepared stages of all token tiles
+    float * y;
+    int64_t ldy;
+    float * part;              // partial tiles of the cut ones: [split][tile][TN tokens][128 rows]
+    int n, m, k;
+    int nchunks, m_tiles;
+    int whole, cut, splits;    // TilePlan
+};
+
+// PREP = false: f32 activation chunks on their way, each lane's own 32 bytes per task (cp.async, read back by the same lane)
+template <int TN, bool PREP>
+struct SplitSmem {
+    static constexpr int B_BYTES = 2 * TN * SP_KC * 2;                  // a stage: [k / 8][xh of TN tokens, xl of TN tokens][8]
+    static constexpr int SB = TN >= 128 ? 6 : 8;
+    static constexpr int ACC_COLS = (TN <= 64 ? 4 : 2) * TN;
+    static constexpr int SA = (512 - ACC_COLS) / SP_A_COLS < 6 ? (512 - ACC_COLS) / SP_A_COLS : 6;
+    static constexpr int XS = 6;                                        // f32 chunks in flight
+    uint8_t b[SB][B_BYTES];
+    float4 x[PREP ? 1 : XS][2][PREP ? 1 : 32 * SP_CONVERT_WARPS];
+    uint64_t full_a[SA], empty_a[SA], full_b[SB], empty_b[SB];
+    uint64_t accum;
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+// The MMAs of a chunk.  All of one shape on an accumulator: the tensor core keeps those in order, it promises nothing for different
+// shapes.  An MMA takes at least about 60 cycles, the time to read its A operand from tensor memory, whatever its columns.
+//   TN <= 64: per 16-weight step two MMAs of 2 TN columns, wh [xh | xl] into D and wl [xh | xl] into the 2 TN columns behind it
+//   TN = 128: three of TN columns, wh xh into D, wh xl and wl xh into the TN columns behind it
+template <int TN>
+__device__ __forceinline__ void mma_chunk_split(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    constexpr uint64_t B_STEP = (uint64_t) (2 * (2 * TN * 16)) >> 4, B_LOW = (uint64_t) (TN * 16) >> 4;
+#pragma unroll
+    for (int ks = 0; ks < SP_KC / 16; ++ks) {
+        const uint32_t acc = ks == 0 ? accumulate : 1u;
+        const uint64_t bh = b_desc + (uint64_t) ks * B_STEP, bl = bh + B_LOW;
+        const uint32_t ah = a + 8u * ks, al = ah + 32u;
+        if constexpr (TN <= 64) {
+            asm volatile(
+                "{\n\t.reg .pred e, pacc;\n\t"
+                "elect.sync _|e, 0xffffffff;\n\t"
+                "setp.ne.b32 pacc, %6, 0;\n\t"
+                "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], %4, %5, pacc;\n\t"
+                "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [%3], %4, %5, pacc;\n\t}" ::"r"(d),
+                "r"(d + 2 * TN), "r"(ah), "r"(al), "l"(bh), "r"(idesc), "r"(acc)
+                : "memory");
+        } else {
+            asm volatile(
+                "{\n\t.reg .pred e, pacc, pone;\n\t"
+                "elect.sync _|e, 0xffffffff;\n\t"
+                "setp.ne.b32 pacc, %7, 0;\n\t"
+                "setp.eq.b32 pone, %7, %7;\n\t"
+                "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], %4, %6, pacc;\n\t"
+                "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %5, %6, pacc;\n\t"
+                "@e tcgen05.mma.cta_group::1.kind::f16 [%1], [%3], %4, %6, pone;\n\t}" ::"r"(d),
+                "r"(d + TN), "r"(ah), "r"(al), "l"(bh), "l"(bl), "r"(idesc), "r"(acc)
+                : "memory");
+        }
+    }
+}
+
+// step ST of a warp's 16 rows: wh into the stage's columns 8 ST .., wl into 32 + 8 ST ..
+template <typename S, int ST>
+__device__ __forceinline__ void put_step(const typename S::Regs & r, int t, const typename S::ScaleSplit (&sc)[2], uint32_t dst) {
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t a[2], b[2];
+        S::template step<ST>(r, h, t, sc[h], a, b);
+        hi[2 * h] = a[0]; hi[2 * h + 1] = a[1];
+        lo[2 * h] = b[0]; lo[2 * h + 1] = b[1];
+    }
+    tmem_st_frag1(dst + 8 * ST, hi);
+    tmem_st_frag1(dst + 32 + 8 * ST, lo);
+}
+
+template <typename S, int TN, bool PREP>
+__global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArgs g) {
+    using Smem = SplitSmem<TN, PREP>;
+    constexpr int SA = Smem::SA, SB = Smem::SB, ACC_COLS = Smem::ACC_COLS;
+    constexpr int SP_GROUPS = sp_groups<PREP>, SP_THREADS = sp_threads<PREP>, PRODUCERS = 8 * SP_GROUPS;
+    constexpr int DEPTH = 2;                                             // chunks of a producer group in flight in registers
+    constexpr int EPI_WARPS = TN >= 64 ? 16 : TN / 4;                    // of the first 16 producer warps
+    constexpr int EPI_COLS = TN / (EPI_WARPS / 4);                       // tokens an epilogue warp reads
+    static_assert(SA >= 2, "at least two weight stages");
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    Smem & sm = *reinterpret_cast<Smem *>(smem_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool in_part = (int) blockIdx.x >= g.whole;
+    const int cut_cta = (int) blockIdx.x - g.whole;
+    const int tile = in_part ? g.whole + cut_cta % g.cut : (int) blockIdx.x, split = in_part ? cut_cta / g.cut : 0, splits = in_part ? g.splits : 1;
+    const int mt = tile % g.m_tiles, nt = tile / g.m_tiles;
+    const int n0 = nt * SP_TM, m0 = mt * TN;
+    const int m_here = g.m - m0 < TN ? g.m - m0 : TN;                    // tokens of this tile
+    const int c_begin = (int) ((int64_t) split * g.nchunks / splits), c_end = (int) ((int64_t) (split + 1) * g.nchunks / splits);
+    volatile int * abort_flag = &sm.abort_flag;
+    auto wait = [&](uint32_t bar, uint32_t parity, int site, bool patient) {
+        return mbar_try_wait(bar, parity) || mbar_wait_bounded(bar, parity, abort_flag, &g_split_fault, site, patient);
+    };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SA; ++s) {
+            mbar_init(smem_addr(&sm.full_a[s]), 8);
+            mbar_init(smem_addr(&sm.empty_a[s]), 1);
+        }
+        for (int s = 0; s < SB; ++s) {
+            mbar_init(smem_addr(&sm.full_b[s]), PREP ? 1 : (m_here + 3) / 4);   // a converting warp has four tokens
+            mbar_init(smem_addr(&sm.empty_b[s]), 1);
+        }
+        mbar_init(smem_addr(&sm.accum), 1);
+        sm.abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (!PREP) {   // padding tokens are zero for good
+        for (int i = threadIdx.x; i < SB * Smem::B_BYTES / 16; i += SP_THREADS) reinterpret_cast<uint4 *>(sm.b)[i] = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async();
+    }
+    if (warp == 0) {
+        tmem_alloc(smem_addr(&sm.tmem_base), 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *(volatile uint32_t *) &sm.tmem_base;
+    const uint32_t full_a0 = smem_addr(&sm.full_a[0]), empty_a0 = smem_addr(&sm.empty_a[0]);
+    const uint32_t full_b0 = smem_addr(&sm.full_b[0]), empty_b0 = smem_addr(&sm.empty_b[0]);
+    const uint32_t b_smem = smem_addr(sm.b);
+
+    if (warp >= SP_FIRST_PRODUCER && warp < SP_FIRST_PRODUCER + PRODUCERS) {
+        // ---- weights (they do not depend on the predecessor on the stream): a group's eight warps take 16 rows each of a chunk
+        // (a warp may write its own quarter of the TMEM lanes only: rows 32 (warp % 4) + 16 (gw / 4) ..) ----
+        const int pw = warp - SP_FIRST_PRODUCER, group = pw >> 3, gw = pw & 7, t = lane & 3;
+        const uint32_t lanes = (uint32_t) (32 * (warp & 3) + 16 * (gw >> 2)) << 16;
+        typename S::Cursor cur;
+        {
+            const int64_t r0 = (int64_t) n0 + 32 * (warp & 3) + 16 * (gw >> 2) + (lane >> 2), last = g.n - 1;
+            const int64_t row[2] = {r0 < last ? r0 : last, r0 + 8 < last ? r0 + 8 : last};   // rows past the tensor: clamped, never stored
+            S::init(cur, g.w, row, t);
+        }
+        typename S::Regs ring[DEPTH];
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) {
+            const int c = c_begin + group + SP_GROUPS * d;
+            S::load(ring[d], cur, c < c_end ? c : c_end - 1);
+        }
+        bool alive = true;
+        for (int cb = c_begin + group; cb < c_end && alive; cb += SP_GROUPS * DEPTH) {
+#pragma unroll
+            for (int d = 0; d < DEPTH; ++d) {
+                const int c = cb + SP_GROUPS * d;
+                if (c >= c_end) break;
+                const int lc = c - c_begin, s = lc % SA;
+                const uint32_t phase = (uint32_t) (lc / SA) & 1u;
+                if (!__all_sync(0xffffffffu, wait(empty_a0 + 8 * s, phase ^ 1u, 0, true))) { alive = false; break; }
+                tc_fence_after();
+                const uint32_t dst = tmem + lanes + (uint32_t) (ACC_COLS + s * SP_A_COLS);
+                typename S::ScaleSplit sc[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) S::scale(ring[d], c, t, h, sc[h]);
+                put_step<S, 0>(ring[d], t, sc, dst);
+                put_step<S, 1>(ring[d], t, sc, dst);
+                put_step<S, 2>(ring[d], t, sc, dst);
+                put_step<S, 3>(ring[d], t, sc, dst);
+                const int cn = c + SP_GROUPS * DEPTH;
+                if (cn < c_end) S::load(ring[d], cur, cn);
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full_a0 + 8 * s);
+            }
+        }
+        pdl_wait();
+        pdl_launch_dependents();
+        // ---- epilogue: lane = row, a quarter (or half, or all) of the tokens per set of four warps ----
+        bool ok = alive && pw < EPI_WARPS;
+        if (ok) ok = wait(smem_addr(&sm.accum), 0u, 1, true);
+        if (__all_sync(0xffffffffu, ok)) {
+            tc_fence_after();
+            const uint32_t quarter = (uint32_t) (32 * (warp & 3)) << 16;
+            const int r_in = 32 * (warp & 3) + lane, col0 = (pw >> 2) * EPI_COLS;
+            const int64_t n_out = (int64_t) n0 + r_in;
+#pragma unroll 1
+            for (int cc = col0; cc < col0 + EPI_COLS && cc < m_here; cc += 16) {
+                uint32_t a[16], b[16];
+                float v[16];
+                tmem_ld16(tmem + quarter + (uint32_t) cc, a);
+                tmem_ld16(tmem + quarter + (uint32_t) (TN + cc), b);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(b[j]);
+                if constexpr (TN <= 64) {
+                    uint32_t c[16], d[16];
+                    tmem_ld16(tmem + quarter + (uint32_t) (2 * TN + cc), c);
+                    tmem_ld16(tmem + quarter + (uint32_t) (3 * TN + cc), d);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(c[j]) + __uint_as_float(d[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(a[j]);
+                if (!in_part) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (cc + j < m_here && n_out < g.n) g.y[(int64_t) (m0 + cc + j) * g.ldy + n_out] = v[j];
+                } else {
+                    float * part = g.part + ((int64_t) cut_cta * TN + cc) * SP_TM + r_in;   // rows past the tensor included: the tile is whole
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (cc + j < m_here) part[j * SP_TM] = v[j];
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp > 0) {
+        pdl_wait();
+        if (PREP) {
+            if (lane == 0 && warp <= SP_BULK_WARPS) {
+                const uint8_t * src = g.image + (int64_t) mt * g.nchunks * Smem::B_BYTES;
+                int last = -1;
+                for (int lc = warp - 1; lc < c_end - c_begin; lc += SP_BULK_WARPS) {
+                    const int s = lc % SB;
+                    if (!wait(empty_b0 + 8 * s, ((uint32_t) (lc / SB) & 1u) ^ 1u, 2, true)) break;
+                    mbar_expect_tx(full_b0 + 8 * s, Smem::B_BYTES);
+                    bulk_g2s(b_smem + s * Smem::B_BYTES, src + (int64_t) (c_begin + lc) * Smem::B_BYTES, Smem::B_BYTES, full_b0 + 8 * s);
+                    last = lc;
+                }
+                if (*abort_flag != 0) {   // giving up: this warp's last copies land before the shared memory goes away
+                    for (int lc = last; lc >= 0 && lc > last - SB; lc -= SP_BULK_WARPS) {
+                        const uint32_t bar = full_b0 + 8 * (lc % SB);
+                        for (uint32_t i = 0; i < (1u << 14) && !mbar_try_wait(bar, (uint32_t) (lc / SB) & 1u); ++i) __nanosleep(64);
+                    }
+                }
+            }
+        } else {
+            // ---- activations: a task is 8 weights of one token (consecutive in the chunk's order of K: eight lanes read a token's
+            // whole chunk), stored as two groups of four of xh and of xl ----
+            constexpr int XS = Smem::XS;
+            const int tid = (warp < SP_FIRST_PRODUCER ? warp - 1 : warp - SP_FIRST_PRODUCER - PRODUCERS + 3) * 32 + lane, tok = tid >> 3, j = tid & 7;
+            const int kk = S::k4(2 * j), p0 = S::pos4(2 * j), p1 = S::pos4(2 * j + 1);
+            const uint32_t at0 = (uint32_t) ((p0 >> 1) * (2 * TN * 16) + (p0 & 1) * 8), at1 = (uint32_t) ((p1 >> 1) * (2 * TN * 16) + (p1 & 1) * 8);
+            const bool live = tok < m_here;
+            const float * src = g.x + (int64_t) (live ? m0 + tok : m0) * g.ldx + kk;
+            const uint32_t dst = b_smem + (uint32_t) tok * 16u, stage = smem_addr(&sm.x[0][0][tid]);
+            constexpr uint32_t X_HALF = 32 * SP_CONVERT_WARPS * 16, X_BYTES = 2 * X_HALF;
+            auto fetch = [&](int c) {
+                if (c < c_end) {
+                    const int base = S::base(c);
+                    const uint32_t to = stage + (uint32_t) ((c - c_begin) % XS) * X_BYTES;
+                    const bool in = live && base + kk < g.k;   // else: zero-filled
+                    const float * from = in ? src + base : g.x;
+                    const int bytes = in ? 16 : 0;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(bytes) : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + X_HALF), "l"(from + 4), "r"(bytes) : "memory");
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");   // one group per chunk, empty ones past the end
+            };
+            if ((tid >> 5) * 4 < m_here) {
+#pragma unroll 1
+                for (int i = 0; i < XS; ++i) fetch(c_begin + i);
+                for (int c = c_begin; c < c_end; ++c) {
+                    const int lc = c - c_begin, s = lc % SB;
+                    asm volatile("cp.async.wait_group %0;" ::"n"(XS - 1) : "memory");
+                    if (!__all_sync(0xffffffffu, wait(empty_b0 + 8 * s, ((uint32_t) (lc / SB) & 1u) ^ 1u, 2, true))) break;
+                    if (live) {
+                        const uint32_t from = stage + (uint32_t) (lc % XS) * X_BYTES, at = dst + (uint32_t) (s * Smem::B_BYTES);
+                        float4 p, q;
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(from) : "memory");
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(from + X_HALF) : "memory");
+                        uint4 h, l;
+                        split_pair(p.x, p.y, h.x, l.x);
+                        split_pair(p.z, p.w, h.y, l.y);
+                        split_pair(q.x, q.y, h.z, l.z);
+                        split_pair(q.z, q.w, h.w, l.w);
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + at0), "r"(h.x), "r"(h.y) : "memory");
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + at1), "r"(h.z), "r"(h.w) : "memory");
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + at0 + TN * 16), "r"(l.x), "r"(l.y) : "memory");
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + at1 + TN * 16), "r"(l.z), "r"(l.w) : "memory");
+                    }
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full_b0 + 8 * s);
+                    fetch(c + XS);
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");   // nothing lands after the CTA is gone
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---- MMA warp: the look at the next chunk's barriers is issued before this chunk's MMAs (see sm100_gemm.cu) ----
+        constexpr uint32_t BF16_AB = (1u << 7) | (1u << 10);
+        constexpr uint32_t IDESC = instr_desc_f16(SP_TM, TN <= 64 ? 2 * TN : TN) | BF16_AB;
+        constexpr uint32_t DESC_HI = (128u >> 4) | (1u << 14);   // 128 bytes between 8-row groups; descriptor version 1
+        const uint32_t b_lo0 = (b_smem >> 4) | ((uint32_t) (2 * TN * 16) >> 4) << 16;
+        const int count = c_end - c_begin;
+        bool alive = true;
+        int sa = 0, sb = 0;
+        uint32_t pa = 0, pb = 0, accumulate = 0;
+        uint32_t ready = (mbar_test_wait(full_b0, 0u) ? 1u : 0u) & (mbar_test_wait(full_a0, 0u) ? 1u : 0u);
+        for (int lc = 0; lc < count; ++lc) {
+            if (ready == 0u) {
+                const bool ok = wait(full_b0 + 8 * sb, pb, 3, false) && wait(full_a0 + 8 * sa, pa, 4, false);
+                if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
+            }
+            tc_fence_after();
+            int sa_n = sa + 1, sb_n = sb + 1;
+            uint32_t pa_n = pa, pb_n = pb;
+            if (sa_n == SA) { sa_n = 0; pa_n ^= 1u; }
+            if (sb_n == SB) { sb_n = 0; pb_n ^= 1u; }
+            const uint32_t rb = mbar_test_wait(full_b0 + 8 * sb_n, pb_n) ? 1u : 0u;
+            const uint32_t ra = mbar_test_wait(full_a0 + 8 * sa_n, pa_n) ? 1u : 0u;
+            const uint64_t b_desc = ((uint64_t) DESC_HI << 32) | (b_lo0 + sb * (Smem::B_BYTES >> 4));
+            mma_chunk_split<TN>(tmem, tmem + ACC_COLS + sa * SP_A_COLS, b_desc, IDESC, accumulate);
+            accumulate = 1u;
+            mma_commit2(empty_a0 + 8 * sa, empty_b0 + 8 * sb, 0u);
+            ready = lc + 1 < count ? (ra & rb) : 1u;
+            sa = sa_n; pa = pa_n; sb = sb_n; pb = pb_n;
+        }
+        __syncwarp();
+        mma_commit(smem_addr(&sm.accum));
+        if (!alive && lane == 0) {
+            for (uint32_t i = 0; i < TC_WAIT_LIMIT && !mbar_try_wait(smem_addr(&sm.accum), 0u); ++i) __nanosleep(64);
+        }
+        __syncwarp();
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+// y of the cut tiles = sum of their parts, in the order of the splits
+template <int TN>
+__global__ void __launch_bounds__(256) split_reduce(const SplitArgs g) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int64_t total = (int64_t) g.cut * (TN * SP_TM);
+    for (int64_t i = (int64_t) blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t) gridDim.x * 256) {
+        const int tile = g.whole + (int) (i / (TN * SP_TM)), in = (int) (i % (TN * SP_TM));
+        const int row = (tile / g.m_tiles) * SP_TM + in % SP_TM, tok = (tile % g.m_tiles) * TN + in / SP_TM;
+        if (row >= g.n || tok >= g.m) continue;
+        float v = 0.f;
+        for (int c = 0; c < g.splits; ++c) v += __ldcg(g.part + (int64_t) c * total + i);
+        g.y[(int64_t) tok * g.ldy + row] = v;
+    }
+}
+
+// f32 [M, K] -> stage images: per (token tile, chunk) [k / 8][xh of TN tokens, xl of TN tokens][8], zero beyond M.
+// A thread takes one token's half chunk: it reads 128 bytes in order of K and stores four 16-byte units of each part in the
+// order of the image; consecutive lanes take consecutive tokens, so the stores of a warp are contiguous.
+template <typename S, int TN>
+__global__ void __launch_bounds__(256) split_prep_x(const float * x, int64_t ldx, int m, int nchunks, int64_t items, uint4 * image) {
+    pdl_wait();
+    pdl_launch_dependents();
+    for (int64_t it = (int64_t) blockIdx.x * 256 + threadIdx.x; it < items; it += (int64_t) gridDim.x * 256) {
+        const int tok_in = (int) (it % TN);
+        const int64_t rest = it / TN;
+        const int half = (int) (rest & 1);                 // units 4 half .. 4 half + 3: steps 2 half, 2 half + 1
+        const int64_t tc = rest >> 1;                      // token tile * nchunks + chunk
+        const int c = (int) (tc % nchunks), tok = (int) (tc / nchunks) * TN + tok_in;
+        float4 v[8];                                       // by place in the image
+        const float * src = x + (int64_t) tok * ldx + S::base(c);
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+            const int q = S::quad_at(8 * half + p);
+            v[p] = tok < m ? __ldcg(reinterpret_cast<const float4 *>(src + S::k4(q))) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        uint4 * dst = image + (tc * 8 + 4 * half) * (2 * TN) + tok_in;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint4 h, l;
+            split_pair(v[2 * i].x, v[2 * i].y, h.x, l.x);
+            split_pair(v[2 * i].z, v[2 * i].w, h.y, l.y);
+            split_pair(v[2 * i + 1].x, v[2 * i + 1].y, h.z, l.z);
+            split_pair(v[2 * i + 1].z, v[2 * i + 1].w, h.w, l.w);
+            dst[(int64_t) i * 2 * TN] = h;
+            dst[(int64_t) i * 2 * TN + TN] = l;
+        }
+    }
+}
+
+std::atomic<bool> g_split_launched[MAX_DEVICES];   // per device, see sm100_common.cuh
+
+template <typename S, int TN, bool PREP>
+int launch_split(cudaStream_t s, SplitArgs g) {
+    const int64_t tiles = (int64_t) ((g.n + SP_TM - 1) / SP_TM) * g.m_tiles;
+    if (tiles > INT32_MAX / 8) return fail(ST_UNSUPPORTED, "mul_mat: too many tiles for one launch");
+    TilePlan plan = plan_tiles(tiles, g.nchunks, TN >= 128 ? 20 : 15, (int64_t) SP_TM * (g.m < TN ? g.m : TN));   // a chunk takes 1.5 to 2 times as long as the f16 GEMM's
+    void * part = nullptr;
+    if (plan.cut > 0 && call_scratch_alloc(s, (size_t) plan.cut * plan.splits * TN * SP_TM * sizeof(float), &part) != ST_OK) plan = {tiles, 0, 1, 0};   // no memory: one CTA per tile needs none
+    g.part = (float *) part;
+    g.whole = (int) plan.whole;
+    g.cut = (int) plan.cut;
+    g.splits = plan.splits;
+    const size_t smem = sizeof(SplitSmem<TN, PREP>);
+    SM100_CUDA(cudaFuncSetAttribute(gemm_split<S, TN, PREP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+    g_split_launched[current_device()].store(true, std::memory_order_relaxed);
+    int st = launch(gemm_split<S, TN, PREP>, dim3((unsigned) plan_ctas(plan)), dim3(sp_threads<PREP>), smem, s, g);
+    if (plan.cut > 0) {
+        const int64_t blocks = plan.cut * (TN * SP_TM / 256), cap = (int64_t) sm_count() * 8;
+        if (st == ST_OK) st = launch(split_reduce<TN>, dim3((unsigned) (blocks < cap ? blocks : cap)), dim3(256), 0, s, g);
+        const int fr = call_scratch_free(s, part);
+        if (st == ST_OK) st = fr;
+    }
+    return st;
+}
+
+template <typename S>
+int batch_split(cudaStream_t s, SplitArgs g) {
+    g.m_tiles = 1;
+    return g.m <= 16 ? launch_split<S, 16, false>(s, g) : launch_split<S, 32, false>(s, g);
+}
+
+template <typename S, int TN>
+int prompt_split(cudaStream_t s, SplitArgs g, const float * x, int64_t ldx, int64_t m, float * y, bool * handled) {
+    // tokens per pass: the images of one pass stay below 64 MiB
+    int64_t pass = ((int64_t) 64 << 20) / ((int64_t) g.nchunks * SP_KC * 4) / TN * TN;
+    if (pass < TN) pass = TN;
+    const int64_t first = m < pass ? (m + TN - 1) / TN * TN : pass;
+    void * image = nullptr;
+    if (call_scratch_alloc(s, (size_t) first * g.nchunks * SP_KC * 4, &image) != ST_OK) return ST_OK;   // no memory for it: the caller's column panels need none
+    int st = ST_OK;
+    for (int64_t c0 = 0; c0 < m && st == ST_OK; c0 += pass) {
+        const int64_t mm = m - c0 < pass ? m - c0 : pass;
+        g.m = (int) mm;
+        g.m_tiles = (int) ((mm + TN - 1) / TN);
+        g.y = y + c0 * g.ldy;
+        g.image = (const uint8_t *) image;
+        const int64_t items = (int64_t) g.m_tiles * TN * g.nchunks * 2;
+        const int64_t blocks = (items + 255) / 256, cap = (int64_t) sm_count() * 16;
+        st = launch(split_prep_x<S, TN>, dim3((unsigned) (blocks < cap ? blocks : cap)), dim3(256), 0, s, x + c0 * ldx, ldx, (int) mm, g.nchunks, items, (uint4 *) image);
+        if (st == ST_OK) st = launch_split<S, TN, true>(s, g);
+    }
+    const int fr = call_scratch_free(s, image);
+    *handled = true;
+    return st != ST_OK ? st : fr;
+}
+
+}  // namespace
+
+// Reads and clears the fault flag of gemm_split on the current device; called after a stream synchronisation.
+int gemm_split_poll_fault() {
+    if (!g_split_launched[current_device()].exchange(false, std::memory_order_relaxed)) return ST_OK;
+    int v = 0;
+    SM100_CUDA(cudaMemcpyFromSymbol(&v, g_split_fault, sizeof(v)));
+    if (v == 0) return ST_OK;
+    const int zero = 0;
+    SM100_CUDA(cudaMemcpyToSymbol(g_split_fault, &zero, sizeof(zero)));
+    return fail(ST_BACKEND, "mul_mat: the split tensor-core GEMM gave up waiting on a pipeline barrier (site %d); its output is incomplete", v - 1);
+}
+
+// Packed Q4_0 / Q8_0 / Q4_K / Q6_K with up to 32 columns, or Q6_K with any number; *handled = false (and ST_OK) when the shape is
+// left to the caller's other kernels.
+int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
+                       bool * handled) {
+    *handled = false;
+    if (!(dtype == DT_Q4_0 || dtype == DT_Q8_0 || dtype == DT_Q4_K || dtype == DT_Q6_K)) return ST_OK;
+    if (k <= 0 || k % block_elems(dtype) != 0 || (m > 32 && dtype != DT_Q6_K)) return ST_OK;
+    if (n > INT32_MAX - SP_TM || k > (1 << 29) || m > INT32_MAX / 2) return ST_OK;
+    if ((((uintptr_t) x) & 15) != 0 || (m > 1 && ldx % 4 != 0) || (((uintptr_t) w) & 31) != 0) return ST_OK;
+    SplitArgs g = {};
+    g.w.base = (const uint8_t *) w;
+    g.w.planes = planes_for(dtype, n, k);
+    g.w.blocks_per_row = k / block_elems(dtype);
+    g.w.n = (int) n;
+    g.w.last_block = (int) (k / 32) - 1;
+    g.x = x;
+    g.ldx = ldx;
+    g.y = y;
+    g.ldy = ldy;
+    g.n = (int) n;
+    g.m = (int) m;
+    g.k = (int) k;
+    g.nchunks = (int) ((k + SP_KC - 1) / SP_KC);
+    if (m > 32) return m <= 64 ? prompt_split<SrcQ6K, 64>(s, g, x, ldx, m, y, handled) : prompt_split<SrcQ6K, 128>(s, g, x, ldx, m, y, handled);
+    int st = ST_OK;
+    switch (dtype) {
+        case DT_Q4_0: st = batch_split<SrcB32<false, true>>(s, g); break;
+        case DT_Q8_0: st = batch_split<SrcB32<true, true>>(s, g); break;
+        case DT_Q4_K: st = batch_split<SrcQ4K>(s, g); break;
+        default: st = batch_split<SrcQ6K>(s, g); break;
+    }
+    *handled = st == ST_OK;
+    return st;
+}
+
+}  // namespace sm100

@@ -30,6 +30,8 @@ int matvec_q4k_imma_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, 
 int matvec_q4k_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
                      bool * handled);
 int q4k_pass_width(int64_t k, int64_t m);
+int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
+                       bool * handled);
 int matvec_q4k_ring_multi(cudaStream_t s, int count, const void * const * ws, const int64_t * ns, int64_t k, const float * x,
                           float * const * ys, bool * handled, const Q4KPrologue * pro, const ArFuse * fuse);
 
@@ -599,6 +601,19 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
             return took("matvec_q4k_mma", ST_OK);
         }
     }
+    // Q4_0 / Q8_0 from 4 columns on, Q6_K at 3 and from 5 on: the split-operand GEMM reads the weights once for all columns.  Measured
+    // against the launches it replaces (one per column, or of 4, 2 and 1 columns with Q6_K), K x N, us:
+    //   Q4_0  4096 x 1024: m = 2  8.6 / 7.5, m = 4  8.8 / 12.6    4096 x 12288: m = 2  29 / 16, m = 4  29.5 / 31.7, m = 8  30 / 62
+    //   Q6_K  4096 x 1024: m = 2 10.8 / 7.9, m = 3 10.7 / 14.3, m = 4 10.7 / 10.5, m = 8 10.7 / 15.9
+    //         12288 x 4096: m = 2  34 / 26, m = 4  35 / 30, m = 8  35 / 59
+    // Below 1024 rows its few tiles cannot fill the GPU, and launches of small products overlap.
+    const bool split_wins = dtype == DT_Q6_K ? m == 3 || m >= 5 : (dtype == DT_Q4_0 || dtype == DT_Q8_0) && m >= 4;
+    if (layout == LAYOUT_PACKED && split_wins && n >= 1024 && x_aligned) {
+        bool handled = false;
+        const int st = gemm_split_mul_mat(s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);
+        if (st != ST_OK) return st;
+        if (handled) return took("gemm_split", ST_OK);
+    }
     // Q6_K with 2..8 columns: the tensor-core kernel assembles the 6-bit weights of a step once and multiplies them with every
     // column (measured on 4096 x 4096: 8 columns in 2.2 times the time of one, where eight single-column launches took 7.4 times)
     if (use_q6k && layout == LAYOUT_PACKED && dtype == DT_Q6_K && x_aligned && m >= 2 && m <= 8) {
@@ -610,7 +625,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
             return full == n ? took("matvec_q6k_imma_cols", ST_OK) : took("matvec_q6k_imma_cols+rows", launch_rows<UnitQ6K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full));
         }
     }
-    // Q6_K / Q4_0 / Q8_0 with 2..8 columns: the single-column tensor-core and wide kernels have no multi-column form yet,
+    // Q6_K / Q4_0 / Q8_0 with few columns or rows: the single-column tensor-core and wide kernels have no multi-column form,
     // and one launch of them per column (weights re-read per column, mostly from L2 for matrices below its size) is still
     // 2-3 times faster than the one-warp-per-row kernel that serves every column in one pass (measured on the sweep
     // shapes: Q6_K 4096 x 4096 at M = 2: 0.93 vs 0.35 TB/s of algorithmic bytes)

@@ -123,7 +123,46 @@ int device_scratch(int slot, size_t bytes, void ** out) {
     return ST_OK;
 }
 
+// Memory of one call, given back in stream order: from a pool of the library's own (per device, at most CALL_POOL_KEEP
+// bytes stay with it between synchronisations).  Concurrent streams and threads get blocks of their own; inside a
+// capture the block belongs to the graph, so a replay on any stream is safe too.
+int call_scratch_alloc(cudaStream_t s, size_t bytes, void ** out) {
+    constexpr uint64_t CALL_POOL_KEEP = (uint64_t) 128 << 20;
+    static std::mutex mu;
+    static cudaMemPool_t pools[MAX_DEVICES] = {};
+    int dev = 0;
+    SM100_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= MAX_DEVICES) return fail(ST_UNSUPPORTED, "device ordinal %d is beyond the table of %d", dev, MAX_DEVICES);
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (pools[dev] == nullptr) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaMemPool_t fresh = nullptr;
+            SM100_CUDA(cudaMemPoolCreate(&fresh, &props));
+            uint64_t keep = CALL_POOL_KEEP;
+            SM100_CUDA(cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep));
+            pools[dev] = fresh;
+        }
+        pool = pools[dev];
+    }
+    const cudaError_t e = cudaMallocFromPoolAsync(out, bytes, pool, s);
+    if (e != cudaSuccess) {
+        (void) cudaGetLastError();
+        return cuda_fail(e, "cudaMallocFromPoolAsync");
+    }
+    return ST_OK;
+}
+int call_scratch_free(cudaStream_t s, void * p) {
+    SM100_CUDA(cudaFreeAsync(p, s));
+    return ST_OK;
+}
+
 int gemm_poll_fault();
+int gemm_split_poll_fault();
 int iq_poll_fault();
 
 // Waits for the stream, then reads the fault words of the kernels with bounded waits on the STREAM's device (they are
@@ -139,6 +178,7 @@ static int sync_and_poll(cudaStream_t st) {
     }
     if (dev != cur) SM100_CUDA(cudaSetDevice(dev));
     int r = gemm_poll_fault();
+    if (r == ST_OK) r = gemm_split_poll_fault();
     if (r == ST_OK) r = iq_poll_fault();
     if (dev != cur) (void) cudaSetDevice(cur);
     return r;

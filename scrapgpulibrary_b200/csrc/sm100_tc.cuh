@@ -83,32 +83,9 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t cols) {
 __host__ __device__ constexpr uint32_t instr_desc_f16(int m, int n) {
     return (1u << 4) | ((uint32_t) (n >> 3) << 17) | ((uint32_t) (m >> 4) << 24);
 }
-// D[tmem] (+)= A . B^T; both descriptors share their high word (same 8-row-group stride and version).
-// Executed by a whole (converged) warp: one elected lane issues.  Keeping the warp converged around the issue lets the
-// operands live in uniform registers - issued from inside a divergent `if (lane == 0)` each MMA cost ~86 cycles.
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 da, {%1, %3};\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// The same with the A operand in tensor memory: lane = row, 32-bit column j of the 8 columns at `a_tmem` = the row's
-// K elements 2j (low half) and 2j + 1.
-__device__ __forceinline__ void mma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, e;\n\t.reg .b64 db;\n\t"
-        "elect.sync _|e, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
+// MMAs are executed by a whole (converged) warp: one elected lane issues.  Keeping the warp converged around the issue lets the
+// operands live in uniform registers - issued from inside a divergent `if (lane == 0)` each MMA cost ~86 cycles.  A in tensor memory:
+// lane = row, 32-bit column j of the 8 columns of a step = the row's K elements 2j (low half) and 2j + 1.
 // The four MMAs of a 64-wide chunk (A in tensor memory) as one block of instructions: the issuing lane is given as a
 // flag, the descriptors and addresses of the K steps are derived inside.  `b_desc` is the whole 64-bit descriptor
 // of the first K step, `b_step` what a K step adds to it.
@@ -142,18 +119,10 @@ __device__ __forceinline__ void mma_commit2(uint32_t bar_a, uint32_t bar_b, uint
         "r"(bar_b), "r"(issuer)
         : "memory");
 }
-// 16 consecutive 32-bit columns of this thread's own TMEM lane (lane = base lane of the warp's quarter + lane id)
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // arrives on `bar` when every MMA issued so far by the elected lane has finished reading shared memory and writing
-// TMEM (whole converged warp, like mma_f16: elect.sync picks the same lane)
+// TMEM (whole converged warp: elect.sync picks the lane that issued them)
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile(
         "{\n\t.reg .pred e;\n\t"
@@ -171,6 +140,35 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
         : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// How the tiles of a launch are dealt: as many as fill whole waves go to one CTA each, the rest - the last wave, or all when there
+// are fewer than SMs - have their K range cut over `splits` CTAs, whose partial tiles a second launch adds in order.  (192 tiles of 64
+// chunks on 148 SMs: 64 + 22 chunks' time with the last 44 cut in three, 128 without.)
+struct TilePlan {
+    int64_t whole;   // tiles [0, whole): one CTA each
+    int64_t cut;     // tiles [whole, whole + cut): `splits` CTAs each
+    int splits;
+    int64_t cost;    // in tenths of a chunk's time of a 128 x 128 tile (about 0.3 us)
+};
+// A wave costs its chunks (`per_chunk` each) plus about eight chunks of start and epilogue; partial tiles cost another six for the
+// launch that adds them and a write and a read of every partial output (`outputs` per tile).  Ties go to fewer CTAs.
+inline TilePlan plan_tiles(int64_t tiles, int nchunks, int per_chunk, int64_t outputs) {
+    const int64_t sms = sm_count();
+    TilePlan p = {tiles / sms * sms, tiles % sms, 1, 0};
+    const int64_t waves = p.whole / sms;
+    int64_t best = 0;
+    if (p.cut > 0) {
+        best = INT64_MAX;
+        for (int s = 1; s <= 8 && s <= nchunks; ++s) {
+            const int64_t cost = (p.cut * s + sms - 1) / sms * ((int64_t) ((nchunks + s - 1) / s) * per_chunk + 80) + (s > 1 ? 60 + s * p.cut * outputs / 20000 : 0);
+            if (cost < best) { best = cost; p.splits = s; }
+        }
+    }
+    p.cost = waves * ((int64_t) nchunks * per_chunk + 80) + best;
+    if (p.splits == 1) p = {tiles, 0, 1, p.cost};
+    return p;
+}
+inline int64_t plan_ctas(const TilePlan & p) { return p.whole + p.cut * p.splits; }
 
 }  // namespace
 }  // namespace sm100

@@ -1,0 +1,121 @@
+"""GPU parity of the split-operand tensor-core MUL_MAT (9..32 columns of packed weights, Q6_K at any width) against the CPU oracle.
+
+Tolerance: both operands are two bf16 numbers (16 bits: relative rounding at most 2^-17, about 2^-18.5 rms) and the product of
+the two small parts is dropped (below 2^-17), so a product is off by 1e-5; the f32
+accumulation in the tensor core truncates (up to 2e-5 over 768 steps, K = 12288).  NMSE bound: (3e-5)^2.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import sgref
+from tests import util as U
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-9
+
+
+def _check(sm100, stream, dtype, k, n, m):
+    wq = U.quantize(dtype, U.seeded_weights(7000 + dtype + k, n, k))
+    x = U.seeded_acts(3 * m + k, m, k)
+    want = sgref.mul_mat(dtype, wq, k, x)
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x)
+    assert np.isfinite(got).all()
+    for t in range(m):   # per token, so that one wrong column cannot hide in the average
+        assert sgref.nmse(got[t], want[t]) <= TOL, (t, sgref.nmse(got[t], want[t]))
+    for r in {0, n // 2, n - 1}:
+        assert sgref.nmse(got[:, r], want[:, r]) <= 4 * TOL, r
+
+
+# rows below, at and past a tile; one block of K, a K range of one chunk per CTA of a cluster, long K; edges of the 16 / 32 column tiles
+@pytest.mark.parametrize("dtype", U.QUANT, ids=lambda d: U.NAMES[d])
+@pytest.mark.parametrize("shape", [(256, 24, 9), (512, 128, 16), (512, 257, 17), (4096, 130, 32), (12288, 48, 24)], ids=lambda s: f"k{s[0]}n{s[1]}m{s[2]}")
+def test_batches(sm100, stream, dtype, shape):
+    _check(sm100, stream, dtype, *shape)
+
+
+@pytest.mark.parametrize("dtype", [U.Q4_0, U.Q8_0], ids=lambda d: U.NAMES[d])
+@pytest.mark.parametrize("shape", [(32, 16, 9), (96, 130, 31)], ids=lambda s: f"k{s[0]}n{s[1]}m{s[2]}")
+def test_half_chunk_at_the_end_of_k(sm100, stream, dtype, shape):
+    _check(sm100, stream, dtype, *shape)
+
+
+@pytest.mark.parametrize("shape", [(256, 24, 33), (512, 130, 64), (512, 257, 65), (4096, 128, 129), (12288, 40, 48)], ids=lambda s: f"k{s[0]}n{s[1]}m{s[2]}")
+def test_q6_k_prompts(sm100, stream, shape):
+    _check(sm100, stream, U.Q6_K, *shape)
+
+
+def test_q6_k_prompt_in_passes(sm100, stream):
+    """More tokens than one pass of prepared activations holds (64 MiB: 1365 tokens at K = 12288)."""
+    _check(sm100, stream, U.Q6_K, 12288, 16, 1400)
+
+
+@pytest.mark.parametrize("dtype,m", [(U.Q4_0, 12), (U.Q8_0, 32), (U.Q4_K, 12), (U.Q6_K, 20), (U.Q6_K, 40)], ids=lambda v: str(v))
+def test_token_magnitudes_and_poison(sm100, stream, dtype, m):
+    """A column keeps its precision whatever its magnitude, and a NaN or an infinity poisons its own column only."""
+    k, n = 1024, 144
+    wq = U.quantize(dtype, U.seeded_weights(5, n, k))
+    x = U.seeded_acts(6, m, k)
+    x[0] *= 1e30
+    x[1] *= 1e-25
+    x[2] = 0.0
+    x[3, 5] = 3e6
+    x[4, 7] = np.nan
+    x[5, 9] = np.inf
+    want = sgref.mul_mat(dtype, wq, k, x)
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x)
+    assert np.all(got[2] == 0.0)
+    assert not np.isfinite(got[4]).any() and not np.isfinite(got[5]).any()
+    for t in [0, 1, 3] + list(range(6, m)):
+        assert sgref.nmse(got[t].astype(np.float64), want[t].astype(np.float64)) <= TOL, t
+
+
+def test_large_scales_stay_finite(sm100, stream):
+    """Block scales near the top of f16: an f16 operand would overflow."""
+    k, n, m = 512, 32, 10
+    wq = U.quantize(U.Q8_0, U.seeded_weights(8, n, k) * np.float32(3e5))
+    x = U.seeded_acts(9, m, k)
+    got = U.device_mul_mat(sm100, stream, U.Q8_0, U.PACKED, wq, k, x)
+    assert np.isfinite(got).all() and sgref.nmse(got, sgref.mul_mat(U.Q8_0, wq, k, x)) <= TOL
+
+
+def test_capture_without_a_call_before_and_two_streams(sm100):
+    """A Q6_K prompt needs memory for its prepared activations: a capture may be the first call, each replay works on the
+    inputs of the moment, and calls on two streams at a time do not share memory."""
+    k, n, m = 768, 200, 200
+    wq = U.quantize(U.Q6_K, U.seeded_weights(11, n, k))
+    streams = [sm100.Stream(0) for _ in range(2)]
+    img = sm100.pack(U.Q6_K, k, wq)
+    wb = U.to_device(sm100, streams[0], img)
+    xs = [U.seeded_acts(20 + i, m, k) for i in range(4)]
+    want = [sgref.mul_mat(U.Q6_K, wq, k, x) for x in xs]
+    xb = [U.to_device(sm100, streams[0], xs[i]) for i in range(2)]
+    yb = [sm100.Buffer(4 * n * m) for _ in range(2)]
+    streams[0].sync()
+    graphs = []
+    for s, x, y in zip(streams, xb, yb):
+        g = sm100.Graph(s)
+        with g:
+            sm100.mul_mat(s, U.Q6_K, U.PACKED, wb, k, n, x, m, y)
+        graphs.append(g)
+    for turn in range(2):
+        for i in range(2):
+            xb[i].upload(streams[i], xs[2 * turn + i])
+        for _ in range(3):
+            for g in graphs:
+                g.launch()
+        for i, s in enumerate(streams):
+            s.sync()
+            got = yb[i].download(s, np.float32, n * m).reshape(m, n)
+            assert sgref.nmse(got, want[2 * turn + i]) <= TOL, (turn, i)
+    for _ in range(4):   # eager, both streams in flight
+        for i, s in enumerate(streams):
+            sm100.mul_mat(s, U.Q6_K, U.PACKED, wb, k, n, xb[i], m, yb[i])
+    for i, s in enumerate(streams):
+        s.sync()
+        assert sgref.nmse(yb[i].download(s, np.float32, n * m).reshape(m, n), want[2 + i]) <= TOL
+    for g in graphs:
+        g.destroy()
+    for s in streams:
+        s.close()
