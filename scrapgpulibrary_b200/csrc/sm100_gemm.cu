@@ -70,13 +70,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // ---------------------------------------------------------------------------------------------
 constexpr int KC = 64;   // weights of a row per chunk
 
-template <int TN, int STAGES, int RT>
+// SUB chunks make a stage of either ring: the MMA warp's hand-over from stage to stage costs about 200 cycles, which four MMAs of 128
+// columns (256 cycles) do not hide.
+template <int TN, int STAGES, int RT, int SUB>
 struct GemmSmem {
-    static constexpr int B_BYTES = TN * KC * 2;
+    static constexpr int CHUNK_BYTES = TN * KC * 2;
+    static constexpr int B_BYTES = SUB * CHUNK_BYTES;
     // Weight stages: as many as the tensor memory columns left by the accumulators hold, at most 8.  The two rings have
     // their own barriers: the activation copies are the long-latency side (~2 us under load) and want every byte of shared
     // memory in flight.
-    static constexpr int SA = (512 - RT * TN) / (RT * (KC / 2)) < 8 ? (512 - RT * TN) / (RT * (KC / 2)) : 8;
+    static constexpr int SA = (512 - RT * TN) / (RT * SUB * (KC / 2)) < 8 ? (512 - RT * TN) / (RT * SUB * (KC / 2)) : 8;
     uint8_t b[STAGES][B_BYTES];  // [k / 8][token][8 halves]
     uint64_t full_a[SA];         // producers -> MMA: one arrival per producer warp and row tile
     uint64_t empty_a[SA];        // MMA commit -> producers
@@ -95,7 +98,7 @@ struct GemmArgs {
     float * y;
     int64_t ldy;
     int n, m;      // weight rows; tokens of this pass
-    int nchunks;   // ceil(K / KC)
+    int nchunks;   // ceil(K / KC), a whole number of stages
     int m_tiles;
 };
 
@@ -105,14 +108,15 @@ struct GemmArgs {
 // The dequantized weights go to tensor memory (tcgen05.st by the producers, A operand of the MMA read from TMEM), so that
 // shared memory carries only the activation stages.  TMEM columns: RT accumulators of TN, then per stage and row tile
 // KC / 2 columns of A (two f16 per column).
-template <typename S, int TN, int STAGES, int RT>
+template <typename S, int TN, int STAGES, int RT, int SUB>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
     constexpr int GROUP_WARPS = 8;                          // a chunk of 128 rows: eight warps of 16 rows each
     constexpr int GROUPS = PRODUCER_WARPS / GROUP_WARPS;    // groups take the chunks in turn
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    using Smem = GemmSmem<TN, STAGES, RT>;
+    using Smem = GemmSmem<TN, STAGES, RT, SUB>;
     constexpr int ACC_COLS = RT * TN;
-    constexpr int A_COLS = KC / 2;                                   // per stage and row tile
+    static_assert(RT == 1 || SUB == 1, "two row tiles per CTA: one chunk per stage");
+    constexpr int A_COLS = SUB * KC / 2;                             // per stage and row tile
     constexpr int SA = Smem::SA;
     static_assert(SA >= 2, "at least two weight stages");
     constexpr int USED_COLS = ACC_COLS + SA * RT * A_COLS;
@@ -159,12 +163,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
         // lanes: rows 32 (warp % 4) + 16 (gw / 4) ..); lane 4 g + t holds 16 weights of rows g and g + 8 (sm100_gemm_src.cuh).
         // DEPTH of the group's chunks are kept in flight in registers to cover the L2/HBM latency.
         constexpr int DEPTH = 2;
+        static_assert(SUB == 1 || SUB == DEPTH, "the chunks of a stage are the chunks in flight");
         const int pw = warp - FIRST_PRODUCER;
         const int group = pw / GROUP_WARPS, gw = pw % GROUP_WARPS, t = lane & 3;
         const int row_in = 32 * (warp & 3) + 16 * (gw >> 2);
         // The work unit is (chunk, row tile): unit u = chunk * RT + row tile, and group g takes the units g, g + GROUPS, ...
         // Rows past the tensor are clamped to the last one: such rows are never stored.
-        const int units = g.nchunks * RT;
+        // With two chunks a stage (RT = 1) the unit is the stage, and the two chunks are the ones in flight.
+        const int units = g.nchunks / SUB * RT;
         typename S::Cursor cur[RT];
 #pragma unroll
         for (int rt = 0; rt < RT; ++rt) {
@@ -172,46 +178,53 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
             const int64_t row[2] = {r0 < last ? r0 : last, r0 + 8 < last ? r0 + 8 : last};
             S::init(cur[rt], g.w, row, t);
         }
-        auto load = [&](typename S::Regs & r, int u) {   // past the end: a clamped, unused load
+        auto load = [&](typename S::Regs & r, int u, int sub) {   // past the end: a clamped, unused load
             const int uu = u < units ? u : units - 1;
-            if (RT == 1) S::load(r, cur[0], uu);
+            if (RT == 1) S::load(r, cur[0], uu * SUB + sub);
             else if (uu % RT == 0) S::load(r, cur[0], uu / RT);
             else S::load(r, cur[RT - 1], uu / RT);
+        };
+        // one chunk of the warp's 16 rows to tensor memory
+        auto put = [&](const typename S::Regs & r, int chunk, uint32_t dst) {
+            uint32_t out[16];   // per step: row g two words, row g + 8 two words
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                typename S::ScaleF16 sc;
+                S::scale(r, chunk, t, h, sc);
+                S::template step<0>(r, h, t, sc, out[2 * h], out[2 * h + 1]);
+                S::template step<1>(r, h, t, sc, out[4 + 2 * h], out[4 + 2 * h + 1]);
+                S::template step<2>(r, h, t, sc, out[8 + 2 * h], out[8 + 2 * h + 1]);
+                S::template step<3>(r, h, t, sc, out[12 + 2 * h], out[12 + 2 * h + 1]);
+            }
+            tmem_st_frag4(dst, out);
         };
         const uint32_t dst0 = tmem + ((uint32_t) row_in << 16) + (uint32_t) ACC_COLS;
         typename S::Regs ring[DEPTH];
 #pragma unroll
-        for (int d = 0; d < DEPTH; ++d) load(ring[d], group + GROUPS * d);
+        for (int d = 0; d < DEPTH; ++d) load(ring[d], SUB == 1 ? group + GROUPS * d : group, SUB == 1 ? 0 : d);
         bool alive = true;
-        for (int u0 = group; u0 < units && alive; u0 += GROUPS * DEPTH) {
+        for (int u0 = group; u0 < units && alive; u0 += GROUPS * (SUB == 1 ? DEPTH : 1)) {
 #pragma unroll
             for (int d = 0; d < DEPTH; ++d) {
-                const int u = u0 + GROUPS * d;
+                const int u = SUB == 1 ? u0 + GROUPS * d : u0;
                 if (u >= units) break;
-                const int c = u / RT, rt = u % RT;
-                uint32_t out[16];   // per step: row g two words, row g + 8 two words
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    typename S::ScaleF16 sc;
-                    S::scale(ring[d], c, t, h, sc);
-                    S::template step<0>(ring[d], h, t, sc, out[2 * h], out[2 * h + 1]);
-                    S::template step<1>(ring[d], h, t, sc, out[4 + 2 * h], out[4 + 2 * h + 1]);
-                    S::template step<2>(ring[d], h, t, sc, out[8 + 2 * h], out[8 + 2 * h + 1]);
-                    S::template step<3>(ring[d], h, t, sc, out[12 + 2 * h], out[12 + 2 * h + 1]);
+                const int st = u / RT, rt = u % RT;
+                const int s = st % SA;
+                if (SUB == 1 || d == 0) {   // the stage is free once the MMAs that used it last have retired
+                    const uint32_t phase = (uint32_t) (st / SA) & 1u;
+                    bool ok = mbar_try_wait(empty_a0 + 8 * s, phase ^ 1u);
+                    if (!ok) ok = mbar_wait(empty_a0 + 8 * s, phase ^ 1u, abort_flag, 0);
+                    if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
+                    tc_fence_after();   // those MMAs (observed through the barrier) precede these stores
                 }
-                load(ring[d], u + GROUPS * DEPTH);
-                // the stage is free once the MMAs of the chunk that used it last have retired
-                const int s = c % SA;
-                const uint32_t phase = (uint32_t) (c / SA) & 1u;
-                bool ok = mbar_try_wait(empty_a0 + 8 * s, phase ^ 1u);
-                if (!ok) ok = mbar_wait(empty_a0 + 8 * s, phase ^ 1u, abort_flag, 0);
-                if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
-                tc_fence_after();   // the stage's previous MMAs (observed through the barrier) precede these stores
-                tmem_st_frag4(dst0 + (uint32_t) ((s * RT + rt) * A_COLS), out);
-                tmem_st_wait();
-                tc_fence_before();   // the stores are ordered before the MMA that the arrival releases
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full_a0 + 8 * s);
+                put(ring[d], SUB == 1 ? st : st * SUB + d, dst0 + (uint32_t) ((s * RT + rt) * A_COLS + (SUB == 1 ? 0 : d * (KC / 2))));
+                load(ring[d], SUB == 1 ? u + GROUPS * DEPTH : u + GROUPS, SUB == 1 ? 0 : d);
+                if (SUB == 1 || d == DEPTH - 1) {
+                    tmem_st_wait();
+                    tc_fence_before();   // the stores are ordered before the MMAs that the arrival releases
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full_a0 + 8 * s);
+                }
             }
         }
         // the dependency wait (long satisfied: the activations have been flowing) comes before the successor is
@@ -257,9 +270,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
         // warps 113 B/cycle), so the chunks go round BULK_WARPS issuing warps. ----
         if (lane == 0) {
             pdl_wait();
-            const uint8_t * src = reinterpret_cast<const uint8_t *>(g.xh) + (int64_t) mt * g.nchunks * Smem::B_BYTES;
+            const uint8_t * src = reinterpret_cast<const uint8_t *>(g.xh) + (int64_t) mt * g.nchunks * Smem::CHUNK_BYTES;
             int last = -1;
-            for (int c = warp - WARP_BULK; c < g.nchunks; c += BULK_WARPS) {
+            for (int c = warp - WARP_BULK; c < g.nchunks / SUB; c += BULK_WARPS) {
                 const int s = c % STAGES;
                 const uint32_t phase = (uint32_t) (c / STAGES) & 1u;
                 if (!mbar_try_wait(empty_b0 + 8 * s, phase ^ 1u) && !mbar_wait(empty_b0 + 8 * s, phase ^ 1u, abort_flag, 2)) break;
@@ -294,7 +307,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
         // the loop).  The look at chunk c + 1's barriers is therefore issued before chunk c's MMAs and its answer
         // used an iteration later; only a "not yet" takes the waiting path.
         uint32_t ready = (mbar_test_wait(full_b0, 0u) ? 1u : 0u) & (mbar_test_wait(full_a0, 0u) ? 1u : 0u);
-        for (int c = 0; c < g.nchunks; ++c) {
+        const int stages = g.nchunks / SUB;
+        for (int c = 0; c < stages; ++c) {
             if (ready == 0u) {
                 bool ok = mbar_try_wait(full_b0 + 8 * sb, pb);
                 if (!ok) ok = mbar_wait(full_b0 + 8 * sb, pb, abort_flag, 3, false);
@@ -314,11 +328,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
             const uint32_t ra = mbar_test_wait(full_a0 + 8 * sa_n, pa_n) ? 1u : 0u;
             const uint64_t b_desc = ((uint64_t) DESC_HI << 32) | (b_lo0 + sb * (Smem::B_BYTES >> 4));
 #pragma unroll
-            for (int rt = 0; rt < RT; ++rt)
-                mma4_f16_ta(tmem + rt * TN, tmem + ACC_COLS + (sa * RT + rt) * A_COLS, b_desc, (uint64_t) (2 * TN * 16 >> 4), IDESC, accumulate, issuer);
+            for (int i = 0; i < RT * SUB; ++i)   // row tiles, or chunks, of the stage
+                mma4_f16_ta(tmem + (RT > 1 ? i * TN : 0), tmem + ACC_COLS + sa * RT * A_COLS + i * (KC / 2), b_desc + (uint64_t) (RT > 1 ? 0 : i * (Smem::CHUNK_BYTES >> 4)),
+                            (uint64_t) (2 * TN * 16 >> 4), IDESC, i == 0 || RT > 1 ? accumulate : 1u, issuer);
             accumulate = 1u;
             mma_commit2(empty_a0 + 8 * sa, empty_b0 + 8 * sb, issuer);   // each commit covers every MMA issued so far
-            ready = c + 1 < g.nchunks ? (ra & rb) : 1u;
+            ready = c + 1 < stages ? (ra & rb) : 1u;
             sa = sa_n; pa = pa_n; sb = sb_n; pb = pb_n;
         }
         __syncwarp();
@@ -419,10 +434,10 @@ __global__ void __launch_bounds__(256) gemm_prep_x(const float * x, int64_t ldx,
 
 std::atomic<bool> g_gemm_launched[MAX_DEVICES];   // per device, see sm100_common.cuh
 
-template <typename S, int TN, int STAGES, int RT>
+template <typename S, int TN, int STAGES, int RT, int SUB>
 int launch_gemm(cudaStream_t s, GemmArgs g, int n_tiles) {
     g.out_scale = 1.0f / S::PRESCALE;
-    using Smem = GemmSmem<TN, STAGES, RT>;
+    using Smem = GemmSmem<TN, STAGES, RT, SUB>;
     static std::mutex mu;
     static std::vector<char> configured;
     int dev = 0;
@@ -431,32 +446,32 @@ int launch_gemm(cudaStream_t s, GemmArgs g, int n_tiles) {
         std::lock_guard<std::mutex> lock(mu);
         if ((int) configured.size() <= dev) configured.resize(dev + 1, 0);
         if (!configured[dev]) {
-            SM100_CUDA(cudaFuncSetAttribute(gemm_tc<S, TN, STAGES, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(Smem)));
+            SM100_CUDA(cudaFuncSetAttribute(gemm_tc<S, TN, STAGES, RT, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(Smem)));
             configured[dev] = 1;
         }
     }
     g_gemm_launched[current_device()].store(true, std::memory_order_relaxed);
-    return launch(gemm_tc<S, TN, STAGES, RT>, dim3((unsigned) (n_tiles * g.m_tiles)), dim3(GEMM_THREADS), sizeof(Smem), s, g);
+    return launch(gemm_tc<S, TN, STAGES, RT, SUB>, dim3((unsigned) (n_tiles * g.m_tiles)), dim3(GEMM_THREADS), sizeof(Smem), s, g);
 }
 
-template <int TN, int STAGES, int RT>
+template <int TN, int STAGES, int RT, int SUB>
 int launch_gemm_dtype(cudaStream_t s, int dtype, int layout, const GemmArgs & g, int n_tiles) {
     const bool packed = layout == LAYOUT_PACKED;
     switch (dtype) {
         case DT_Q8_0:
-            return packed ? launch_gemm<SrcB32<true, true>, TN, STAGES, RT>(s, g, n_tiles) : launch_gemm<SrcB32<true, false>, TN, STAGES, RT>(s, g, n_tiles);
+            return packed ? launch_gemm<SrcB32<true, true>, TN, STAGES, RT, SUB>(s, g, n_tiles) : launch_gemm<SrcB32<true, false>, TN, STAGES, RT, SUB>(s, g, n_tiles);
         case DT_Q4_0:
-            return packed ? launch_gemm<SrcB32<false, true>, TN, STAGES, RT>(s, g, n_tiles) : launch_gemm<SrcB32<false, false>, TN, STAGES, RT>(s, g, n_tiles);
-        case DT_Q4_K: return launch_gemm<SrcQ4K, TN, STAGES, RT>(s, g, n_tiles);
-        case DT_F16: return launch_gemm<SrcF16, TN, STAGES, RT>(s, g, n_tiles);
+            return packed ? launch_gemm<SrcB32<false, true>, TN, STAGES, RT, SUB>(s, g, n_tiles) : launch_gemm<SrcB32<false, false>, TN, STAGES, RT, SUB>(s, g, n_tiles);
+        case DT_Q4_K: return launch_gemm<SrcQ4K, TN, STAGES, RT, SUB>(s, g, n_tiles);
+        case DT_F16: return launch_gemm<SrcF16, TN, STAGES, RT, SUB>(s, g, n_tiles);
     }
     return fail(ST_UNSUPPORTED, "gemm: no tensor-core source for dtype %d", dtype);
 }
 
-template <int TN, int STAGES, int RT>
+template <int TN, int STAGES, int RT, int SUB>
 int gemm_passes(cudaStream_t s, int dtype, int layout, GemmArgs g, const float * x, int64_t ldx, int64_t m, int64_t k, float * y) {
     const int n_tiles = (g.n + TM * RT - 1) / (TM * RT);
-    g.nchunks = (int) ((k + KC - 1) / KC);
+    g.nchunks = (int) ((k + SUB * KC - 1) / (SUB * KC)) * SUB;
     // tokens per pass: the prepared activations of one pass stay below 64 MiB
     int64_t pass = ((int64_t) 64 << 20) / ((int64_t) g.nchunks * KC * 2) / TN * TN;
     if (pass < TN) pass = TN;
@@ -482,7 +497,7 @@ int gemm_passes(cudaStream_t s, int dtype, int layout, GemmArgs g, const float *
         g.y = y + c0 * g.ldy;
         g.m = (int) mm;
         g.m_tiles = m_tiles;
-        st = launch_gemm_dtype<TN, STAGES, RT>(s, dtype, layout, g, n_tiles);
+        st = launch_gemm_dtype<TN, STAGES, RT, SUB>(s, dtype, layout, g, n_tiles);
         if (st != ST_OK) return st;
     }
     return ST_OK;
@@ -527,8 +542,9 @@ int gemm_tc_mul_mat(cudaStream_t s, int dtype, int layout, const void * w, int64
     g.n = (int) n;
     g.ldy = ldy;
     // Tile choice.  128 weight rows x 256 tokens per CTA once such tiles fill the SMs: a chunk of 64 weights takes 517 cycles (its
-    // MMAs: 512), 128 x 128 takes 446 for half the work (256), because the MMA warp's hand-over from chunk to chunk shows.  Two row
-    // tiles per CTA (256 x 128) are bound by the dequantizing warps instead; they stay selectable for experiments.
+    // MMAs: 512), 128 x 128 takes more than half of that, because the MMA warp's hand-over from stage to stage shows (446 cycles
+    // with one chunk a stage, MMAs 256; two chunks a stage: Q4_0 5003 x 77 tokens 26.2 -> 23.3 us, 4096 x 512 30.8 -> 27.7 us).  Two
+    // row tiles per CTA (256 x 128) are bound by the dequantizing warps instead; they stay selectable for experiments.
     static const int forced_tn = [] { const char * e = getenv("SM100_GEMM_TN"); return e != nullptr ? atoi(e) : 0; }();
     static const int forced_rt = [] { const char * e = getenv("SM100_GEMM_RT"); return e != nullptr ? atoi(e) : 0; }();
     int tn = (int64_t) n_tiles * ((m + 255) / 256) >= (int64_t) sm_count() ? 256 : 128;
@@ -536,8 +552,8 @@ int gemm_tc_mul_mat(cudaStream_t s, int dtype, int layout, const void * w, int64
     const int rt = forced_rt == 2 ? 2 : 1;
     int st;
     // more activation stages than these in flight slow the weight loads down by more than they hide
-    if (rt == 2) st = gemm_passes<128, 8, 2>(s, dtype, layout, g, x, ldx, m, k, y);   // 2 x 128 accumulator columns + 4 weight stages
-    else st = tn == 256 ? gemm_passes<256, 6, 1>(s, dtype, layout, g, x, ldx, m, k, y) : gemm_passes<128, 8, 1>(s, dtype, layout, g, x, ldx, m, k, y);
+    if (rt == 2) st = gemm_passes<128, 8, 2, 1>(s, dtype, layout, g, x, ldx, m, k, y);   // 2 x 128 accumulator columns + 4 weight stages
+    else st = tn == 256 ? gemm_passes<256, 6, 1, 1>(s, dtype, layout, g, x, ldx, m, k, y) : gemm_passes<128, 6, 1, 2>(s, dtype, layout, g, x, ldx, m, k, y);
     if (st != ST_OK) return st;
     *handled = true;
     return ST_OK;
