@@ -38,7 +38,7 @@ int sm100_mul_mat(sm100_stream_t s, int dtype, int layout, const void * w, int64
         if (st != ST_OK || handled) return st;
     }
     // narrow batches of packed weights, and Q6_K at any width: the split-operand GEMM, at the column kernels' precision and one pass
-    // over the weights instead of one per 8 columns (Q4_K 12288 x 4096, 24 columns: 36 us, 63 in panels)
+    // over the weights instead of one per 8 columns (Q4_K 12288 x 4096, 24 columns: 34 us, 63 in panels)
     if (layout == LAYOUT_PACKED && is_quant(dtype) && w != nullptr && x != nullptr && y != nullptr && k > 0 && n > 0) {
         bool handled = false;
         const int st = gemm_split_mul_mat((cudaStream_t) s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);

@@ -20,7 +20,7 @@
 //
 // What bounds it: up to 32 tokens the hand-over from chunk to chunk and the dequantizing warps (about 900 cycles a chunk of 64
 // weights x 128 rows), with prompts the tensor core (12 MMAs of 64 cycles in a chunk's 1090).  Measured, us, before / now: Q4_0
-// 4096 x 12288, 8 columns 64 / 30; Q4_K 12288 x 4096, 24 columns 63 / 37; Q6_K 12288 x 4096, 512 columns 3740 / 168 (before: one
+// 4096 x 12288, 8 columns 64 / 28; Q4_K 12288 x 4096, 24 columns 63 / 34; Q6_K 12288 x 4096, 512 columns 3740 / 168 (before: one
 // launch per 8 or 4 columns).  Tried: K over a cluster with the exchange in distributed shared memory (wrong sums; taken out),
 // three converting warps with their loads in registers (Q4_K, 24 columns: 41).
 //
@@ -67,10 +67,15 @@ struct SplitArgs {
 // PREP = false: f32 activation chunks on their way, each lane's own 32 bytes per task (cp.async, read back by the same lane)
 template <int TN, bool PREP>
 struct SplitSmem {
-    static constexpr int B_BYTES = 2 * TN * SP_KC * 2;                  // a stage: [k / 8][xh of TN tokens, xl of TN tokens][8]
-    static constexpr int SB = TN >= 128 ? 6 : 8;
+    // Chunks per stage of either ring: the MMA warp's hand-over from stage to stage (about 200 cycles) shows behind the short MMAs of few
+    // columns (one / two chunks, us: Q4_0 4096 x 12288, 8 columns 29.5 / 27.6; Q4_K 12288 x 4096, 24 columns 36.5 / 34.0; Q6_K 4096 x
+    // 12288, 16 columns 41.4 / 39.0, 12288 x 4096, 8 columns 34.8 / 35.2).
+    static constexpr int SUB = PREP ? 1 : 2;
+    static constexpr int CHUNK_BYTES = 2 * TN * SP_KC * 2;              // of activations: [k / 8][xh of TN tokens, xl of TN tokens][8]
+    static constexpr int B_BYTES = SUB * CHUNK_BYTES;
+    static constexpr int SB = PREP ? (TN >= 128 ? 6 : 8) : 4;
     static constexpr int ACC_COLS = (TN <= 64 ? 4 : 2) * TN;
-    static constexpr int SA = (512 - ACC_COLS) / SP_A_COLS < 6 ? (512 - ACC_COLS) / SP_A_COLS : 6;
+    static constexpr int SA = (512 - ACC_COLS) / (SUB * SP_A_COLS) < 6 ? (512 - ACC_COLS) / (SUB * SP_A_COLS) : 6;
     static constexpr int XS = 6;                                        // f32 chunks in flight
     uint8_t b[SB][B_BYTES];
     float4 x[PREP ? 1 : XS][2][PREP ? 1 : 32 * SP_CONVERT_WARPS];
@@ -134,7 +139,7 @@ __device__ __forceinline__ void put_step(const typename S::Regs & r, int t, cons
 template <typename S, int TN, bool PREP>
 __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArgs g) {
     using Smem = SplitSmem<TN, PREP>;
-    constexpr int SA = Smem::SA, SB = Smem::SB, ACC_COLS = Smem::ACC_COLS;
+    constexpr int SUB = Smem::SUB, SA = Smem::SA, SB = Smem::SB, ACC_COLS = Smem::ACC_COLS;
     constexpr int SP_GROUPS = sp_groups<PREP>, SP_THREADS = sp_threads<PREP>, PRODUCERS = 8 * SP_GROUPS;
     constexpr int DEPTH = 2;                                             // chunks of a producer group in flight in registers
     constexpr int EPI_WARPS = TN >= 64 ? 16 : TN / 4;                    // of the first 16 producer warps
@@ -149,7 +154,8 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
     const int mt = tile % g.m_tiles, nt = tile / g.m_tiles;
     const int n0 = nt * SP_TM, m0 = mt * TN;
     const int m_here = g.m - m0 < TN ? g.m - m0 : TN;                    // tokens of this tile
-    const int c_begin = (int) ((int64_t) split * g.nchunks / splits), c_end = (int) ((int64_t) (split + 1) * g.nchunks / splits);
+    const int stages = g.nchunks / SUB, st_begin = (int) ((int64_t) split * stages / splits), st_count = (int) ((int64_t) (split + 1) * stages / splits) - st_begin;
+    const int c_begin = st_begin * SUB, c_end = c_begin + st_count * SUB;
     volatile int * abort_flag = &sm.abort_flag;
     auto wait = [&](uint32_t bar, uint32_t parity, int site, bool patient) {
         return mbar_try_wait(bar, parity) || mbar_wait_bounded(bar, parity, abort_flag, &g_split_fault, site, patient);
@@ -195,23 +201,28 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
             const int64_t row[2] = {r0 < last ? r0 : last, r0 + 8 < last ? r0 + 8 : last};   // rows past the tensor: clamped, never stored
             S::init(cur, g.w, row, t);
         }
+        // the chunks in flight in registers: two of the group's, or the two of its stage
+        static_assert(SUB == 1 || SUB == DEPTH, "the chunks of a stage are the chunks in flight");
         typename S::Regs ring[DEPTH];
+        auto load = [&](typename S::Regs & r, int st, int sub) {   // past the end: a clamped, unused load
+            const int c = c_begin + st * SUB + sub;
+            S::load(r, cur, c < c_end ? c : c_end - 1);
+        };
 #pragma unroll
-        for (int d = 0; d < DEPTH; ++d) {
-            const int c = c_begin + group + SP_GROUPS * d;
-            S::load(ring[d], cur, c < c_end ? c : c_end - 1);
-        }
+        for (int d = 0; d < DEPTH; ++d) load(ring[d], SUB == 1 ? group + SP_GROUPS * d : group, SUB == 1 ? 0 : d);
         bool alive = true;
-        for (int cb = c_begin + group; cb < c_end && alive; cb += SP_GROUPS * DEPTH) {
+        for (int s0 = group; s0 < st_count && alive; s0 += SP_GROUPS * (SUB == 1 ? DEPTH : 1)) {
 #pragma unroll
             for (int d = 0; d < DEPTH; ++d) {
-                const int c = cb + SP_GROUPS * d;
-                if (c >= c_end) break;
-                const int lc = c - c_begin, s = lc % SA;
-                const uint32_t phase = (uint32_t) (lc / SA) & 1u;
-                if (!__all_sync(0xffffffffu, wait(empty_a0 + 8 * s, phase ^ 1u, 0, true))) { alive = false; break; }
-                tc_fence_after();
-                const uint32_t dst = tmem + lanes + (uint32_t) (ACC_COLS + s * SP_A_COLS);
+                const int st = SUB == 1 ? s0 + SP_GROUPS * d : s0;
+                if (st >= st_count) break;
+                const int s = st % SA;
+                if (SUB == 1 || d == 0) {
+                    if (!__all_sync(0xffffffffu, wait(empty_a0 + 8 * s, ((uint32_t) (st / SA) & 1u) ^ 1u, 0, true))) { alive = false; break; }
+                    tc_fence_after();
+                }
+                const int c = c_begin + st * SUB + (SUB == 1 ? 0 : d);
+                const uint32_t dst = tmem + lanes + (uint32_t) (ACC_COLS + (s * SUB + (SUB == 1 ? 0 : d)) * SP_A_COLS);
                 typename S::ScaleSplit sc[2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) S::scale(ring[d], c, t, h, sc[h]);
@@ -219,12 +230,13 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
                 put_step<S, 1>(ring[d], t, sc, dst);
                 put_step<S, 2>(ring[d], t, sc, dst);
                 put_step<S, 3>(ring[d], t, sc, dst);
-                const int cn = c + SP_GROUPS * DEPTH;
-                if (cn < c_end) S::load(ring[d], cur, cn);
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full_a0 + 8 * s);
+                load(ring[d], SUB == 1 ? st + SP_GROUPS * DEPTH : st + SP_GROUPS, SUB == 1 ? 0 : d);
+                if (SUB == 1 || d == DEPTH - 1) {
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full_a0 + 8 * s);
+                }
             }
         }
         pdl_wait();
@@ -316,11 +328,11 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
 #pragma unroll 1
                 for (int i = 0; i < XS; ++i) fetch(c_begin + i);
                 for (int c = c_begin; c < c_end; ++c) {
-                    const int lc = c - c_begin, s = lc % SB;
+                    const int lc = c - c_begin, st = lc / SUB, s = st % SB;
                     asm volatile("cp.async.wait_group %0;" ::"n"(XS - 1) : "memory");
-                    if (!__all_sync(0xffffffffu, wait(empty_b0 + 8 * s, ((uint32_t) (lc / SB) & 1u) ^ 1u, 2, true))) break;
+                    if (lc % SUB == 0 && !__all_sync(0xffffffffu, wait(empty_b0 + 8 * s, ((uint32_t) (st / SB) & 1u) ^ 1u, 2, true))) break;
                     if (live) {
-                        const uint32_t from = stage + (uint32_t) (lc % XS) * X_BYTES, at = dst + (uint32_t) (s * Smem::B_BYTES);
+                        const uint32_t from = stage + (uint32_t) (lc % XS) * X_BYTES, at = dst + (uint32_t) (s * Smem::B_BYTES + lc % SUB * Smem::CHUNK_BYTES);
                         float4 p, q;
                         asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "r"(from) : "memory");
                         asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(q.x), "=f"(q.y), "=f"(q.z), "=f"(q.w) : "r"(from + X_HALF) : "memory");
@@ -334,9 +346,11 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
                         asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + at0 + TN * 16), "r"(l.x), "r"(l.y) : "memory");
                         asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at + at1 + TN * 16), "r"(l.z), "r"(l.w) : "memory");
                     }
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(full_b0 + 8 * s);
+                    if (lc % SUB == SUB - 1) {
+                        fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(full_b0 + 8 * s);
+                    }
                     fetch(c + XS);
                 }
                 asm volatile("cp.async.wait_all;" ::: "memory");   // nothing lands after the CTA is gone
@@ -349,7 +363,7 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
         constexpr uint32_t IDESC = instr_desc_f16(SP_TM, TN <= 64 ? 2 * TN : TN) | BF16_AB;
         constexpr uint32_t DESC_HI = (128u >> 4) | (1u << 14);   // 128 bytes between 8-row groups; descriptor version 1
         const uint32_t b_lo0 = (b_smem >> 4) | ((uint32_t) (2 * TN * 16) >> 4) << 16;
-        const int count = c_end - c_begin;
+        const int count = st_count;
         bool alive = true;
         int sa = 0, sb = 0;
         uint32_t pa = 0, pb = 0, accumulate = 0;
@@ -367,7 +381,9 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
             const uint32_t rb = mbar_test_wait(full_b0 + 8 * sb_n, pb_n) ? 1u : 0u;
             const uint32_t ra = mbar_test_wait(full_a0 + 8 * sa_n, pa_n) ? 1u : 0u;
             const uint64_t b_desc = ((uint64_t) DESC_HI << 32) | (b_lo0 + sb * (Smem::B_BYTES >> 4));
-            mma_chunk_split<TN>(tmem, tmem + ACC_COLS + sa * SP_A_COLS, b_desc, IDESC, accumulate);
+#pragma unroll
+            for (int i = 0; i < SUB; ++i)
+                mma_chunk_split<TN>(tmem, tmem + ACC_COLS + (sa * SUB + i) * SP_A_COLS, b_desc + (uint64_t) (i * (Smem::CHUNK_BYTES >> 4)), IDESC, i == 0 ? accumulate : 1u);
             accumulate = 1u;
             mma_commit2(empty_a0 + 8 * sa, empty_b0 + 8 * sb, 0u);
             ready = lc + 1 < count ? (ra & rb) : 1u;
@@ -445,7 +461,8 @@ template <typename S, int TN, bool PREP>
 int launch_split(cudaStream_t s, SplitArgs g) {
     const int64_t tiles = (int64_t) ((g.n + SP_TM - 1) / SP_TM) * g.m_tiles;
     if (tiles > INT32_MAX / 8) return fail(ST_UNSUPPORTED, "mul_mat: too many tiles for one launch");
-    TilePlan plan = plan_tiles(tiles, g.nchunks, TN >= 128 ? 20 : 15, (int64_t) SP_TM * (g.m < TN ? g.m : TN));   // a chunk takes 1.5 to 2 times as long as the f16 GEMM's
+    constexpr int SUB = SplitSmem<TN, PREP>::SUB;
+    TilePlan plan = plan_tiles(tiles, g.nchunks / SUB, (TN >= 128 ? 20 : 15) * SUB, (int64_t) SP_TM * (g.m < TN ? g.m : TN));   // a chunk takes 1.5 to 2 times as long as the f16 GEMM's
     void * part = nullptr;
     if (plan.cut > 0 && call_scratch_alloc(s, (size_t) plan.cut * plan.splits * TN * SP_TM * sizeof(float), &part) != ST_OK) plan = {tiles, 0, 1, 0};   // no memory: one CTA per tile needs none
     g.part = (float *) part;
@@ -468,6 +485,7 @@ int launch_split(cudaStream_t s, SplitArgs g) {
 template <typename S>
 int batch_split(cudaStream_t s, SplitArgs g) {
     g.m_tiles = 1;
+    g.nchunks = (g.nchunks + 1) / 2 * 2;   // whole stages of two chunks
     return g.m <= 16 ? launch_split<S, 16, false>(s, g) : launch_split<S, 32, false>(s, g);
 }
 
