@@ -131,7 +131,10 @@ SM100_API int sm100_graph_destroy(sm100_graph_t g);
  * graphs captured earlier stay valid when a later, larger call makes the library allocate a bigger block.  Allocation
  * is impossible during stream capture; a caller that captures reserves the largest size it will need beforehand, either
  * by issuing the call once outside the capture or with sm100_scratch_reserve on the device in question.  No
- * counterpart in the reference (its backends allocate per call: src/core/attention.cpp:576). */
+ * counterpart in the reference (its backends allocate per call: src/core/attention.cpp:576).
+ * MUL_MAT of packed weights with 3..32 columns, and of Q6_K with more, takes what it needs per call from a stream-ordered pool of
+ * the library instead (nothing to reserve; inside a capture the memory belongs to the graph; where there is none the call
+ * runs without it, slower). */
 SM100_API int sm100_scratch_reserve(int slot, size_t bytes);
 /* number of kernels of this library launched (or captured) by the calling process so far */
 SM100_API uint64_t sm100_launch_count(void);
