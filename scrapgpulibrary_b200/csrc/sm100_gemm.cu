@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
         uint32_t ready = (mbar_test_wait(full_b0, 0u) ? 1u : 0u) & (mbar_test_wait(full_a0, 0u) ? 1u : 0u);
         const int stages = g.nchunks / SUB;
         for (int c = 0; c < stages; ++c) {
-            if (ready == 0u) {
+            if (!__all_sync(0xffffffffu, ready != 0u)) {   // one answer for the warp: a lane may have looked before a phase completed, another after
                 bool ok = mbar_try_wait(full_b0 + 8 * sb, pb);
                 if (!ok) ok = mbar_wait(full_b0 + 8 * sb, pb, abort_flag, 3, false);
                 if (ok) {

@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
         uint32_t pa = 0, pb = 0, accumulate = 0;
         uint32_t ready = (mbar_test_wait(full_b0, 0u) ? 1u : 0u) & (mbar_test_wait(full_a0, 0u) ? 1u : 0u);
         for (int lc = 0; lc < count; ++lc) {
-            if (ready == 0u) {
+            if (!__all_sync(0xffffffffu, ready != 0u)) {   // one answer for the warp (see sm100_gemm.cu)
                 const bool ok = wait(full_b0 + 8 * sb, pb, 3, false) && wait(full_a0 + 8 * sa, pa, 4, false);
                 if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
             }
