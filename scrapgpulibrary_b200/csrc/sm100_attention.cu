@@ -52,6 +52,14 @@ __device__ __forceinline__ int64_t scratch_index(const AttnArgs & a, int64_t q, 
     return ((q * a.hq + h) * a.splits + split) * (a.dv + ATT_HDR);
 }
 
+// The larger of two scores, NaN if either is NaN: a row whose scores hold a NaN ends as NaN, like the reference's
+// (fmaxf drops NaNs, and a row of nothing else would pass for one without a visible key).
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 __device__ __forceinline__ int64_t visible_keys(const AttnArgs & a, int64_t q) {
     if (!a.causal) return a.nk;
     const int64_t off = a.positions != nullptr ? (int64_t) a.positions[0] : a.offset;
@@ -119,9 +127,9 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_partial_kernel(AttnArgs a) {
     // per head: max, exponentials, sum (warp g handles head g; group <= 8 = warps)
     for (int g = warp; g < group; g += nwarps) {
         float m = -INFINITY;
-        for (int64_t kk = lane; kk < count; kk += 32) m = fmaxf(m, ss[g * a.chunk + kk]);
+        for (int64_t kk = lane; kk < count; kk += 32) m = max_nan(m, ss[g * a.chunk + kk]);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        for (int o = 16; o > 0; o >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
         float l = 0.f;
         for (int64_t kk = lane; kk < count; kk += 32) {
             const float e = m == -INFINITY ? 0.f : expf(ss[g * a.chunk + kk] - m);
@@ -183,14 +191,14 @@ __device__ __forceinline__ void attn_merge_head(const AttnArgs & a, int64_t q, i
     for (int s = tid; s < a.splits; s += blockDim.x) {
         const float ms = __ldcg(base + s * stride);
         s_w[s] = ms;
-        m = fmaxf(m, ms);
+        m = max_nan(m, ms);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = 16; o > 0; o >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (lane == 0) s_red[0][warp] = m;
     __syncthreads();
     m = -INFINITY;
-    for (int w = 0; w < nwarps; ++w) m = fmaxf(m, s_red[0][w]);
+    for (int w = 0; w < nwarps; ++w) m = max_nan(m, s_red[0][w]);
     float l = 0.f;
     for (int s = tid; s < a.splits; s += blockDim.x) {
         const float ms = s_w[s];
@@ -253,10 +261,10 @@ __device__ __forceinline__ void attn_merge_group(const AttnArgs & a, int64_t q, 
         for (int i = 0; i < ATT_FUSED_SPLITS / 32; ++i) {
             const int sp = lane + 32 * i;
             ml[i] = sp < a.splits ? __ldcg(reinterpret_cast<const float2 *>(base + (int64_t) sp * stride)) : make_float2(-INFINITY, 0.f);
-            m = fmaxf(m, ml[i].x);
+            m = max_nan(m, ml[i].x);
         }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+        for (int off = 16; off > 0; off >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, off));
         float l = 0.f;
 #pragma unroll
         for (int i = 0; i < ATT_FUSED_SPLITS / 32; ++i) {
@@ -570,7 +578,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_fast_kernel(AttnArgs a) {
                     sc[j] += a.mask[(mh * a.nq + q) * a.nk + k0 + kb + j];
                 }
                 if (kb + j >= count) sc[j] = -INFINITY;
-                mx = fmaxf(mx, sc[j]);
+                mx = max_nan(mx, sc[j]);
             }
             if (mx != -INFINITY) {   // warp-uniform: every lane holds the same scores
                 const float corr = m[g] == -INFINITY ? 0.f : expf(m[g] - mx);
@@ -616,7 +624,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_fast_kernel(AttnArgs a) {
         const int g = tid / NW, w = tid % NW;
         float mm = -INFINITY;
 #pragma unroll
-        for (int w2 = 0; w2 < NW; ++w2) mm = fmaxf(mm, smem[(w2 * G + g) * SROW]);
+        for (int w2 = 0; w2 < NW; ++w2) mm = max_nan(mm, smem[(w2 * G + g) * SROW]);
         const float mw = smem[(w * G + g) * SROW];
         s_f[tid] = mw == -INFINITY ? 0.f : expf(mw - mm);
     }
@@ -637,7 +645,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_fast_kernel(AttnArgs a) {
             float mm = -INFINITY, ll = 0.f;
 #pragma unroll
             for (int w = 0; w < NW; ++w) {
-                mm = fmaxf(mm, smem[(w * G + g) * SROW]);
+                mm = max_nan(mm, smem[(w * G + g) * SROW]);
                 ll = fmaf(smem[(w * G + g) * SROW + 1], s_f[g * NW + w], ll);
             }
             *reinterpret_cast<float2 *>(dst) = make_float2(mm, ll);
@@ -827,10 +835,10 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
                 } else {
                     sc[j] = -INFINITY;
                 }
-                mx = fmaxf(mx, sc[j]);
+                mx = max_nan(mx, sc[j]);
             }
 #pragma unroll
-            for (int off = 1; off < 8; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+            for (int off = 1; off < 8; off <<= 1) mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, off));
             corr[i] = 1.f;
             float pr[4] = {0.f, 0.f, 0.f, 0.f};
             if (mx != -INFINITY) {   // a row without a visible key so far keeps m = -inf, l = 0

@@ -72,3 +72,35 @@ def test_rows_without_keys_and_hidden_values(sm100, stream):
     got2 = _run(sm100, stream, q, k, bad, True, -20)
     assert np.array_equal(got2[:, :120], got[:, :120])
     assert np.isnan(got2[:, 120:, 5]).all() and not np.isfinite(got2[:, 130:, 9]).any()
+
+
+# many-query kernel, decode kernel with the splits merged in the launch and by a second one (more than 128 splits), generic kernel
+@pytest.mark.parametrize("hq,hkv,nq,nk,d", [(32, 8, 128, 200, 128), (32, 8, 2, 600, 128), (8, 8, 3, 300, 256), (4, 4, 1, 5000, 128), (6, 2, 3, 200, 64)], ids=lambda v: str(v))
+def test_nan_scores_stay_visible(sm100, stream, hq, hkv, nq, nk, d):
+    """A NaN in a query or in any key that it sees makes the whole row NaN, wherever it stands: a row (or the part of one that a
+    warp, a tile or a split sees) that holds nothing but NaN must not pass for one without a visible key."""
+    rng = np.random.default_rng(hq + nq + nk)
+    q, k, v = (rng.standard_normal(s).astype(np.float32) for s in ((hq, nq, d), (hkv, nk, d), (hkv, nk, d)))
+    off, g = nk - nq, hq // hkv
+
+    def run(q, k):
+        qb, kb, vb = (U.to_device(sm100, stream, a) for a in (q, k, v))
+        ob, optr = U.guarded_output(sm100, stream, hq * nq * d)
+        sm100.check(sm100.lib().sm100_attention(stream.handle, qb.at(), kb.at(), vb.at(), None, 1, C.c_void_p(optr), d, d, nq, nk, hq, hkv, 1, off, None, SCALE), "attention")
+        stream.sync()
+        return U.read_guarded(sm100, stream, ob, hq * nq * d).reshape(hq, nq, d).copy()
+
+    clean = run(q, k)
+    bad = q.copy()
+    bad[1, nq - 1, 3] = np.nan
+    got = run(bad, k)
+    assert np.isnan(got[1, nq - 1]).all()
+    rest = np.ones((hq, nq), bool)
+    rest[1, nq - 1] = False
+    assert np.array_equal(got[rest], clean[rest])
+    for first, last in ((0, 40), (off, off + 1), (0, off + 1)):   # every query sees them
+        bad = k.copy()
+        bad[hkv - 1, first:last, 7] = np.nan
+        got = run(q, bad)
+        assert np.isnan(got[(hkv - 1) * g:]).all(), (first, last)
+        assert np.array_equal(got[:(hkv - 1) * g], clean[:(hkv - 1) * g])
