@@ -11,6 +11,7 @@
 // scratch buffer; kernel 2 merges the splits.  HBM-bound: algorithmic bytes = 2 * 4 * D * visible keys * Hkv.
 #include "sm100_common.cuh"
 
+#include <cfloat>
 #include <cstdlib>
 #include <mutex>
 #include <vector>
@@ -674,16 +675,22 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_fast_kernel(AttnArgs a) {
 // The decode kernel above reads every visible key once per query, which is right for one query and bound by L1/L2 traffic
 // for hundreds.  Here a CTA takes AP_ROWS rows - (query, head of the KV group) pairs, heads fastest, so that one K/V
 // tile serves the whole group - and walks the visible keys in tiles of AP_KEYS, double buffered by cp.async, with the
-// online softmax per row.  It is bound by the f32 FMA units: 4 D flops per (row, key) as packed f32x2 FMAs.  A warp owns 16
-// rows: S as 4 rows x 4 keys per lane (8 x 16 bytes from shared memory per 64 FMAs; K and Q chunks are XOR-swizzled by row so
-// the eight rows a warp reads together lie in different banks), then the probabilities pass through the warp's own slot of
-// shared memory and every lane accumulates 16 rows x 4 output elements.  A tile's sums are taken on their own and then added
-// to the rest, and a score is added up from four parts: short chains keep the rounding error at that of the split decode
-// kernel (2.3e-7 against 2.0e-7 at 1024 keys).  No scratch, no second launch.
-// Measured, 32 / 8 heads: 512 queries behind 512 keys 261 us (decode kernel 715), 2048 queries 1133 us (3915).  Tried: the second
-// product as packed FMAs over (even, odd) keys, 397 us.
+// online softmax per row.  A warp owns 16 rows: S as 4 rows x 4 keys per lane (8 x 16 bytes from shared memory per 64
+// packed f32x2 FMAs; K and Q chunks are XOR-swizzled by row so the eight rows a warp reads together lie in different banks), then the
+// probabilities pass through the warp's own slot of shared memory and every lane accumulates 16 rows x 4 output elements.  No
+// scratch, no second launch.
+// Rounding: every chain of additions is short.  A score is added up from eight parts of 16 elements (even and odd ones apart), the
+// outputs from 16 keys at a time, `span` tiles of those in registers and the rest through a.out; the sum of the probabilities is
+// compensated.  Relative error against float64 behind 512 / 4096 / 32768 keys: 1.9e-7 / 2.1e-7 / 2.6e-7, the decode kernel
+// 2.0e-7 / 2.2e-7 / 2.5e-7 (with one chain over all tiles 2.3e-7 / 3.0e-7 / 6.5e-7); without a prefix, 128 / 512 / 2048
+// queries, 1.2e-7 / 1.4e-7 / 1.6e-7, the decode kernel 1.2e-7 / 1.3e-7 / 1.5e-7.
+// Bound by the f32 FMA units and the instruction issue in front of them (4 D flops per (row, key)); with one CTA per SM by
+// latency, where the size of the unrolled loops counts (128 queries behind 512 keys: 130 us, 155 with the loops over parts and halves unrolled).
+// Measured, 32 / 8 heads: 512 queries behind 512 keys 290 us (decode kernel 716), 2048 queries 1270 us (3930).  Tried: the second
+// product as packed FMAs over (even, odd) keys, 397 us; compensated sums of the outputs in registers, 303 us and 158 behind 512 for 128 queries.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int AP_ROWS = 64, AP_KEYS = 32, AP_WARPS = 4, AP_D = 128;
+constexpr int AP_SPAN = 8;                // key tiles added up in registers at a time, at least
 constexpr int AP_PSTRIDE = AP_KEYS + 8;   // floats per probability row: conflict-free stores, 16-byte rows
 
 struct ApSmem {
@@ -691,6 +698,7 @@ struct ApSmem {
     float4 k[2][AP_KEYS][AP_D / 4];
     float4 v[2][AP_KEYS][AP_D / 4];
     float p[AP_WARPS][16][AP_PSTRIDE];
+    int64_t mask_row[AP_ROWS];   // offset of the row's mask values
     int vis[AP_ROWS];   // visible keys per row
 };
 
@@ -704,6 +712,19 @@ __device__ __forceinline__ void ap_unpack(ap_pair v, float & a, float & b) { asm
 __device__ __forceinline__ void ap_fma(ap_pair & acc, ap_pair a, ap_pair b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
 __device__ __forceinline__ void ap_lds(uint32_t addr, ap_pair & a, ap_pair & b) {
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ap_mul(ap_pair & r, ap_pair a, ap_pair b) { asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); }
+__device__ __forceinline__ void ap_add2(ap_pair & acc, ap_pair a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc) : "l"(a)); }
+// sum += v; what the addition rounds away is gathered in `low` (compensated summation, Kahan 1965)
+__device__ __forceinline__ void ap_add(float & sum, float & low, float v) {
+    const float t = __fadd_rn(sum, v);
+    low = __fadd_rn(low, __fsub_rn(v, __fsub_rn(t, sum)));
+    sum = t;
+}
+// an infinity or NaN in the sum leaves NaN in `low`
+__device__ __forceinline__ float ap_total(float sum, float low) { return fabsf(sum) <= FLT_MAX ? sum + low : sum; }
+__device__ __forceinline__ void ap_lds4(uint32_t addr, float4 & v) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
 }
 __device__ __forceinline__ void ap_cp16(uint32_t dst, const void * src, bool in) {
     const int bytes = in ? 16 : 0;   // rows past the last visible key are zero-filled
@@ -750,22 +771,23 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
         sm.q[i][lane ^ (i & 7)] = t;
     }
 
-    if (tid < AP_ROWS) sm.vis[tid] = (int) visible_keys(a, (r_base + tid < rows ? r_base + tid : rows - 1) / group);
+    for (int i = tid; i < AP_ROWS; i += AP_WARPS * 32) {
+        const int r = r_base + i < rows ? r_base + i : rows - 1, qi = r / group;
+        sm.vis[i] = (int) visible_keys(a, qi);
+        sm.mask_row[i] = ((a.mask_heads == 1 ? 0 : hk * group + r % group) * a.nq + qi) * a.nk;
+    }
+    __syncthreads();
 
     // this lane's rows of S: 16 warp + ly + 4 i; its keys of a tile: lx + 8 j
-    int vis[4];
-    const float * mrow[4];
-    float m[4], l[4];
+    const int * vis = sm.vis + 16 * warp + ly;
+    const int64_t * mask_row = sm.mask_row + 16 * warp + ly;
+    float m[4], l[4], l_low[4], m_out[4];   // m_out: the maximum that the sums in a.out are relative to
     int least = INT32_MAX;   // keys that every row of the warp sees
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int r = r_base + 16 * warp + ly + 4 * i, rr = r < rows ? r : rows - 1, qi = rr / group;
-        vis[i] = (int) visible_keys(a, qi);
-        least = vis[i] < least ? vis[i] : least;
-        const int64_t mh = a.mask_heads == 1 ? 0 : hk * group + rr % group;
-        mrow[i] = a.mask != nullptr ? a.mask + (mh * a.nq + qi) * a.nk : nullptr;
-        m[i] = -INFINITY;
-        l[i] = 0.f;
+        least = vis[4 * i] < least ? vis[4 * i] : least;
+        m[i] = m_out[i] = -INFINITY;
+        l[i] = l_low[i] = 0.f;
     }
     least = __reduce_min_sync(0xffffffffu, least);
     float o[16][4];   // row 16 warp + r, output elements 4 lane .. 4 lane + 3
@@ -773,6 +795,33 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
     for (int r = 0; r < 16; ++r)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[r][e] = 0.f;
+    // Long contexts: the sums of `span` tiles at a time are added to a.out, whose rows are this warp's own, so that no chain of
+    // additions is longer than about the square root of the tiles.
+    int span = AP_SPAN;
+    while (span * span < tiles) ++span;
+    auto out_row = [&](int r) {
+        const int row = r_base + 16 * warp + r;
+        return row < rows ? reinterpret_cast<float4 *>(a.out + ((hk * group + row % group) * a.nq + row / group) * AP_D) + lane : nullptr;
+    };
+    bool in_out = false;
+    auto add_up = [&]() {   // o += what a.out holds, and back into it
+        float f[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[i] = m_out[i] == -INFINITY ? 0.f : expf(m_out[i] - m[i]);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            const float c = __shfl_sync(0xffffffffu, f[r >> 2], (r & 3) * 8);
+            float4 * p = out_row(r);
+            if (p == nullptr) continue;
+            if (in_out) {
+                const float4 v = *p;
+                o[r][0] = fmaf(v.x, c, o[r][0]); o[r][1] = fmaf(v.y, c, o[r][1]);
+                o[r][2] = fmaf(v.z, c, o[r][2]); o[r][3] = fmaf(v.w, c, o[r][3]);
+            }
+            *p = make_float4(o[r][0], o[r][1], o[r][2], o[r][3]);
+        }
+        in_out = true;
+    };
     // swizzled offset of 16-byte chunk c (low three bits) for rows with row & 7 = lx (K) and ly (Q, even i; odd i: c ^ 4)
     const uint32_t q_row = q0 + (uint32_t) (16 * warp + ly) * 512u, k_row = k0 + (uint32_t) lx * 512u;
 
@@ -782,56 +831,56 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
         __syncthreads();   // tile t is in place for everyone, and everyone is done with tile t - 1
         if (t + 1 < tiles) fetch(t + 1, buf ^ 1);
 
-        float sum[4][4];
+        ap_pair sum[4][4];   // (even, odd) elements
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) sum[i][j] = 0.f;
+            for (int j = 0; j < 4; ++j) sum[i][j] = 0ull;
         const uint32_t kb = k_row + buf * TILE_BYTES;
 #pragma unroll 1
         for (int hi = 0; hi < 4; ++hi) {
-            ap_pair s2[4][4];
+#pragma unroll 1
+            for (int part = 0; part < 2; ++part) {
+                ap_pair s2[4][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+                for (int l4 = 0; l4 < 4; ++l4) {
+                    const int lo = l4 + 4 * part;
+                    const uint32_t ko = (uint32_t) (hi * 128 + ((lo ^ lx) << 4)), qo = (uint32_t) (hi * 128 + ((lo ^ ly) << 4));
+                    ap_pair qa[4], qb[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
+                    for (int i = 0; i < 4; ++i) ap_lds(q_row + (uint32_t) (i * 4 * 512) + (i & 1 ? qo ^ 64u : qo), qa[i], qb[i]);
 #pragma unroll
-            for (int lo = 0; lo < 8; ++lo) {
-                const uint32_t ko = (uint32_t) (hi * 128 + ((lo ^ lx) << 4)), qo = (uint32_t) (hi * 128 + ((lo ^ ly) << 4));
-                ap_pair qa[4], qb[4];
+                    for (int j = 0; j < 4; ++j) {
+                        ap_pair ka, kc;
+                        ap_lds(kb + (uint32_t) (j * 8 * 512) + ko, ka, kc);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) ap_lds(q_row + (uint32_t) (i * 4 * 512) + (i & 1 ? qo ^ 64u : qo), qa[i], qb[i]);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    ap_pair ka, kc;
-                    ap_lds(kb + (uint32_t) (j * 8 * 512) + ko, ka, kc);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        ap_fma(s2[i][j], qa[i], ka);
-                        ap_fma(s2[i][j], qb[i], kc);
+                        for (int i = 0; i < 4; ++i) {
+                            if (l4 == 0) ap_mul(s2[i][j], qa[i], ka);
+                            else ap_fma(s2[i][j], qa[i], ka);
+                            ap_fma(s2[i][j], qb[i], kc);
+                        }
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) ap_add2(sum[i][j], s2[i][j]);
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float x, y;
-                    ap_unpack(s2[i][j], x, y);
-                    sum[i][j] += x + y;
-                }
         }
         // online softmax: a row is spread over the eight lanes of equal ly
         float corr[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             float sc[4], mx = m[i];
+            const int seen = vis[4 * i];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int key = t * AP_KEYS + lx + 8 * j;
-                sc[j] = sum[i][j] * a.scale;
-                if (key < vis[i]) {
-                    if (mrow[i] != nullptr) sc[j] += mrow[i][key];
+                float even, odd;
+                ap_unpack(sum[i][j], even, odd);
+                sc[j] = (even + odd) * a.scale;
+                if (key < seen) {
+                    if (a.mask != nullptr) sc[j] += a.mask[mask_row[4 * i] + key];
                 } else {
                     sc[j] = -INFINITY;
                 }
@@ -849,7 +898,9 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
                     pr[j] = expf(sc[j] - mx);
                     psum += pr[j];
                 }
-                l[i] = fmaf(l[i], corr[i], psum);   // this lane's keys; the lanes of a row are added at the end
+                l[i] *= corr[i];   // this lane's keys; the lanes of a row are added at the end
+                l_low[i] *= corr[i];
+                ap_add(l[i], l_low[i], psum);
                 m[i] = mx;
             }
 #pragma unroll
@@ -857,51 +908,45 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
         }
         __syncwarp();   // the warp's probabilities are visible to its lanes
         const uint32_t vb = v0 + buf * TILE_BYTES + (uint32_t) lane * 16u;
-        if ((t + 1) * AP_KEYS > least && least < n_keys) {
-            // some row does not see every key here: its value rows are left out, not multiplied by zero (they may hold anything)
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                const float c = __shfl_sync(0xffffffffu, corr[r >> 2], (r & 3) * 8);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) o[r][e] *= c;
-            }
+        const bool ragged = (t + 1) * AP_KEYS > least && least < n_keys;
 #pragma unroll 1
-            for (int kk = 0; kk < AP_KEYS; ++kk) {
-                ap_pair va, vc;
-                float vx, vy, vz, vw;
-                ap_lds(vb + (uint32_t) kk * 512u, va, vc);
-                ap_unpack(va, vx, vy);
-                ap_unpack(vc, vz, vw);
-#pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    if (t * AP_KEYS + kk < sm.vis[16 * warp + r]) {
-                        const float pj = sm.p[warp][r][kk];
-                        o[r][0] = fmaf(pj, vx, o[r][0]); o[r][1] = fmaf(pj, vy, o[r][1]);
-                        o[r][2] = fmaf(pj, vz, o[r][2]); o[r][3] = fmaf(pj, vw, o[r][3]);
-                    }
-                }
-            }
-        } else {
+        for (int half = 0; half < 2; ++half) {   // 16 keys at a time are summed on their own
             float part[16][4];
 #pragma unroll
             for (int r = 0; r < 16; ++r)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) part[r][e] = 0.f;
+            if (ragged) {
+                // some row does not see every key here: its value rows are left out, not multiplied by zero (they may hold anything)
+#pragma unroll 1
+                for (int kk = 16 * half; kk < 16 * half + 16; ++kk) {
+                    float4 v;
+                    ap_lds4(vb + (uint32_t) kk * 512u, v);
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        if (t * AP_KEYS + kk < sm.vis[16 * warp + r]) {
+                            const float pj = sm.p[warp][r][kk];
+                            part[r][0] = fmaf(pj, v.x, part[r][0]); part[r][1] = fmaf(pj, v.y, part[r][1]);
+                            part[r][2] = fmaf(pj, v.z, part[r][2]); part[r][3] = fmaf(pj, v.w, part[r][3]);
+                        }
+                    }
+                }
+            } else {
 #pragma unroll 2
-            for (int k4 = 0; k4 < AP_KEYS; k4 += 4) {
-                float4 v[4];
+                for (int k4 = 16 * half; k4 < 16 * half + 16; k4 += 4) {
+                    float4 v[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w) : "r"(vb + (uint32_t) (k4 + j) * 512u) : "memory");
+                    for (int j = 0; j < 4; ++j) ap_lds4(vb + (uint32_t) (k4 + j) * 512u, v[j]);
 #pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    float4 pv;
-                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(pv.x), "=f"(pv.y), "=f"(pv.z), "=f"(pv.w) : "r"(p0 + (uint32_t) (r * AP_PSTRIDE + k4) * 4u) : "memory");
-                    const float pj[4] = {pv.x, pv.y, pv.z, pv.w};
+                    for (int r = 0; r < 16; ++r) {
+                        float4 pv;
+                        ap_lds4(p0 + (uint32_t) (r * AP_PSTRIDE + k4) * 4u, pv);
+                        const float pj[4] = {pv.x, pv.y, pv.z, pv.w};
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        part[r][0] = fmaf(pj[j], v[j].x, part[r][0]); part[r][1] = fmaf(pj[j], v[j].y, part[r][1]);
-                        part[r][2] = fmaf(pj[j], v[j].z, part[r][2]); part[r][3] = fmaf(pj[j], v[j].w, part[r][3]);
+                        for (int j = 0; j < 4; ++j) {
+                            part[r][0] = fmaf(pj[j], v[j].x, part[r][0]); part[r][1] = fmaf(pj[j], v[j].y, part[r][1]);
+                            part[r][2] = fmaf(pj[j], v[j].z, part[r][2]); part[r][3] = fmaf(pj[j], v[j].w, part[r][3]);
+                        }
                     }
                 }
             }
@@ -911,26 +956,38 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
 #pragma unroll
                 for (int e = 0; e < 4; ++e) o[r][e] = fmaf(o[r][e], c, part[r][e]);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) corr[i] = 1.f;
+        }
+        if ((t + 1) % span == 0 && t + 1 < tiles) {
+            add_up();
+#pragma unroll
+            for (int r = 0; r < 16; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[r][e] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) m_out[i] = m[i];
         }
         __syncwarp();   // the slot is read before the next tile's probabilities go in
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
+        l[i] = ap_total(l[i], l_low[i]);
 #pragma unroll
         for (int off = 1; off < 8; off <<= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], off);
+    }
+    if (in_out) add_up();
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
         const float lr = __shfl_sync(0xffffffffu, l[r >> 2], (r & 3) * 8), mr = __shfl_sync(0xffffffffu, m[r >> 2], (r & 3) * 8);
-        const int row = r_base + 16 * warp + r;
-        if (row < rows)
-            reinterpret_cast<float4 *>(a.out + ((hk * group + row % group) * a.nq + row / group) * AP_D)[lane] =
-                mr == -INFINITY ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(o[r][0] / lr, o[r][1] / lr, o[r][2] / lr, o[r][3] / lr);
+        float4 * p = out_row(r);
+        if (p != nullptr) *p = mr == -INFINITY ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(o[r][0] / lr, o[r][1] / lr, o[r][2] / lr, o[r][3] / lr);
     }
 }
 
 // Which calls take it: head dimension 128 and at least 64 row tiles over the KV heads.  With 32 of them (64 queries, 32 / 8 heads,
-// 576 keys) a CTA's serial walk over the keys takes 100 us where the splits of the decode kernel take 77; with 64 (128 queries, 640
-// keys) 113 against 147, and without a prefix 33 against 35.
+// 576 keys) a CTA's serial walk over the keys takes 100 us or more where the splits of the decode kernel take 77; with 64 (128 queries)
+// 130 against 148 behind 512 keys, 756 against 916 behind 4096, 2830 against 4030 behind 16384, and without a prefix 34 against 35.
 static bool attention_is_prompt(const AttnArgs & a) {
     if (a.d != AP_D || a.dv != AP_D || a.k_new != nullptr || a.nk > INT32_MAX / 2) return false;
     if ((((uintptr_t) a.q | (uintptr_t) a.k | (uintptr_t) a.v | (uintptr_t) a.out) & 15) != 0) return false;

@@ -75,7 +75,7 @@ def test_rows_without_keys_and_hidden_values(sm100, stream):
 
 
 # many-query kernel, decode kernel with the splits merged in the launch and by a second one (more than 128 splits), generic kernel
-@pytest.mark.parametrize("hq,hkv,nq,nk,d", [(32, 8, 128, 200, 128), (32, 8, 2, 600, 128), (8, 8, 3, 300, 256), (4, 4, 1, 5000, 128), (6, 2, 3, 200, 64)], ids=lambda v: str(v))
+@pytest.mark.parametrize("hq,hkv,nq,nk,d", [(32, 8, 128, 200, 128), (32, 8, 128, 600, 128), (32, 8, 2, 600, 128), (8, 8, 3, 300, 256), (4, 4, 1, 5000, 128), (6, 2, 3, 200, 64)], ids=lambda v: str(v))
 def test_nan_scores_stay_visible(sm100, stream, hq, hkv, nq, nk, d):
     """A NaN in a query or in any key that it sees makes the whole row NaN, wherever it stands: a row (or the part of one that a
     warp, a tile or a split sees) that holds nothing but NaN must not pass for one without a visible key."""
@@ -104,3 +104,32 @@ def test_nan_scores_stay_visible(sm100, stream, hq, hkv, nq, nk, d):
         got = run(q, bad)
         assert np.isnan(got[(hkv - 1) * g:]).all(), (first, last)
         assert np.array_equal(got[:(hkv - 1) * g], clean[:(hkv - 1) * g])
+
+
+def test_keys_hidden_beyond_the_first_span_of_tiles(sm100, stream):
+    """The first 18 of 20 key tiles are masked: the sums set aside after eight of them belong to no visible key yet."""
+    q, k, v = _inputs(32, 8, 128, 640)
+    mask = np.zeros((1, 128, 640), np.float32)
+    mask[0, :, :576] = -np.inf
+    mask[0, 5] = -np.inf
+    mask[0, 7, :] = 0
+    got = _run(sm100, stream, q, k, v, False, 0, mask=mask)
+    rows = [i for i in range(128) if i not in (5, 7)]
+    assert sgref.nmse(got[:, rows], sgref.attention(np.ascontiguousarray(q[:, rows]), k[:, 576:], v[:, 576:], False, 0, SCALE)) <= TOL
+    assert np.all(got[:, 5] == 0.0)
+    assert sgref.nmse(got[:, 7:8], sgref.attention(np.ascontiguousarray(q[:, 7:8]), k, v, False, 0, SCALE)) <= TOL
+
+
+@pytest.mark.parametrize("nk,bound", [(576, 2.0e-7), (8192, 2.4e-7)], ids=["576", "8192"])
+def test_rounding_does_not_grow_with_the_context(sm100, stream, nk, bound):
+    """Against float64.  The bounds are what the decode kernel leaves on these calls (1.9e-7 to 2.0e-7, 2.3e-7); one chain of additions
+    over all key tiles left 2.3e-7 and 3.7e-7."""
+    hq, hkv, nq = 64, 8, 64
+    q, k, v = _inputs(hq, hkv, nq, nk)
+    off, g = nk - nq, hq // hkv
+    s = q[:g].astype(np.float64) @ k[0].astype(np.float64).T * SCALE
+    s[:, np.arange(nk)[None] > off + np.arange(nq)[:, None]] = -np.inf
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = (p / p.sum(-1, keepdims=True)) @ v[0].astype(np.float64)
+    err = np.linalg.norm(_run(sm100, stream, q, k, v, True, off)[:g] - want) / np.linalg.norm(want)
+    assert err <= bound, err
