@@ -132,9 +132,11 @@ SM100_API int sm100_graph_destroy(sm100_graph_t g);
  * is impossible during stream capture; a caller that captures reserves the largest size it will need beforehand, either
  * by issuing the call once outside the capture or with sm100_scratch_reserve on the device in question.  No
  * counterpart in the reference (its backends allocate per call: src/core/attention.cpp:576).
- * MUL_MAT of packed weights with 3..32 columns, and of Q6_K with more, takes what it needs per call from a stream-ordered pool of
- * the library instead (nothing to reserve; inside a capture the memory belongs to the graph; where there is none the call
- * runs without it, slower). */
+ * MUL_MAT of packed weights with 9..32 columns (Q4_0, Q8_0 and Q6_K also with 3..8) and of Q6_K with more takes what it needs per
+ * call instead and needs nothing reserved: outside a capture from a stream-ordered pool of the library, inside one from a block
+ * that belongs to the captured graph and to all that is instantiated or copied from it (instances that run at the same time share it, as
+ * they share the outputs).  Where there is no memory the call runs without it, slower.  Q4_K with 3..8 columns uses slot 2, F16
+ * activations of prompts (Q4_0, Q8_0, Q4_K, F16 weights, more than 32 columns) slot 1. */
 SM100_API int sm100_scratch_reserve(int slot, size_t bytes);
 /* number of kernels of this library launched (or captured) by the calling process so far */
 SM100_API uint64_t sm100_launch_count(void);

@@ -95,6 +95,17 @@ int stream_tail(cudaStream_t stream);
 // launches of the calling thread without programmatic dependent launch while `on` (sm100_launch_serialized)
 void thread_serialized(bool on);
 
+// Device memory for the length of one call (sm100_runtime.cu).  An error means "take the path that needs none": nothing has been
+// enqueued and a capture is still whole.  To be given back behind the call's last launch.
+struct GraphBlock;
+struct CallScratch {
+    void * ptr = nullptr;
+    bool pooled = false;
+    GraphBlock * block = nullptr;   // a captured graph's
+};
+int call_scratch_alloc(cudaStream_t s, size_t bytes, CallScratch * out);
+int call_scratch_free(cudaStream_t s, const CallScratch & m);
+
 // Launches `kernel` on `stream`; with programmatic dependent launch when enabled, so the kernel may
 // start (and prefetch) while its predecessor on the stream drains.  Kernels launched through this
 // must execute griddepcontrol.wait before they read anything a predecessor wrote or write anything.

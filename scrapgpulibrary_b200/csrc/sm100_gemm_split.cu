@@ -34,9 +34,6 @@
 
 namespace sm100 {
 
-int call_scratch_alloc(cudaStream_t s, size_t bytes, void ** out);
-int call_scratch_free(cudaStream_t s, void * p);
-
 namespace {
 
 constexpr int SP_TM = 128;             // weight rows per CTA = TMEM lanes
@@ -457,14 +454,18 @@ __global__ void __launch_bounds__(256) split_prep_x(const float * x, int64_t ldx
 
 std::atomic<bool> g_split_launched[MAX_DEVICES];   // per device, see sm100_common.cuh
 
-template <typename S, int TN, bool PREP>
-int launch_split(cudaStream_t s, SplitArgs g) {
-    const int64_t tiles = (int64_t) ((g.n + SP_TM - 1) / SP_TM) * g.m_tiles;
-    if (tiles > INT32_MAX / 8) return fail(ST_UNSUPPORTED, "mul_mat: too many tiles for one launch");
+// how the tiles of g's tokens are dealt, and the memory that the partial tiles need
+template <int TN, bool PREP>
+TilePlan split_plan(const SplitArgs & g) {
     constexpr int SUB = SplitSmem<TN, PREP>::SUB;
-    TilePlan plan = plan_tiles(tiles, g.nchunks / SUB, (TN >= 128 ? 20 : 15) * SUB, (int64_t) SP_TM * (g.m < TN ? g.m : TN));   // a chunk takes 1.5 to 2 times as long as the f16 GEMM's
-    void * part = nullptr;
-    if (plan.cut > 0 && call_scratch_alloc(s, (size_t) plan.cut * plan.splits * TN * SP_TM * sizeof(float), &part) != ST_OK) plan = {tiles, 0, 1, 0};   // no memory: one CTA per tile needs none
+    const int64_t tiles = (int64_t) ((g.n + SP_TM - 1) / SP_TM) * g.m_tiles;
+    return plan_tiles(tiles, g.nchunks / SUB, (TN >= 128 ? 20 : 15) * SUB, (int64_t) SP_TM * (g.m < TN ? g.m : TN));   // a chunk takes 1.5 to 2 times as long as the f16 GEMM's
+}
+template <int TN>
+size_t part_bytes(const TilePlan & plan) { return (size_t) plan.cut * plan.splits * TN * SP_TM * sizeof(float); }
+
+template <typename S, int TN, bool PREP>
+int launch_split(cudaStream_t s, SplitArgs g, const TilePlan & plan, void * part) {
     g.part = (float *) part;
     g.whole = (int) plan.whole;
     g.cut = (int) plan.cut;
@@ -473,20 +474,27 @@ int launch_split(cudaStream_t s, SplitArgs g) {
     SM100_CUDA(cudaFuncSetAttribute(gemm_split<S, TN, PREP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
     g_split_launched[current_device()].store(true, std::memory_order_relaxed);
     int st = launch(gemm_split<S, TN, PREP>, dim3((unsigned) plan_ctas(plan)), dim3(sp_threads<PREP>), smem, s, g);
-    if (plan.cut > 0) {
+    if (st == ST_OK && plan.cut > 0) {
         const int64_t blocks = plan.cut * (TN * SP_TM / 256), cap = (int64_t) sm_count() * 8;
-        if (st == ST_OK) st = launch(split_reduce<TN>, dim3((unsigned) (blocks < cap ? blocks : cap)), dim3(256), 0, s, g);
-        const int fr = call_scratch_free(s, part);
-        if (st == ST_OK) st = fr;
+        st = launch(split_reduce<TN>, dim3((unsigned) (blocks < cap ? blocks : cap)), dim3(256), 0, s, g);
     }
     return st;
 }
 
+template <typename S, int TN>
+int batch_split(cudaStream_t s, SplitArgs g) {
+    TilePlan plan = split_plan<TN, false>(g);
+    CallScratch mem;
+    if (plan.cut > 0 && call_scratch_alloc(s, part_bytes<TN>(plan), &mem) != ST_OK) plan = {plan.whole + plan.cut, 0, 1};   // no memory: one CTA per tile needs none
+    const int st = launch_split<S, TN, false>(s, g, plan, mem.ptr);
+    const int fr = call_scratch_free(s, mem);
+    return st != ST_OK ? st : fr;
+}
 template <typename S>
 int batch_split(cudaStream_t s, SplitArgs g) {
     g.m_tiles = 1;
     g.nchunks = (g.nchunks + 1) / 2 * 2;   // whole stages of two chunks
-    return g.m <= 16 ? launch_split<S, 16, false>(s, g) : launch_split<S, 32, false>(s, g);
+    return g.m <= 16 ? batch_split<S, 16>(s, g) : batch_split<S, 32>(s, g);
 }
 
 template <typename S, int TN>
@@ -494,22 +502,26 @@ int prompt_split(cudaStream_t s, SplitArgs g, const float * x, int64_t ldx, int6
     // tokens per pass: the images of one pass stay below 64 MiB
     int64_t pass = ((int64_t) 64 << 20) / ((int64_t) g.nchunks * SP_KC * 4) / TN * TN;
     if (pass < TN) pass = TN;
-    const int64_t first = m < pass ? (m + TN - 1) / TN * TN : pass;
-    void * image = nullptr;
-    if (call_scratch_alloc(s, (size_t) first * g.nchunks * SP_KC * 4, &image) != ST_OK) return ST_OK;   // no memory for it: the caller's column panels need none
+    auto tokens = [&](int64_t c0) {
+        g.m = (int) (m - c0 < pass ? m - c0 : pass);
+        g.m_tiles = (g.m + TN - 1) / TN;
+        return split_plan<TN, true>(g);
+    };
+    const int64_t first = m < pass ? (m + TN - 1) / TN * TN : pass, last = (m - 1) / pass * pass;
+    const size_t image_bytes = (size_t) first * g.nchunks * SP_KC * 4, part0 = part_bytes<TN>(tokens(0)), part1 = part_bytes<TN>(tokens(last));
+    CallScratch mem;   // the stage images, then the partial tiles
+    if (call_scratch_alloc(s, image_bytes + (part0 > part1 ? part0 : part1), &mem) != ST_OK) return ST_OK;   // no memory: the caller's column panels need none
     int st = ST_OK;
     for (int64_t c0 = 0; c0 < m && st == ST_OK; c0 += pass) {
-        const int64_t mm = m - c0 < pass ? m - c0 : pass;
-        g.m = (int) mm;
-        g.m_tiles = (int) ((mm + TN - 1) / TN);
+        const TilePlan plan = tokens(c0);
         g.y = y + c0 * g.ldy;
-        g.image = (const uint8_t *) image;
+        g.image = (const uint8_t *) mem.ptr;
         const int64_t items = (int64_t) g.m_tiles * TN * g.nchunks * 2;
         const int64_t blocks = (items + 255) / 256, cap = (int64_t) sm_count() * 16;
-        st = launch(split_prep_x<S, TN>, dim3((unsigned) (blocks < cap ? blocks : cap)), dim3(256), 0, s, x + c0 * ldx, ldx, (int) mm, g.nchunks, items, (uint4 *) image);
-        if (st == ST_OK) st = launch_split<S, TN, true>(s, g);
+        st = launch(split_prep_x<S, TN>, dim3((unsigned) (blocks < cap ? blocks : cap)), dim3(256), 0, s, x + c0 * ldx, ldx, g.m, g.nchunks, items, (uint4 *) mem.ptr);
+        if (st == ST_OK) st = launch_split<S, TN, true>(s, g, plan, (uint8_t *) mem.ptr + image_bytes);
     }
-    const int fr = call_scratch_free(s, image);
+    const int fr = call_scratch_free(s, mem);
     *handled = true;
     return st != ST_OK ? st : fr;
 }

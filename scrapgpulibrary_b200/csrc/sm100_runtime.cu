@@ -2,7 +2,9 @@
 // vtable that is not arithmetic: include/scrapgpu/backend.h:33-44 of the reference).
 #include "sm100_common.cuh"
 
+#include <algorithm>
 #include <atomic>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -123,41 +125,175 @@ int device_scratch(int slot, size_t bytes, void ** out) {
     return ST_OK;
 }
 
-// Memory of one call, given back in stream order: from a pool of the library's own (per device, at most CALL_POOL_KEEP
-// bytes stay with it between synchronisations).  Concurrent streams and threads get blocks of their own; inside a
-// capture the block belongs to the graph, so a replay on any stream is safe too.
-int call_scratch_alloc(cudaStream_t s, size_t bytes, void ** out) {
-    constexpr uint64_t CALL_POOL_KEEP = (uint64_t) 128 << 20;
-    static std::mutex mu;
-    static cudaMemPool_t pools[MAX_DEVICES] = {};
+// For the duration of a scope the calling thread may allocate and create although a stream is capturing (its own, or
+// another thread's in the global mode): calls that CUDA otherwise refuses, which would invalidate the capture.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    const bool set = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    ~RelaxedCapture() {
+        if (set) (void) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+};
+
+// ---- memory of one call ----
+// Outside a capture: from a stream-ordered pool of the library's own (per device, at most CALL_POOL_KEEP bytes stay with it
+// between synchronisations), given back in stream order: concurrent streams and threads get blocks of their own.
+// Inside a capture: a block that lives as long as the captured graph and everything instantiated or copied from it (a user
+// object of the graph), so that the graph holds kernel nodes only.  A later call of the same capture shares the block if the
+// graph orders it behind the block's last user, as it does for calls on one stream.
+constexpr uint64_t CALL_POOL_KEEP = (uint64_t) 128 << 20;
+struct GraphBlock {
+    unsigned long long capture;   // id, never used twice
+    void * ptr;
+    size_t bytes;
+    cudaGraphNode_t last;         // the last kernel that uses it; null while a call is being recorded
+};
+struct CallMemory {
+    std::mutex mu;
+    cudaMemPool_t pools[MAX_DEVICES] = {};
+    std::vector<GraphBlock *> blocks;     // of graphs that are alive
+    std::mutex dead_mu;                   // nothing of CUDA is called while it is held
+    std::vector<GraphBlock *> dead;       // of graphs that are gone: their destructor may not call CUDA
+    std::atomic<int> dead_count{0};
+};
+static CallMemory & call_memory() {
+    static CallMemory * m = new CallMemory;   // graphs may be destroyed after this library's static objects
+    return *m;
+}
+static void CUDART_CB graph_block_dead(void * p) {
+    CallMemory & cm = call_memory();
+    std::lock_guard<std::mutex> lock(cm.dead_mu);
+    cm.dead.push_back((GraphBlock *) p);
+    cm.dead_count.fetch_add(1, std::memory_order_release);
+}
+// frees the blocks of destroyed graphs; the caller holds cm.mu and a RelaxedCapture
+static void free_dead_blocks(CallMemory & cm) {
+    std::vector<GraphBlock *> gone;
+    {
+        std::lock_guard<std::mutex> lock(cm.dead_mu);
+        gone.swap(cm.dead);
+        cm.dead_count.store(0, std::memory_order_release);
+    }
+    for (GraphBlock * b : gone) {
+        for (size_t i = 0; i < cm.blocks.size(); ++i)
+            if (cm.blocks[i] == b) { cm.blocks[i] = cm.blocks.back(); cm.blocks.pop_back(); break; }
+        if (cudaFree(b->ptr) != cudaSuccess) (void) cudaGetLastError();
+        delete b;
+    }
+}
+// Does the graph order `node` before a node that depends on `deps`?  Looks at 64 nodes at most: "no" only costs a block.
+static bool precedes(cudaGraphNode_t node, const cudaGraphNode_t * deps, size_t count) {
+    std::vector<cudaGraphNode_t> seen(deps, deps + count);
+    for (size_t i = 0; i < seen.size() && i < 64; ++i) {
+        if (seen[i] == node) return true;
+        size_t n = 0;
+        if (cudaGraphNodeGetDependencies_v2(seen[i], nullptr, nullptr, &n) != cudaSuccess) { (void) cudaGetLastError(); return false; }
+        std::vector<cudaGraphNode_t> from(n);
+        std::vector<cudaGraphEdgeData> edges(n);
+        if (n > 0 && cudaGraphNodeGetDependencies_v2(seen[i], from.data(), edges.data(), &n) != cudaSuccess) { (void) cudaGetLastError(); return false; }
+        for (size_t j = 0; j < n; ++j)
+            if (std::find(seen.begin(), seen.end(), from[j]) == seen.end()) seen.push_back(from[j]);
+    }
+    return false;
+}
+void call_scratch_collect() {
+    CallMemory & cm = call_memory();
+    if (cm.dead_count.load(std::memory_order_acquire) == 0) return;
+    std::lock_guard<std::mutex> lock(cm.mu);
+    RelaxedCapture relaxed;
+    free_dead_blocks(cm);
+}
+
+// SM100_CALL_SCRATCH=0: every call takes the path that needs no memory (for tests)
+int call_scratch_alloc(cudaStream_t s, size_t bytes, CallScratch * out) {
+    static const bool off = [] { const char * e = getenv("SM100_CALL_SCRATCH"); return e != nullptr && e[0] == '0'; }();
+    *out = CallScratch{};
+    if (off) return ST_OOM;
     int dev = 0;
     SM100_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= MAX_DEVICES) return fail(ST_UNSUPPORTED, "device ordinal %d is beyond the table of %d", dev, MAX_DEVICES);
-    cudaMemPool_t pool;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (pools[dev] == nullptr) {
-            cudaMemPoolProps props = {};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            cudaMemPool_t fresh = nullptr;
-            SM100_CUDA(cudaMemPoolCreate(&fresh, &props));
-            uint64_t keep = CALL_POOL_KEEP;
-            SM100_CUDA(cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep));
-            pools[dev] = fresh;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    cudaGraph_t graph = nullptr;
+    const cudaGraphNode_t * deps = nullptr;
+    const cudaGraphEdgeData * edges = nullptr;
+    size_t dep_count = 0;
+    SM100_CUDA(cudaStreamGetCaptureInfo_v3(s, &status, &capture, &graph, &deps, &edges, &dep_count));
+    CallMemory & cm = call_memory();
+    std::lock_guard<std::mutex> lock(cm.mu);
+    RelaxedCapture relaxed;
+    free_dead_blocks(cm);
+    if (status == cudaStreamCaptureStatusActive) {
+        size_t want = bytes;
+        for (GraphBlock * b : cm.blocks) {
+            if (b->capture != capture || b->last == nullptr || !precedes(b->last, deps, dep_count)) continue;
+            if (b->bytes >= bytes) {
+                b->last = nullptr;
+                out->ptr = b->ptr;
+                out->block = b;
+                return ST_OK;
+            }
+            if (want < 2 * b->bytes) want = 2 * b->bytes;   // the smaller ones add up to less than the largest
         }
-        pool = pools[dev];
+        GraphBlock * block = new GraphBlock{capture, nullptr, want, nullptr};
+        cudaError_t e = cudaMalloc(&block->ptr, want);
+        if (e != cudaSuccess) {
+            (void) cudaGetLastError();
+            delete block;
+            return cuda_fail(e, "cudaMalloc(memory of a captured call)");
+        }
+        cudaUserObject_t owner = nullptr;
+        e = cudaUserObjectCreate(&owner, block, graph_block_dead, 1, cudaUserObjectNoDestructorSync);
+        if (e == cudaSuccess) {
+            e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+            if (e != cudaSuccess) {
+                (void) cudaGetLastError();
+                (void) cudaUserObjectRelease(owner, 1);   // the destructor gives the block back
+                return cuda_fail(e, "cudaGraphRetainUserObject");
+            }
+        } else {
+            (void) cudaGetLastError();
+            (void) cudaFree(block->ptr);
+            delete block;
+            return cuda_fail(e, "cudaUserObjectCreate");
+        }
+        cm.blocks.push_back(block);
+        out->ptr = block->ptr;
+        out->block = block;
+        return ST_OK;
     }
-    const cudaError_t e = cudaMallocFromPoolAsync(out, bytes, pool, s);
+    if (cm.pools[dev] == nullptr) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t fresh = nullptr;
+        SM100_CUDA(cudaMemPoolCreate(&fresh, &props));
+        uint64_t keep = CALL_POOL_KEEP;
+        SM100_CUDA(cudaMemPoolSetAttribute(fresh, cudaMemPoolAttrReleaseThreshold, &keep));
+        cm.pools[dev] = fresh;
+    }
+    const cudaError_t e = cudaMallocFromPoolAsync(&out->ptr, bytes, cm.pools[dev], s);
     if (e != cudaSuccess) {
         (void) cudaGetLastError();
+        out->ptr = nullptr;
         return cuda_fail(e, "cudaMallocFromPoolAsync");
     }
+    out->pooled = true;
     return ST_OK;
 }
-int call_scratch_free(cudaStream_t s, void * p) {
-    SM100_CUDA(cudaFreeAsync(p, s));
+int call_scratch_free(cudaStream_t s, const CallScratch & m) {
+    if (m.pooled) SM100_CUDA(cudaFreeAsync(m.ptr, s));
+    if (m.block != nullptr) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        const cudaGraphNode_t * deps = nullptr;
+        const cudaGraphEdgeData * edges = nullptr;
+        size_t dep_count = 0;
+        SM100_CUDA(cudaStreamGetCaptureInfo_v3(s, &status, nullptr, nullptr, &deps, &edges, &dep_count));
+        CallMemory & cm = call_memory();
+        std::lock_guard<std::mutex> lock(cm.mu);
+        if (status == cudaStreamCaptureStatusActive && dep_count == 1) m.block->last = deps[0];   // the call's last kernel
+    }
     return ST_OK;
 }
 
@@ -169,6 +305,7 @@ int iq_poll_fault();
 // per-device variables; the current device may be another one in a process that drives several GPUs).
 static int sync_and_poll(cudaStream_t st) {
     SM100_CUDA(cudaStreamSynchronize(st));
+    call_scratch_collect();
     int cur = 0, dev = 0;
     SM100_CUDA(cudaGetDevice(&cur));
     dev = cur;
@@ -406,6 +543,7 @@ int sm100_graph_launch(sm100_graph_t g, sm100_stream_t s) {
 
 int sm100_graph_destroy(sm100_graph_t g) {
     if (g != nullptr) SM100_CUDA(cudaGraphExecDestroy((cudaGraphExec_t) g));
+    call_scratch_collect();
     return ST_OK;
 }
 

@@ -80,9 +80,9 @@ def test_large_scales_stay_finite(sm100, stream):
     assert np.isfinite(got).all() and sgref.nmse(got, sgref.mul_mat(U.Q8_0, wq, k, x)) <= TOL
 
 
-def test_capture_without_a_call_before_and_two_streams(sm100):
-    """A Q6_K prompt needs memory for its prepared activations: a capture may be the first call, each replay works on the
-    inputs of the moment, and calls on two streams at a time do not share memory."""
+def test_captures_on_two_streams(sm100):
+    """A Q6_K prompt needs memory for its prepared activations: each replay works on the inputs of the moment, and calls on two
+    streams at a time do not share memory."""
     k, n, m = 768, 200, 200
     wq = U.quantize(U.Q6_K, U.seeded_weights(11, n, k))
     streams = [sm100.Stream(0) for _ in range(2)]
@@ -119,3 +119,21 @@ def test_capture_without_a_call_before_and_two_streams(sm100):
         g.destroy()
     for s in streams:
         s.close()
+
+
+# the second environment: as if there were no memory to be had
+@pytest.mark.parametrize("env", [{}, {"SM100_CALL_SCRATCH": "0"}], ids=["", "no_memory"])
+@pytest.mark.parametrize("dtype,m", [(U.Q6_K, 8), (U.Q6_K, 200), (U.Q4_0, 8), (U.Q4_K, 24)], ids=lambda v: str(v))
+def test_first_product_of_a_process_is_captured(dtype, m, env):
+    """Nothing has to come before the capture, and the graph holds kernel nodes only (kind 0): it can be copied, be part of another
+    graph and have several instances."""
+    import json
+    import os
+    import subprocess
+    import sys
+    worker = os.path.join(os.path.dirname(os.path.abspath(__file__)), "capture_worker.py")
+    r = subprocess.run([sys.executable, worker, str(dtype), str(m)], capture_output=True, text=True, timeout=300, env=dict(os.environ, **env))
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    res = json.loads(r.stdout.strip().splitlines()[-1])
+    assert res["kinds"] == [0], res
+    assert res["worst"] <= TOL, res
