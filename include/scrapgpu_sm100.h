@@ -122,6 +122,9 @@ SM100_API int sm100_event_record(sm100_event_t e, sm100_stream_t s);
 SM100_API int sm100_stream_wait_event(sm100_stream_t s, sm100_event_t e);
 SM100_API int sm100_event_sync(sm100_event_t e);
 SM100_API int sm100_event_elapsed_ms(sm100_event_t start, sm100_event_t stop, float * ms);
+/* Host word that a kernel of a family (0: tensor-core GEMM, 1: split GEMM, 2: Q4_K matvecs) sets when it gives up on a bounded wait.
+ * sm100_stream_sync and the blocking reads report and clear the words of their device; a supervisor may read them at any time. */
+SM100_API int sm100_fault_word(int device, int family, int ** word_out);
 SM100_API int sm100_graph_begin(sm100_stream_t s);
 SM100_API int sm100_graph_end(sm100_stream_t s, sm100_graph_t * out);
 SM100_API int sm100_graph_launch(sm100_graph_t g, sm100_stream_t s);

@@ -50,6 +50,7 @@ def lib() -> C.CDLL:
         L.sm100_stream_wait_event.argtypes = [vp, vp]
         L.sm100_event_sync.argtypes = [vp]
         L.sm100_event_elapsed_ms.argtypes = [vp, vp, C.POINTER(C.c_float)]
+        L.sm100_fault_word.argtypes = [i32, i32, C.POINTER(C.POINTER(i32))]
         L.sm100_graph_begin.argtypes = [vp]
         L.sm100_graph_end.argtypes = [vp, pv]
         L.sm100_graph_launch.argtypes = [vp, vp]

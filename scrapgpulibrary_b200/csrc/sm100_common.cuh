@@ -4,7 +4,6 @@
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 
-#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -80,9 +79,11 @@ bool allreduce_fuse_args(void * ctx, ArFuse * out);   // false when ctx is null
 int sm_count();          // SMs of the current device (cached per device)
 int current_device();    // ordinal of the current device (0 when it cannot be read)
 
-// One "a kernel with bounded waits was launched" mark per device: the kernel's fault word is a __device__ variable,
-// i.e. one copy per device, and it is read back after a stream synchronisation only on devices that launched one.
 constexpr int MAX_DEVICES = 64;
+// Where a kernel with bounded waits reports that it gave up: the current device's word of its family, in mapped host memory
+// (sm100_runtime.cu); the kernel gets the address as an argument.
+enum { FAULT_GEMM = 0, FAULT_SPLIT = 1, FAULT_Q4K = 2, FAULT_FAMILIES = 3 };
+int fault_word(int family, int ** out);
 bool pdl_enabled();
 void count_launch();
 // What the library launched last on a stream, as far as the dispatcher of the Q4_K matvec cares: TAIL_Q4K_MATVEC after

@@ -32,7 +32,6 @@
 #include "sm100_gemm_src.cuh"
 #include "sm100_tc.cuh"
 
-#include <atomic>
 #include <cstdlib>
 #include <mutex>
 #include <vector>
@@ -56,14 +55,6 @@ constexpr int FIRST_PRODUCER = 4;  // warps 4.. dequantize; the first 16 of them
 constexpr int PRODUCER_WARPS = 24;
 constexpr int EPILOGUE_WARPS = 16;
 constexpr int GEMM_THREADS = 32 * (FIRST_PRODUCER + PRODUCER_WARPS);
-
-__device__ int g_gemm_fault;  // 0, or 1 + the wait site that gave up
-
-
-// bounded wait with this file's fault word
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int * abort_flag, int site, bool patient = true) {
-    return mbar_wait_bounded(bar, parity, abort_flag, &g_gemm_fault, site, patient);
-}
 
 // ---------------------------------------------------------------------------------------------
 // Shared memory of one CTA
@@ -97,6 +88,7 @@ struct GemmArgs {
     float out_scale;         // 1 / weight prescale
     float * y;
     int64_t ldy;
+    int * fault;
     int n, m;      // weight rows; tokens of this pass
     int nchunks;   // ceil(K / KC), a whole number of stages
     int m_tiles;
@@ -213,7 +205,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
                 if (SUB == 1 || d == 0) {   // the stage is free once the MMAs that used it last have retired
                     const uint32_t phase = (uint32_t) (st / SA) & 1u;
                     bool ok = mbar_try_wait(empty_a0 + 8 * s, phase ^ 1u);
-                    if (!ok) ok = mbar_wait(empty_a0 + 8 * s, phase ^ 1u, abort_flag, 0);
+                    if (!ok) ok = mbar_wait_bounded(empty_a0 + 8 * s, phase ^ 1u, abort_flag, g.fault, 0, true);
                     if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
                     tc_fence_after();   // those MMAs (observed through the barrier) precede these stores
                 }
@@ -237,7 +229,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
         bool acc_ok = alive;
         if (acc_ok) {
             acc_ok = mbar_try_wait(smem_addr(&sm.accum), 0u);
-            if (!acc_ok) acc_ok = mbar_wait(smem_addr(&sm.accum), 0u, abort_flag, 1);
+            if (!acc_ok) acc_ok = mbar_wait_bounded(smem_addr(&sm.accum), 0u, abort_flag, g.fault, 1, true);
         }
         if (__all_sync(0xffffffffu, acc_ok) && pw < EPILOGUE_WARPS) {
             tc_fence_after();
@@ -275,7 +267,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
             for (int c = warp - WARP_BULK; c < g.nchunks / SUB; c += BULK_WARPS) {
                 const int s = c % STAGES;
                 const uint32_t phase = (uint32_t) (c / STAGES) & 1u;
-                if (!mbar_try_wait(empty_b0 + 8 * s, phase ^ 1u) && !mbar_wait(empty_b0 + 8 * s, phase ^ 1u, abort_flag, 2)) break;
+                if (!mbar_try_wait(empty_b0 + 8 * s, phase ^ 1u) && !mbar_wait_bounded(empty_b0 + 8 * s, phase ^ 1u, abort_flag, g.fault, 2, true)) break;
                 mbar_expect_tx(full_b0 + 8 * s, Smem::B_BYTES);
                 bulk_g2s(b_smem + s * Smem::B_BYTES, src + (int64_t) c * Smem::B_BYTES, Smem::B_BYTES, full_b0 + 8 * s);
                 last = c;
@@ -311,10 +303,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
         for (int c = 0; c < stages; ++c) {
             if (!__all_sync(0xffffffffu, ready != 0u)) {   // one answer for the warp: a lane may have looked before a phase completed, another after
                 bool ok = mbar_try_wait(full_b0 + 8 * sb, pb);
-                if (!ok) ok = mbar_wait(full_b0 + 8 * sb, pb, abort_flag, 3, false);
+                if (!ok) ok = mbar_wait_bounded(full_b0 + 8 * sb, pb, abort_flag, g.fault, 3, false);
                 if (ok) {
                     ok = mbar_try_wait(full_a0 + 8 * sa, pa);
-                    if (!ok) ok = mbar_wait(full_a0 + 8 * sa, pa, abort_flag, 4, false);
+                    if (!ok) ok = mbar_wait_bounded(full_a0 + 8 * sa, pa, abort_flag, g.fault, 4, false);
                 }
                 if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
             }
@@ -432,8 +424,6 @@ __global__ void __launch_bounds__(256) gemm_prep_x(const float * x, int64_t ldx,
     }
 }
 
-std::atomic<bool> g_gemm_launched[MAX_DEVICES];   // per device, see sm100_common.cuh
-
 template <typename S, int TN, int STAGES, int RT, int SUB>
 int launch_gemm(cudaStream_t s, GemmArgs g, int n_tiles) {
     g.out_scale = 1.0f / S::PRESCALE;
@@ -450,7 +440,6 @@ int launch_gemm(cudaStream_t s, GemmArgs g, int n_tiles) {
             configured[dev] = 1;
         }
     }
-    g_gemm_launched[current_device()].store(true, std::memory_order_relaxed);
     return launch(gemm_tc<S, TN, STAGES, RT, SUB>, dim3((unsigned) (n_tiles * g.m_tiles)), dim3(GEMM_THREADS), sizeof(Smem), s, g);
 }
 
@@ -505,19 +494,6 @@ int gemm_passes(cudaStream_t s, int dtype, int layout, GemmArgs g, const float *
 
 }  // namespace
 
-// Reads and clears the fault flag of the tensor-core GEMM on the current device; called after a stream
-// synchronisation.  Costs nothing until a GEMM has been launched.
-
-int gemm_poll_fault() {
-    if (!g_gemm_launched[current_device()].exchange(false, std::memory_order_relaxed)) return ST_OK;
-    int v = 0;
-    SM100_CUDA(cudaMemcpyFromSymbol(&v, g_gemm_fault, sizeof(v)));
-    if (v == 0) return ST_OK;
-    const int zero = 0;
-    SM100_CUDA(cudaMemcpyToSymbol(g_gemm_fault, &zero, sizeof(zero)));
-    return fail(ST_BACKEND, "mul_mat: the tensor-core GEMM gave up waiting on a pipeline barrier (site %d); its output is incomplete", v - 1);
-}
-
 // Tensor-core MUL_MAT.  *handled = false (and ST_OK) when the shape or dtype is left to the caller's fallback.
 int gemm_tc_mul_mat(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_stride, int64_t k, int64_t n, const float * x,
                     int64_t ldx, int64_t m, float * y, int64_t ldy, bool * handled) {
@@ -533,6 +509,8 @@ int gemm_tc_mul_mat(cudaStream_t s, int dtype, int layout, const void * w, int64
 
     const int n_tiles = (int) ((n + TM - 1) / TM);
     GemmArgs g = {};
+    const int fw = fault_word(FAULT_GEMM, &g.fault);
+    if (fw != ST_OK) return fw;
     g.w.base = (const uint8_t *) w;
     g.w.planes = packed ? planes_for(dtype, n, k) : Planes{};
     g.w.row_stride = w_row_stride;

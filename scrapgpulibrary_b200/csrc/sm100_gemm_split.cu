@@ -30,8 +30,6 @@
 #include "sm100_gemm_src.cuh"
 #include "sm100_tc.cuh"
 
-#include <atomic>
-
 namespace sm100 {
 
 namespace {
@@ -46,8 +44,6 @@ template <bool PREP> constexpr int sp_threads = 32 * (SP_FIRST_PRODUCER + 8 * sp
 constexpr int SP_BULK_WARPS = 3, SP_CONVERT_WARPS = 8;
 constexpr int SP_A_COLS = 64;          // TMEM columns of a weight stage: wh (32), wl (32)
 
-__device__ int g_split_fault;   // 0, or 1 + the wait site that gave up
-
 struct SplitArgs {
     WeightRef w;
     const float * x;           // PREP = false: activations, column stride ldx
@@ -56,6 +52,7 @@ struct SplitArgs {
     float * y;
     int64_t ldy;
     float * part;              // partial tiles of the cut ones: [split][tile][TN tokens][128 rows]
+    int * fault;
     int n, m, k;
     int nchunks, m_tiles;
     int whole, cut, splits;    // TilePlan
@@ -155,7 +152,7 @@ __global__ void __launch_bounds__(sp_threads<PREP>, 1) gemm_split(const SplitArg
     const int c_begin = st_begin * SUB, c_end = c_begin + st_count * SUB;
     volatile int * abort_flag = &sm.abort_flag;
     auto wait = [&](uint32_t bar, uint32_t parity, int site, bool patient) {
-        return mbar_try_wait(bar, parity) || mbar_wait_bounded(bar, parity, abort_flag, &g_split_fault, site, patient);
+        return mbar_try_wait(bar, parity) || mbar_wait_bounded(bar, parity, abort_flag, g.fault, site, patient);
     };
 
     if (threadIdx.x == 0) {
@@ -452,8 +449,6 @@ __global__ void __launch_bounds__(256) split_prep_x(const float * x, int64_t ldx
     }
 }
 
-std::atomic<bool> g_split_launched[MAX_DEVICES];   // per device, see sm100_common.cuh
-
 // how the tiles of g's tokens are dealt, and the memory that the partial tiles need
 template <int TN, bool PREP>
 TilePlan split_plan(const SplitArgs & g) {
@@ -472,7 +467,6 @@ int launch_split(cudaStream_t s, SplitArgs g, const TilePlan & plan, void * part
     g.splits = plan.splits;
     const size_t smem = sizeof(SplitSmem<TN, PREP>);
     SM100_CUDA(cudaFuncSetAttribute(gemm_split<S, TN, PREP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
-    g_split_launched[current_device()].store(true, std::memory_order_relaxed);
     int st = launch(gemm_split<S, TN, PREP>, dim3((unsigned) plan_ctas(plan)), dim3(sp_threads<PREP>), smem, s, g);
     if (st == ST_OK && plan.cut > 0) {
         const int64_t blocks = plan.cut * (TN * SP_TM / 256), cap = (int64_t) sm_count() * 8;
@@ -528,17 +522,6 @@ int prompt_split(cudaStream_t s, SplitArgs g, const float * x, int64_t ldx, int6
 
 }  // namespace
 
-// Reads and clears the fault flag of gemm_split on the current device; called after a stream synchronisation.
-int gemm_split_poll_fault() {
-    if (!g_split_launched[current_device()].exchange(false, std::memory_order_relaxed)) return ST_OK;
-    int v = 0;
-    SM100_CUDA(cudaMemcpyFromSymbol(&v, g_split_fault, sizeof(v)));
-    if (v == 0) return ST_OK;
-    const int zero = 0;
-    SM100_CUDA(cudaMemcpyToSymbol(g_split_fault, &zero, sizeof(zero)));
-    return fail(ST_BACKEND, "mul_mat: the split tensor-core GEMM gave up waiting on a pipeline barrier (site %d); its output is incomplete", v - 1);
-}
-
 // Packed Q4_0 / Q8_0 / Q4_K / Q6_K with up to 32 columns, or Q6_K with any number; *handled = false (and ST_OK) when the shape is
 // left to the caller's other kernels.
 int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
@@ -549,6 +532,8 @@ int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int
     if (n > INT32_MAX - SP_TM || k > (1 << 29) || m > INT32_MAX / 2) return ST_OK;
     if ((((uintptr_t) x) & 15) != 0 || (m > 1 && ldx % 4 != 0) || (((uintptr_t) w) & 31) != 0) return ST_OK;
     SplitArgs g = {};
+    const int fw = fault_word(FAULT_SPLIT, &g.fault);
+    if (fw != ST_OK) return fw;
     g.w.base = (const uint8_t *) w;
     g.w.planes = planes_for(dtype, n, k);
     g.w.blocks_per_row = k / block_elems(dtype);

@@ -22,7 +22,6 @@
 // blocks; weight tiles are prefetched one chunk ahead and the first chunk is issued before griddepcontrol.wait.
 #include "sm100_quant_units.cuh"
 
-#include <atomic>
 #include <cstdlib>
 
 namespace sm100 {
@@ -53,6 +52,7 @@ struct IqArgs {
     const float * pa; const float * pb; const float * pw;
     float * sum_out; float * x_out;
     float eps;
+    int * fault;         // set when a wait ran out
     int n_tiles;         // full 16-row tiles of all tensors
     int pairs;           // K / 64
     int blocks;          // K / 256
@@ -149,8 +149,6 @@ __device__ __forceinline__ void imma_16832_zero(int (&c)[4], uint32_t a0, uint32
 }
 
 constexpr uint32_t IQ_WAIT_LIMIT = 1u << 22;         // polls of one barrier before the warp gives up
-
-__device__ int g_iq_fault;
 
 // Shared memory of one CTA:
 //   xq    [M][K/64][128 B]    quantized activations in B-fragment order: per pair [plane h, l][t][low sub-block b0, b1,
@@ -430,7 +428,7 @@ __global__ void __launch_bounds__(IQ_THREADS, NB == 1 ? 2 : 1) matvec_q4k_imma(I
                 bool ok = iq_bar_try_wait(bar, cphase);
                 for (uint32_t i = 0; !ok && i < IQ_WAIT_LIMIT; ++i) ok = iq_bar_try_wait(bar, cphase);
                 if (!__all_sync(0xffffffffu, ok)) {
-                    if (lane == 0) atomicExch(&g_iq_fault, 1);
+                    if (lane == 0) *(volatile int *) p.fault = 1;
                     alive = false;
                     break;
                 }
@@ -647,7 +645,7 @@ __global__ void __launch_bounds__(IQ_THREADS, 1) matvec_q4k_imma_cols(IqArgs p, 
     {
         bool ok = iq_bar_try_wait(img_bar, 0u);
         for (uint32_t i = 0; !ok && i < IQ_WAIT_LIMIT; ++i) ok = iq_bar_try_wait(img_bar, 0u);
-        if (!ok) atomicExch(&g_iq_fault, 2);
+        if (!ok) *(volatile int *) p.fault = 2;
     }
     pdl_launch_dependents();
 
@@ -671,7 +669,7 @@ __global__ void __launch_bounds__(IQ_THREADS, 1) matvec_q4k_imma_cols(IqArgs p, 
                 bool ok = iq_bar_try_wait(bar, cphase);
                 for (uint32_t i = 0; !ok && i < IQ_WAIT_LIMIT; ++i) ok = iq_bar_try_wait(bar, cphase);
                 if (!__all_sync(0xffffffffu, ok)) {
-                    if (lane == 0) atomicExch(&g_iq_fault, 1);
+                    if (lane == 0) *(volatile int *) p.fault = 1;
                     alive = false;
                     break;
                 }
@@ -779,22 +777,8 @@ int launch_iq(cudaStream_t s, const IqArgs & a, size_t smem, int grid) {
     return a.blocks % NB == 0 ? launch_iq_full<M, NB, true>(s, a, smem, grid) : launch_iq_full<M, NB, false>(s, a, smem, grid);
 }
 
-std::atomic<bool> g_iq_launched[MAX_DEVICES];   // per device, see sm100_common.cuh
-
 }  // namespace
 
-
-// Reads and clears the kernel's fault flag on the current device (set when a warp gave up waiting for a copy);
-// called after a stream synchronisation.
-int iq_poll_fault() {
-    if (!g_iq_launched[current_device()].exchange(false, std::memory_order_relaxed)) return ST_OK;
-    int v = 0;
-    SM100_CUDA(cudaMemcpyFromSymbol(&v, g_iq_fault, sizeof(v)));
-    if (v == 0) return ST_OK;
-    const int zero = 0;
-    SM100_CUDA(cudaMemcpyToSymbol(g_iq_fault, &zero, sizeof(zero)));
-    return fail(ST_BACKEND, "mul_mat: the Q4_K matvec gave up waiting for a weight copy; its output is incomplete");
-}
 
 // Q4_K packed matvec (1 or 2 activation columns) over the full 16-row tiles of up to three tensors that share
 // the activations; *handled = false when the shapes are left to the caller's other kernels.
@@ -859,8 +843,8 @@ int matvec_q4k_imma_multi(cudaStream_t s, int count, const void * const * ws, co
     int64_t grid = (int64_t) sm_count() * (nb == 1 ? 2 : 1);   // resident CTAs: each quantizes the activations once
     const int64_t rounds = (tiles + IQ_GROUPS - 1) / IQ_GROUPS;
     if (grid > rounds) grid = rounds;
-    g_iq_launched[current_device()].store(true, std::memory_order_relaxed);
-    int st;
+    int st = fault_word(FAULT_Q4K, &a.fault);
+    if (st != ST_OK) return st;
     if (nb == 1) st = m == 1 ? launch_iq<1, 1>(s, a, smem, (int) grid) : launch_iq<2, 1>(s, a, smem, (int) grid);
     else st = m == 1 ? launch_iq<1, 2>(s, a, smem, (int) grid) : launch_iq<2, 2>(s, a, smem, (int) grid);
     *handled = st == ST_OK;
@@ -898,10 +882,11 @@ int matvec_q4k_imma_cols_tiles(cudaStream_t s, const void * w, int64_t k, int64_
     int64_t grid = sm_count();
     const int64_t rounds = (tiles + IQ_GROUPS - 1) / IQ_GROUPS;
     if (grid > rounds) grid = rounds;
-    g_iq_launched[current_device()].store(true, std::memory_order_relaxed);
     const int mt = 4 * mg;
     void * img = nullptr;
-    int st = device_scratch(2, (size_t) mt * (pairs * 128 + (pairs + 1) * 16), &img);
+    int st = fault_word(FAULT_Q4K, &a.fault);
+    if (st != ST_OK) return st;
+    st = device_scratch(2, (size_t) mt * (pairs * 128 + (pairs + 1) * 16), &img);
     if (st != ST_OK) return st;
     const int q_items = mt * pairs * 16;
     st = launch(q4k_quantize_cols, dim3((unsigned) ((q_items + 255) / 256)), dim3(256), 0, s, x, ldx, (int) m, mt, pairs, (uint32_t *) img);

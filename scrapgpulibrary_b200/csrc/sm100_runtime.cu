@@ -297,28 +297,57 @@ int call_scratch_free(cudaStream_t s, const CallScratch & m) {
     return ST_OK;
 }
 
-int gemm_poll_fault();
-int gemm_split_poll_fault();
-int iq_poll_fault();
+// ---- fault words ----
+// One word per device and kernel family in mapped host memory: a kernel that gives up on a bounded wait writes its wait site + 1
+// there (it goes on to the end, so the word has arrived when the stream is synchronised).  Reading them costs no call, so every
+// synchronisation looks at all of them, whatever was launched and however: directly, from a graph, on another stream.
+struct FaultWords { int word[MAX_DEVICES][16]; };   // a cache line per device
+static std::atomic<FaultWords *> g_faults{nullptr};
+static int fault_words(FaultWords ** out) {
+    static std::mutex mu;
+    FaultWords * f = g_faults.load(std::memory_order_acquire);
+    if (f == nullptr) {
+        std::lock_guard<std::mutex> lock(mu);
+        f = g_faults.load(std::memory_order_acquire);
+        if (f == nullptr) {
+            RelaxedCapture relaxed;
+            SM100_CUDA(cudaHostAlloc((void **) &f, sizeof(FaultWords), cudaHostAllocPortable | cudaHostAllocMapped));
+            std::memset(f, 0, sizeof(FaultWords));
+            g_faults.store(f, std::memory_order_release);
+        }
+    }
+    *out = f;
+    return ST_OK;
+}
+int fault_word(int family, int ** out) {
+    FaultWords * f = nullptr;
+    const int st = fault_words(&f);
+    *out = st == ST_OK ? &f->word[current_device()][family] : nullptr;
+    return st;
+}
+static int poll_faults(int dev) {
+    FaultWords * f = g_faults.load(std::memory_order_acquire);
+    if (f == nullptr || dev < 0 || dev >= MAX_DEVICES) return ST_OK;
+    static const char * const what[FAULT_FAMILIES] = {"the tensor-core GEMM gave up waiting on a pipeline barrier", "the split tensor-core GEMM gave up waiting on a pipeline barrier",
+                                                      "the Q4_K matvec gave up waiting for a weight copy"};
+    for (int i = 0; i < FAULT_FAMILIES; ++i) {
+        const int v = __atomic_load_n(&f->word[dev][i], __ATOMIC_ACQUIRE) == 0 ? 0 : __atomic_exchange_n(&f->word[dev][i], 0, __ATOMIC_ACQ_REL);
+        if (v != 0) return fail(ST_BACKEND, "mul_mat: %s (site %d); its output is incomplete", what[i], v - 1);
+    }
+    return ST_OK;
+}
 
-// Waits for the stream, then reads the fault words of the kernels with bounded waits on the STREAM's device (they are
-// per-device variables; the current device may be another one in a process that drives several GPUs).
+// Waits for the stream, then reads the fault words of the STREAM's device (the current device may be another one in a process
+// that drives several GPUs).
 static int sync_and_poll(cudaStream_t st) {
     SM100_CUDA(cudaStreamSynchronize(st));
     call_scratch_collect();
-    int cur = 0, dev = 0;
-    SM100_CUDA(cudaGetDevice(&cur));
-    dev = cur;
-    if (st != nullptr && cudaStreamGetDevice(st, &dev) != cudaSuccess) {
-        (void) cudaGetLastError();
-        dev = cur;
+    int dev = 0;
+    if (st == nullptr || cudaStreamGetDevice(st, &dev) != cudaSuccess) {
+        if (st != nullptr) (void) cudaGetLastError();
+        dev = current_device();
     }
-    if (dev != cur) SM100_CUDA(cudaSetDevice(dev));
-    int r = gemm_poll_fault();
-    if (r == ST_OK) r = gemm_split_poll_fault();
-    if (r == ST_OK) r = iq_poll_fault();
-    if (dev != cur) (void) cudaSetDevice(cur);
-    return r;
+    return poll_faults(dev);
 }
 
 }  // namespace sm100
@@ -516,6 +545,14 @@ int sm100_event_sync(sm100_event_t e) {
 int sm100_event_elapsed_ms(sm100_event_t start, sm100_event_t stop, float * ms) {
     SM100_CUDA(cudaEventElapsedTime(ms, (cudaEvent_t) start, (cudaEvent_t) stop));
     return ST_OK;
+}
+
+int sm100_fault_word(int device, int family, int ** word_out) {
+    if (word_out == nullptr || device < 0 || device >= MAX_DEVICES || family < 0 || family >= FAULT_FAMILIES) return fail(ST_INVALID, "fault_word: bad argument");
+    FaultWords * f = nullptr;
+    const int st = fault_words(&f);
+    if (st == ST_OK) *word_out = &f->word[device][family];
+    return st;
 }
 
 int sm100_graph_begin(sm100_stream_t s) {

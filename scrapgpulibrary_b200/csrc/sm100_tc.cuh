@@ -52,7 +52,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
         }
     }
     *abort_flag = 1 + site;
-    atomicCAS(fault, 0, 1 + site);
+    *(volatile int *) fault = 1 + site;
     return false;
 }
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }

@@ -137,3 +137,34 @@ def test_first_product_of_a_process_is_captured(dtype, m, env):
     res = json.loads(r.stdout.strip().splitlines()[-1])
     assert res["kinds"] == [0], res
     assert res["worst"] <= TOL, res
+
+
+@pytest.mark.parametrize("family,dtype,m", [(0, U.Q8_0, 40), (1, U.Q4_0, 12), (2, U.Q4_K, 1), (2, U.Q4_K, 4)], ids=lambda v: str(v))
+def test_give_ups_of_replays_are_reported(sm100, stream, family, dtype, m):
+    """A kernel that gives up on a wait leaves its mark in a host word (written here by the test): every synchronisation and blocking
+    read of the device reports it once, also when the kernel came from a graph that was captured long before."""
+    k, n = 512, 96
+    wb = U.to_device(sm100, stream, sm100.pack(dtype, k, U.quantize(dtype, U.seeded_weights(3, n, k))))
+    xb, yb = U.to_device(sm100, stream, U.seeded_acts(4, m, k)), sm100.Buffer(4 * n * m)
+    sm100.mul_mat(stream, dtype, U.PACKED, wb, k, n, xb, m, yb)
+    stream.sync()
+    graph = sm100.Graph(stream)
+    with graph:
+        sm100.mul_mat(stream, dtype, U.PACKED, wb, k, n, xb, m, yb)
+    word = C.POINTER(C.c_int)()
+    sm100.check(sm100.lib().sm100_fault_word(0, family, C.byref(word)), "fault_word")
+    graph.launch()
+    stream.sync()
+    other = sm100.Stream(0)
+    for wait in (stream.sync, lambda: yb.download(stream, np.float32, 1), other.sync):
+        graph.launch()
+        assert word[0] == 0
+        word[0] = 4
+        with pytest.raises(sm100.Sm100Error, match="gave up.*site 3") as e:
+            wait()
+        assert e.value.status == 4 and word[0] == 0
+        stream.sync()
+    graph.destroy()
+    other.close()
+    for b in (wb, xb, yb):
+        b.free()
