@@ -103,11 +103,12 @@ struct SrcB32 {
             }
         }
         u.off = t >> 1;
-        u.last = W.last_block;   // a half chunk at the end of K re-reads the last block: the activation image is zero there
+        u.last = W.last_block;
     }
     __device__ static __forceinline__ void load(Regs & r, const Cursor & u, int c) {
         int b = 2 * c + u.off;
-        b = b < u.last ? b : u.last;
+        const bool in = b <= u.last;   // past the end of K (a half chunk, or a whole one of the last stage): weights of scale zero
+        b = in ? b : u.last;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             if (PACKED) {
@@ -118,12 +119,12 @@ struct SrcB32 {
                     const uint2 v = __ldg((const uint2 *) (u.q[h] + (int64_t) b * 16));
                     r.q[h][0] = v.x; r.q[h][1] = v.y;
                 }
-                r.d[h] = ld_u16_any(u.d[h] + (int64_t) b * 2);
+                r.d[h] = in ? ld_u16_any(u.d[h] + (int64_t) b * 2) : 0u;
             } else {
                 const uint8_t * p = u.q[h] + (int64_t) b * (Q8 ? 34 : 18);
 #pragma unroll
                 for (int i = 0; i < (Q8 ? 4 : 2); ++i) r.q[h][i] = ld_u16_any(p + 4 * i) | ld_u16_any(p + 4 * i + 2) << 16;
-                r.d[h] = ld_u16_any(u.d[h] + (int64_t) b * (Q8 ? 34 : 18));
+                r.d[h] = in ? ld_u16_any(u.d[h] + (int64_t) b * (Q8 ? 34 : 18)) : 0u;
             }
         }
     }
@@ -171,12 +172,15 @@ struct SrcF16 {
         u.last = W.last_block;
     }
     __device__ static __forceinline__ void load(Regs & r, const Cursor & u, int c) {
-        int b = 2 * c + u.off;
-        b = b < u.last ? b : u.last;
+        const int b = 2 * c + u.off;
+        const bool in = b <= u.last;   // past the end of K: zero (an infinity read twice would meet the zero activations)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint8_t * p = u.p[h] + (int64_t) b * 64;
-            if ((((uintptr_t) p) & 15) == 0) {
+            if (!in) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) r.h[h][i] = 0u;
+            } else if ((((uintptr_t) p) & 15) == 0) {
                 const uint4 a = __ldg((const uint4 *) p), e = __ldg((const uint4 *) p + 1);
                 r.h[h][0] = a.x; r.h[h][1] = a.y; r.h[h][2] = a.z; r.h[h][3] = a.w;
                 r.h[h][4] = e.x; r.h[h][5] = e.y; r.h[h][6] = e.z; r.h[h][7] = e.w;

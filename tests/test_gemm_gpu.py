@@ -114,3 +114,22 @@ def test_gemm_forced_tiles(sm100, tn, rt, tmem_a):
     res = json.loads(r.stdout.strip().splitlines()[-1])
     assert res["cases"] == 6
     assert res["worst"] <= TOL, res
+
+
+@pytest.mark.parametrize("k", [160, 192, 224, 256])
+@pytest.mark.parametrize("dtype", [U.F16, U.Q8_0], ids=lambda d: U.NAMES[d])
+def test_infinite_weight_in_the_last_block(sm100, stream, dtype, k):
+    """K is padded to whole stages of 128 weights with weights of zero: an infinity in a row's last 32 weights is multiplied by
+    activations only, and the row is infinite as in the reference, not NaN."""
+    n, m = 40, 77
+    w = np.abs(U.seeded_weights(k, n, k)) + np.float32(0.01)
+    wq = U.quantize(dtype, w)
+    if dtype == U.F16:
+        wq.view(np.float16).reshape(n, k)[7, k - 3] = np.inf
+    else:
+        wq.reshape(n, k // 32, 34)[7, -1, :2] = np.frombuffer(np.float16(np.inf).tobytes(), np.uint8)
+    x = np.abs(U.seeded_acts(k, m, k)) + np.float32(0.01)
+    got = U.device_mul_mat(sm100, stream, dtype, U.NATURAL if dtype == U.F16 else U.PACKED, wq, k, x)
+    assert np.all(got[:, 7] == np.inf)
+    rest = [r for r in range(n) if r != 7]
+    assert sgref.nmse(got[:, rest], sgref.mul_mat(dtype, np.ascontiguousarray(wq[rest]), k, x)) <= TOL
