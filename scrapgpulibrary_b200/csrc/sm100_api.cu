@@ -35,6 +35,7 @@ int sm100_mul_mat(sm100_stream_t s, int dtype, int layout, const void * w, int64
         if (k <= 0 || n <= 0) return fail(ST_INVALID, "mul_mat: K, N and M must be positive");
         bool handled = false;
         const int st = gemm_tc_mul_mat((cudaStream_t) s, dtype, layout, w, w_row_stride, k, n, x, ldx, m, y, ldy, &handled);
+        if (handled) matvec_note_kernel("gemm_tc");
         if (st != ST_OK || handled) return st;
     }
     // narrow batches of packed weights, and Q6_K at any width: the split-operand GEMM, at the column kernels' precision and one pass
@@ -42,6 +43,7 @@ int sm100_mul_mat(sm100_stream_t s, int dtype, int layout, const void * w, int64
     if (layout == LAYOUT_PACKED && is_quant(dtype) && w != nullptr && x != nullptr && y != nullptr && k > 0 && n > 0) {
         bool handled = false;
         const int st = gemm_split_mul_mat((cudaStream_t) s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);
+        if (handled) matvec_note_kernel(n % 16 == 0 ? "gemm_split" : "gemm_split+rows");
         if (st != ST_OK || handled) return st;
     }
     // narrow batches, and shapes or dtypes the tensor-core path leaves alone: column panels of 8 through the matvec

@@ -365,6 +365,59 @@ __global__ void __launch_bounds__(256) matvec_rows(const uint8_t * __restrict__ 
     }
 }
 
+// ---- kernel C: the last few rows of a packed tensor, any number of columns ----------------------------
+// A CTA takes 4 rows x 2 or 4 columns; its threads share K.  There is little of it, and what counts is the length of a thread's own
+// instruction stream: 11 rows of 4096 (Q4_0), 8 columns 2.5 us, 14 with 8 columns per CTA; 15 rows of 12288 (Q6_K), 512 columns 26 us, 78.
+constexpr int TAIL_ROWS = 4, TAIL_THREADS = 256;   // at most: a thread per unit of K
+
+template <class U, int TAIL_COLS>
+__global__ void __launch_bounds__(TAIL_THREADS) matvec_tail(const uint8_t * __restrict__ w, Planes P, const float * x, int64_t ldx, float * y, int64_t ldy,
+                                                            int row_begin, int n_rows, int units_per_row, int m_cols) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ float part[TAIL_THREADS / 32][TAIL_ROWS * TAIL_COLS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r0 = row_begin + blockIdx.x * TAIL_ROWS, c0 = blockIdx.y * TAIL_COLS;
+    const int64_t bpr = units_per_row / U::UNITS_PER_BLOCK;
+    float acc[TAIL_ROWS][TAIL_COLS];
+#pragma unroll
+    for (int i = 0; i < TAIL_ROWS; ++i)
+#pragma unroll
+        for (int c = 0; c < TAIL_COLS; ++c) acc[i][c] = 0.f;
+    for (int cu = threadIdx.x; cu < units_per_row; cu += blockDim.x) {
+        typename U::Data d[TAIL_ROWS];
+#pragma unroll
+        for (int i = 0; i < TAIL_ROWS; ++i) U::load(w, P, min(r0 + i, n_rows - 1), bpr, cu, d[i]);
+#pragma unroll
+        for (int c = 0; c < TAIL_COLS; ++c) {
+            if (c0 + c < m_cols) {
+                float xr[U::WEIGHTS], sums[U::XSUMS];
+                load_x_unit<U>(x + (int64_t) (c0 + c) * ldx, cu, xr, sums);
+#pragma unroll
+                for (int i = 0; i < TAIL_ROWS; ++i) acc[i][c] += U::dot(d[i], cu, xr, sums);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TAIL_ROWS; ++i)
+#pragma unroll
+        for (int c = 0; c < TAIL_COLS; ++c) {
+            float v = acc[i][c];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) part[warp][i * TAIL_COLS + c] = v;
+        }
+    __syncthreads();
+    if (threadIdx.x < TAIL_ROWS * TAIL_COLS) {
+        const int r = r0 + threadIdx.x / TAIL_COLS, c = c0 + threadIdx.x % TAIL_COLS;
+        float v = 0.f;
+#pragma unroll
+        for (int i = 0; i < TAIL_THREADS / 32; ++i)
+            if (i < blockDim.x / 32) v += part[i][threadIdx.x];
+        if (r < n_rows && c < m_cols) y[(int64_t) c * ldy + r] = v;
+    }
+}
+
 // scalar tail for rows whose K is not a whole number of units or whose x is not 16-byte aligned
 // (F32 / F16 weights only; quantized rows are whole blocks by contract)
 template <int DT>
@@ -476,6 +529,34 @@ static int launch_rows(cudaStream_t s, const void * w, int64_t w_row_stride, int
     }
 #undef SM100_ROWS_CASE
     return fail(ST_INVALID, "matvec: M must be 1..8");
+}
+
+template <class U, int COLS>
+static int launch_tail_cols(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
+    const int units = (int) (k / U::WEIGHTS), threads = units >= TAIL_THREADS ? TAIL_THREADS : (units + 31) / 32 * 32;
+    constexpr int64_t MAX_COLS = 65535 * COLS;   // 65535 panels fit the y dimension of a launch
+    for (int64_t c = 0; c < m; c += MAX_COLS) {
+        const int64_t mm = m - c < MAX_COLS ? m - c : MAX_COLS;
+        const dim3 grid((unsigned) ((n - row_begin + TAIL_ROWS - 1) / TAIL_ROWS), (unsigned) ((mm + COLS - 1) / COLS));
+        const int st = launch(matvec_tail<U, COLS>, grid, dim3((unsigned) threads), 0, s, (const uint8_t *) w, planes_for(dtype, n, k), x + c * ldx, ldx, y + c * ldy, ldy,
+                              (int) row_begin, (int) n, units, (int) mm);
+        if (st != ST_OK) return st;
+    }
+    return ST_OK;
+}
+template <class U>
+static int launch_tail(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
+    return m <= 64 ? launch_tail_cols<U, 2>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy) : launch_tail_cols<U, 4>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
+}
+// rows row_begin .. n - 1 of a packed tensor in f32, m columns, x 16-byte aligned
+int tail_rows(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
+    switch (dtype) {
+        case DT_Q4_0: return launch_tail<UnitQ40>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
+        case DT_Q8_0: return launch_tail<UnitQ80>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
+        case DT_Q4_K: return launch_tail<UnitQ4K>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
+        case DT_Q6_K: return launch_tail<UnitQ6K>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
+    }
+    return fail(ST_UNSUPPORTED, "mul_mat: no packed rows of dtype %d", dtype);
 }
 
 template <class U>
@@ -612,7 +693,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         bool handled = false;
         const int st = gemm_split_mul_mat(s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);
         if (st != ST_OK) return st;
-        if (handled) return took("gemm_split", ST_OK);
+        if (handled) return took(n % 16 == 0 ? "gemm_split" : "gemm_split+rows", ST_OK);
     }
     // Q6_K with 2..8 columns: the tensor-core kernel assembles the 6-bit weights of a step once and multiplies them with every
     // column (measured on 4096 x 4096: 8 columns in 2.2 times the time of one, where eight single-column launches took 7.4 times)

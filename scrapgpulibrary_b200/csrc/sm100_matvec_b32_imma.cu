@@ -321,17 +321,18 @@ int launch_bq(cudaStream_t s, const BqArgs & a, size_t smem, int grid) {
 
 }  // namespace
 
+bool b32_imma_serves(int64_t k) { return k % 128 == 0 && k <= (int64_t) 1 << 20 && bq_smem_bytes((int) (k / 32)) <= (size_t) 227 * 1024; }
+
 // Q4_0 / Q8_0 packed matvec, one activation column, over the full 16-row tiles of the tensor; *handled = false
 // when the shape is left to the caller's other kernels.
 int matvec_b32_imma_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, float * y, bool * handled) {
     *handled = false;
     const int64_t tiles = n / 16;
-    if (tiles == 0 || k % 128 != 0 || k > (int64_t) 1 << 20 || tiles > INT32_MAX / 2) return ST_OK;
+    if (tiles == 0 || !b32_imma_serves(k) || tiles > INT32_MAX / 2) return ST_OK;
     if (dtype != DT_Q4_0 && dtype != DT_Q8_0) return ST_OK;
     if (((uintptr_t) w & 31) != 0 || ((uintptr_t) x & 15) != 0) return ST_OK;
     const int blocks = (int) (k / 32);
     const size_t smem = bq_smem_bytes(blocks);
-    if (smem > (size_t) 227 * 1024) return ST_OK;
     BqArgs a;
     a.w = (const uint8_t *) w;
     a.d_off = n * (int64_t) blocks * (dtype == DT_Q8_0 ? 32 : 16);

@@ -851,6 +851,9 @@ int matvec_q4k_imma_multi(cudaStream_t s, int count, const void * const * ws, co
     return st;
 }
 
+// Do 3 or more columns of rows of length k go to the integer kernel below (all at once or four at a time)?
+bool q4k_cols_serves(int64_t k) { return k % 256 == 0 && k / 64 <= 4096 && iq_cols_smem_bytes((int) (k / 64), 4, 2) <= (size_t) 227 * 1024; }
+
 // 3..8 activation columns of one packed Q4_K tensor over its full 16-row tiles; *handled = false when the shape
 // (or the shared memory the quantized columns need) is left to the caller's other kernels.
 int matvec_q4k_imma_cols_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,

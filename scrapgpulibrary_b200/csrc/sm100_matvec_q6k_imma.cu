@@ -342,16 +342,17 @@ size_t sq_smem_bytes(int units, int cols = 1) { return (size_t) cols * ((size_t)
 
 }  // namespace
 
+bool q6k_imma_serves(int64_t k) { return k % 256 == 0 && k <= (int64_t) 1 << 18 && sq_smem_bytes((int) (k / 64)) <= (size_t) 227 * 1024; }
+
 // Q6_K packed matvec, one activation column, over the full 16-row tiles of the tensor; *handled = false when the
 // shape is left to the caller's other kernels.
 int matvec_q6k_imma_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, float * y, bool * handled) {
     *handled = false;
     const int64_t tiles = n / 16;
-    if (tiles == 0 || k % 256 != 0 || k > (int64_t) 1 << 18 || tiles > INT32_MAX / 2) return ST_OK;
+    if (tiles == 0 || !q6k_imma_serves(k) || tiles > INT32_MAX / 2) return ST_OK;
     if (((uintptr_t) w & 15) != 0 || ((uintptr_t) x & 15) != 0) return ST_OK;
     const int units = (int) (k / 64);
     const size_t smem = sq_smem_bytes(units);
-    if (smem > (size_t) 227 * 1024) return ST_OK;
     const Planes P = planes_for(DT_Q6_K, n, k);
     SqArgs a;
     a.w = (const uint8_t *) w;
@@ -394,10 +395,9 @@ static int launch_q6k_cols(cudaStream_t s, SqArgs a, int grid) {
 int matvec_q6k_imma_cols(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int m, float * y, int64_t ldy, bool * handled) {
     *handled = false;
     const int64_t tiles = n / 16;
-    if (m < 2 || m > 8 || tiles == 0 || k % 256 != 0 || k > (int64_t) 1 << 18 || tiles > INT32_MAX / 2) return ST_OK;
+    if (m < 2 || m > 8 || tiles == 0 || !q6k_imma_serves(k) || tiles > INT32_MAX / 2) return ST_OK;
     if (((uintptr_t) w & 15) != 0 || ((uintptr_t) x & 15) != 0 || ldx % 4 != 0) return ST_OK;
     const int units = (int) (k / 64);
-    if (sq_smem_bytes(units, 1) > (size_t) 227 * 1024) return ST_OK;
     const Planes P = planes_for(DT_Q6_K, n, k);
     SqArgs a;
     a.w = (const uint8_t *) w;

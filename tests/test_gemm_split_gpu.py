@@ -121,6 +121,25 @@ def test_captures_on_two_streams(sm100):
         s.close()
 
 
+# the last N mod 16 rows behind whole tiles (one row, 15 rows; one panel of 8 columns, a ragged one, many), fewer rows than a tile, rows
+# that are not whole units of the integer kernels, rows too long for them
+@pytest.mark.parametrize("dtype,k,n,m,tail", [(U.Q4_0, 1024, 1025, 5, 1), (U.Q8_0, 4096, 47, 17, 15), (U.Q4_K, 512, 140, 9, 12), (U.Q4_K, 12288, 24, 32, 8),
+                                              (U.Q6_K, 768, 1031, 3, 7), (U.Q6_K, 4096, 29, 12, 13), (U.Q6_K, 4096, 520, 300, 8), (U.Q6_K, 12288, 31, 40, 15),
+                                              (U.Q4_K, 1024, 8, 9, 8), (U.Q6_K, 4096, 15, 64, 15), (U.Q4_0, 160, 48, 31, 48), (U.Q8_0, 4064, 64, 12, 64),
+                                              (U.Q4_K, 14592, 32, 12, 32)], ids=lambda v: str(v))
+def test_rows_that_stay_in_f32(sm100, stream, dtype, k, n, m, tail):
+    """What the f32 kernels serve of a batch keeps their precision.  Against float64: 2e-7 to 1.2e-6 measured; the split GEMM, whose
+    operands have 16 bits, leaves 5e-6 or more."""
+    wq = U.quantize(dtype, U.seeded_weights(7000 + dtype + k, n, k))
+    x = U.seeded_acts(3 * m + k, m, k)
+    want = x.astype(np.float64) @ sgref.dequantize(dtype, wq, k).astype(np.float64).T
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x)
+    part = slice(n - tail, n)
+    err = np.linalg.norm(got[:, part] - want[:, part]) / np.linalg.norm(want[:, part])
+    assert err <= 2e-6, err
+    assert sgref.nmse(got.astype(np.float64), want) <= 4 * TOL
+
+
 # the second environment: as if there were no memory to be had
 @pytest.mark.parametrize("env", [{}, {"SM100_CALL_SCRATCH": "0"}], ids=["", "no_memory"])
 @pytest.mark.parametrize("dtype,m", [(U.Q6_K, 8), (U.Q6_K, 200), (U.Q4_0, 8), (U.Q4_K, 24)], ids=lambda v: str(v))
