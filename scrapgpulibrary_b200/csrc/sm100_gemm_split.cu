@@ -48,6 +48,9 @@ template <bool PREP> constexpr int sp_groups = PREP ? 3 : 2;
 template <bool PREP> constexpr int sp_threads = 32 * (SP_FIRST_PRODUCER + 8 * sp_groups<PREP> + (PREP ? 0 : 5));
 constexpr int SP_BULK_WARPS = 3, SP_CONVERT_WARPS = 8;
 constexpr int SP_A_COLS = 64;          // TMEM columns of a weight stage: wh (32), wl (32)
+// Chunks that one CTA adds up at most.  The tensor core truncates, so the error grows with the chain: Q6_K, 512 columns, 12288 weights
+// 1.68e-5, 14336 1.88e-5, 28672 3.4e-5, where the integer column kernels have 1.83e-5 at any length.
+constexpr int SP_CHAIN = 208;
 
 struct SplitArgs {
     WeightRef w;
@@ -459,7 +462,7 @@ template <int TN, bool PREP>
 TilePlan split_plan(const SplitArgs & g) {
     constexpr int SUB = SplitSmem<TN, PREP>::SUB;
     const int64_t tiles = (int64_t) ((g.n + SP_TM - 1) / SP_TM) * g.m_tiles;
-    return plan_tiles(tiles, g.nchunks / SUB, (TN >= 128 ? 20 : 15) * SUB, (int64_t) SP_TM * (g.m < TN ? g.m : TN));   // a chunk takes 1.5 to 2 times as long as the f16 GEMM's
+    return plan_tiles(tiles, g.nchunks / SUB, (TN >= 128 ? 20 : 15) * SUB, (int64_t) SP_TM * (g.m < TN ? g.m : TN), (g.nchunks + SP_CHAIN - 1) / SP_CHAIN);   // a chunk takes 1.5 to 2 times as long as the f16 GEMM's
 }
 template <int TN>
 size_t part_bytes(const TilePlan & plan) { return (size_t) plan.cut * plan.splits * TN * SP_TM * sizeof(float); }
@@ -481,25 +484,34 @@ int launch_split(cudaStream_t s, SplitArgs g, const TilePlan & plan, void * part
 }
 
 template <typename S, int TN>
-int batch_split(cudaStream_t s, SplitArgs g) {
+int batch_split(cudaStream_t s, SplitArgs g, bool * handled) {
     TilePlan plan = split_plan<TN, false>(g);
     CallScratch mem;
-    if (plan.cut > 0 && call_scratch_alloc(s, part_bytes<TN>(plan), &mem) != ST_OK) plan = {plan.whole + plan.cut, 0, 1};   // no memory: one CTA per tile needs none
+    if (plan.cut > 0 && call_scratch_alloc(s, part_bytes<TN>(plan), &mem) != ST_OK) {   // no memory: one CTA per tile needs none
+        if (g.nchunks > SP_CHAIN) return ST_OK;
+        plan = {plan.whole + plan.cut, 0, 1};
+    }
+    *handled = true;
     const int st = launch_split<S, TN, false>(s, g, plan, mem.ptr);
     const int fr = call_scratch_free(s, mem);
     return st != ST_OK ? st : fr;
 }
 template <typename S>
-int batch_split(cudaStream_t s, SplitArgs g) {
+int batch_split(cudaStream_t s, SplitArgs g, bool * handled) {
     g.m_tiles = 1;
     g.nchunks = (g.nchunks + 1) / 2 * 2;   // whole stages of two chunks
-    return g.m <= 16 ? batch_split<S, 16>(s, g) : batch_split<S, 32>(s, g);
+    return g.m <= 16 ? batch_split<S, 16>(s, g, handled) : batch_split<S, 32>(s, g, handled);
 }
 
 template <typename S, int TN>
 int prompt_split(cudaStream_t s, SplitArgs g, const float * x, int64_t ldx, int64_t m, float * y, bool * handled) {
-    // tokens per pass: the images of one pass stay below 64 MiB
+    // tokens per pass: the images of one pass stay below 64 MiB, and where every tile is cut its partial tiles below 256 MiB
     int64_t pass = ((int64_t) 64 << 20) / ((int64_t) g.nchunks * SP_KC * 4) / TN * TN;
+    if (g.nchunks > SP_CHAIN) {
+        const int64_t rows = ((int64_t) g.n + SP_TM - 1) / SP_TM * SP_TM * ((g.nchunks + SP_CHAIN - 1) / SP_CHAIN);
+        const int64_t fit = ((int64_t) 256 << 20) / (rows * 4) / TN * TN;
+        if (pass > fit) pass = fit;
+    }
     if (pass < TN) pass = TN;
     auto tokens = [&](int64_t c0) {
         g.m = (int) (m - c0 < pass ? m - c0 : pass);
@@ -565,16 +577,16 @@ int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int
     int st = ST_OK;
     if (m > 32) {
         st = m <= 64 ? prompt_split<SrcQ6K, 64>(s, g, x, ldx, m, y, handled) : prompt_split<SrcQ6K, 128>(s, g, x, ldx, m, y, handled);
-        if (st != ST_OK || !*handled) return st;
     } else {
         switch (dtype) {
-            case DT_Q4_0: st = batch_split<SrcB32<false, true>>(s, g); break;
-            case DT_Q8_0: st = batch_split<SrcB32<true, true>>(s, g); break;
-            case DT_Q4_K: st = batch_split<SrcQ4K>(s, g); break;
-            default: st = batch_split<SrcQ6K>(s, g); break;
+            case DT_Q4_0: st = batch_split<SrcB32<false, true>>(s, g, handled); break;
+            case DT_Q8_0: st = batch_split<SrcB32<true, true>>(s, g, handled); break;
+            case DT_Q4_K: st = batch_split<SrcQ4K>(s, g, handled); break;
+            default: st = batch_split<SrcQ6K>(s, g, handled); break;
         }
     }
-    if (st == ST_OK && full < n) st = tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy);
+    if (st != ST_OK || !*handled) return st;
+    if (full < n) st = tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy);
     *handled = st == ST_OK;
     return st;
 }

@@ -151,12 +151,13 @@ struct TilePlan {
 };
 // Costs in tenths of a chunk's time of a 128 x 128 tile (about 0.3 us).  A wave costs its chunks (`per_chunk` each) plus about eight chunks of start and epilogue; partial tiles cost another six for the
 // launch that adds them and a write and a read of every partial output (`outputs` per tile).  Ties go to fewer CTAs.
-inline TilePlan plan_tiles(int64_t tiles, int nchunks, int per_chunk, int64_t outputs) {
+// `least` > 1: no CTA may take the whole of K, every tile is cut.
+inline TilePlan plan_tiles(int64_t tiles, int nchunks, int per_chunk, int64_t outputs, int least) {
     const int64_t sms = sm_count();
-    TilePlan p = {tiles / sms * sms, tiles % sms, 1};
+    TilePlan p = {least > 1 ? 0 : tiles / sms * sms, least > 1 ? tiles : tiles % sms, 1};
     if (p.cut > 0) {
         int64_t best = INT64_MAX;
-        for (int s = 1; s <= 8 && s <= nchunks; ++s) {
+        for (int s = least; s <= least + 7 && s <= nchunks; ++s) {
             const int64_t cost = (p.cut * s + sms - 1) / sms * ((int64_t) ((nchunks + s - 1) / s) * per_chunk + 80) + (s > 1 ? 60 + s * p.cut * outputs / 20000 : 0);
             if (cost < best) { best = cost; p.splits = s; }
         }

@@ -121,6 +121,21 @@ def test_captures_on_two_streams(sm100):
         s.close()
 
 
+# whole tiles only where nothing needs cutting, tiles of a prompt; and one shape below the limit
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 28672, 148 * 128, 4), (U.Q6_K, 28672, 1024, 130), (U.Q6_K, 14336, 512, 300), (U.Q6_K, 12288, 512, 300)], ids=lambda v: str(v))
+def test_error_does_not_grow_with_k(sm100, stream, dtype, k, n, m):
+    """The tensor core truncates when it adds: K is cut so that no chain is longer than 13312 weights, and the error against float64 stays
+    below that of the integer column kernels (1.8e-5 to 2.1e-5 at any K; 3.1e-5 and more were seen at 28672 in one chain)."""
+    wq = U.quantize(dtype, U.seeded_weights(7000 + dtype + k, min(n, 640), k))
+    wq = np.ascontiguousarray(np.resize(wq, (n, wq.shape[1])))
+    x = U.seeded_acts(3 * m + k, m, k)
+    rows = np.r_[0:256, n - 256:n]
+    want = x.astype(np.float64) @ sgref.dequantize(dtype, np.ascontiguousarray(wq[rows]), k).astype(np.float64).T
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x)[:, rows]
+    err = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert err <= 1.8e-5, err
+
+
 # the last N mod 16 rows behind whole tiles (one row, 15 rows; one panel of 8 columns, a ragged one, many), fewer rows than a tile, rows
 # that are not whole units of the integer kernels, rows too long for them
 @pytest.mark.parametrize("dtype,k,n,m,tail", [(U.Q4_0, 1024, 1025, 5, 1), (U.Q8_0, 4096, 47, 17, 15), (U.Q4_K, 512, 140, 9, 12), (U.Q4_K, 12288, 24, 32, 8),
