@@ -136,6 +136,16 @@ def test_error_does_not_grow_with_k(sm100, stream, dtype, k, n, m):
     assert err <= 1.8e-5, err
 
 
+@pytest.mark.parametrize("dtype,k,n", [(U.Q4_0, 4096, 1040), (U.Q8_0, 2048, 3000), (U.Q4_K, 4096, 300), (U.Q6_K, 6144, 2064)], ids=lambda v: str(v))
+def test_columns_do_not_depend_on_their_batch(sm100, stream, dtype, k, n):
+    """Bit for bit, over the 16 and 32 column tiles (Q4_K: from 17 columns on, fewer belong to the column kernel)."""
+    wq = U.quantize(dtype, U.seeded_weights(dtype + k, n, k))
+    x = U.seeded_acts(k, 32, k)
+    all_ = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x)
+    for m in [24, 17] + ([] if dtype == U.Q4_K else [16, 9]) + ([7] if n >= 1024 and dtype != U.Q4_K else []):
+        assert np.array_equal(U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x[:m]), all_[:m]), m
+
+
 # the last N mod 16 rows behind whole tiles (one row, 15 rows; one panel of 8 columns, a ragged one, many), fewer rows than a tile, rows
 # that are not whole units of the integer kernels, rows too long for them
 @pytest.mark.parametrize("dtype,k,n,m,tail", [(U.Q4_0, 1024, 1025, 5, 1), (U.Q8_0, 4096, 47, 17, 15), (U.Q4_K, 512, 140, 9, 12), (U.Q4_K, 12288, 24, 32, 8),
