@@ -15,6 +15,7 @@ int matvec_q4k_ring_multi(cudaStream_t s, int count, const void * const * ws, co
                           float * const * ys, bool * handled, const Q4KPrologue * pro, const ArFuse * fuse);
 int gemm_tc_mul_mat(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_stride, int64_t k, int64_t n, const float * x,
                     int64_t ldx, int64_t m, float * y, int64_t ldy, bool * handled);
+int q4k_batch(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy, bool * handled);
 int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
                        bool * handled);
 }
@@ -39,10 +40,14 @@ int sm100_mul_mat(sm100_stream_t s, int dtype, int layout, const void * w, int64
         if (st != ST_OK || handled) return st;
     }
     // narrow batches of packed weights, and Q6_K at any width: the split-operand GEMM, at the column kernels' precision and one pass
-    // over the weights instead of one per 8 columns (Q4_K 12288 x 4096, 24 columns: 34 us, 63 in panels)
+    // over the weights instead of one per 8 columns (Q4_K 12288 x 4096, 24 columns: 34 us, 63 in panels); Q4_K batches that are faster in
+    // panels all the same stay there
     if (layout == LAYOUT_PACKED && is_quant(dtype) && w != nullptr && x != nullptr && y != nullptr && k > 0 && n > 0) {
         bool handled = false;
-        const int st = gemm_split_mul_mat((cudaStream_t) s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);
+        int st = ST_OK;
+        if (dtype == DT_Q4_K) st = q4k_batch((cudaStream_t) s, w, k, n, x, ldx, m, y, ldy, &handled);
+        if (st != ST_OK || handled) return st;
+        st = gemm_split_mul_mat((cudaStream_t) s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);
         if (handled) matvec_note_kernel(n % 16 == 0 ? "gemm_split" : "gemm_split+rows");
         if (st != ST_OK || handled) return st;
     }

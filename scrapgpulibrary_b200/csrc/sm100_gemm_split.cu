@@ -33,7 +33,7 @@
 namespace sm100 {
 
 bool b32_imma_serves(int64_t k);
-bool q4k_cols_serves(int64_t k);
+int q4k_cols_width(int64_t k);
 bool q6k_imma_serves(int64_t k);
 int tail_rows(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy);
 
@@ -491,7 +491,7 @@ int batch_split(cudaStream_t s, SplitArgs g, bool * handled) {
     CallScratch mem;
     if (plan.cut > 0 && call_scratch_alloc(s, part_bytes<TN>(plan), &mem) != ST_OK) {   // no memory: one CTA per tile needs none
         if (g.nchunks > SP_CHAIN) return ST_OK;
-        plan = {plan.whole + plan.cut, 0, 1};
+        plan = {plan.whole + plan.cut, 0, 1, plan.cost};
     }
     *handled = true;
     const int st = launch_split<S, TN, false>(s, g, plan, mem.ptr);
@@ -541,6 +541,32 @@ int prompt_split(cudaStream_t s, SplitArgs g, const float * x, int64_t ldx, int6
 
 }  // namespace
 
+// Is a batch faster in the integer column kernels, `width` columns a launch, than in one pass of the split GEMM?  Both times as measured
+// (us, within 8 % or so over K 1024 .. 12288, N 64 .. 151936; what the rule picks was at most 5 % slower than the other way):
+//   columns    a launch of 8 columns: 3.05 and, for every round of 16-row tiles (two per SM), 0.385 + 0.695 K / 1024 with Q4_K; 2.8 + K / 1024
+//              and 0.9 + 2.35 K / 1024 with Q6_K; of a round of a narrower Q4_K launch 0.58 + 0.056 per column; where rows are so long that
+//              only four columns fit, 8 % more
+//   split GEMM the cost of its plan times 0.031 + 0.0004 per column (Q4_K), 0.041 (Q6_K)
+// Measured, columns / split: Q4_K 4096 x 12288, 9 columns 21.6 / 32.9, 16 columns 26.9 / 35.6, 20 columns 37.6 / 37.2; 4096 x 4096, 16 columns
+// 13.0 / 15.3; 4096 x 1024, 16 columns 11.7 / 9.4; 12288 x 4096, 12 columns 31.4 / 30.9; Q6_K 5120 x 13824, 8 columns 47.0 / 53.0,
+// 4096 x 4096 17.2 / 16.1.
+bool columns_faster(int dtype, int64_t k, int64_t n, int64_t m, int width) {
+    if (m > 32) return false;
+    SplitArgs g = {};
+    g.n = (int) (n / 16 * 16);
+    g.m_tiles = 1;
+    g.nchunks = (int) ((k + 2 * SP_KC - 1) / (2 * SP_KC)) * 2;
+    const double cost = (double) split_plan<16, false>(g).cost, kk = (double) k / 1024;
+    const int64_t at_once = 2 * (int64_t) sm_count(), rounds = (n / 16 + at_once - 1) / at_once;
+    if (dtype == DT_Q6_K) return 2.8 + kk + (double) rounds * (0.9 + 2.35 * kk) < 0.041 * cost;
+    double columns = 0;
+    for (int64_t c = 0; c < m; c += width) {
+        const int64_t mm = m - c < width ? m - c : width;
+        columns += 3.05 + (double) rounds * (0.385 + 0.695 * kk) * (mm == 8 ? 1.0 : 0.58 + 0.056 * (double) mm);
+    }
+    return columns * (width == 8 ? 1.0 : 1.08) < cost * (0.031 + 0.0004 * (double) m);
+}
+
 // Packed Q4_0 / Q8_0 / Q4_K / Q6_K with up to 32 columns, or Q6_K with any number; *handled = false (and ST_OK) when the shape is
 // left to the caller's other kernels.
 // It takes the place of the integer column kernels only, whose 16-bit activations are coarser than its operands (relative error
@@ -553,7 +579,7 @@ int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int
     if (n < 16 || k <= 0 || (m > 32 && dtype != DT_Q6_K)) return ST_OK;
     switch (dtype) {
         case DT_Q4_0: case DT_Q8_0: if (!b32_imma_serves(k)) return ST_OK; break;
-        case DT_Q4_K: if (!q4k_cols_serves(k)) return ST_OK; break;
+        case DT_Q4_K: if (q4k_cols_width(k) == 0) return ST_OK; break;
         case DT_Q6_K: if (!q6k_imma_serves(k)) return ST_OK; break;
         default: return ST_OK;
     }

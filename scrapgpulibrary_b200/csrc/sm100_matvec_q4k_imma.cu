@@ -851,13 +851,21 @@ int matvec_q4k_imma_multi(cudaStream_t s, int count, const void * const * ws, co
     return st;
 }
 
-// Do 3 or more columns of rows of length k go to the integer kernel below (all at once or four at a time)?
-bool q4k_cols_serves(int64_t k) { return k % 256 == 0 && k / 64 <= 4096 && iq_cols_smem_bytes((int) (k / 64), 4, 2) <= (size_t) 227 * 1024; }
+// How many columns of rows of length k the integer kernel below takes in a launch: 8, 4, or 0 if it leaves them alone
+int q4k_cols_width(int64_t k) {
+    if (k <= 0 || k % 256 != 0 || k / 64 > 4096) return 0;
+    for (int cols = 8; cols >= 4; cols -= 4)
+        if (iq_cols_smem_bytes((int) (k / 64), cols, 2) <= (size_t) 227 * 1024) return cols;
+    return 0;
+}
+// bytes of the prepared image of 1..8 columns
+size_t q4k_cols_image_bytes(int64_t k, int64_t cols) { return (size_t) (cols > 4 ? 8 : 4) * (size_t) (k / 64 * 128 + (k / 64 + 1) * 16); }
 
 // 3..8 activation columns of one packed Q4_K tensor over its full 16-row tiles; *handled = false when the shape
-// (or the shared memory the quantized columns need) is left to the caller's other kernels.
+// (or the shared memory the quantized columns need) is left to the caller's other kernels.  img: memory for the quantized columns
+// (q4k_cols_image_bytes), or null for the library's scratch.
 int matvec_q4k_imma_cols_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
-                               bool * handled) {
+                               bool * handled, void * img) {
     *handled = false;
     const int64_t tiles = n / 16;
     if (tiles == 0 || m < 3 || m > 8 || k % 256 != 0 || k / 64 > 4096 || tiles > INT32_MAX / 2) return ST_OK;
@@ -886,10 +894,8 @@ int matvec_q4k_imma_cols_tiles(cudaStream_t s, const void * w, int64_t k, int64_
     const int64_t rounds = (tiles + IQ_GROUPS - 1) / IQ_GROUPS;
     if (grid > rounds) grid = rounds;
     const int mt = 4 * mg;
-    void * img = nullptr;
     int st = fault_word(FAULT_Q4K, &a.fault);
-    if (st != ST_OK) return st;
-    st = device_scratch(2, (size_t) mt * (pairs * 128 + (pairs + 1) * 16), &img);
+    if (st == ST_OK && img == nullptr) st = device_scratch(2, q4k_cols_image_bytes(k, m), &img);
     if (st != ST_OK) return st;
     const int q_items = mt * pairs * 16;
     st = launch(q4k_quantize_cols, dim3((unsigned) ((q_items + 255) / 256)), dim3(256), 0, s, x, ldx, (int) m, mt, pairs, (uint32_t *) img);

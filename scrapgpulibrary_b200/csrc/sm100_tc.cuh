@@ -148,21 +148,26 @@ struct TilePlan {
     int64_t whole;   // tiles [0, whole): one CTA each
     int64_t cut;     // tiles [whole, whole + cut): `splits` CTAs each
     int splits;
+    int64_t cost;    // of the whole launch
 };
-// Costs in tenths of a chunk's time of a 128 x 128 tile (about 0.3 us).  A wave costs its chunks (`per_chunk` each) plus about eight chunks of start and epilogue; partial tiles cost another six for the
-// launch that adds them and a write and a read of every partial output (`outputs` per tile).  Ties go to fewer CTAs.
+// Costs in tenths of a chunk's time of a 128 x 128 tile (about 0.3 us).  A wave costs its chunks (`per_chunk` each) plus about eight chunks of
+// start and epilogue; partial tiles cost another six for the launch that adds them and a write and a read of every partial output
+// (`outputs` per tile).  Ties go to fewer CTAs.
 // `least` > 1: no CTA may take the whole of K, every tile is cut.
 inline TilePlan plan_tiles(int64_t tiles, int nchunks, int per_chunk, int64_t outputs, int least) {
     const int64_t sms = sm_count();
-    TilePlan p = {least > 1 ? 0 : tiles / sms * sms, least > 1 ? tiles : tiles % sms, 1};
+    TilePlan p = {least > 1 ? 0 : tiles / sms * sms, least > 1 ? tiles : tiles % sms, 1, 0};
+    const int64_t waves = p.whole / sms;
+    int64_t best = 0;
     if (p.cut > 0) {
-        int64_t best = INT64_MAX;
+        best = INT64_MAX;
         for (int s = least; s <= least + 7 && s <= nchunks; ++s) {
             const int64_t cost = (p.cut * s + sms - 1) / sms * ((int64_t) ((nchunks + s - 1) / s) * per_chunk + 80) + (s > 1 ? 60 + s * p.cut * outputs / 20000 : 0);
             if (cost < best) { best = cost; p.splits = s; }
         }
     }
-    if (p.splits == 1) p = {tiles, 0, 1};
+    p.cost = waves * ((int64_t) nchunks * per_chunk + 80) + best;
+    if (p.splits == 1) p = {tiles, 0, 1, p.cost};
     return p;
 }
 inline int64_t plan_ctas(const TilePlan & p) { return p.whole + p.cut * p.splits; }

@@ -1,5 +1,5 @@
 """Worker of tests/test_gemm_split_gpu.py::test_first_product_of_a_process_is_captured: the process' first product is recorded into a
-graph (argument: dtype, columns), which is then looked at and run through the driver API, as a program does that has graphs of
+graph (arguments: dtype, columns, K, N), which is then looked at and run through the driver API, as a program does that has graphs of
 its own.  Prints one JSON line with the worst NMSE and what the graph is made of."""
 import ctypes as C
 import json
@@ -16,14 +16,13 @@ from scrapgpulibrary_b200 import capi  # noqa: E402
 from tests import util as U  # noqa: E402
 
 
-def main(dtype, m):
+def main(dtype, m, k, n):
     capi.require_device()
     cu = C.CDLL("libcuda.so.1")
 
     def ok(status):
         assert status == 0, f"driver API: {status}"
 
-    k, n = 768, 1061
     wq = U.quantize(dtype, U.seeded_weights(11 + dtype, n, k))
     xs = [U.seeded_acts(20 + i, m, k) for i in range(3)]
     want = [sgref.mul_mat(dtype, wq, k, x) for x in xs]
@@ -91,4 +90,4 @@ def main(dtype, m):
 
 
 if __name__ == "__main__":
-    main(int(sys.argv[1]), int(sys.argv[2]))
+    main(*(int(a) for a in sys.argv[1:5]))
