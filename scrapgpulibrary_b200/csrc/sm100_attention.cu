@@ -995,6 +995,20 @@ static bool attention_is_prompt(const AttnArgs & a) {
     return rows >= AP_ROWS && (rows + AP_ROWS - 1) / AP_ROWS * a.hkv >= 64;
 }
 
+// Causal prompts whose last tiles see many more keys than the first leave most SMs idle when there is one round of few tiles; with heads in
+// groups of 2 or 4 the decode kernel, whose work follows the visible keys, is the faster one then.  Measured, decode (with the zeroing of its
+// counters) / prompt kernel, us, at `tiles` times mean over most visible keys: group 4 (8 / 2 heads) 512 queries, no prefix (32) 91 / 106, behind 256
+// keys (43) 147 / 152, 576 queries behind 128 (43) 141 / 143, 704 queries (44) 151 / 143, (4 / 1 heads) 1024 queries (32) 151 / 198, behind 512 (43) 259 / 291, (16 / 4 heads)
+// 320 queries behind 64 (47) 99 / 86, (32 / 8 heads) 128 queries behind 64 keys (43) 58 / 49; group 2 (4 / 2 heads) 1024 queries (32) 185 / 199; group 8,
+// 512 queries (32) 118 / 106; 288 queries, no prefix (16 / 4 heads, 36) 71 / 70.
+static bool attention_prompt_uneven(const AttnArgs & a) {
+    const int64_t group = a.hq / a.hkv;
+    if (!a.causal || a.positions != nullptr || (group != 2 && group != 4)) return false;
+    const int64_t tiles = (a.nq * group + AP_ROWS - 1) / AP_ROWS * a.hkv;
+    const int64_t first = a.offset + 1 < 0 ? 0 : a.offset + 1 < a.nk ? a.offset + 1 : a.nk, last = a.offset + a.nq < 0 ? 0 : a.offset + a.nq < a.nk ? a.offset + a.nq : a.nk;
+    return last > 320 && tiles * (first + last) < 2 * (group == 2 ? 35 : last < 768 ? 42 : 46) * last;
+}
+
 static int attention_prompt_launch(cudaStream_t s, const AttnArgs & a) {
     const int64_t rows = a.nq * (a.hq / a.hkv);
     SM100_CUDA(cudaFuncSetAttribute(attn_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(ApSmem)));
@@ -1003,6 +1017,7 @@ static int attention_prompt_launch(cudaStream_t s, const AttnArgs & a) {
 
 
 int device_scratch(int slot, size_t bytes, void ** out);
+void matvec_note_kernel(const char * name);
 
 static int workspace(size_t bytes, float ** out) {
     void * p = nullptr;
@@ -1086,6 +1101,23 @@ void attention_plan(AttnArgs & a) {
     a.splits = (int) ((a.nk + chunk - 1) / chunk);
 }
 
+// An uneven prompt in the decode kernel.  Its partials are memory of the call, so that prompts on several streams share nothing as with
+// the prompt kernel; *handled = false where there is none, and in a capture, which keeps the kernel that needs none.
+static int attention_uneven_launch(cudaStream_t s, AttnArgs a, bool * handled) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    SM100_CUDA(cudaStreamIsCapturing(s, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return ST_OK;
+    attention_plan(a);
+    CallScratch mem;
+    if (call_scratch_alloc(s, attention_scratch_bytes(a), &mem) != ST_OK) return ST_OK;
+    *handled = true;
+    matvec_note_kernel("attn_splits");
+    const cudaError_t e = cudaMemsetAsync(mem.ptr, 0, (size_t) (a.nq * a.hkv < ATT_COUNTER_SLOTS ? a.nq * a.hkv : ATT_COUNTER_SLOTS) * sizeof(int), s);
+    const int st = e == cudaSuccess ? attention_launch(s, a, (float *) mem.ptr) : cuda_fail(e, "cudaMemsetAsync(attention counters)");
+    const int fr = call_scratch_free(s, mem);
+    return st != ST_OK ? st : fr;
+}
+
 }  // namespace sm100
 
 using namespace sm100;
@@ -1101,11 +1133,18 @@ static int attention_entry(sm100_stream_t s, const float * q, const float * k, c
     a.fresh_keys = fresh_keys;
     const int st = attention_check(a);
     if (st != ST_OK) return st;
-    if (attention_is_prompt(a)) return attention_prompt_launch((cudaStream_t) s, a);
+    if (attention_is_prompt(a)) {
+        bool handled = false;
+        const int su = attention_prompt_uneven(a) ? attention_uneven_launch((cudaStream_t) s, a, &handled) : ST_OK;
+        if (su != ST_OK || handled) return su;
+        matvec_note_kernel("attn_prompt");
+        return attention_prompt_launch((cudaStream_t) s, a);
+    }
     attention_plan(a);
     float * ws = nullptr;
     const int sw = workspace(attention_scratch_bytes(a), &ws);
     if (sw != ST_OK) return sw;
+    matvec_note_kernel("attn_splits");
     return attention_launch((cudaStream_t) s, a, ws);
 }
 

@@ -133,3 +133,38 @@ def test_rounding_does_not_grow_with_the_context(sm100, stream, nk, bound):
     want = (p / p.sum(-1, keepdims=True)) @ v[0].astype(np.float64)
     err = np.linalg.norm(_run(sm100, stream, q, k, v, True, off)[:g] - want) / np.linalg.norm(want)
     assert err <= bound, err
+
+
+# few tiles whose rows see very different numbers of keys; more tiles, a long prefix, heads in groups of 8 and 1, no causal mask, few keys
+@pytest.mark.parametrize("hq,hkv,nq,nk,causal,name", [(8, 2, 512, 512, True, "attn_splits"), (4, 1, 1024, 1300, True, "attn_splits"), (12, 3, 345, 400, True, "attn_splits"),
+                                                      (4, 2, 1024, 1024, True, "attn_splits"), (8, 2, 768, 768, True, "attn_prompt"), (8, 2, 512, 1536, True, "attn_prompt"),
+                                                      (8, 1, 512, 512, True, "attn_prompt"), (8, 8, 512, 512, True, "attn_prompt"), (8, 2, 512, 512, False, "attn_prompt"),
+                                                      (32, 8, 128, 128, True, "attn_prompt")], ids=lambda v: str(v))
+def test_uneven_prompts_take_the_faster_kernel(sm100, stream, hq, hkv, nq, nk, causal, name):
+    """Same values whichever kernel serves a call; a captured one always has the kernel that needs no memory.  Calls on two streams
+    share nothing."""
+    q, k, v = _inputs(hq, hkv, nq, nk)
+    off = nk - nq if causal else 0
+    want = sgref.attention(q, k, v, causal, off, SCALE)
+    assert sgref.nmse(_run(sm100, stream, q, k, v, causal, off), want) <= TOL
+    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == name
+    qb, kb, vb = (U.to_device(sm100, stream, a) for a in (q, k, v))
+    ob, optr = U.guarded_output(sm100, stream, hq * nq * 128)
+    stream.sync()
+    graph = sm100.Graph(stream)
+    with graph:
+        sm100.check(sm100.lib().sm100_attention(stream.handle, qb.at(), kb.at(), vb.at(), None, 1, C.c_void_p(optr), 128, 128, nq, nk, hq, hkv, int(causal), off, None, SCALE), "attention")
+    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == "attn_prompt"
+    graph.launch()
+    stream.sync()
+    assert sgref.nmse(U.read_guarded(sm100, stream, ob, hq * nq * 128).reshape(hq, nq, 128), want) <= TOL
+    graph.destroy()
+    streams, outs = [stream, sm100.Stream(0)], [U.guarded_output(sm100, stream, hq * nq * 128) for _ in range(2)]
+    stream.sync()
+    for _ in range(3):
+        for s, (_, p) in zip(streams, outs):
+            sm100.check(sm100.lib().sm100_attention(s.handle, qb.at(), kb.at(), vb.at(), None, 1, C.c_void_p(p), 128, 128, nq, nk, hq, hkv, int(causal), off, None, SCALE), "attention")
+    for s, (b, _) in zip(streams, outs):
+        s.sync()
+        assert sgref.nmse(U.read_guarded(sm100, s, b, hq * nq * 128).reshape(hq, nq, 128), want) <= TOL
+    streams[1].close()
