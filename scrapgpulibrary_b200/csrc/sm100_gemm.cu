@@ -1,4 +1,4 @@
-// Prefill MUL_MAT (M > 8 activation columns) on the fifth-generation tensor cores.
+// Prefill MUL_MAT (33 activation columns and more) on the fifth-generation tensor cores.
 //
 //   y[N, M] = W[K, N] . x[K, M]      W quantized (Q8_0, Q4_0, Q4_K) or F16, x and y f32
 //
@@ -63,16 +63,16 @@ constexpr int KC = 64;   // weights of a row per chunk
 
 // SUB chunks make a stage of either ring: the MMA warp's hand-over from stage to stage costs about 200 cycles, which four MMAs of 128
 // columns (256 cycles) do not hide.
-template <int TN, int STAGES, int RT, int SUB>
+template <int TN, int STAGES, int SUB>
 struct GemmSmem {
     static constexpr int CHUNK_BYTES = TN * KC * 2;
     static constexpr int B_BYTES = SUB * CHUNK_BYTES;
-    // Weight stages: as many as the tensor memory columns left by the accumulators hold, at most 8.  The two rings have
+    // Weight stages: as many as the tensor memory columns left by the accumulator hold, at most 8.  The two rings have
     // their own barriers: the activation copies are the long-latency side (~2 us under load) and want every byte of shared
     // memory in flight.
-    static constexpr int SA = (512 - RT * TN) / (RT * SUB * (KC / 2)) < 8 ? (512 - RT * TN) / (RT * SUB * (KC / 2)) : 8;
+    static constexpr int SA = (512 - TN) / (SUB * (KC / 2)) < 8 ? (512 - TN) / (SUB * (KC / 2)) : 8;
     uint8_t b[STAGES][B_BYTES];  // [k / 8][token][8 halves]
-    uint64_t full_a[SA];         // producers -> MMA: one arrival per producer warp and row tile
+    uint64_t full_a[SA];         // producers -> MMA: one arrival per producer warp of a group
     uint64_t empty_a[SA];        // MMA commit -> producers
     uint64_t full_b[STAGES];     // bulk copy -> MMA: the issuing lane's expect_tx arrival + the bytes
     uint64_t empty_b[STAGES];    // MMA commit -> bulk warp
@@ -94,35 +94,31 @@ struct GemmArgs {
     int m_tiles;
 };
 
-// RT row tiles of 128 weight rows per CTA (RT accumulators of TN columns in TMEM) share one activation stage: the
-// activation bytes a CTA pulls from L2 per multiply-add halve with RT = 2.
-//
 // The dequantized weights go to tensor memory (tcgen05.st by the producers, A operand of the MMA read from TMEM), so that
-// shared memory carries only the activation stages.  TMEM columns: RT accumulators of TN, then per stage and row tile
-// KC / 2 columns of A (two f16 per column).
-template <typename S, int TN, int STAGES, int RT, int SUB>
+// shared memory carries only the activation stages.  TMEM columns: the accumulator of TN, then per chunk of a stage KC / 2 columns of A
+// (two f16 per column).
+template <typename S, int TN, int STAGES, int SUB>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
     constexpr int GROUP_WARPS = 8;                          // a chunk of 128 rows: eight warps of 16 rows each
     constexpr int GROUPS = PRODUCER_WARPS / GROUP_WARPS;    // groups take the chunks in turn
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    using Smem = GemmSmem<TN, STAGES, RT, SUB>;
-    constexpr int ACC_COLS = RT * TN;
-    static_assert(RT == 1 || SUB == 1, "two row tiles per CTA: one chunk per stage");
-    constexpr int A_COLS = SUB * KC / 2;                             // per stage and row tile
+    using Smem = GemmSmem<TN, STAGES, SUB>;
+    constexpr int ACC_COLS = TN;
+    constexpr int A_COLS = SUB * KC / 2;                             // per stage
     constexpr int SA = Smem::SA;
     static_assert(SA >= 2, "at least two weight stages");
-    constexpr int USED_COLS = ACC_COLS + SA * RT * A_COLS;
+    constexpr int USED_COLS = ACC_COLS + SA * A_COLS;
     constexpr int TMEM_COLS = USED_COLS <= 32 ? 32 : USED_COLS <= 64 ? 64 : USED_COLS <= 128 ? 128 : USED_COLS <= 256 ? 256 : 512;
-    static_assert(USED_COLS <= 512, "accumulators and weight stages exceed the tensor memory");
+    static_assert(USED_COLS <= 512, "accumulator and weight stages exceed the tensor memory");
     Smem & sm = *reinterpret_cast<Smem *>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int mt = blockIdx.x % g.m_tiles, nt = blockIdx.x / g.m_tiles;
-    const int n0 = nt * (TM * RT), m0 = mt * TN;
+    const int n0 = nt * TM, m0 = mt * TN;
     volatile int * abort_flag = &sm.abort_flag;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < SA; ++s) {
-            mbar_init(smem_addr(&sm.full_a[s]), RT * GROUP_WARPS);
+            mbar_init(smem_addr(&sm.full_a[s]), GROUP_WARPS);
             mbar_init(smem_addr(&sm.empty_a[s]), 1);
         }
         for (int s = 0; s < STAGES; ++s) {
@@ -159,22 +155,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
         const int pw = warp - FIRST_PRODUCER;
         const int group = pw / GROUP_WARPS, gw = pw % GROUP_WARPS, t = lane & 3;
         const int row_in = 32 * (warp & 3) + 16 * (gw >> 2);
-        // The work unit is (chunk, row tile): unit u = chunk * RT + row tile, and group g takes the units g, g + GROUPS, ...
-        // Rows past the tensor are clamped to the last one: such rows are never stored.
-        // With two chunks a stage (RT = 1) the unit is the stage, and the two chunks are the ones in flight.
-        const int units = g.nchunks / SUB * RT;
-        typename S::Cursor cur[RT];
-#pragma unroll
-        for (int rt = 0; rt < RT; ++rt) {
-            const int64_t r0 = (int64_t) n0 + rt * TM + row_in + (lane >> 2), last = g.n - 1;
+        // Group g takes the stages g, g + GROUPS, ...  Rows past the tensor are clamped to the last one: such rows are never stored.
+        // With two chunks a stage these are the chunks in flight.
+        const int units = g.nchunks / SUB;
+        typename S::Cursor cur;
+        {
+            const int64_t r0 = (int64_t) n0 + row_in + (lane >> 2), last = g.n - 1;
             const int64_t row[2] = {r0 < last ? r0 : last, r0 + 8 < last ? r0 + 8 : last};
-            S::init(cur[rt], g.w, row, t);
+            S::init(cur, g.w, row, t);
         }
-        auto load = [&](typename S::Regs & r, int u, int sub) {   // past the end: a clamped, unused load
-            const int uu = u < units ? u : units - 1;
-            if (RT == 1) S::load(r, cur[0], uu * SUB + sub);
-            else if (uu % RT == 0) S::load(r, cur[0], uu / RT);
-            else S::load(r, cur[RT - 1], uu / RT);
+        auto load = [&](typename S::Regs & r, int st, int sub) {   // past the end: a clamped, unused load
+            S::load(r, cur, (st < units ? st : units - 1) * SUB + sub);
         };
         // one chunk of the warp's 16 rows to tensor memory
         auto put = [&](const typename S::Regs & r, int chunk, uint32_t dst) {
@@ -198,9 +189,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
         for (int u0 = group; u0 < units && alive; u0 += GROUPS * (SUB == 1 ? DEPTH : 1)) {
 #pragma unroll
             for (int d = 0; d < DEPTH; ++d) {
-                const int u = SUB == 1 ? u0 + GROUPS * d : u0;
-                if (u >= units) break;
-                const int st = u / RT, rt = u % RT;
+                const int st = SUB == 1 ? u0 + GROUPS * d : u0;
+                if (st >= units) break;
                 const int s = st % SA;
                 if (SUB == 1 || d == 0) {   // the stage is free once the MMAs that used it last have retired
                     const uint32_t phase = (uint32_t) (st / SA) & 1u;
@@ -209,8 +199,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
                     if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
                     tc_fence_after();   // those MMAs (observed through the barrier) precede these stores
                 }
-                put(ring[d], SUB == 1 ? st : st * SUB + d, dst0 + (uint32_t) ((s * RT + rt) * A_COLS + (SUB == 1 ? 0 : d * (KC / 2))));
-                load(ring[d], SUB == 1 ? u + GROUPS * DEPTH : u + GROUPS, SUB == 1 ? 0 : d);
+                put(ring[d], SUB == 1 ? st : st * SUB + d, dst0 + (uint32_t) (s * A_COLS + (SUB == 1 ? 0 : d * (KC / 2))));
+                load(ring[d], SUB == 1 ? st + GROUPS * DEPTH : st + GROUPS, SUB == 1 ? 0 : d);
                 if (SUB == 1 || d == DEPTH - 1) {
                     tmem_st_wait();
                     tc_fence_before();   // the stores are ordered before the MMAs that the arrival releases
@@ -235,24 +225,21 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
             tc_fence_after();
             const int lane_base = 32 * (warp & 3);
             const int col_base = (pw >> 2) * (TN / 4);
+            const int64_t n_out = (int64_t) n0 + lane_base + lane;
 #pragma unroll 1
-            for (int rt = 0; rt < RT; ++rt) {
-                const int64_t n_out = (int64_t) n0 + rt * TM + lane_base + lane;
-#pragma unroll 1
-                for (int cc = 0; cc < TN / 4; cc += 16) {
-                    uint32_t r[16];
-                    tmem_ld16(tmem + ((uint32_t) lane_base << 16) + (uint32_t) (rt * TN + col_base + cc), r);
-                    // the token factors are fetched before any store: a load after a store to memory that may alias
-                    // is not moved up by the compiler, and 16 dependent trips to L2 per pass cost ~5 us per CTA
-                    float f[16];
+            for (int cc = 0; cc < TN / 4; cc += 16) {
+                uint32_t r[16];
+                tmem_ld16(tmem + ((uint32_t) lane_base << 16) + (uint32_t) (col_base + cc), r);
+                // the token factors are fetched before any store: a load after a store to memory that may alias
+                // is not moved up by the compiler, and 16 dependent trips to L2 per pass cost ~5 us per CTA
+                float f[16];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) f[j] = __ldcg(g.tokscale + m0 + col_base + cc + j) * g.out_scale;   // allocated for whole tiles
-                    tmem_ld_wait();
+                for (int j = 0; j < 16; ++j) f[j] = __ldcg(g.tokscale + m0 + col_base + cc + j) * g.out_scale;   // allocated for whole tiles
+                tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int tok = m0 + col_base + cc + j;
-                        if (tok < g.m && n_out < g.n) g.y[(int64_t) tok * g.ldy + n_out] = __uint_as_float(r[j]) * f[j];
-                    }
+                for (int j = 0; j < 16; ++j) {
+                    const int tok = m0 + col_base + cc + j;
+                    if (tok < g.m && n_out < g.n) g.y[(int64_t) tok * g.ldy + n_out] = __uint_as_float(r[j]) * f[j];
                 }
             }
         }
@@ -320,9 +307,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
             const uint32_t ra = mbar_test_wait(full_a0 + 8 * sa_n, pa_n) ? 1u : 0u;
             const uint64_t b_desc = ((uint64_t) DESC_HI << 32) | (b_lo0 + sb * (Smem::B_BYTES >> 4));
 #pragma unroll
-            for (int i = 0; i < RT * SUB; ++i)   // row tiles, or chunks, of the stage
-                mma4_f16_ta(tmem + (RT > 1 ? i * TN : 0), tmem + ACC_COLS + sa * RT * A_COLS + i * (KC / 2), b_desc + (uint64_t) (RT > 1 ? 0 : i * (Smem::CHUNK_BYTES >> 4)),
-                            (uint64_t) (2 * TN * 16 >> 4), IDESC, i == 0 || RT > 1 ? accumulate : 1u, issuer);
+            for (int i = 0; i < SUB; ++i)   // chunks of the stage
+                mma4_f16_ta(tmem, tmem + ACC_COLS + sa * A_COLS + i * (KC / 2), b_desc + (uint64_t) (i * (Smem::CHUNK_BYTES >> 4)), (uint64_t) (2 * TN * 16 >> 4), IDESC,
+                            i == 0 ? accumulate : 1u, issuer);
             accumulate = 1u;
             mma_commit2(empty_a0 + 8 * sa, empty_b0 + 8 * sb, issuer);   // each commit covers every MMA issued so far
             ready = c + 1 < stages ? (ra & rb) : 1u;
@@ -424,10 +411,10 @@ __global__ void __launch_bounds__(256) gemm_prep_x(const float * x, int64_t ldx,
     }
 }
 
-template <typename S, int TN, int STAGES, int RT, int SUB>
+template <typename S, int TN, int STAGES, int SUB>
 int launch_gemm(cudaStream_t s, GemmArgs g, int n_tiles) {
     g.out_scale = 1.0f / S::PRESCALE;
-    using Smem = GemmSmem<TN, STAGES, RT, SUB>;
+    using Smem = GemmSmem<TN, STAGES, SUB>;
     static std::mutex mu;
     static std::vector<char> configured;
     int dev = 0;
@@ -436,30 +423,30 @@ int launch_gemm(cudaStream_t s, GemmArgs g, int n_tiles) {
         std::lock_guard<std::mutex> lock(mu);
         if ((int) configured.size() <= dev) configured.resize(dev + 1, 0);
         if (!configured[dev]) {
-            SM100_CUDA(cudaFuncSetAttribute(gemm_tc<S, TN, STAGES, RT, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(Smem)));
+            SM100_CUDA(cudaFuncSetAttribute(gemm_tc<S, TN, STAGES, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(Smem)));
             configured[dev] = 1;
         }
     }
-    return launch(gemm_tc<S, TN, STAGES, RT, SUB>, dim3((unsigned) (n_tiles * g.m_tiles)), dim3(GEMM_THREADS), sizeof(Smem), s, g);
+    return launch(gemm_tc<S, TN, STAGES, SUB>, dim3((unsigned) (n_tiles * g.m_tiles)), dim3(GEMM_THREADS), sizeof(Smem), s, g);
 }
 
-template <int TN, int STAGES, int RT, int SUB>
+template <int TN, int STAGES, int SUB>
 int launch_gemm_dtype(cudaStream_t s, int dtype, int layout, const GemmArgs & g, int n_tiles) {
     const bool packed = layout == LAYOUT_PACKED;
     switch (dtype) {
         case DT_Q8_0:
-            return packed ? launch_gemm<SrcB32<true, true>, TN, STAGES, RT, SUB>(s, g, n_tiles) : launch_gemm<SrcB32<true, false>, TN, STAGES, RT, SUB>(s, g, n_tiles);
+            return packed ? launch_gemm<SrcB32<true, true>, TN, STAGES, SUB>(s, g, n_tiles) : launch_gemm<SrcB32<true, false>, TN, STAGES, SUB>(s, g, n_tiles);
         case DT_Q4_0:
-            return packed ? launch_gemm<SrcB32<false, true>, TN, STAGES, RT, SUB>(s, g, n_tiles) : launch_gemm<SrcB32<false, false>, TN, STAGES, RT, SUB>(s, g, n_tiles);
-        case DT_Q4_K: return launch_gemm<SrcQ4K, TN, STAGES, RT, SUB>(s, g, n_tiles);
-        case DT_F16: return launch_gemm<SrcF16, TN, STAGES, RT, SUB>(s, g, n_tiles);
+            return packed ? launch_gemm<SrcB32<false, true>, TN, STAGES, SUB>(s, g, n_tiles) : launch_gemm<SrcB32<false, false>, TN, STAGES, SUB>(s, g, n_tiles);
+        case DT_Q4_K: return launch_gemm<SrcQ4K, TN, STAGES, SUB>(s, g, n_tiles);
+        case DT_F16: return launch_gemm<SrcF16, TN, STAGES, SUB>(s, g, n_tiles);
     }
     return fail(ST_UNSUPPORTED, "gemm: no tensor-core source for dtype %d", dtype);
 }
 
-template <int TN, int STAGES, int RT, int SUB>
+template <int TN, int STAGES, int SUB>
 int gemm_passes(cudaStream_t s, int dtype, int layout, GemmArgs g, const float * x, int64_t ldx, int64_t m, int64_t k, float * y) {
-    const int n_tiles = (g.n + TM * RT - 1) / (TM * RT);
+    const int n_tiles = (g.n + TM - 1) / TM;
     g.nchunks = (int) ((k + SUB * KC - 1) / (SUB * KC)) * SUB;
     // tokens per pass: the prepared activations of one pass stay below 64 MiB
     int64_t pass = ((int64_t) 64 << 20) / ((int64_t) g.nchunks * KC * 2) / TN * TN;
@@ -486,7 +473,7 @@ int gemm_passes(cudaStream_t s, int dtype, int layout, GemmArgs g, const float *
         g.y = y + c0 * g.ldy;
         g.m = (int) mm;
         g.m_tiles = m_tiles;
-        st = launch_gemm_dtype<TN, STAGES, RT, SUB>(s, dtype, layout, g, n_tiles);
+        st = launch_gemm_dtype<TN, STAGES, SUB>(s, dtype, layout, g, n_tiles);
         if (st != ST_OK) return st;
     }
     return ST_OK;
@@ -519,19 +506,14 @@ int gemm_tc_mul_mat(cudaStream_t s, int dtype, int layout, const void * w, int64
     g.w.last_block = (int) (k / 32) - 1;
     g.n = (int) n;
     g.ldy = ldy;
-    // Tile choice.  128 weight rows x 256 tokens per CTA once such tiles fill the SMs: a chunk of 64 weights takes 517 cycles (its
-    // MMAs: 512), 128 x 128 takes more than half of that, because the MMA warp's hand-over from stage to stage shows (446 cycles
-    // with one chunk a stage, MMAs 256; two chunks a stage: Q4_0 5003 x 77 tokens 26.2 -> 23.3 us, 4096 x 512 30.8 -> 27.7 us).  Two
-    // row tiles per CTA (256 x 128) are bound by the dequantizing warps instead; they stay selectable for experiments.
+    // Tile choice.  128 weight rows x 256 tokens per CTA once such tiles fill the SMs: a 128 x 128 tile takes more than half the time, because
+    // the MMA warp's hand-over from stage to stage shows (446 cycles a chunk with one chunk a stage, MMAs 256; two chunks a stage:
+    // Q4_0 5003 x 77 tokens 26.2 -> 23.3 us, 4096 x 512 30.8 -> 27.7 us).
     static const int forced_tn = [] { const char * e = getenv("SM100_GEMM_TN"); return e != nullptr ? atoi(e) : 0; }();
-    static const int forced_rt = [] { const char * e = getenv("SM100_GEMM_RT"); return e != nullptr ? atoi(e) : 0; }();
     int tn = (int64_t) n_tiles * ((m + 255) / 256) >= (int64_t) sm_count() ? 256 : 128;
     if (forced_tn == 128 || forced_tn == 256) tn = forced_tn;
-    const int rt = forced_rt == 2 ? 2 : 1;
-    int st;
     // more activation stages than these in flight slow the weight loads down by more than they hide
-    if (rt == 2) st = gemm_passes<128, 8, 2, 1>(s, dtype, layout, g, x, ldx, m, k, y);   // 2 x 128 accumulator columns + 4 weight stages
-    else st = tn == 256 ? gemm_passes<256, 6, 1, 1>(s, dtype, layout, g, x, ldx, m, k, y) : gemm_passes<128, 6, 1, 2>(s, dtype, layout, g, x, ldx, m, k, y);
+    const int st = tn == 256 ? gemm_passes<256, 6, 1>(s, dtype, layout, g, x, ldx, m, k, y) : gemm_passes<128, 6, 2>(s, dtype, layout, g, x, ldx, m, k, y);
     if (st != ST_OK) return st;
     *handled = true;
     return ST_OK;
