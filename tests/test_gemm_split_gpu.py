@@ -1,7 +1,7 @@
 """GPU parity of the split-operand tensor-core MUL_MAT (batches of packed weights, Q6_K at any width) against the CPU oracle.
 
-Tolerance: both operands are two bf16 numbers (16 bits: relative rounding at most 2^-17, about 2^-18.5 rms) and the product of
-the two small parts is dropped (below 2^-17), so a product is off by 1e-5; the f32
+Tolerance: both operands are two bf16 numbers (16 bits: relative rounding at most 2^-17, about 2^-18.5 rms) and with more than 64 columns
+the product of the two small parts is dropped (below 2^-17), so a product is off by 1e-5; the f32
 accumulation in the tensor core truncates (up to 2e-5 over 768 steps, K = 12288).  NMSE bound: (3e-5)^2.
 """
 import ctypes as C
@@ -22,6 +22,7 @@ def _check(sm100, stream, dtype, k, n, m):
     x = U.seeded_acts(3 * m + k, m, k)
     want = sgref.mul_mat(dtype, wq, k, x)
     got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x)
+    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == ("gemm_split" if n % 16 == 0 else "gemm_split+rows")
     assert np.isfinite(got).all()
     for t in range(m):   # per token, so that one wrong column cannot hide in the average
         assert sgref.nmse(got[t], want[t]) <= TOL, (t, sgref.nmse(got[t], want[t]))
@@ -29,17 +30,53 @@ def _check(sm100, stream, dtype, k, n, m):
         assert sgref.nmse(got[:, r], want[:, r]) <= 4 * TOL, r
 
 
-# rows below, at and past a tile; one block of K, a K range of one chunk per CTA of a cluster, long K; edges of the 16 / 32 column tiles
+# rows below, at and past a tile; one block of K, a K range of one stage per CTA, long K; edges of the 16 / 32 column tiles
 @pytest.mark.parametrize("dtype", U.QUANT, ids=lambda d: U.NAMES[d])
 @pytest.mark.parametrize("shape", [(256, 24, 9), (512, 128, 16), (512, 257, 17), (4096, 130, 32), (12288, 48, 24)], ids=lambda s: f"k{s[0]}n{s[1]}m{s[2]}")
 def test_batches(sm100, stream, dtype, shape):
     _check(sm100, stream, dtype, *shape)
 
 
+# three to eight columns, from 1024 rows on: the matvec's own way here; rows at and past a tile of 128, a tail, K of one stage and more
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 1024, 1030, 4), (U.Q4_0, 128, 1024, 7), (U.Q8_0, 1024, 1030, 7), (U.Q8_0, 2176, 1152, 4),
+                                         (U.Q6_K, 1024, 1030, 3), (U.Q6_K, 256, 1040, 5), (U.Q6_K, 4096, 1030, 8)], ids=lambda v: str(v))
+def test_few_columns(sm100, stream, dtype, k, n, m):
+    _check(sm100, stream, dtype, k, n, m)
+
+
+# more tiles than SMs: whole waves of one CTA per tile, and the rest with K cut; row and token tiles ragged
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 512, 128 * 160 + 16, 24), (U.Q4_K, 1024, 128 * 150 + 5, 32), (U.Q8_0, 512, 128 * 297, 5), (U.Q6_K, 512, 4100, 700), (U.Q6_K, 1024, 6400, 200)],
+                         ids=lambda v: str(v))
+def test_whole_waves_and_cut_tiles(sm100, stream, dtype, k, n, m):
+    """Rows repeat every 360 (no multiple of a tile), so that the oracle has few to multiply while every tile differs from its neighbours."""
+    few = 360
+    wq = U.quantize(dtype, U.seeded_weights(dtype + k, few, k))
+    x = U.seeded_acts(k + m, m, k)
+    want = sgref.mul_mat(dtype, wq, k, x)[:, np.arange(n) % few]
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, np.ascontiguousarray(np.resize(wq, (n, wq.shape[1]))), k, x)
+    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == ("gemm_split" if n % 16 == 0 else "gemm_split+rows")
+    for r0 in range(0, n, 128):
+        for t0 in range(0, m, 64):
+            part = np.s_[t0:t0 + 64, r0:r0 + 128]
+            assert sgref.nmse(got[part], want[part]) <= TOL, (r0, t0)
+
+
+@pytest.mark.parametrize("dtype", [U.Q4_0, U.Q8_0], ids=lambda d: U.NAMES[d])
+@pytest.mark.parametrize("shape", [(128, 16, 9), (384, 144, 31)], ids=lambda s: f"k{s[0]}n{s[1]}m{s[2]}")
+def test_an_odd_number_of_chunk_pairs(sm100, stream, dtype, shape):
+    """One stage of two chunks, and three."""
+    _check(sm100, stream, dtype, *shape)
+
+
+# rows that are not whole stages stay with the other kernels
 @pytest.mark.parametrize("dtype", [U.Q4_0, U.Q8_0], ids=lambda d: U.NAMES[d])
 @pytest.mark.parametrize("shape", [(32, 16, 9), (96, 130, 31)], ids=lambda s: f"k{s[0]}n{s[1]}m{s[2]}")
-def test_half_chunk_at_the_end_of_k(sm100, stream, dtype, shape):
-    _check(sm100, stream, dtype, *shape)
+def test_short_rows(sm100, stream, dtype, shape):
+    k, n, m = shape
+    wq = U.quantize(dtype, U.seeded_weights(7000 + dtype + k, n, k))
+    x = U.seeded_acts(3 * m + k, m, k)
+    assert sgref.nmse(U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x), sgref.mul_mat(dtype, wq, k, x)) <= TOL
+    assert "gemm_split" not in (sm100.lib().sm100_matvec_last_kernel() or b"").decode()
 
 
 @pytest.mark.parametrize("shape", [(256, 24, 33), (512, 130, 64), (512, 257, 65), (4096, 128, 129), (12288, 40, 48)], ids=lambda s: f"k{s[0]}n{s[1]}m{s[2]}")
