@@ -684,8 +684,8 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_fast_kernel(AttnArgs a) {
 // compensated.  Relative error against float64 behind 512 / 4096 / 32768 keys: 1.9e-7 / 2.1e-7 / 2.6e-7, the decode kernel
 // 2.0e-7 / 2.2e-7 / 2.5e-7 (with one chain over all tiles 2.3e-7 / 3.0e-7 / 6.5e-7); without a prefix, 128 / 512 / 2048
 // queries, 1.2e-7 / 1.4e-7 / 1.6e-7, the decode kernel 1.2e-7 / 1.3e-7 / 1.5e-7.
-// Bound by the f32 FMA units and the instruction issue in front of them (4 D flops per (row, key)); with one CTA per SM by
-// latency, where the size of the unrolled loops counts (128 queries behind 512 keys: 130 us, 155 with the loops over parts and halves unrolled).
+// Bound by the instruction stream of two warps per scheduler (512 queries behind 512 keys: issue slots 53 % busy, the heavy FMA pipe 49 %); with
+// one CTA per SM by latency, where the size of the unrolled loops counts (128 queries behind 512 keys: 130 us, 155 with the loops over parts and halves unrolled).
 // Measured, 32 / 8 heads: 512 queries behind 512 keys 290 us (decode kernel 716), 2048 queries 1270 us (3930).  Tried: the second
 // product as packed FMAs over (even, odd) keys, 397 us; compensated sums of the outputs in registers, 303 us and 158 behind 512 for 128 queries.
 // ---------------------------------------------------------------------------------------------------------

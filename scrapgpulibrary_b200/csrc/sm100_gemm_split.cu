@@ -1,5 +1,6 @@
 // MUL_MAT of packed quantized weights on the fifth-generation tensor cores at the precision of the integer matvecs:
-// batches of up to 32 activation columns, and prompts of any length over Q6_K weights.
+// batches of up to 32 activation columns (those that the integer column kernels serve faster stay there: columns_faster), and prompts
+// of any length over Q6_K weights.
 //
 //   y[N, M] = W[K, N] . x[K, M]      values of src/core/ref/quant.cpp:30-108 and src/core/ref/ops.cpp:891-984
 //
@@ -19,7 +20,8 @@
 // tiles go to scratch memory of the call; split_reduce adds them in a fixed order.
 //
 // What bounds it: up to 32 tokens the hand-over from chunk to chunk and the dequantizing warps (about 900 cycles a chunk of 64
-// weights x 128 rows), with prompts the tensor core (12 MMAs of 64 cycles in a chunk's 1090).  Measured, us, before / now: Q4_0
+// weights x 128 rows; tensor pipe 12 to 21 % busy, issue slots 53 to 66 %), with prompts the tensor core (71 % busy while a CTA is
+// resident: 12 MMAs of 64 cycles in a chunk's 1090).  Measured, us, before / now: Q4_0
 // 4096 x 12288, 8 columns 64 / 28; Q4_K 12288 x 4096, 24 columns 63 / 34; Q6_K 12288 x 4096, 512 columns 3740 / 168 (before: one
 // launch per 8 or 4 columns).  Tried: K over a cluster with the exchange in distributed shared memory (wrong sums; taken out),
 // three converting warps with their loads in registers (Q4_K, 24 columns: 41).

@@ -267,7 +267,7 @@ __device__ __forceinline__ float transpose_reduce<4>(const float (&v)[4], int la
 
 // The warps of a CTA meet once per WIDE_SPAN batches, not once per batch: a warp leaves its partial sums in shared memory
 // ([row][warp of the row]) and goes on, and a row's slot is reloaded as soon as the row has been multiplied, so that the
-// weight stream has fewer bubbles (vocabulary head, Q6_K 4096 x 151936: 122.5 us, 124.0 with two barriers per batch of 4 rows; what
+// weight stream has fewer bubbles (vocabulary head, Q6_K 4096 x 151936: 123.5 us, 124.9 with two barriers per batch of 4 rows and the reload after all four; what
 // is left is the instructions of the unpacking, about 3 per weight).
 constexpr int WIDE_SPAN = 32;
 

@@ -142,8 +142,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // How the tiles of a launch are dealt: as many as fill whole waves go to one CTA each, the rest - the last wave, or all when there
-// are fewer than SMs - have their K range cut over `splits` CTAs, whose partial tiles a second launch adds in order.  (192 tiles of 64
-// chunks on 148 SMs: 64 + 22 chunks' time with the last 44 cut in three, 128 without.)
+// are fewer than SMs - have their K range cut over `splits` CTAs, whose partial tiles a second launch adds in order.  (160 tiles of 96
+// chunks on 148 SMs: 96 + 12 chunks' time with the last 12 cut in eight, 192 without.)
 struct TilePlan {
     int64_t whole;   // tiles [0, whole): one CTA each
     int64_t cut;     // tiles [whole, whole + cut): `splits` CTAs each
