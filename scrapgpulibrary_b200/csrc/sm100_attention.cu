@@ -684,9 +684,9 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_fast_kernel(AttnArgs a) {
 // compensated.  Relative error against float64 behind 512 / 4096 / 32768 keys: 1.9e-7 / 2.1e-7 / 2.6e-7, the decode kernel
 // 2.0e-7 / 2.2e-7 / 2.5e-7 (with one chain over all tiles 2.3e-7 / 3.0e-7 / 6.5e-7); without a prefix, 128 / 512 / 2048
 // queries, 1.2e-7 / 1.4e-7 / 1.6e-7, the decode kernel 1.2e-7 / 1.3e-7 / 1.5e-7.
-// Bound by the instruction stream of two warps per scheduler (512 queries behind 512 keys: issue slots 53 % busy, the heavy FMA pipe 49 %); with
-// one CTA per SM by latency, where the size of the unrolled loops counts (128 queries behind 512 keys: 130 us, 155 with the loops over parts and halves unrolled).
-// Measured, 32 / 8 heads: 512 queries behind 512 keys 290 us (decode kernel 716), 2048 queries 1270 us (3930).  Tried: the second
+// Bound by the instruction stream of two warps per scheduler (512 queries behind 512 keys: issue slots 55 % busy, the heavy FMA pipe 51 %); with
+// one CTA per SM by latency, where the size of the unrolled loops counts (128 queries behind 512 keys: 119 us, 134 with the loop over parts unrolled).
+// Measured, 32 / 8 heads: 512 queries behind 512 keys 268 us (decode kernel 716), 2048 queries 1172 us (3930).  Tried: the second
 // product as packed FMAs over (even, odd) keys, 397 us; compensated sums of the outputs in registers, 303 us and 158 behind 512 for 128 queries.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int AP_ROWS = 64, AP_KEYS = 32, AP_WARPS = 4, AP_D = 128;
@@ -699,6 +699,7 @@ struct ApSmem {
     float4 v[2][AP_KEYS][AP_D / 4];
     float p[AP_WARPS][16][AP_PSTRIDE];
     int64_t mask_row[AP_ROWS];   // offset of the row's mask values
+    int64_t out_at[AP_ROWS];     // offset of the row's output, in float4; negative past the last row
     int vis[AP_ROWS];   // visible keys per row
 };
 
@@ -774,6 +775,7 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
     for (int i = tid; i < AP_ROWS; i += AP_WARPS * 32) {
         const int r = r_base + i < rows ? r_base + i : rows - 1, qi = r / group;
         sm.vis[i] = (int) visible_keys(a, qi);
+        sm.out_at[i] = r_base + i < rows ? ((hk * group + r % group) * a.nq + qi) * (AP_D / 4) : -1;
         sm.mask_row[i] = ((a.mask_heads == 1 ? 0 : hk * group + r % group) * a.nq + qi) * a.nk;
     }
     __syncthreads();
@@ -799,26 +801,32 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
     // additions is longer than about the square root of the tiles.
     int span = AP_SPAN;
     while (span * span < tiles) ++span;
-    auto out_row = [&](int r) {
-        const int row = r_base + 16 * warp + r;
-        return row < rows ? reinterpret_cast<float4 *>(a.out + ((hk * group + row % group) * a.nq + row / group) * AP_D) + lane : nullptr;
-    };
+    const int64_t * out_at = sm.out_at + 16 * warp;
+    float4 * out_lane = reinterpret_cast<float4 *>(a.out) + lane;
     bool in_out = false;
     auto add_up = [&]() {   // o += what a.out holds, and back into it
         float f[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) f[i] = m_out[i] == -INFINITY ? 0.f : expf(m_out[i] - m[i]);
+        // two rows at a time, their loads before the stores: with one row after the other, each a trip to L2, 512 queries behind 512 keys took 292 us,
+        // now 268; with 4, 8 or 16 rows the code of the loop grows and it is 274, 279, 294
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const float c = __shfl_sync(0xffffffffu, f[r >> 2], (r & 3) * 8);
-            float4 * p = out_row(r);
-            if (p == nullptr) continue;
+        for (int r0 = 0; r0 < 16; r0 += 2) {
+            float4 v[2];
             if (in_out) {
-                const float4 v = *p;
-                o[r][0] = fmaf(v.x, c, o[r][0]); o[r][1] = fmaf(v.y, c, o[r][1]);
-                o[r][2] = fmaf(v.z, c, o[r][2]); o[r][3] = fmaf(v.w, c, o[r][3]);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) v[r] = out_at[r0 + r] >= 0 ? __ldcg(out_lane + out_at[r0 + r]) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            *p = make_float4(o[r][0], o[r][1], o[r][2], o[r][3]);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int rr = r0 + r;
+                const float c = __shfl_sync(0xffffffffu, f[rr >> 2], (rr & 3) * 8);
+                if (in_out) {
+                    o[rr][0] = fmaf(v[r].x, c, o[rr][0]); o[rr][1] = fmaf(v[r].y, c, o[rr][1]);
+                    o[rr][2] = fmaf(v[r].z, c, o[rr][2]); o[rr][3] = fmaf(v[r].w, c, o[rr][3]);
+                }
+                if (out_at[rr] >= 0) out_lane[out_at[rr]] = make_float4(o[rr][0], o[rr][1], o[rr][2], o[rr][3]);
+            }
         }
         in_out = true;
     };
@@ -980,14 +988,13 @@ __global__ void __launch_bounds__(AP_WARPS * 32, 2) attn_prompt_kernel(AttnArgs 
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
         const float lr = __shfl_sync(0xffffffffu, l[r >> 2], (r & 3) * 8), mr = __shfl_sync(0xffffffffu, m[r >> 2], (r & 3) * 8);
-        float4 * p = out_row(r);
-        if (p != nullptr) *p = mr == -INFINITY ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(o[r][0] / lr, o[r][1] / lr, o[r][2] / lr, o[r][3] / lr);
+        if (out_at[r] >= 0) out_lane[out_at[r]] = mr == -INFINITY ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(o[r][0] / lr, o[r][1] / lr, o[r][2] / lr, o[r][3] / lr);
     }
 }
 
 // Which calls take it: head dimension 128 and at least 64 row tiles over the KV heads.  With 32 of them (64 queries, 32 / 8 heads,
-// 576 keys) a CTA's serial walk over the keys takes 100 us or more where the splits of the decode kernel take 77; with 64 (128 queries)
-// 130 against 148 behind 512 keys, 756 against 916 behind 4096, 2830 against 4030 behind 16384, and without a prefix 34 against 35.
+// 576 keys) a CTA's serial walk over the keys takes about 100 us where the splits of the decode kernel take 77; with 64 (128 queries)
+// 120 against 148 behind 512 keys, 697 against 916 behind 4096, 2638 against 4030 behind 16384, and without a prefix 34 against 35.
 static bool attention_is_prompt(const AttnArgs & a) {
     if (a.d != AP_D || a.dv != AP_D || a.k_new != nullptr || a.nk > INT32_MAX / 2) return false;
     if ((((uintptr_t) a.q | (uintptr_t) a.k | (uintptr_t) a.v | (uintptr_t) a.out) & 15) != 0) return false;
@@ -996,17 +1003,17 @@ static bool attention_is_prompt(const AttnArgs & a) {
 }
 
 // Causal prompts whose last tiles see many more keys than the first leave most SMs idle when there is one round of few tiles; with heads in
-// groups of 2 or 4 the decode kernel, whose work follows the visible keys, is the faster one then.  Measured, decode (with the zeroing of its
-// counters) / prompt kernel, us, at `tiles` times mean over most visible keys: group 4 (8 / 2 heads) 512 queries, no prefix (32) 91 / 106, behind 256
-// keys (43) 147 / 152, 576 queries behind 128 (43) 141 / 143, 704 queries (44) 151 / 143, (4 / 1 heads) 1024 queries (32) 151 / 198, behind 512 (43) 259 / 291, (16 / 4 heads)
-// 320 queries behind 64 (47) 99 / 86, (32 / 8 heads) 128 queries behind 64 keys (43) 58 / 49; group 2 (4 / 2 heads) 1024 queries (32) 185 / 199; group 8,
-// 512 queries (32) 118 / 106; 288 queries, no prefix (16 / 4 heads, 36) 71 / 70.
+// groups of 4 the decode kernel, whose work follows the visible keys, is the faster one then, the more the longer the rows.  Measured, decode
+// (with the zeroing of its counters) / prompt kernel, us, at `tiles` times mean over most visible keys: 4 / 1 heads, 1024 queries, no prefix (32)
+// 149 / 179, behind 256 keys (38) 207 / 221, behind 384 (41) 233 / 242, behind 512 (43) 259 / 262, 1280 queries (40) 221 / 222; 8 / 2 heads, 512
+// queries (32) 90 / 96, behind 64 (36) 107 / 109, behind 128 (38) 120 / 119; 12 / 3 heads, 342 queries (33) 71 / 71; groups of 2 (4 / 2 heads), 1024
+// queries (32) 186 / 181; of 8 (8 / 1 heads), 512 queries (32) 118 / 100.
 static bool attention_prompt_uneven(const AttnArgs & a) {
     const int64_t group = a.hq / a.hkv;
-    if (!a.causal || a.positions != nullptr || (group != 2 && group != 4)) return false;
+    if (!a.causal || a.positions != nullptr || group != 4) return false;
     const int64_t tiles = (a.nq * group + AP_ROWS - 1) / AP_ROWS * a.hkv;
     const int64_t first = a.offset + 1 < 0 ? 0 : a.offset + 1 < a.nk ? a.offset + 1 : a.nk, last = a.offset + a.nq < 0 ? 0 : a.offset + a.nq < a.nk ? a.offset + a.nq : a.nk;
-    return last > 320 && tiles * (first + last) < 2 * (group == 2 ? 35 : last < 768 ? 42 : 46) * last;
+    return last >= 512 && tiles * (first + last) < 2 * (last < 1024 ? 36 : 41) * last;
 }
 
 static int attention_prompt_launch(cudaStream_t s, const AttnArgs & a) {

@@ -135,9 +135,9 @@ def test_rounding_does_not_grow_with_the_context(sm100, stream, nk, bound):
     assert err <= bound, err
 
 
-# few tiles whose rows see very different numbers of keys; more tiles, a long prefix, heads in groups of 8 and 1, no causal mask, few keys
-@pytest.mark.parametrize("hq,hkv,nq,nk,causal,name", [(8, 2, 512, 512, True, "attn_splits"), (4, 1, 1024, 1300, True, "attn_splits"), (12, 3, 345, 400, True, "attn_splits"),
-                                                      (4, 2, 1024, 1024, True, "attn_splits"), (8, 2, 768, 768, True, "attn_prompt"), (8, 2, 512, 1536, True, "attn_prompt"),
+# few tiles whose rows see very different numbers of keys; short rows, more tiles, a long prefix, heads in groups of 2, 8 and 1, no causal mask
+@pytest.mark.parametrize("hq,hkv,nq,nk,causal,name", [(8, 2, 512, 512, True, "attn_splits"), (4, 1, 1024, 1300, True, "attn_splits"), (8, 2, 520, 560, True, "attn_splits"),
+                                                      (12, 3, 345, 400, True, "attn_prompt"), (4, 2, 1024, 1024, True, "attn_prompt"), (8, 2, 768, 768, True, "attn_prompt"), (8, 2, 512, 1536, True, "attn_prompt"),
                                                       (8, 1, 512, 512, True, "attn_prompt"), (8, 8, 512, 512, True, "attn_prompt"), (8, 2, 512, 512, False, "attn_prompt"),
                                                       (32, 8, 128, 128, True, "attn_prompt")], ids=lambda v: str(v))
 def test_uneven_prompts_take_the_faster_kernel(sm100, stream, hq, hkv, nq, nk, causal, name):
