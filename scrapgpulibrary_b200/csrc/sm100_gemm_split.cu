@@ -1,5 +1,5 @@
 // MUL_MAT of packed quantized weights on the fifth-generation tensor cores at the precision of the integer matvecs:
-// batches of up to 32 activation columns (those that the integer column kernels serve faster stay there: columns_faster), and prompts
+// batches of up to 32 activation columns (those that the integer column kernels serve faster stay there: q4k_columns_faster), and prompts
 // of any length over Q6_K weights.
 //
 //   y[N, M] = W[K, N] . x[K, M]      values of src/core/ref/quant.cpp:30-108 and src/core/ref/ops.cpp:891-984
@@ -543,24 +543,20 @@ int prompt_split(cudaStream_t s, SplitArgs g, const float * x, int64_t ldx, int6
 
 }  // namespace
 
-// Is a batch faster in the integer column kernels, `width` columns a launch, than in one pass of the split GEMM?  Both times as measured
-// (us, within 8 % or so over K 1024 .. 12288, N 64 .. 151936; what the rule picks was at most 5 % slower than the other way):
-//   columns    a launch of 8 columns: 3.05 and, for every round of 16-row tiles (two per SM), 0.385 + 0.695 K / 1024 with Q4_K; 2.8 + K / 1024
-//              and 0.9 + 2.35 K / 1024 with Q6_K; of a round of a narrower Q4_K launch 0.58 + 0.056 per column; where rows are so long that
-//              only four columns fit, 8 % more
-//   split GEMM the cost of its plan times 0.031 + 0.0004 per column (Q4_K), 0.041 (Q6_K)
-// Measured, columns / split: Q4_K 4096 x 12288, 9 columns 21.6 / 32.9, 16 columns 26.9 / 35.6, 20 columns 37.6 / 37.2; 4096 x 4096, 16 columns
-// 13.0 / 15.3; 4096 x 1024, 16 columns 11.7 / 9.4; 12288 x 4096, 12 columns 31.4 / 30.9; Q6_K 5120 x 13824, 8 columns 47.0 / 53.0,
-// 4096 x 4096 17.2 / 16.1.
-bool columns_faster(int dtype, int64_t k, int64_t n, int64_t m, int width) {
-    if (m > 32) return false;
-    SplitArgs g = {};
-    g.n = (int) (n / 16 * 16);
-    g.m_tiles = 1;
-    g.nchunks = (int) ((k + 2 * SP_KC - 1) / (2 * SP_KC)) * 2;
-    const double cost = (double) split_plan<16, false>(g).cost, kk = (double) k / 1024;
+// Are 9..16 columns of Q4_K faster in the integer column kernel, `width` columns a launch, than in one pass of the split GEMM?  Both times as
+// measured (us, within 8 % or so over K 1024 .. 12288, N 64 .. 151936; what the rule picks was at most 5 % slower than the other way):
+//   columns    a launch of 8 columns: 3.05 and, for every round of 16-row tiles (two per SM), 0.385 + 0.695 K / 1024; of a round of a narrower
+//              launch 0.58 + 0.056 per column; where rows are so long that only four columns fit, 8 % more
+//   split GEMM the cost of its plan times 0.031 + 0.0004 per column
+// Measured, columns / split: 4096 x 12288, 9 columns 21.6 / 32.9, 16 columns 26.9 / 35.6; 4096 x 4096, 16 columns 13.0 / 15.3; 4096 x 1024,
+// 16 columns 11.7 / 9.4; 12288 x 4096, 12 columns 31.4 / 30.9.  The line is drawn at 16 columns because the split GEMM is the more accurate way (error
+// 7e-6; 4e-5 to 1e-4 with the column kernel): beyond, and for 8 columns of Q6_K, the column kernels win little and seldom (Q4_K 5120 x 13824,
+// 17 columns 43.4 / 49.7, 24 columns 49.4 / 51.4, 4096 x 4096, 17 columns 16.9 / 15.7; Q6_K 5120 x 13824, 8 columns 47.0 / 53.0, 4096 x 4096 17.2 / 16.1).
+bool q4k_columns_faster(int64_t k, int64_t n, int64_t m, int width) {
+    if (m > 16) return false;
+    const int chunks = (int) ((k + 2 * SP_KC - 1) / (2 * SP_KC)) * 2;
+    const double cost = (double) plan_tiles((n / 16 * 16 + SP_TM - 1) / SP_TM, chunks / 2, 30, SP_TM * 32, (chunks + SP_CHAIN - 1) / SP_CHAIN).cost, kk = (double) k / 1024;
     const int64_t at_once = 2 * (int64_t) sm_count(), rounds = (n / 16 + at_once - 1) / at_once;
-    if (dtype == DT_Q6_K) return 2.8 + kk + (double) rounds * (0.9 + 2.35 * kk) < 0.041 * cost;
     double columns = 0;
     for (int64_t c = 0; c < m; c += width) {
         const int64_t mm = m - c < width ? m - c : width;

@@ -27,8 +27,7 @@ int matvec_q4k_imma_cols_tiles(cudaStream_t s, const void * w, int64_t k, int64_
                                bool * handled, void * img = nullptr);
 int q4k_cols_width(int64_t k);
 size_t q4k_cols_image_bytes(int64_t k, int64_t cols);
-bool q6k_cols8_serves(int64_t k);
-bool columns_faster(int dtype, int64_t k, int64_t n, int64_t m, int width);
+bool q4k_columns_faster(int64_t k, int64_t n, int64_t m, int width);
 int matvec_q4k_imma_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
                           bool * handled);
 int matvec_q4k_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
@@ -691,11 +690,9 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
     //   Q4_0  4096 x 1024: m = 2  8.6 / 7.5, m = 4  8.8 / 12.6    4096 x 12288: m = 2  29 / 16, m = 4  29.5 / 31.7, m = 8  28 / 62
     //   Q6_K  4096 x 1024: m = 2 10.8 / 7.9, m = 3 10.7 / 14.3, m = 4 10.7 / 10.5, m = 8 10.7 / 15.9
     //         12288 x 4096: m = 2  34 / 26, m = 4  35 / 30, m = 8  35 / 59
-    // Below 1024 rows its few tiles cannot fill the GPU, and launches of small products overlap.  Eight columns of Q6_K are one launch of the
-    // column kernel where they fit, and that is the faster one for some shapes (columns_faster).
+    // Below 1024 rows its few tiles cannot fill the GPU, and launches of small products overlap.
     const bool split_wins = dtype == DT_Q6_K ? m == 3 || m >= 5 : (dtype == DT_Q4_0 || dtype == DT_Q8_0) && m >= 4;
-    const bool eight = use_q6k && dtype == DT_Q6_K && m == 8 && q6k_cols8_serves(k) && columns_faster(dtype, k, n, m, 8);
-    if (layout == LAYOUT_PACKED && split_wins && !eight && n >= 1024 && x_aligned) {
+    if (layout == LAYOUT_PACKED && split_wins && n >= 1024 && x_aligned) {
         bool handled = false;
         const int st = gemm_split_mul_mat(s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);
         if (st != ST_OK) return st;
@@ -758,14 +755,14 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
     return fail(ST_UNSUPPORTED, "mul_mat: unsupported weight dtype %d", dtype);
 }
 
-// 9..32 columns of a packed Q4_K tensor in the integer column kernel, 8 or 4 per launch, where that is the faster way (columns_faster);
+// 9..16 columns of a packed Q4_K tensor in the integer column kernel, 8 or 4 per launch, where that is the faster way (q4k_columns_faster);
 // *handled = false otherwise.  The quantized columns are memory of the call: nothing has to be reserved, and streams share nothing.
 int q4k_batch(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy, bool * handled) {
     static const int use_imma = env_int("SM100_Q4K_IMMA", 1);
     *handled = false;
     const int width = q4k_cols_width(k);
-    if (!use_imma || width == 0 || n < 16 || n > INT32_MAX / 2 || m < 9 || m > 32 || (((uintptr_t) w | (uintptr_t) x) & 15) != 0 || ldx % 4 != 0) return ST_OK;
-    if (!columns_faster(DT_Q4_K, k, n, m, width)) return ST_OK;
+    if (!use_imma || width == 0 || n < 16 || n > INT32_MAX / 2 || m < 9 || m > 16 || (((uintptr_t) w | (uintptr_t) x) & 15) != 0 || ldx % 4 != 0) return ST_OK;
+    if (!q4k_columns_faster(k, n, m, width)) return ST_OK;
     CallScratch mem;
     if (call_scratch_alloc(s, q4k_cols_image_bytes(k, width), &mem) != ST_OK) return ST_OK;   // no memory: the split GEMM can do without
     const int64_t rest = m % width < 3 ? m % width : 0, cols = m - rest, full = n / 16 * 16;

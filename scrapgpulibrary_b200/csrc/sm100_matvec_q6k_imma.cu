@@ -343,7 +343,6 @@ size_t sq_smem_bytes(int units, int cols = 1) { return (size_t) cols * ((size_t)
 }  // namespace
 
 bool q6k_imma_serves(int64_t k) { return k % 256 == 0 && k <= (int64_t) 1 << 18 && sq_smem_bytes((int) (k / 64)) <= (size_t) 227 * 1024; }
-bool q6k_cols8_serves(int64_t k) { return q6k_imma_serves(k) && sq_smem_bytes((int) (k / 64), 8) <= (size_t) 227 * 1024; }   // 8 columns in one launch
 
 // Q6_K packed matvec, one activation column, over the full 16-row tiles of the tensor; *handled = false when the
 // shape is left to the caller's other kernels.

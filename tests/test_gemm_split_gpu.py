@@ -184,13 +184,13 @@ def test_columns_do_not_depend_on_their_batch(sm100, stream, dtype, k, n):
         assert np.array_equal(U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x[:m]), all_[:m]), m
 
 
-# few rows, a filled wave of the split GEMM, a long row; many rows, up to 16 columns in two launches, 17 in three; rows that fit four at a
-# time; a tail; Q6_K where one launch of eight columns is the faster one, and where it is not
+# few rows, a filled wave of the split GEMM, a long row; many rows and up to 16 columns in two launches; rows that fit four at a
+# time; a tail; more columns, and Q6_K, stay with the more accurate kernel
 @pytest.mark.parametrize("dtype,k,n,m,name", [(U.Q4_K, 4096, 1024, 16, "gemm_split"), (U.Q4_K, 2048, 8192, 24, "gemm_split"), (U.Q4_K, 12288, 2048, 9, "gemm_split"),
                                               (U.Q4_K, 1024, 8192, 9, "matvec_q4k_imma_cols"), (U.Q4_K, 4096, 4096, 16, "matvec_q4k_imma_cols"),
-                                              (U.Q4_K, 1024, 65536, 12, "matvec_q4k_imma_cols"), (U.Q4_K, 5120, 13824, 17, "matvec_q4k_imma_cols"),
+                                              (U.Q4_K, 1024, 65536, 12, "matvec_q4k_imma_cols"), (U.Q4_K, 5120, 13824, 17, "gemm_split"),
                                               (U.Q4_K, 8192, 28672, 11, "matvec_q4k_imma_cols"), (U.Q4_K, 1024, 8203, 10, "matvec_q4k_imma_cols+rows"),
-                                              (U.Q6_K, 5120, 13824, 8, "matvec_q6k_imma_cols"), (U.Q6_K, 4096, 4096, 8, "gemm_split")], ids=lambda v: str(v))
+                                              (U.Q6_K, 5120, 13824, 8, "gemm_split")], ids=lambda v: str(v))
 def test_batches_take_the_faster_kernel(sm100, stream, dtype, k, n, m, name):
     """Batches that the integer column kernels serve faster than one pass of the split GEMM stay with them.  Rows repeat every 480 (not a
     multiple of any tile), so that the oracle has few to multiply."""
