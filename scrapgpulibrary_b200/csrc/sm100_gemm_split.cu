@@ -22,7 +22,7 @@
 // What bounds it: up to 32 tokens the hand-over from chunk to chunk and the dequantizing warps (about 900 cycles a chunk of 64
 // weights x 128 rows; tensor pipe 12 to 21 % busy, issue slots 53 to 66 %), with prompts the tensor core (71 % busy while a CTA is
 // resident: 12 MMAs of 64 cycles in a chunk's 1090).  Measured, us, before / now: Q4_0
-// 4096 x 12288, 8 columns 64 / 28; Q4_K 12288 x 4096, 24 columns 63 / 34; Q6_K 12288 x 4096, 512 columns 3740 / 168 (before: one
+// 4096 x 12288, 8 columns 64 / 28; Q4_K 12288 x 4096, 24 columns 63 / 34; Q6_K 12288 x 4096, 512 columns 3740 / 157 (before: one
 // launch per 8 or 4 columns).  Tried: K over a cluster with the exchange in distributed shared memory (wrong sums; taken out),
 // three converting warps with their loads in registers (Q4_K, 24 columns: 41).
 //
@@ -552,7 +552,7 @@ int prompt_split(cudaStream_t s, SplitArgs g, const float * x, int64_t ldx, int6
 // Measured, columns / split: 4096 x 12288, 9 columns 21.6 / 32.9, 16 columns 26.9 / 35.6; 4096 x 4096, 16 columns 13.0 / 15.3; 4096 x 1024,
 // 16 columns 11.7 / 9.4; 12288 x 4096, 12 columns 31.4 / 30.9.  The line is drawn at 16 columns because the split GEMM is the more accurate way (error
 // 7e-6; 4e-5 to 1e-4 with the column kernel): beyond, and for 8 columns of Q6_K, the column kernels win little and seldom (Q4_K 5120 x 13824,
-// 17 columns 43.4 / 49.7, 24 columns 49.4 / 51.4, 4096 x 4096, 17 columns 16.9 / 15.7; Q6_K 5120 x 13824, 8 columns 47.0 / 53.0, 4096 x 4096 17.2 / 16.1).
+// 17 columns 43.4 / 49.7, 24 columns 49.4 / 51.4, 4096 x 4096, 17 columns 16.9 / 15.7; Q6_K 5120 x 13824, 8 columns 47.0 / 48.5, 4096 x 4096 17.2 / 15.0).
 bool q4k_columns_faster(int64_t k, int64_t n, int64_t m, int width) {
     if (m > 16) return false;
     const int chunks = (int) ((k + 2 * SP_KC - 1) / (2 * SP_KC)) * 2;

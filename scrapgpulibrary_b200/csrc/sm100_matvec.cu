@@ -689,7 +689,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
     // against the launches it replaces (one per column, or of 4, 2 and 1 columns with Q6_K), K x N, us:
     //   Q4_0  4096 x 1024: m = 2  8.6 / 7.5, m = 4  8.8 / 12.6    4096 x 12288: m = 2  29 / 16, m = 4  29.5 / 31.7, m = 8  28 / 62
     //   Q6_K  4096 x 1024: m = 2 10.8 / 7.9, m = 3 10.7 / 14.3, m = 4 10.7 / 10.5, m = 8 10.7 / 15.9
-    //         12288 x 4096: m = 2  34 / 26, m = 4  35 / 30, m = 8  35 / 59
+    //         12288 x 4096: m = 2  34 / 26, m = 4  31 / 30, m = 8  32 / 59
     // Below 1024 rows its few tiles cannot fill the GPU, and launches of small products overlap.
     const bool split_wins = dtype == DT_Q6_K ? m == 3 || m >= 5 : (dtype == DT_Q4_0 || dtype == DT_Q8_0) && m >= 4;
     if (layout == LAYOUT_PACKED && split_wins && n >= 1024 && x_aligned) {
