@@ -32,7 +32,11 @@ int matvec_q4k_imma_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, 
                           bool * handled);
 int matvec_q4k_tiles(cudaStream_t s, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
                      bool * handled);
+bool b32_imma_serves(int64_t k);
+bool q6k_imma_serves(int64_t k);
 int q4k_pass_width(int64_t k, int64_t m);
+int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
+                     bool fine, bool * handled);
 int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
                        bool * handled);
 int matvec_q4k_ring_multi(cudaStream_t s, int count, const void * const * ws, const int64_t * ns, int64_t k, const float * x,
@@ -573,6 +577,32 @@ static int matvec_dispatch(cudaStream_t s, int layout, const void * w, int64_t w
     return took("matvec_rows_natural", launch_rows<U, false>(s, w, w_row_stride, k, n, x, ldx, m, y, ldy));
 }
 
+// Weights up to which the single-column Q6_K tensor-core kernel beats the streaming kernel: it wins on small tensors and on short rows (4096 x 4096:
+// 1.9 vs 1.25 TB/s, 4096 x 12288: 2.45 vs 2.29), the streaming kernel on long rows (12288 x 4096: 2.98 vs 2.35 TB/s), where its lower instruction count per byte pays.
+static int64_t q6k_imma_limit(int64_t k) { return k <= 4096 ? (int64_t) 64 << 20 : (int64_t) 20 << 20; }
+
+// Does the column kernel (sm100_cols.cu) take this product?  Where the integer kernels, the split GEMM, or with Q6_K and one column the f32
+// kernels were slower; not where f32 kernels serve a batch, whose error (2e-7) is below its own (up to 1.3e-6).  Measured, us, before / after:
+//   Q6_K  1 column    4096 x 1024 7.0 / 5.9, 4096 x 12288 16.6 / 13.2, 12288 x 1024 16.3 / 7.9, 5120 x 5120 49.1 / 10.6, 8192 x 28672 61.9 / 49.6; but 2048 x 1024
+//                     7.0 / 7.3, and in the streaming kernel 12288 x 4096 12.4 / 15.0, 4096 x 151936 123 / 124 (118 / 104 in short bursts, at higher clocks)
+//         4 columns   4096 x 4096 13.2 / 8.2, 4096 x 12288 29.7 / 13.8, 12288 x 4096 31.5 / 15.6;  8 columns 15.4 / 9.3, 34.4 / 17.8, 32.1 / 21.2
+//   Q4_0  4 columns   4096 x 1024 9.0 / 5.5, 4096 x 12288 27.5 / 10.4, 12288 x 4096 24.5 / 11.7;  8 columns 9.1 / 5.7, 28.1 / 13.5, 25.1 / 15.1; Q8_0 alike;
+//                     but 1 column 4096 x 4096 5.4 / 6.0
+//   Q4_K  2 columns   4096 x 4096 5.9 / 6.4, 5120 x 5120 9.4 / 8.6, 12288 x 1024 12.6 / 6.7;  3 columns 4096 x 4096 8.2 / 6.7, 12288 x 4096 11.1 / 12.3
+//                     (four columns are one launch of the integer kernel there);  8 columns 4096 x 4096 8.0 / 7.6, 12288 x 4096 21.8 / 15.1
+// Below 4096 rows five to eight columns stay with the split GEMM, where a column's result does not depend on its batch.
+static bool cols_win(int dtype, int64_t k, int64_t n, int64_t m, bool split_wins) {
+    if (n < (split_wins && m >= 5 ? 4096 : 1024)) return false;
+    switch (dtype) {
+        case DT_Q4_0: case DT_Q8_0: return m >= 2 && b32_imma_serves(k);
+        case DT_Q4_K: return q4k_cols_width(k) != 0 && (m == 2 ? k > 4096 : m >= 5 || (m >= 3 && (k <= 8192 || n < 2048)));
+        case DT_Q6_K:
+            if (!q6k_imma_serves(k) || n * k < (int64_t) 4 << 20) return false;
+            return m > 1 || n * k <= q6k_imma_limit(k) || !wide_ok<WideQ6K>(k, m) || (k > 4096 && k <= 8192);
+    }
+    return false;
+}
+
 // Decode matvec entry used by sm100_mul_mat for m <= 8.  w_row_stride (bytes) only matters for the
 // natural layout; 0 means dense rows.
 int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_stride, int64_t k, int64_t n, const float * x,
@@ -589,6 +619,19 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
     if (layout == LAYOUT_PACKED && !is_quant(dtype)) return fail(ST_UNSUPPORTED, "mul_mat: only quantized weights have a packed layout");
     if (layout != LAYOUT_PACKED && layout != LAYOUT_NATURAL) return fail(ST_INVALID, "mul_mat: unknown layout %d", layout);
     if (is_quant(dtype) && !x_aligned) return fail(ST_UNSUPPORTED, "mul_mat: activations must be 16-byte aligned (columns too)");
+    // the batches that the split GEMM serves (further down)
+    const bool split_wins = dtype == DT_Q6_K ? m == 3 || m >= 5 : (dtype == DT_Q4_0 || dtype == DT_Q8_0) && m >= 4;
+    if (layout == LAYOUT_PACKED && x_aligned && cols_win(dtype, k, n, m, split_wins)) {
+        const bool fine = m == 1 && !wide_ok<WideQ6K>(k, m) && n * k > q6k_imma_limit(k);   // f32 kernels' precision where they served
+        bool handled = false;
+        const int st = quant_cols_tiles(s, dtype, w, k, n, x, ldx, m, y, ldy, fine, &handled);
+        if (st != ST_OK) return st;
+        if (handled) {   // it goes by the name of the split-operand GEMM where it stands in for that
+            const int64_t full = n / 16 * 16;
+            if (full == n) return took(split_wins ? "gemm_split" : "quant_cols", ST_OK);
+            return took(split_wins ? "gemm_split+rows" : "quant_cols+rows", tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
+        }
+    }
     static const int use_imma = env_int("SM100_Q4K_IMMA", 1);
     if (use_imma && layout == LAYOUT_PACKED && dtype == DT_Q4_K && x_aligned && m == 1) {
         // the ring kernel (consecutive launches overlap; it declines unless the stream's last launch was such a matvec);
@@ -627,11 +670,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         }
     }
     static const int use_q6k = env_int("SM100_Q6K_IMMA", 1);
-    // measured: the tensor-core kernel wins on small tensors and on short rows (4096 x 4096: 1.9 vs 1.25 TB/s,
-    // 4096 x 12288: 2.45 vs 2.29), the streaming kernel on long rows and large tensors (12288 x 4096: 2.98 vs 2.35,
-    // vocabulary head: 4.1 vs 3.1 TB/s), where its lower instruction count per byte pays
-    const int64_t q6k_limit = k <= 4096 ? (int64_t) 64 << 20 : (int64_t) 20 << 20;
-    if (use_q6k && layout == LAYOUT_PACKED && dtype == DT_Q6_K && x_aligned && m == 1 && (use_q6k > 1 || n * k <= q6k_limit)) {
+    if (use_q6k && layout == LAYOUT_PACKED && dtype == DT_Q6_K && x_aligned && m == 1 && (use_q6k > 1 || n * k <= q6k_imma_limit(k))) {
         bool handled = false;
         const int st = matvec_q6k_imma_tiles(s, w, k, n, x, y, &handled);
         if (st != ST_OK) return st;
@@ -691,7 +730,6 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
     //   Q6_K  4096 x 1024: m = 2 10.8 / 7.9, m = 3 10.7 / 14.3, m = 4 10.7 / 10.5, m = 8 10.7 / 15.9
     //         12288 x 4096: m = 2  34 / 26, m = 4  31 / 30, m = 8  32 / 59
     // Below 1024 rows its few tiles cannot fill the GPU, and launches of small products overlap.
-    const bool split_wins = dtype == DT_Q6_K ? m == 3 || m >= 5 : (dtype == DT_Q4_0 || dtype == DT_Q8_0) && m >= 4;
     if (layout == LAYOUT_PACKED && split_wins && n >= 1024 && x_aligned) {
         bool handled = false;
         const int st = gemm_split_mul_mat(s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);

@@ -1,0 +1,87 @@
+"""GPU parity of the column kernel (packed weights, up to 8 columns, integers times two f16 numbers on mma.sync) against float64.
+
+Tolerance: activations have 22 bits (2^-23), block scales and block sums are f32; the tensor core truncates its sums (2^-23 of the
+largest term, two to four MMAs a block), and the integers' offsets (8, 32, 128, the minima of Q4_K) make the terms up to three times as large as what is left of
+them: 3 (2^-23 + 4 2^-23) is 1.8e-6 at most per block, measured 2e-7 to 1.3e-6 over whole rows.  Bound: 4e-6, so NMSE 1.6e-11.
+"""
+import numpy as np
+import pytest
+
+from oracle import sgref
+from tests import util as U
+
+pytestmark = pytest.mark.gpu
+TOL = 1.6e-11
+
+
+def _want(dtype, wq, k, x):
+    return x.astype(np.float64) @ sgref.dequantize(dtype, wq, k).astype(np.float64).T
+
+
+def _name(n, m, dtype):
+    split = m in (3, 5, 6, 7, 8) if dtype == U.Q6_K else m >= 4 and dtype != U.Q4_K
+    return ("gemm_split" if split else "quant_cols") + ("" if n % 16 == 0 else "+rows")
+
+
+def _check(sm100, stream, dtype, k, n, m, seed=0):
+    few = min(n, 416)   # rows repeat, not in step with any tile, so that the oracle has few to multiply
+    wq = U.quantize(dtype, U.seeded_weights(900 + dtype + k, few, k))
+    x = U.seeded_acts(3 * m + k + seed, m, k)
+    want = _want(dtype, wq, k, x)[:, np.arange(n) % few]
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, np.ascontiguousarray(np.resize(wq, (n, wq.shape[1]))), k, x)
+    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == _name(n, m, dtype)
+    for t in range(m):
+        assert sgref.nmse(got[t].astype(np.float64), want[t]) <= TOL, (t, sgref.nmse(got[t].astype(np.float64), want[t]))
+    for r0 in range(0, n, 16):   # every row tile on its own
+        assert sgref.nmse(got[:, r0:r0 + 16].astype(np.float64), want[:, r0:r0 + 16]) <= 4 * TOL, r0
+
+
+# one unit of K, an odd number of units, 17 (two CTAs, uneven), 48 (three); fewer and more row tiles than CTAs, rows behind the last
+# whole tile; one window of row tiles and several
+SHAPES = [(256, 16384 + 16), (1280, 4096 + 5), (4352, 4096), (12288, 4096 + 48), (4096, 12288 + 16), (2048, 148 * 16 * 16)]
+
+
+@pytest.mark.parametrize("dtype", U.QUANT, ids=lambda d: U.NAMES[d])
+@pytest.mark.parametrize("m", [3, 4, 5, 8])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"k{s[0]}n{s[1]}")
+def test_shapes(sm100, stream, dtype, shape, m):
+    k, n = shape
+    if dtype == U.Q4_K and k > 8192 and m < 5:
+        pytest.skip("one launch of the integer kernel is faster there and serves it")
+    _check(sm100, stream, dtype, k, n, m)
+
+
+# the longest rows, few tiles, one and two columns; one column of Q6_K where an f32 kernel served before (signed integers)
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q6_K, 16384, 1024, 2), (U.Q4_0, 512, 1024, 3), (U.Q8_0, 8192, 1040, 2), (U.Q4_K, 13824, 1024, 8), (U.Q4_K, 6400, 2048, 2),
+                                         (U.Q6_K, 4096, 8192, 1), (U.Q6_K, 12288, 1040, 1), (U.Q6_K, 4352, 5008, 1), (U.Q6_K, 1280, 52016, 1)], ids=lambda v: str(v))
+def test_longest_rows_few_tiles_one_column(sm100, stream, dtype, k, n, m):
+    _check(sm100, stream, dtype, k, n, m)
+
+
+def test_one_column_keeps_the_precision_of_f32(sm100, stream):
+    """Rows that the f32 kernels served (2.3e-7 against float64)."""
+    k, n = 5120, 5120
+    wq = U.quantize(U.Q6_K, U.seeded_weights(1, n, k))
+    x = U.seeded_acts(2, 1, k)
+    got, want = U.device_mul_mat(sm100, stream, U.Q6_K, U.PACKED, wq, k, x), _want(U.Q6_K, wq, k, x)
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-7
+
+
+@pytest.mark.parametrize("dtype", U.QUANT, ids=lambda d: U.NAMES[d])
+@pytest.mark.parametrize("m", [4, 8])
+def test_magnitudes_and_poison(sm100, stream, dtype, m):
+    """A column keeps its precision whatever its magnitude, a NaN or an infinity poisons its own column only, and large block scales stay finite."""
+    k, n = 1024, 4096
+    wq = np.ascontiguousarray(np.resize(U.quantize(dtype, U.seeded_weights(5, 416, k) * np.float32(1e4 if dtype in (U.Q4_0, U.Q8_0) else 1.0)), (n, U.quantize(dtype, U.seeded_weights(5, 1, k)).shape[1])))
+    for poison in (np.nan, np.inf, -np.inf):
+        x = U.seeded_acts(6, m, k)
+        x[0] *= 1e30
+        x[1] *= 1e-25
+        x[1, 300:400] = 0.0
+        x[2, 5] = 3e6
+        x[3, 777] = poison
+        got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x).astype(np.float64)
+        want = _want(dtype, wq[:416], k, np.where(np.isfinite(x), x, 0))[:, np.arange(n) % 416]
+        assert not np.isfinite(got[3]).any()
+        for t in [0, 1, 2] + list(range(4, m)):
+            assert sgref.nmse(got[t], want[t]) <= TOL, t
