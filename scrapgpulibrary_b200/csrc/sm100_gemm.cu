@@ -336,14 +336,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
 // Activation preparation: f32 [M, K] (column stride ldx) -> normalised f16 stage images + token factors
 // ---------------------------------------------------------------------------------------------
 // A CTA takes `toks` consecutive tokens (a power of two, 1..8) with 256 / toks threads each and keeps their rows in
-// registers (up to PREP_MAX_V float4 per thread, all requested at once): one trip to memory gives both the
+// registers (up to V float4 per thread, all requested at once): one trip to memory gives both the
 // token's largest magnitude and, after the scale is known, the f16 image.  Rows too long for the registers
-// (K > 32768 / toks at toks = 1) take the two-pass path: the same loop twice.
+// (K > 32768) take the two-pass path: the same loop twice.
+// What bounds it is the number of CTAs and of bytes in flight: few float4 a thread (V = 4 up to K = 4096) and so many CTAs, of few registers each, rather than
+// eight tokens a CTA with 32 float4 a thread.  Products of 77 tokens (Q4_0, 4096 x 5003):
+// 23.2 -> 21.1 us, of 512 (Q8_0, 4096 x 12288) 74.0 -> 73.0; the preparation alone, cold, 6.5 -> 4.1 and 8.0 -> 6.0.
 constexpr int PREP_MAX_V = 32;
 
 // `order`: places of the groups of four weights in a chunk (pos4 of the weight source): 0 = in order of K, 1 = as Q8_0 and F16
 // weights want them, 2 = Q4_0.
-template <int TN>
+template <int TN, int V>
 __global__ void __launch_bounds__(256) gemm_prep_x(const float * x, int64_t ldx, int m, int k, int nchunks, int toks, int order, float * tokscale,
                                                    __half * xh) {
     pdl_wait();
@@ -355,19 +358,19 @@ __global__ void __launch_bounds__(256) gemm_prep_x(const float * x, int64_t ldx,
     const int r = threadIdx.x % tpt;
     const int kpad4 = nchunks * (KC / 4);        // float4 per token in the image (K padded to whole chunks)
     const int k4 = k / 4;
-    const bool in_regs = kpad4 <= PREP_MAX_V * tpt;
+    const bool in_regs = kpad4 <= V * tpt;
     const float4 * row = reinterpret_cast<const float4 *>(x + (int64_t) tok * ldx);
     const bool tok_ok = tok < m;
-    float4 v[PREP_MAX_V];
+    float4 v[V];
     float amax = 0.0f;
     if (in_regs) {
 #pragma unroll
-        for (int i = 0; i < PREP_MAX_V; ++i) {
+        for (int i = 0; i < V; ++i) {
             const int idx = r + i * tpt;
             v[i] = tok_ok && idx < k4 ? __ldcg(row + idx) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
-        for (int i = 0; i < PREP_MAX_V; ++i)
+        for (int i = 0; i < V; ++i)
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
     } else if (tok_ok) {
 #pragma unroll 8
@@ -401,7 +404,7 @@ __global__ void __launch_bounds__(256) gemm_prep_x(const float * x, int64_t ldx,
     };
     if (in_regs) {
 #pragma unroll
-        for (int i = 0; i < PREP_MAX_V; ++i) {
+        for (int i = 0; i < V; ++i) {
             const int idx = r + i * tpt;
             if (idx < kpad4) put(idx, v[i]);
         }
@@ -462,11 +465,13 @@ int gemm_passes(cudaStream_t s, int dtype, int layout, GemmArgs g, const float *
         if (st != ST_OK) return st;
         float * tokscale = (float *) ws;
         __half * xh = (__half *) ((uint8_t *) ws + scale_bytes);
-        // tokens per CTA: as many (up to 8) as keep a token's share of the row within the registers of its threads
+        // tokens per CTA: as many (up to 8) as leave at most four float4 to a thread
         int toks = 8;
-        while (toks > 1 && (int64_t) g.nchunks * (KC / 4) > (int64_t) PREP_MAX_V * (256 / toks)) toks >>= 1;
-        st = launch(gemm_prep_x<TN>, dim3((unsigned) (mpad / toks)), dim3(256), 0, s, x + c0 * ldx, ldx, (int) mm, (int) k, g.nchunks,
-                    toks, dtype == DT_Q4_K ? 0 : dtype == DT_Q4_0 ? 2 : 1, tokscale, xh);
+        while (toks > 1 && g.nchunks * (KC / 4) > 4 * (256 / toks)) toks >>= 1;
+        const int per = (g.nchunks * (KC / 4) * toks + 255) / 256;
+        auto prep = per <= 4 ? gemm_prep_x<TN, 4> : per <= 8 ? gemm_prep_x<TN, 8> : per <= 16 ? gemm_prep_x<TN, 16> : gemm_prep_x<TN, PREP_MAX_V>;
+        st = launch(prep, dim3((unsigned) (mpad / toks)), dim3(256), 0, s, x + c0 * ldx, ldx, (int) mm, (int) k, g.nchunks, toks,
+                    dtype == DT_Q4_K ? 0 : dtype == DT_Q4_0 ? 2 : 1, tokscale, xh);
         if (st != ST_OK) return st;
         g.xh = xh;
         g.tokscale = tokscale;

@@ -1,0 +1,27 @@
+"""The activation preparation of the tensor-core GEMM: one to eight tokens a CTA, 4 to 32 float4 a thread, two passes for the longest rows.
+
+Tolerance: f16 roundings of both operands, NMSE about 2e-7 (bar of the GEMM: 1e-6).
+"""
+import numpy as np
+import pytest
+
+from oracle import sgref
+from tests import util as U
+
+pytestmark = pytest.mark.gpu
+
+
+# eight, four, two tokens a CTA; one token with 4, 8, 16 and 32 float4 a thread (and just past each); two passes
+@pytest.mark.parametrize("k", [96, 512, 544, 1024, 1056, 2048, 4096, 4128, 8192, 8224, 16384, 16416, 32768, 32800])
+def test_row_lengths(sm100, stream, k):
+    n, m = 24, 37
+    wq = U.quantize(U.Q8_0, U.seeded_weights(k, n, k))
+    x = U.seeded_acts(k, m, k)
+    x[3] *= 1e6
+    x[5] = 0.0
+    x[7, k - 1] = 1e4   # the largest magnitude in the last element
+    want = sgref.mul_mat(U.Q8_0, wq, k, x)
+    got = U.device_mul_mat(sm100, stream, U.Q8_0, U.PACKED, wq, k, x)
+    assert np.all(got[5] == 0.0)
+    for t in [0, 3, 7, m - 1]:
+        assert sgref.nmse(got[t], want[t]) <= 1e-6, t
