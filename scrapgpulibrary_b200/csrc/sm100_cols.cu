@@ -513,7 +513,8 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
 struct ColsPlan { int cluster, wk, wr_log, at_once; };
 
 // The time of a plan goes with the row tiles that a warp walks down (`iters`) and with the warps that share an SM while it does so, plus
-// start and exchange.  12288 x 4096 (Q6_K, 4 columns), us: clusters of 3 with 16 warps a CTA 15.5, of 6 16.8, of 5 with 10 warps 18.6.
+// start and exchange.  12288 x 4096 (Q6_K, 4 columns), us: clusters of 3 with 16 warps a CTA 15.5, of 6 16.8, of 5 with 10 warps 18.6.  A CTA more
+// in the cluster counts 5 %: Q4_K, 2 columns, 3072 x 14336 with one CTA of 12 warps 9.6, three of 16 13.2; 5120 x 6144 two of 10 9.3, three of 14 10.6.
 // at_once: clusters that run at a time where every CTA has an SM of its own; SMs lie in groups that a cluster does not cross, so it is
 // fewer than 148 / cluster (a 7 x 17 grid took twice as long as one of 15).
 inline bool plan_cols(int units, int tiles, ColsPlan & p) {
@@ -524,7 +525,7 @@ inline bool plan_cols(int units, int tiles, ColsPlan & p) {
         if (wk > CO_WARPS || at_once < 1) continue;
         for (int wl = 0; wk << wl <= CO_WARPS; ++wl) {
             const int64_t groups = (tiles + (1 << wl) - 1) >> wl, iters = (groups + at_once - 1) / at_once;
-            const int64_t cost = iters * ((wk << wl) + 4) + (c > 1 ? 6 : 0);
+            const int64_t cost = iters * ((wk << wl) + 4) * (19 + c) / 20 + (c > 1 ? 6 : 0);
             if (cost < best) { best = cost; p = {c, wk, wl, at_once}; }
         }
     }

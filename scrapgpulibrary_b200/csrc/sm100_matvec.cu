@@ -338,13 +338,13 @@ __global__ void __launch_bounds__(MAXT, MINB) matvec_wide(const uint8_t * __rest
 template <class U, int M, bool PACKED>
 __global__ void __launch_bounds__(256) matvec_rows(const uint8_t * __restrict__ w, Planes P, int64_t w_row_stride,
                                                    const float * x, int64_t ldx, float * y, int64_t ldy,
-                                                   int row_begin, int n_rows, int units_per_row) {
+                                                   int n_rows, int units_per_row) {
     pdl_wait();
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int warps = blockDim.x >> 5;
     const int64_t bpr = units_per_row / U::UNITS_PER_BLOCK;
-    for (int r = row_begin + blockIdx.x * warps + (threadIdx.x >> 5); r < n_rows; r += gridDim.x * warps) {
+    for (int r = blockIdx.x * warps + (threadIdx.x >> 5); r < n_rows; r += gridDim.x * warps) {
         float acc[M];
 #pragma unroll
         for (int m = 0; m < M; ++m) acc[m] = 0.f;
@@ -518,18 +518,18 @@ static bool wide_ok(int64_t k, int64_t m) {
 
 template <class U, bool PACKED>
 static int launch_rows(cudaStream_t s, const void * w, int64_t w_row_stride, int64_t k, int64_t n, const float * x, int64_t ldx,
-                       int64_t m, float * y, int64_t ldy, int64_t row_begin = 0) {
+                       int64_t m, float * y, int64_t ldy) {
     const int upr = (int) (k / U::WEIGHTS);
     Planes P = {};
     if (PACKED) P = planes_for(U::DTYPE, n, k);
     const int threads = 256, warps = threads / 32;
-    int64_t grid = (n - row_begin + warps - 1) / warps;
+    int64_t grid = (n + warps - 1) / warps;
     const int64_t cap = (int64_t) sm_count() * 8;
     if (grid > cap) grid = cap;
     const dim3 g((unsigned) grid), b(threads);
     const uint8_t * wp = (const uint8_t *) w;
 #define SM100_ROWS_CASE(MM) \
-    case MM: return launch(matvec_rows<U, MM, PACKED>, g, b, 0, s, wp, P, w_row_stride, x, ldx, y, ldy, (int) row_begin, (int) n, upr);
+    case MM: return launch(matvec_rows<U, MM, PACKED>, g, b, 0, s, wp, P, w_row_stride, x, ldx, y, ldy, (int) n, upr);
     switch (m) {
         SM100_ROWS_CASE(1) SM100_ROWS_CASE(2) SM100_ROWS_CASE(3) SM100_ROWS_CASE(4)
         SM100_ROWS_CASE(5) SM100_ROWS_CASE(6) SM100_ROWS_CASE(7) SM100_ROWS_CASE(8)
@@ -555,7 +555,8 @@ template <class U>
 static int launch_tail(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
     return m <= 64 ? launch_tail_cols<U, 2>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy) : launch_tail_cols<U, 4>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
 }
-// rows row_begin .. n - 1 of a packed tensor in f32, m columns, x 16-byte aligned
+// Rows row_begin .. n - 1 of a packed tensor in f32, m columns, x 16-byte aligned.  Behind a single column too it takes half the time of matvec_rows, whose warps walk
+// along K alone (Q4_0 5120 x 5003, 11 rows, TAIL_FIGURES).
 int tail_rows(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
     switch (dtype) {
         case DT_Q4_0: return launch_tail<UnitQ40>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
@@ -582,23 +583,34 @@ static int matvec_dispatch(cudaStream_t s, int layout, const void * w, int64_t w
 static int64_t q6k_imma_limit(int64_t k) { return k <= 4096 ? (int64_t) 64 << 20 : (int64_t) 20 << 20; }
 
 // Does the column kernel (sm100_cols.cu) take this product?  Where the integer kernels, the split GEMM, or with Q6_K and one column the f32
-// kernels were slower; not where f32 kernels serve a batch, whose error (2e-7) is below its own (up to 1.3e-6).  Measured, us, before / after:
-//   Q6_K  1 column    4096 x 1024 7.0 / 5.9, 4096 x 12288 16.6 / 13.2, 12288 x 1024 16.3 / 7.9, 5120 x 5120 49.1 / 10.6, 8192 x 28672 61.9 / 49.6; but 2048 x 1024
-//                     7.0 / 7.3, and in the streaming kernel 12288 x 4096 12.4 / 15.0, 4096 x 151936 123 / 124 (118 / 104 in short bursts, at higher clocks)
-//         4 columns   4096 x 4096 13.2 / 8.2, 4096 x 12288 29.7 / 13.8, 12288 x 4096 31.5 / 15.6;  8 columns 15.4 / 9.3, 34.4 / 17.8, 32.1 / 21.2
-//   Q4_0  4 columns   4096 x 1024 9.0 / 5.5, 4096 x 12288 27.5 / 10.4, 12288 x 4096 24.5 / 11.7;  8 columns 9.1 / 5.7, 28.1 / 13.5, 25.1 / 15.1; Q8_0 alike;
-//                     but 1 column 4096 x 4096 5.4 / 6.0
-//   Q4_K  2 columns   4096 x 4096 5.9 / 6.4, 5120 x 5120 9.4 / 8.6, 12288 x 1024 12.6 / 6.7;  3 columns 4096 x 4096 8.2 / 6.7, 12288 x 4096 11.1 / 12.3
-//                     (four columns are one launch of the integer kernel there);  8 columns 4096 x 4096 8.0 / 7.6, 12288 x 4096 21.8 / 15.1
+// kernels were slower; not where f32 kernels serve a batch, whose error (2e-7) is below its own (up to 1.3e-6).  Measured over 250 shapes, K x N, us, before / after:
+//   Q4_0  4 columns   4096 x 1024 9.0 / 5.5, 4096 x 12288 27.5 / 10.4, 12288 x 4096 24.5 / 12.5;  8 columns 9.1 / 5.7, 28.1 / 13.5, 25.1 / 15.1; Q8_0 alike
+//         1 column    the integer kernel is at its best where K is a multiple of 4096: 4096 x 4096 5.4 / 6.0, 8192 x 8192 11.5 / 12.3, 12288 x 4096 10.2 / 12.0, but
+//                     12288 x 1024 8.6 / 6.4; else 5120 x 6144 11.1 / 9.0, 7168 x 12288 21.2 / 15.2, 3072 x 6144 7.4 / 6.2, 6144 x 2048 7.2 / 6.2; 6144 x 4096 7.5 / 9.4,
+//                     2048 x 8192 6.5 / 6.0 (Q8_0 6.5 / 6.8)
+//   Q4_K  2 columns   4096 x 4096 5.9 / 6.4, 4096 x 14336 12.8 / 11.1, 5120 x 6144 9.5 / 9.3, 12288 x 6144 18.8 / 15.9, 10240 x 14336 26.0 / 28.9
+//         4 columns   4096 x 4096 8.2 / 6.7, 6144 x 14336 20.1 / 15.5, 10240 x 2048 9.3 / 10.3, 10240 x 6144 17.2 / 15.6, 12288 x 14336 32.5 / 32.3
+//         8 columns   4096 x 4096 8.0 / 7.6, 10240 x 6144 33.5 / 20.3, 12288 x 4096 21.8 / 15.1
+//   Q6_K  1 column    4096 x 1024 7.0 / 5.9, 4096 x 12288 16.6 / 13.2, 2048 x 4096 5.1 / 5.8, 7168 x 8192 81.7 / 17.1 (an f32 kernel for rows of any length before);
+//                     in the streaming kernel 6144 x 4096 9.1 / 11.3, 8192 x 8192 20.5 / 16.8, 12288 x 4096 12.4 / 16.2, 4096 x 151936 123 / 124
+//         4 columns   4096 x 4096 13.2 / 8.2, 4096 x 12288 29.7 / 13.8, 12288 x 4096 31.6 / 17.2;  8 columns 15.4 / 9.3, 34.4 / 17.8, 32.1 / 21.2
 // Below 4096 rows five to eight columns stay with the split GEMM, where a column's result does not depend on its batch.
 static bool cols_win(int dtype, int64_t k, int64_t n, int64_t m, bool split_wins) {
     if (n < (split_wins && m >= 5 ? 4096 : 1024)) return false;
     switch (dtype) {
-        case DT_Q4_0: case DT_Q8_0: return m >= 2 && b32_imma_serves(k);
-        case DT_Q4_K: return q4k_cols_width(k) != 0 && (m == 2 ? k > 4096 : m >= 5 || (m >= 3 && (k <= 8192 || n < 2048)));
+        case DT_Q4_0: case DT_Q8_0:
+            if (!b32_imma_serves(k)) return false;
+            if (m >= 2) return true;
+            if (k % 4096 == 0) return k >= 12288 && n < 2048;
+            return n >= (k >= 2560 ? 6144 : 12288) || (n <= 2048 && k >= 5120);
+        case DT_Q4_K:
+            if (q4k_cols_width(k) == 0) return false;
+            if (m == 2) return k > 4096 ? k <= 8192 || n <= 8192 : k >= 2560 && n >= 12288;
+            return m >= 5 || (m >= 3 && (k <= 8192 || n < 2048 || n >= 6144));
         case DT_Q6_K:
             if (!q6k_imma_serves(k) || n * k < (int64_t) 4 << 20) return false;
-            return m > 1 || n * k <= q6k_imma_limit(k) || !wide_ok<WideQ6K>(k, m) || (k > 4096 && k <= 8192);
+            if (m > 1) return true;
+            return n * k > q6k_imma_limit(k) && wide_ok<WideQ6K>(k, m) ? k > 6144 && k <= 8192 : k >= 2560 || n >= 12288;
     }
     return false;
 }
@@ -641,7 +653,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            if (full < n) return took("matvec_q4k_ring+rows", launch_rows<UnitQ4K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full));
+            if (full < n) return took("matvec_q4k_ring+rows", tail_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
             return took("matvec_q4k_ring", ST_OK);
         }
     }
@@ -652,7 +664,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            if (full < n) return took("matvec_q4k_imma+rows", launch_rows<UnitQ4K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full));
+            if (full < n) return took("matvec_q4k_imma+rows", tail_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
             if (m == 1) stream_tail_set(s, TAIL_Q4K_MATVEC);   // a second plain Q4_K matvec right behind this one starts a run of the ring kernel
             return took("matvec_q4k_imma", ST_OK);
         }
@@ -665,8 +677,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (handled) {
             const int64_t full = (n / 16) * 16;
             if (full == n) return took("matvec_b32_imma", ST_OK);
-            return took("matvec_b32_imma+rows", dtype == DT_Q4_0 ? launch_rows<UnitQ40, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full)
-                                                                 : launch_rows<UnitQ80, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full));
+            return took("matvec_b32_imma+rows", tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
     static const int use_q6k = env_int("SM100_Q6K_IMMA", 1);
@@ -676,7 +687,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            return full == n ? took("matvec_q6k_imma", ST_OK) : took("matvec_q6k_imma+rows", launch_rows<UnitQ6K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full));
+            return full == n ? took("matvec_q6k_imma", ST_OK) : took("matvec_q6k_imma+rows", tail_rows(s, DT_Q6_K, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
     if (use_imma && layout == LAYOUT_PACKED && dtype == DT_Q4_K && x_aligned && m >= 3) {
@@ -698,7 +709,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         }
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            if (full < n) return took("matvec_q4k_imma_cols+rows", launch_rows<UnitQ4K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full));
+            if (full < n) return took("matvec_q4k_imma_cols+rows", tail_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
             return took("matvec_q4k_imma_cols", ST_OK);
         }
     }
@@ -720,7 +731,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         }
         if (all) {
             const int64_t full = (n / 16) * 16;
-            if (full < n) return took("matvec_q4k_mma+rows", launch_rows<UnitQ4K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full));
+            if (full < n) return took("matvec_q4k_mma+rows", tail_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
             return took("matvec_q4k_mma", ST_OK);
         }
     }
@@ -744,7 +755,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            return full == n ? took("matvec_q6k_imma_cols", ST_OK) : took("matvec_q6k_imma_cols+rows", launch_rows<UnitQ6K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, full));
+            return full == n ? took("matvec_q6k_imma_cols", ST_OK) : took("matvec_q6k_imma_cols+rows", tail_rows(s, DT_Q6_K, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
     // Q6_K / Q4_0 / Q8_0 with few columns or rows: the single-column tensor-core and wide kernels have no multi-column form,
