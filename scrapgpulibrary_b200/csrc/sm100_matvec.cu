@@ -556,7 +556,7 @@ static int launch_tail(cudaStream_t s, int dtype, const void * w, int64_t k, int
     return m <= 64 ? launch_tail_cols<U, 2>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy) : launch_tail_cols<U, 4>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
 }
 // Rows row_begin .. n - 1 of a packed tensor in f32, m columns, x 16-byte aligned.  Behind a single column too it takes half the time of matvec_rows, whose warps walk
-// along K alone (Q4_0 5120 x 5003, 11 rows, TAIL_FIGURES).
+// along K alone (Q8_0 4096 x 5003, 11 rows: the whole product 17.0 -> 10.4 us).
 int tail_rows(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
     switch (dtype) {
         case DT_Q4_0: return launch_tail<UnitQ40>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
@@ -588,9 +588,10 @@ static int64_t q6k_imma_limit(int64_t k) { return k <= 4096 ? (int64_t) 64 << 20
 //         1 column    the integer kernel is at its best where K is a multiple of 4096: 4096 x 4096 5.4 / 6.0, 8192 x 8192 11.5 / 12.3, 12288 x 4096 10.2 / 12.0, but
 //                     12288 x 1024 8.6 / 6.4; else 5120 x 6144 11.1 / 9.0, 7168 x 12288 21.2 / 15.2, 3072 x 6144 7.4 / 6.2, 6144 x 2048 7.2 / 6.2; 6144 x 4096 7.5 / 9.4,
 //                     2048 x 8192 6.5 / 6.0 (Q8_0 6.5 / 6.8)
-//   Q4_K  2 columns   4096 x 4096 5.9 / 6.4, 4096 x 14336 12.8 / 11.1, 5120 x 6144 9.5 / 9.3, 12288 x 6144 18.8 / 15.9, 10240 x 14336 26.0 / 28.9
-//         4 columns   4096 x 4096 8.2 / 6.7, 6144 x 14336 20.1 / 15.5, 10240 x 2048 9.3 / 10.3, 10240 x 6144 17.2 / 15.6, 12288 x 14336 32.5 / 32.3
-//         8 columns   4096 x 4096 8.0 / 7.6, 10240 x 6144 33.5 / 20.3, 12288 x 4096 21.8 / 15.1
+//   Q4_K  2..4 columns  the integer kernels' launches overlap in a graph; three layers' projections, hidden / FFN, 4 columns 2048 / 6144 47.3 / 52.4, 4096 / 12288 86.1 / 87.8,
+//                     4864 / 12288 126 / 133, 5120 / 14336 146 / 117 (single launches 4096 x 4096 8.2 / 6.7, 6144 x 14336 20.1 / 15.5, 12288 x 14336 32.5 / 32.3)
+//         5..8 columns  the same graphs, 8 columns 57.4 / 57.8, 126 / 120, 5120 / 14336 224 / 147; single launches 4096 x 4096 8.0 / 7.6, 10240 x 6144 33.5 / 20.3,
+//                     12288 x 4096 21.8 / 15.1; the one loss seen is 5 columns at 3840 / 11264, 115 / 123 (8 columns 121 / 120)
 //   Q6_K  1 column    4096 x 1024 7.0 / 5.9, 4096 x 12288 16.6 / 13.2, 2048 x 4096 5.1 / 5.8, 7168 x 8192 81.7 / 17.1 (an f32 kernel for rows of any length before);
 //                     in the streaming kernel 6144 x 4096 9.1 / 11.3, 8192 x 8192 20.5 / 16.8, 12288 x 4096 12.4 / 16.2, 4096 x 151936 123 / 124
 //         4 columns   4096 x 4096 13.2 / 8.2, 4096 x 12288 29.7 / 13.8, 12288 x 4096 31.6 / 17.2;  8 columns 15.4 / 9.3, 34.4 / 17.8, 32.1 / 21.2
@@ -605,8 +606,7 @@ static bool cols_win(int dtype, int64_t k, int64_t n, int64_t m, bool split_wins
             return n >= (k >= 2560 ? 6144 : 12288) || (n <= 2048 && k >= 5120);
         case DT_Q4_K:
             if (q4k_cols_width(k) == 0) return false;
-            if (m == 2) return k > 4096 ? k <= 8192 || n <= 8192 : k >= 2560 && n >= 12288;
-            return m >= 5 || (m >= 3 && (k <= 8192 || n < 2048 || n >= 6144));
+            return m >= 5 || (m >= 2 && k > 12288);
         case DT_Q6_K:
             if (!q6k_imma_serves(k) || n * k < (int64_t) 4 << 20) return false;
             if (m > 1) return true;
