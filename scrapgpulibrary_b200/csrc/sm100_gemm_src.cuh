@@ -293,7 +293,6 @@ struct SrcQ6K {
     struct Regs { uint4 n[2], b[2]; uint32_t sc[2], d[2]; };
     struct ScaleSplit { __nv_bfloat162 d1, d2; };
     __host__ __device__ static __forceinline__ int pos4(int q) { return 4 * (q & 3) + (q >> 2); }
-    __host__ __device__ static __forceinline__ int quad_at(int p) { return 4 * (p & 3) + (p >> 2); }   // inverse of pos4
     __host__ __device__ static __forceinline__ int base(int c) { return (c >> 2) * 256 + ((c >> 1) & 1) * 128 + (c & 1) * 16; }
     __host__ __device__ static __forceinline__ int k4(int q) { return 32 * (q >> 2) + 4 * (q & 3); }   // first weight of group q from base(c)
     __device__ static __forceinline__ void init(Cursor & u, const WeightRef & W, const int64_t (&row)[2], int t) {

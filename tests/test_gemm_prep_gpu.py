@@ -25,3 +25,17 @@ def test_row_lengths(sm100, stream, k):
     assert np.all(got[5] == 0.0)
     for t in [0, 3, 7, m - 1]:
         assert sgref.nmse(got[t], want[t]) <= 1e-6, t
+
+
+# eight tokens a CTA (up to 64) and 32: one CTA's tokens, one more, one less; one block of K and several
+@pytest.mark.parametrize("m", [33, 40, 41, 63, 64, 65, 96, 97, 128, 129, 160])
+@pytest.mark.parametrize("k", [256, 1280])
+def test_stage_images_of_q6_k_prompts(sm100, stream, k, m):
+    """Both operands as two bf16 numbers: 16 bits each, NMSE (3e-5)^2 as for the split GEMM."""
+    n = 32
+    wq = U.quantize(U.Q6_K, U.seeded_weights(k, n, k))
+    x = U.seeded_acts(m, m, k)
+    want = sgref.mul_mat(U.Q6_K, wq, k, x)
+    got = U.device_mul_mat(sm100, stream, U.Q6_K, U.PACKED, wq, k, x)
+    for t in range(m):
+        assert sgref.nmse(got[t], want[t]) <= 1e-9, t
