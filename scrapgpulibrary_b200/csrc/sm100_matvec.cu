@@ -735,7 +735,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
             return took("matvec_q4k_mma", ST_OK);
         }
     }
-    // Q4_0 / Q8_0 from 4 columns on, Q6_K at 3 and from 5 on: the split-operand GEMM reads the weights once for all columns.  Measured
+    // Q4_0 / Q8_0 from 4 columns on, Q6_K at 3 and from 5 on, where the column kernel has not taken them: the split-operand GEMM reads the weights once for all columns.  Measured
     // against the launches it replaces (one per column, or of 4, 2 and 1 columns with Q6_K), K x N, us:
     //   Q4_0  4096 x 1024: m = 2  8.6 / 7.5, m = 4  8.8 / 12.6    4096 x 12288: m = 2  29 / 16, m = 4  29.5 / 31.7, m = 8  28 / 62
     //   Q6_K  4096 x 1024: m = 2 10.8 / 7.9, m = 3 10.7 / 14.3, m = 4 10.7 / 10.5, m = 8 10.7 / 15.9
