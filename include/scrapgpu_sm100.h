@@ -180,7 +180,7 @@ SM100_API int sm100_pack_device_range(sm100_stream_t s, int dtype, int64_t k, in
 SM100_API int sm100_mul_mat(sm100_stream_t s, int dtype, int layout, const void * w, int64_t w_row_stride, int64_t k,
                             int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy);
 /* Name of the kernel family that served the calling thread's last sm100_mul_mat ("matvec_q4k_imma", "matvec_wide", "matvec_rows",
- * "gemm_split", "gemm_tc", ...; "+rows" when leftover rows took the row kernel) or sm100_attention ("attn_prompt", "attn_splits").  The reference reports its kernel
+ * "quant_cols", "gemm_split", "gemm_tc", ...; "+rows" when leftover rows took the row kernel) or sm100_attention ("attn_prompt", "attn_splits").  The reference reports its kernel
  * choice per op key in its profile table (src/backends/opencl11/executor.h:41-112); here the parity tests use it to
  * prove that every branch of the dispatcher is exercised. */
 SM100_API const char * sm100_matvec_last_kernel(void);

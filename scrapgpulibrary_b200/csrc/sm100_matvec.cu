@@ -638,10 +638,10 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         bool handled = false;
         const int st = quant_cols_tiles(s, dtype, w, k, n, x, ldx, m, y, ldy, fine, &handled);
         if (st != ST_OK) return st;
-        if (handled) {   // it goes by the name of the split-operand GEMM where it stands in for that
+        if (handled) {
             const int64_t full = n / 16 * 16;
-            if (full == n) return took(split_wins ? "gemm_split" : "quant_cols", ST_OK);
-            return took(split_wins ? "gemm_split+rows" : "quant_cols+rows", tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
+            if (full == n) return took("quant_cols", ST_OK);
+            return took("quant_cols+rows", tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
     static const int use_imma = env_int("SM100_Q4K_IMMA", 1);

@@ -91,7 +91,7 @@ def _kernel(sm100):
 FORCED = [
     ({}, ["q4_k:matvec_q4k_imma", "q4_k:matvec_q4k_imma+rows", "q4_k:matvec_q4k_imma_cols+rows",
           "q6_k:matvec_q6k_imma", "q4_0:matvec_b32_imma", "q8_0:matvec_b32_imma", "q6_k:matvec_q6k_imma_cols", "q4_0:matvec_per_column",
-          "q6_k:matvec_rows", "q8_0:matvec_rows", "q4_0:gemm_split+rows", "q8_0:gemm_split", "q6_k:gemm_split+rows"]),
+          "q6_k:matvec_rows", "q8_0:matvec_rows", "q4_0:quant_cols+rows", "q4_0:gemm_split+rows", "q8_0:gemm_split", "q6_k:gemm_split+rows"]),
     ({"SM100_Q4K_RING": "2"}, ["q4_k:matvec_q4k_ring", "q4_k:matvec_q4k_ring+rows", "q4_k:matvec_q4k_imma"]),   # 2: the ring kernel wherever its shapes allow
     ({"SM100_Q4K_RING": "0"}, ["q4_k:matvec_q4k_imma", "q4_k:matvec_q4k_imma+rows"]),
     ({"SM100_Q6K_IMMA": "0", "SM100_B32_IMMA": "0"}, ["q6_k:matvec_wide", "q4_0:matvec_wide", "q8_0:matvec_wide", "q6_k:matvec_rows", "q6_k:matvec_per_column"]),

@@ -18,18 +18,13 @@ def _want(dtype, wq, k, x):
     return x.astype(np.float64) @ sgref.dequantize(dtype, wq, k).astype(np.float64).T
 
 
-def _name(n, m, dtype):
-    split = m in (3, 5, 6, 7, 8) if dtype == U.Q6_K else m >= 4 and dtype != U.Q4_K
-    return ("gemm_split" if split else "quant_cols") + ("" if n % 16 == 0 else "+rows")
-
-
 def _check(sm100, stream, dtype, k, n, m, seed=0):
     few = min(n, 416)   # rows repeat, not in step with any tile, so that the oracle has few to multiply
     wq = U.quantize(dtype, U.seeded_weights(900 + dtype + k, few, k))
     x = U.seeded_acts(3 * m + k + seed, m, k)
     want = _want(dtype, wq, k, x)[:, np.arange(n) % few]
     got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, np.ascontiguousarray(np.resize(wq, (n, wq.shape[1]))), k, x)
-    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == _name(n, m, dtype)
+    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == ("quant_cols" if n % 16 == 0 else "quant_cols+rows")
     for t in range(m):
         assert sgref.nmse(got[t].astype(np.float64), want[t]) <= TOL, (t, sgref.nmse(got[t].astype(np.float64), want[t]))
     for r0 in range(0, n, 16):   # every row tile on its own
