@@ -22,7 +22,8 @@ CASES = [(U.Q4_K, 4096, 272, 1), (U.Q4_K, 4096, 264, 2), (U.Q4_K, 2048, 40, 4), 
          (U.Q6_K, 4096, 272, 1), (U.Q6_K, 2048, 40, 1), (U.Q6_K, 12288, 528, 1), (U.Q6_K, 4096, 64, 4), (U.Q6_K, 768, 24, 1), (U.Q6_K, 768, 8, 2),
          (U.Q4_0, 4096, 272, 1), (U.Q4_0, 2048, 33, 1), (U.Q4_0, 4096, 64, 3), (U.Q4_0, 96, 24, 1),
          (U.Q8_0, 4096, 272, 1), (U.Q8_0, 1024, 40, 1), (U.Q8_0, 4096, 64, 8), (U.Q8_0, 160, 17, 1), (U.Q8_0, 160, 17, 3),
-         (U.Q4_0, 512, 1030, 4), (U.Q4_0, 640, 1030, 4), (U.Q8_0, 640, 1024, 7), (U.Q6_K, 512, 1030, 5)]
+         (U.Q4_0, 512, 1030, 4), (U.Q8_0, 512, 1024, 7), (U.Q6_K, 512, 1030, 5),
+         (U.Q4_0, 640, 1030, 4)]   # rows that are no multiple of 256: the column kernel declines them
 
 
 def main():

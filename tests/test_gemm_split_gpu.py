@@ -15,6 +15,12 @@ from tests import util as U
 pytestmark = pytest.mark.gpu
 TOL = 1e-9
 COLUMNS_TOL = 2e-8   # the integer column kernels: 16-bit activations per 64 weights, their bound in test_matvec_gpu.py is 1e-6
+# shapes of the lists below that the column kernel (test_quant_cols_gpu.py) serves instead
+COLUMN_KERNEL = {(U.Q4_0, 1024, 1030, 4), (U.Q8_0, 512, 128 * 297, 5), (U.Q6_K, 5120, 13824, 8)}
+
+
+def _name(dtype, k, n, m):
+    return ("quant_cols" if (dtype, k, n, m) in COLUMN_KERNEL else "gemm_split") + ("" if n % 16 == 0 else "+rows")
 
 
 def _check(sm100, stream, dtype, k, n, m):
@@ -22,7 +28,7 @@ def _check(sm100, stream, dtype, k, n, m):
     x = U.seeded_acts(3 * m + k, m, k)
     want = sgref.mul_mat(dtype, wq, k, x)
     got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x)
-    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == ("gemm_split" if n % 16 == 0 else "gemm_split+rows")
+    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == _name(dtype, k, n, m)
     assert np.isfinite(got).all()
     for t in range(m):   # per token, so that one wrong column cannot hide in the average
         assert sgref.nmse(got[t], want[t]) <= TOL, (t, sgref.nmse(got[t], want[t]))
@@ -37,16 +43,17 @@ def test_batches(sm100, stream, dtype, shape):
     _check(sm100, stream, dtype, *shape)
 
 
-# three to eight columns, from 1024 rows on: the matvec's own way here; rows at and past a tile of 128, a tail, K of one stage and more.  The column
-# kernel is ahead where K is a multiple of 256 (Q4_0, Q8_0) and from 4 M weights on (Q6_K)
-@pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 1152, 1030, 4), (U.Q4_0, 128, 1024, 7), (U.Q8_0, 1152, 1030, 7), (U.Q8_0, 2176, 1152, 4),
-                                         (U.Q6_K, 1024, 1030, 3), (U.Q6_K, 256, 1040, 5), (U.Q6_K, 3840, 1030, 8)], ids=lambda v: str(v))
+# three to eight columns, from 1024 rows on: the matvec's own way here; rows at and past a tile of 128, a tail, K of one stage and more
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 1024, 1030, 4), (U.Q4_0, 128, 1024, 7), (U.Q8_0, 1024, 1030, 7), (U.Q8_0, 2176, 1152, 4),
+                                         (U.Q6_K, 1024, 1030, 3), (U.Q6_K, 256, 1040, 5), (U.Q6_K, 4096, 1030, 8),
+                                         (U.Q4_0, 1152, 1030, 4)], ids=lambda v: str(v))
 def test_few_columns(sm100, stream, dtype, k, n, m):
     _check(sm100, stream, dtype, k, n, m)
 
 
 # more tiles than SMs: whole waves of one CTA per tile, and the rest with K cut; row and token tiles ragged
-@pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 512, 128 * 160 + 16, 24), (U.Q4_K, 1024, 128 * 150 + 5, 32), (U.Q8_0, 640, 128 * 297, 5), (U.Q6_K, 512, 4100, 700), (U.Q6_K, 1024, 6400, 200)],
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 512, 128 * 160 + 16, 24), (U.Q4_K, 1024, 128 * 150 + 5, 32), (U.Q8_0, 512, 128 * 297, 5), (U.Q6_K, 512, 4100, 700), (U.Q6_K, 1024, 6400, 200),
+                                         (U.Q8_0, 640, 128 * 297, 5)],
                          ids=lambda v: str(v))
 def test_whole_waves_and_cut_tiles(sm100, stream, dtype, k, n, m):
     """Rows repeat every 360 (no multiple of a tile), so that the oracle has few to multiply while every tile differs from its neighbours."""
@@ -55,7 +62,7 @@ def test_whole_waves_and_cut_tiles(sm100, stream, dtype, k, n, m):
     x = U.seeded_acts(k + m, m, k)
     want = sgref.mul_mat(dtype, wq, k, x)[:, np.arange(n) % few]
     got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, np.ascontiguousarray(np.resize(wq, (n, wq.shape[1]))), k, x)
-    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == ("gemm_split" if n % 16 == 0 else "gemm_split+rows")
+    assert (sm100.lib().sm100_matvec_last_kernel() or b"").decode() == _name(dtype, k, n, m)
     for r0 in range(0, n, 128):
         for t0 in range(0, m, 64):
             part = np.s_[t0:t0 + 64, r0:r0 + 128]
@@ -191,7 +198,7 @@ def test_columns_do_not_depend_on_their_batch(sm100, stream, dtype, k, n):
                                               (U.Q4_K, 1024, 8192, 9, "matvec_q4k_imma_cols"), (U.Q4_K, 4096, 4096, 16, "matvec_q4k_imma_cols"),
                                               (U.Q4_K, 1024, 65536, 12, "matvec_q4k_imma_cols"), (U.Q4_K, 5120, 13824, 17, "gemm_split"),
                                               (U.Q4_K, 8192, 28672, 11, "matvec_q4k_imma_cols"), (U.Q4_K, 1024, 8203, 10, "matvec_q4k_imma_cols+rows"),
-                                              (U.Q6_K, 5120, 13824, 9, "gemm_split"), (U.Q6_K, 5120, 13824, 8, "quant_cols")], ids=lambda v: str(v))
+                                              (U.Q6_K, 5120, 13824, 8, "quant_cols"), (U.Q6_K, 5120, 13824, 9, "gemm_split")], ids=lambda v: str(v))
 def test_batches_take_the_faster_kernel(sm100, stream, dtype, k, n, m, name):
     """Batches that the integer column kernels serve faster than one pass of the split GEMM stay with them.  Rows repeat every 480 (not a
     multiple of any tile), so that the oracle has few to multiply."""
