@@ -634,7 +634,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
     // the batches that the split GEMM serves (further down)
     const bool split_wins = dtype == DT_Q6_K ? m == 3 || m >= 5 : (dtype == DT_Q4_0 || dtype == DT_Q8_0) && m >= 4;
     if (layout == LAYOUT_PACKED && x_aligned && cols_win(dtype, k, n, m, split_wins)) {
-        const bool fine = m == 1 && !wide_ok<WideQ6K>(k, m) && n * k > q6k_imma_limit(k);   // f32 kernels' precision where they served
+        const bool fine = dtype == DT_Q6_K && m == 1 && n * k > q6k_imma_limit(k);   // f32 kernels' precision where they served
         bool handled = false;
         const int st = quant_cols_tiles(s, dtype, w, k, n, x, ldx, m, y, ldy, fine, &handled);
         if (st != ST_OK) return st;

@@ -18,6 +18,10 @@ def _want(dtype, wq, k, x):
     return x.astype(np.float64) @ sgref.dequantize(dtype, wq, k).astype(np.float64).T
 
 
+def _served(sm100):
+    return (sm100.lib().sm100_matvec_last_kernel() or b"").decode()
+
+
 def _check(sm100, stream, dtype, k, n, m, seed=0):
     few = min(n, 416)   # rows repeat, not in step with any tile, so that the oracle has few to multiply
     wq = U.quantize(dtype, U.seeded_weights(900 + dtype + k, few, k))
@@ -82,3 +86,13 @@ def test_magnitudes_and_poison(sm100, stream, dtype, m):
         assert not np.isfinite(got[3]).any()
         for t in [0, 1, 2] + list(range(4, m)):
             assert sgref.nmse(got[t], want[t]) <= TOL, t
+
+
+@pytest.mark.parametrize("k,n", [(8192, 5120), (4352, 5008), (7168, 4096)])
+def test_one_column_of_every_row_that_f32_kernels_served(sm100, stream, k, n):
+    """K = 8192 among them, which the streaming kernel would serve: the bound of the rows above."""
+    wq = np.ascontiguousarray(np.resize(U.quantize(U.Q6_K, U.seeded_weights(k, 416, k)), (n, k // 256 * 210)))
+    x = U.seeded_acts(n, 1, k)
+    got, want = U.device_mul_mat(sm100, stream, U.Q6_K, U.PACKED, wq, k, x), _want(U.Q6_K, wq[:416], k, x)[:, np.arange(n) % 416]
+    assert _served(sm100).startswith("quant_cols")
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-7
