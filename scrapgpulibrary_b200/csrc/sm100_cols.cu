@@ -6,8 +6,9 @@
 // A warp owns 256 weights of K (a unit) for the whole launch: its activations are B fragments in registers.  It walks down row
 // tiles of 16 rows, whose bytes it copies to a ring of its own in shared memory (cp.async: whole lines of the row-major planes, no registers
 // for what is in flight) and reads back as A fragments (ldmatrix: a matrix row is 16 bytes of a weight row).  The integers need no conversion:
-// a bit field under a zero exponent is a subnormal f16 number.  A block (32 weights, Q6_K 16) is multiplied into a fresh accumulator, which
-// times the block's scale goes to f32 sums: no weight is scaled or rounded, and the tensor core's truncation sees 32 products at most.
+// a bit field under the exponent of 1024 is an f16 number, and one packed addition takes 1024 and the format's offset (8, 32, 128) off, exactly; the unsigned
+// ones of Q4_K stand under a zero exponent, subnormal numbers.  A block (32 weights, Q6_K 16) is multiplied into a fresh accumulator, which times the block's
+// scale goes to f32 sums: no weight is scaled or rounded, and the tensor core's truncation sees 32 products at most.
 //
 // Activations: per column and unit one power of two brings the largest to [2^13, 2^14), then x = xh + xl, both f16 (22 bits).
 //   M <= 4: the eight columns of an MMA are xh and xl of four tokens; M <= 8: two MMAs, xh and xl of eight
@@ -42,6 +43,7 @@ struct ColsArgs {
     int wk, wr_log; // warps of a CTA: wk units x 2^wr_log row tiles
     int iters;      // row tiles of a warp
     int window;     // of them, as many whose partial sums meet at once
+    uint32_t k1024; // CO_1024
 };
 
 __device__ __forceinline__ uint32_t co_smem(const void * p) { return (uint32_t) __cvta_generic_to_shared(p); }
@@ -83,14 +85,25 @@ __device__ __forceinline__ uint32_t co_add2(uint32_t a, uint32_t b) { uint32_t d
 __device__ __forceinline__ uint32_t h2(__half2 h) { return *reinterpret_cast<uint32_t *>(&h); }
 __device__ __forceinline__ float co_half(uint32_t h) { return __half2float(__ushort_as_half((unsigned short) h)); }
 
-// An integer below 1024 in the low bits of a half IS a (subnormal) f16 number, the integer times 2^-24: no conversion.  Bits 4 .. 7 hold 16 times
-// a nibble, whose step's activations are a 16th instead.  What the integers are too large by (8, 32, 128; the minima of Q4_K) is
-// one more step over a unit: the sums of x over the blocks times the scales or minima, small integers or f16 numbers themselves.
+// An integer below 1024 in the low bits of a half, under the exponent of 1024, is 1024 + the integer: no conversion.  Bits 4 .. 7 hold 16 times
+// a nibble, whose step's activations are a 16th instead.  What the integers are too large by is subtracted from them, with the 1024, and not from the products: a
+// weight of zero then multiplies by zero.  With the offset taken off afterwards, as the sum of x over the block times the scale, an activation 1e3
+// times the others left an error of 6e-4 (Q4_0) in rows where its weight is zero, one of 1e5 times 9e-2.  The instruction that masks the bits also
+// sets the exponent, and the sums need not be made: 4096 x 12288, us before / now: Q4_0 4 columns 10.1 / 10.3, 8 columns 13.5 / 13.1; Q8_0 8 columns 14.3 / 13.4;
+// Q6_K 1 column 13.3 / 12.4, 4 columns 13.9 / 12.9, 8 columns 17.6 / 17.1.
+// Q4_K, whose minima are part of the weights' values, has unsigned integers as subnormal numbers (they count 2^-24) and one more step over a
+// unit: the sums of x over the blocks times the minima, small integers themselves.  Subnormal numbers in place of the signed ones' 1024: the tensor core's truncation
+// costs more, 2e-7 instead of 1.2e-7 for a column of Q6_K and 4.4e-6 for eight of Q4_0 with an outlier of 3e6.
 constexpr float CO_2_24 = 16777216.0f;
+constexpr uint32_t CO_1024 = 0x64006400u;   // an argument of the launch: with two constants in it, masking and setting would be two instructions
+// (a & MASK) | c in one instruction
+template <uint32_t MASK>
+__device__ __forceinline__ uint32_t co_pick(uint32_t a, uint32_t c) { uint32_t d; asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "n"(MASK), "r"(c)); return d; }
+__device__ __forceinline__ uint32_t co_less1032(uint32_t a) { return co_add2(a, 0xe408e408u); }
+__device__ __forceinline__ uint32_t co_less1152(uint32_t a) { return co_add2(a, 0xe480e480u); }
 
-// B: the activations, per step of 16 weights pairs (0, 2) and (1, 3) of the lane's four, and the sums over the blocks (pairs of
-// blocks 2 t, 2 t + 1 and 2 t + 8, 2 t + 9)
-template <bool P4> struct CoB { uint32_t h[16][2], l[P4 ? 1 : 16][P4 ? 1 : 2]; uint32_t sum_h[2], sum_l[2]; };
+// B: the activations, per step of 16 weights pairs (0, 2) and (1, 3) of the lane's four, and of Q4_K the sums over the blocks (2 t, 2 t + 1)
+template <bool P4> struct CoB { uint32_t h[16][2], l[P4 ? 1 : 16][P4 ? 1 : 2]; uint32_t sum_h, sum_l, k1024; };
 
 template <bool P4>
 __device__ __forceinline__ void co_mul0(float (&acc)[4], const uint32_t (&a)[4], const CoB<P4> & b, int s) {
@@ -110,12 +123,13 @@ __device__ __forceinline__ void co_scale(float (&sum)[4], const float (&acc)[4],
 }
 
 // What a format does: a Cursor holds a lane's addresses of a unit in the row tile that is fetched next, fetch() copies that to a slot (cp.async) and goes
-// `step` tiles on, run() multiplies.  sum += 2^-24 times the products.
+// `step` tiles on, run() multiplies.  sum = 1 / COUNT times the products.
 // Q4_0 and Q8_0: per row the unit's quants and its eight f16 scales
 template <bool Q8>
 struct CoB32 {
     static constexpr int QB = Q8 ? 256 : 128, PITCH = QB + 16, SLOT = 16 * PITCH, SLOTS = Q8 ? 2 : 4, TABLE = 0;
-    static constexpr int BLOCKS = 8;
+    static constexpr bool SUMS = false;
+    static constexpr float COUNT = 1.0f;
     struct Cursor { const uint8_t * q; const uint8_t * d; };
     __device__ static __forceinline__ int k_of(int s) { return 16 * s; }
     __device__ static __forceinline__ bool sixteenth(int s) { return !Q8 && (s & 1); }
@@ -140,15 +154,8 @@ struct CoB32 {
     __device__ static __forceinline__ void run(uint32_t slot, uint32_t, int, int lane, const CoB<P4> & b, float (&sum)[4]) {
         // matrices: rows 0-7, rows 8-15 of one 16-byte piece, then of the next
         const uint32_t at = slot + (lane & 15) * PITCH + (lane >> 4) * 16;
-        {
-            uint32_t d[2];
-            co_ldsm2(d, at + QB);
-            const uint32_t a[4] = {d[0], d[1], 0u, 0u};
-            co_mma0(sum, a, b.sum_h[0], 0u);
-            if constexpr (!P4) co_mma(sum, a, b.sum_l[0], 0u);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) sum[j] *= (Q8 ? -128.0f : -8.0f) * 32.0f / CO_2_24;
-        }
+        for (int j = 0; j < 4; ++j) sum[j] = 0.f;
         const uint4 s0 = co_lds4(slot + (lane >> 2) * PITCH + QB), s1 = co_lds4(slot + (8 + (lane >> 2)) * PITCH + QB);
         const uint32_t d0[4] = {s0.x, s0.y, s0.z, s0.w}, d1[4] = {s1.x, s1.y, s1.z, s1.w};
         auto scale = [&](const float (&acc)[4], int blk) {
@@ -160,17 +167,20 @@ struct CoB32 {
             co_ldsm4(v, at + 32 * i);
             const uint32_t u[4] = {v[0] >> 8, v[1] >> 8, v[2] >> 8, v[3] >> 8};
             float acc[4];
-            if constexpr (Q8) {   // a block: its two pieces; the signed bytes with 128 added
-                const uint32_t a[4] = {(v[0] & 0x00ff00ffu) ^ 0x00800080u, (v[1] & 0x00ff00ffu) ^ 0x00800080u, (u[0] & 0x00ff00ffu) ^ 0x00800080u, (u[1] & 0x00ff00ffu) ^ 0x00800080u};
-                const uint32_t c[4] = {(v[2] & 0x00ff00ffu) ^ 0x00800080u, (v[3] & 0x00ff00ffu) ^ 0x00800080u, (u[2] & 0x00ff00ffu) ^ 0x00800080u, (u[3] & 0x00ff00ffu) ^ 0x00800080u};
+            if constexpr (Q8) {   // a block: its two pieces; the signed bytes, 1024 + 128 added and taken off again
+                const uint32_t k1152 = b.k1024 ^ 0x00800080u;
+                auto sb = [&](uint32_t q) { return co_less1152((q & 0x00ff00ffu) ^ k1152); };
+                const uint32_t a[4] = {sb(v[0]), sb(v[1]), sb(u[0]), sb(u[1])}, c[4] = {sb(v[2]), sb(v[3]), sb(u[2]), sb(u[3])};
                 co_mul0<P4>(acc, a, b, 2 * i);
                 co_mul<P4>(acc, c, b, 2 * i + 1);
                 scale(acc, i);
             } else {              // two blocks of 16 bytes
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const uint32_t a[4] = {v[2 * e] & 0x000f000fu, v[2 * e + 1] & 0x000f000fu, u[2 * e] & 0x000f000fu, u[2 * e + 1] & 0x000f000fu};
-                    const uint32_t c[4] = {v[2 * e] & 0x00f000f0u, v[2 * e + 1] & 0x00f000f0u, u[2 * e] & 0x00f000f0u, u[2 * e + 1] & 0x00f000f0u};
+                    auto lo = [&](uint32_t q) { return co_less1032(co_pick<0x000f000fu>(q, b.k1024)); };
+                    auto hi = [&](uint32_t q) { return co_less1152(co_pick<0x00f000f0u>(q, b.k1024)); };
+                    const uint32_t a[4] = {lo(v[2 * e]), lo(v[2 * e + 1]), lo(u[2 * e]), lo(u[2 * e + 1])};
+                    const uint32_t c[4] = {hi(v[2 * e]), hi(v[2 * e + 1]), hi(u[2 * e]), hi(u[2 * e + 1])};
                     co_mul0<P4>(acc, a, b, 4 * i + 2 * e);
                     co_mul<P4>(acc, c, b, 4 * i + 2 * e + 1);
                     scale(acc, 2 * i + e);
@@ -183,7 +193,8 @@ struct CoB32 {
 // Q4_K: four lane-ordered tiles of 512 bytes, then the rows' headers.  Table: d sc of [16 rows][8 sub-blocks], padded to 12.
 struct CoQ4K {
     static constexpr int SLOT = 4 * 512 + 256, SLOTS = 4, TABLE = 16 * 12 * 4;
-    static constexpr int BLOCKS = 8;
+    static constexpr bool SUMS = true;
+    static constexpr float COUNT = CO_2_24;
     struct Cursor { const uint8_t * q; const uint8_t * h; };
     __device__ static __forceinline__ int k_of(int s) { return 16 * s; }
     __device__ static __forceinline__ bool sixteenth(int s) { return s & 2; }
@@ -214,8 +225,8 @@ struct CoQ4K {
             asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to + 8 * 48), "f"(d1 * (float) (f1 & 63u)), "f"(d1 * (float) ((f1 >> 12) & 63u)) : "memory");
             const uint32_t a[4] = {((f0 >> 6) & 63u) | ((f0 >> 2) & 0x003f0000u), ((f1 >> 6) & 63u) | ((f1 >> 2) & 0x003f0000u), 0u, 0u};
             float acc[4];
-            co_mma0(acc, a, b.sum_h[0], 0u);
-            if constexpr (!P4) co_mma(acc, a, b.sum_l[0], 0u);
+            co_mma0(acc, a, b.sum_h, 0u);
+            if constexpr (!P4) co_mma(acc, a, b.sum_l, 0u);
             sum[0] = m0 * acc[0]; sum[1] = m0 * acc[1]; sum[2] = m1 * acc[2]; sum[3] = m1 * acc[3];
         }
         __syncwarp();
@@ -247,12 +258,11 @@ struct CoQ4K {
 };
 
 // Q6_K: per row 128 bytes of nibbles, 64 of bit pairs, 16 scales; then the words that hold the rows' d.  Table: d sc of
-// [16 rows][16 groups], padded to 20.  SIGNED: the integers less 32, made with a magic exponent and a packed addition or FMA, so that nothing is to be
-// taken off afterwards: 1.2e-7 instead of 2e-7 to 4e-7 of error, for the rows that f32 kernels served before.
-template <bool SIGNED>
+// [16 rows][16 groups], padded to 20.
 struct CoQ6K {
     static constexpr int PITCH = 208, SLOT = 16 * PITCH + 64, SLOTS = 3, TABLE = 16 * 20 * 4;
-    static constexpr int BLOCKS = 16;
+    static constexpr bool SUMS = false;
+    static constexpr float COUNT = 1.0f;
     struct Cursor { const uint8_t * q; const uint8_t * x; const uint8_t * s; const uint8_t * d; };
     __device__ static __forceinline__ int k_of(int s) { return 128 * (s >> 3) + 16 * ((s >> 2) & 1) + 32 * (s & 3); }
     __device__ static __forceinline__ bool sixteenth(int s) { return s & 2; }
@@ -286,25 +296,17 @@ struct CoQ6K {
     __device__ static __forceinline__ void run(uint32_t slot, uint32_t table, int odd, int lane, const CoB<P4> & b, float (&sum)[4]) {
         const int gr = lane >> 2, t = lane & 3;
         const uint32_t at = slot + (lane & 15) * PITCH;   // matrices of rows 0-7 and 8-15
-        {   // lane (g, t): scales 4 t .. 4 t + 3 of rows g and g + 8, for the table and, as f16 integers, times the sums of x
+        {   // lane (g, t): scales 4 t .. 4 t + 3 of rows g and g + 8
             uint32_t v[2];
             co_ldsm2(v, at + 192);
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            const uint32_t a[4] = {co_add2((v[0] & 0x00ff00ffu) ^ 0x64806480u, 0xe480e480u), co_add2((v[1] & 0x00ff00ffu) ^ 0x64806480u, 0xe480e480u),   // 1024 + 128 + sc, - 1152
-                                   co_add2(((v[0] >> 8) & 0x00ff00ffu) ^ 0x64806480u, 0xe480e480u), co_add2(((v[1] >> 8) & 0x00ff00ffu) ^ 0x64806480u, 0xe480e480u)};
-            if constexpr (!SIGNED) {
-                co_mma0(acc, a, b.sum_h[0], b.sum_h[1]);
-                if constexpr (!P4) co_mma(acc, a, b.sum_l[0], b.sum_l[1]);
-            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const float dd = co_half(co_lds(slot + 16 * PITCH + (gr + 8 * h) * 4) >> ((odd >> gr & 1) * 16) & 0xffffu);   // `odd`: bit r = row r's block has an odd number (row r + 8 like row r)
+                const float d = co_half(co_lds(slot + 16 * PITCH + (gr + 8 * h) * 4) >> ((odd >> gr & 1) * 16) & 0xffffu);   // `odd`: bit r = row r's block has an odd number (row r + 8 like row r)
                 const int w = (int) v[h];
-                const float d = SIGNED ? dd * (1.0f / CO_2_24) : dd;
                 co_sts4f(table + (gr + 8 * h) * 80 + t * 16, d * (float) (w << 24 >> 24), d * (float) (w << 16 >> 24), d * (float) (w << 8 >> 24), d * (float) (w >> 24));
-                sum[2 * h] = dd * (-1024.0f / CO_2_24) * acc[2 * h];
-                sum[2 * h + 1] = dd * (-1024.0f / CO_2_24) * acc[2 * h + 1];
             }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum[j] = 0.f;
         }
         __syncwarp();
 #pragma unroll
@@ -317,21 +319,19 @@ struct CoQ6K {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t n0 = n[h], n1 = n[2 + h], m0 = n0 >> 8, m1 = n1 >> 8, y = x[h] >> 8, xa = x[h] << 4, xb = x[h] << 2, ya = y << 4, yb = y << 2;
-                a[0][h] = (n0 & 0x000f000fu) | (xa & 0x00300030u);
-                a[0][2 + h] = (m0 & 0x000f000fu) | (ya & 0x00300030u);
-                a[1][h] = (n1 & 0x000f000fu) | (xb & 0x00300030u);
-                a[1][2 + h] = (m1 & 0x000f000fu) | (yb & 0x00300030u);
-                a[2][h] = (n0 & 0x00f000f0u) | (xa & 0x03000300u);
-                a[2][2 + h] = (m0 & 0x00f000f0u) | (ya & 0x03000300u);
-                a[3][h] = (n1 & 0x00f000f0u) | (xb & 0x03000300u);
-                a[3][2 + h] = (m1 & 0x00f000f0u) | (yb & 0x03000300u);
+                a[0][h] = co_pick<0x000f000fu>(n0, co_pick<0x00300030u>(xa, b.k1024));
+                a[0][2 + h] = co_pick<0x000f000fu>(m0, co_pick<0x00300030u>(ya, b.k1024));
+                a[1][h] = co_pick<0x000f000fu>(n1, co_pick<0x00300030u>(xb, b.k1024));
+                a[1][2 + h] = co_pick<0x000f000fu>(m1, co_pick<0x00300030u>(yb, b.k1024));
+                a[2][h] = co_pick<0x00f000f0u>(n0, co_pick<0x03000300u>(xa, b.k1024));
+                a[2][2 + h] = co_pick<0x00f000f0u>(m0, co_pick<0x03000300u>(ya, b.k1024));
+                a[3][h] = co_pick<0x00f000f0u>(n1, co_pick<0x03000300u>(xb, b.k1024));
+                a[3][2 + h] = co_pick<0x00f000f0u>(m1, co_pick<0x03000300u>(yb, b.k1024));
             }
-            if constexpr (SIGNED) {   // 1024 + q - 1056 as 2^24 times what the sums count in; (1024 + 16 q) - 1536
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < 4; ++j)   // 1024 + q - 1056, 1024 + 16 q - 1536
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) a[j][i] = co_add2(a[j][i] | 0x64006400u, j < 2 ? 0xe420e420u : 0xe600e600u);
-            }
+                for (int i = 0; i < 4; ++i) a[j][i] = co_add2(a[j][i], j < 2 ? 0xe420e420u : 0xe600e600u);
             const float s0[4] = {e0.x, e0.y, e0.z, e0.w}, s1[4] = {e1.x, e1.y, e1.z, e1.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -377,6 +377,7 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
     pdl_wait();
     // ---- activations: lane (g, t) holds column g's weights k_of(s) + 4 t .. + 3 of each step (M <= 4: column g % 4, high parts for g < 4, low parts beyond) ----
     CoB<P4> b;
+    b.k1024 = g.k1024;
     float back[2];   // of the lane's two result columns: 1 / scale
     {
         const int col = P4 ? (lane >> 2) & 3 : lane >> 2;
@@ -399,13 +400,14 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
         back[1] = __shfl_sync(0xffffffffu, inv, P4 ? (8 * t + 4) & 15 : 8 * t + 4);
         const float less = lo_lane ? -1.0f : 0.0f;
         const __half2 z = __float2half2_rn(0.0625f);
-        float sums[F::BLOCKS];
+        float sums[8];
 #pragma unroll
         for (int s = 0; s < 16; ++s) {
             const float f[4] = {v[s].x * scale, v[s].z * scale, v[s].y * scale, v[s].w * scale};
-            const float q = (f[0] + f[1]) + (f[2] + f[3]);
-            constexpr int PER = 16 / F::BLOCKS;
-            sums[s / PER] = s % PER ? sums[s / PER] + q : q;
+            if constexpr (F::SUMS) {
+                const float q = (f[0] + f[1]) + (f[2] + f[3]);
+                sums[s / 2] = s % 2 ? sums[s / 2] + q : q;
+            }
             __half2 h[2] = {__floats2half2_rn(f[0], f[1]), __floats2half2_rn(f[2], f[3])};
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
@@ -420,27 +422,21 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 }
             }
         }
-        // over the lanes that share a block, a 32nd of them.  Lane t holds blocks 2 t and 2 t + 1 of eight; of sixteen 4 t and 4 t + 2, and 4 t + 1 and 4 t + 3
+        if constexpr (F::SUMS) {   // over the lanes that share a block, a 32nd of them; lane t holds blocks 2 t and 2 t + 1
 #pragma unroll
-        for (int i = 0; i < F::BLOCKS; ++i) {
-            sums[i] += __shfl_xor_sync(0xffffffffu, sums[i], 1);
-            sums[i] += __shfl_xor_sync(0xffffffffu, sums[i], 2);
-            sums[i] *= 0.03125f;
-        }
-#pragma unroll
-        for (int i = 0; i < F::BLOCKS / 8; ++i) {
+            for (int i = 0; i < 8; ++i) {
+                sums[i] += __shfl_xor_sync(0xffffffffu, sums[i], 1);
+                sums[i] += __shfl_xor_sync(0xffffffffu, sums[i], 2);
+                sums[i] *= 0.03125f;
+            }
             float a[2];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                constexpr int N = F::BLOCKS / 4;   // blocks of a lane
-                const int o = F::BLOCKS == 8 ? j : 2 * j + i;
-                a[j] = t == 0 ? sums[o] : t == 1 ? sums[N + o] : t == 2 ? sums[2 * N + o] : sums[3 * N + o];
-            }
+            for (int j = 0; j < 2; ++j) a[j] = t == 0 ? sums[j] : t == 1 ? sums[2 + j] : t == 2 ? sums[4 + j] : sums[6 + j];
             const __half2 hh = __floats2half2_rn(a[0], a[1]);
             const float2 r = __half22float2(hh);
             const __half2 ll = __floats2half2_rn(a[0] - r.x, a[1] - r.y);
-            b.sum_h[i] = h2(lo_lane ? ll : hh);
-            if constexpr (!P4) b.sum_l[i] = h2(ll);
+            b.sum_h = h2(lo_lane ? ll : hh);
+            if constexpr (!P4) b.sum_l = h2(ll);
         }
     }
     pdl_launch_dependents();
@@ -468,7 +464,7 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 if (!P4 || t < 2) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 4u * (uint32_t) ((2 * t + (j & 1)) * 16 + (lane >> 2) + 8 * (j >> 1))), "f"(sum[j] * CO_2_24 * back[j & 1]) : "memory");
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + 4u * (uint32_t) ((2 * t + (j & 1)) * 16 + (lane >> 2) + 8 * (j >> 1))), "f"(sum[j] * F::COUNT * back[j & 1]) : "memory");
                 }
             }
             slot = slot + 1 == F::SLOTS ? 0 : slot + 1;
@@ -560,10 +556,10 @@ int launch_cols(cudaStream_t s, const ColsArgs & g) { return g.m <= 4 ? launch_c
 
 }  // namespace
 
-// The full 16-row tiles of a packed tensor, 1..8 columns; `fine`: Q6_K, up to 4 columns, at the error of an f32 kernel.  *handled = false (and ST_OK) for
+// The full 16-row tiles of a packed tensor, 1..8 columns.  *handled = false (and ST_OK) for
 // rows that are not whole units, or longer than four CTAs' units: larger clusters leave too many SMs idle (28672 x 8192, Q6_K, 1 column: 122 us with
 // clusters of 7, the f32 kernel 66).
-int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy, bool fine, bool * handled) {
+int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy, bool * handled) {
     *handled = false;
     if (k % CO_UNIT != 0 || k > CO_MOST_K || n < 16 || n > INT32_MAX - 16 || m < 1 || m > 8) return ST_OK;
     if ((((uintptr_t) x) & 15) != 0 || (m > 1 && ldx % 4 != 0) || (((uintptr_t) w) & 31) != 0) return ST_OK;
@@ -580,12 +576,13 @@ int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64
     g.m = (int) m;
     g.units = (int) (k / CO_UNIT);
     g.tiles = (int) (n / 16);
+    g.k1024 = CO_1024;
     *handled = true;
     switch (dtype) {
         case DT_Q4_0: return launch_cols<CoB32<false>>(s, g);
         case DT_Q8_0: return launch_cols<CoB32<true>>(s, g);
         case DT_Q4_K: return launch_cols<CoQ4K>(s, g);
-        case DT_Q6_K: return fine && m <= 4 ? launch_cols<CoQ6K<true>, true>(s, g) : launch_cols<CoQ6K<false>>(s, g);
+        case DT_Q6_K: return launch_cols<CoQ6K>(s, g);
     }
     *handled = false;
     return ST_OK;

@@ -96,3 +96,29 @@ def test_one_column_of_every_row_that_f32_kernels_served(sm100, stream, k, n):
     got, want = U.device_mul_mat(sm100, stream, U.Q6_K, U.PACKED, wq, k, x), _want(U.Q6_K, wq[:416], k, x)[:, np.arange(n) % 416]
     assert _served(sm100).startswith("quant_cols")
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-7
+
+
+def _zero_columns(dtype, k, n, large):
+    """Packed rows (416, repeated) whose weights `large` are zero: the integer 0 in the three formats without minima."""
+    w = U.seeded_weights(77 + dtype + k, 416, k)
+    w[:, large] = 0.0
+    wq = U.quantize(dtype, w)
+    assert not sgref.dequantize(dtype, wq, k)[:, large].any()
+    return wq, np.ascontiguousarray(np.resize(wq, (n, wq.shape[1])))
+
+
+@pytest.mark.parametrize("ratio", [1e3], ids=lambda v: f"{v:.0e}")
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 1024, 4096, 4), (U.Q4_0, 1024, 4096, 8), (U.Q8_0, 1024, 4096, 4), (U.Q8_0, 1024, 4096, 8),
+                                         (U.Q6_K, 1024, 4096, 3), (U.Q6_K, 1024, 4096, 8), (U.Q4_0, 5120, 6144, 1)], ids=lambda v: str(v))
+def test_large_activations_at_zero_weights(sm100, stream, dtype, k, n, m, ratio):
+    """A weight of zero leaves nothing of its activation, however large that is beside the 255 others of its unit.  No offset is cancelled
+    afterwards: the bound of ordinary inputs."""
+    large = np.arange(7, k, 256)
+    wq, full = _zero_columns(dtype, k, n, large)
+    x = U.seeded_acts(m + k, m, k)
+    x[:, large] = np.float32(ratio) * np.where(np.arange(large.size) % 2, -1.0, 1.0).astype(np.float32)
+    want = _want(dtype, wq, k, x)[:, np.arange(n) % 416]
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, full, k, x)
+    assert _served(sm100).startswith("quant_cols")
+    for t in range(m):
+        assert sgref.nmse(got[t].astype(np.float64), want[t]) <= TOL, (t, sgref.nmse(got[t].astype(np.float64), want[t]))
