@@ -10,7 +10,9 @@
 // ones of Q4_K stand under a zero exponent, subnormal numbers.  A block (32 weights, Q6_K 16) is multiplied into a fresh accumulator, which times the block's
 // scale goes to f32 sums: no weight is scaled or rounded, and the tensor core's truncation sees 32 products at most.
 //
-// Activations: per column and unit one power of two brings the largest to [2^13, 2^14), then x = xh + xl, both f16 (22 bits).
+// Activations: per column and unit one power of two brings the largest to [2^13, 2^14), then x = xh + 2^-11 xl, both f16: 22 bits, and because the low part is
+// scaled up they are there down to 2^-35 of the largest (2^-31 for half of Q4_0's).  Not with M > 4 of Q4_K, 2^-24 there: it replaces kernels of 16-bit
+// integers to the largest of 64 and would lose 0.4 us of 7.1 (4096 x 4096, 8 columns).
 //   M <= 4: the eight columns of an MMA are xh and xl of four tokens; M <= 8: two MMAs, xh and xl of eight
 // Error against float64: 2e-7 to 1.3e-6 (the integer column kernels 2e-5 to 6e-5, the split GEMM 5e-6, the f32 matvec of the vocabulary head 9e-7).
 //
@@ -105,6 +107,37 @@ __device__ __forceinline__ uint32_t co_less1152(uint32_t a) { return co_add2(a, 
 // B: the activations, per step of 16 weights pairs (0, 2) and (1, 3) of the lane's four, and of Q4_K the sums over the blocks (2 t, 2 t + 1)
 template <bool P4> struct CoB { uint32_t h[16][2], l[P4 ? 1 : 16][P4 ? 1 : 2]; uint32_t sum_h, sum_l, k1024; };
 
+// What the low parts are multiplied by: as they are, the low part of an activation 2^-14 of the largest would be a subnormal number, with fewer bits (an activation
+// 1e7 times the others left 2e-4 of them).  4096 x 12288, us before / now: Q8_0 4 columns 12.1 / 12.3, 8 columns 13.4 / 14.1; Q6_K 4 columns 12.9 / 13.4, 8 columns 17.1 / 17.7.
+constexpr float CO_LOW = 2048.0f;
+
+// acc = the products of a step; of two.  M <= 8: the low parts' come first, since the accumulator then is divided by what they are multiplied by (four
+// multiplications; two accumulators would not leave enough registers).  M <= 4: the low parts have columns of their own.
+template <bool P4>
+__device__ __forceinline__ void co_block(float (&acc)[4], const uint32_t (&a)[4], const CoB<P4> & b, int s) {
+    if constexpr (P4) {
+        co_mma0(acc, a, b.h[s][0], b.h[s][1]);
+    } else {
+        co_mma0(acc, a, b.l[s][0], b.l[s][1]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] *= 1.0f / CO_LOW;
+        co_mma(acc, a, b.h[s][0], b.h[s][1]);
+    }
+}
+template <bool P4>
+__device__ __forceinline__ void co_block2(float (&acc)[4], const uint32_t (&a)[4], const uint32_t (&c)[4], const CoB<P4> & b, int s) {
+    if constexpr (P4) {
+        co_mma0(acc, a, b.h[s][0], b.h[s][1]);
+    } else {
+        co_mma0(acc, a, b.l[s][0], b.l[s][1]);
+        co_mma(acc, c, b.l[s + 1][0], b.l[s + 1][1]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] *= 1.0f / CO_LOW;
+        co_mma(acc, a, b.h[s][0], b.h[s][1]);
+    }
+    co_mma(acc, c, b.h[s + 1][0], b.h[s + 1][1]);
+}
+// Q4_K, whose low parts are as they are with eight columns
 template <bool P4>
 __device__ __forceinline__ void co_mul0(float (&acc)[4], const uint32_t (&a)[4], const CoB<P4> & b, int s) {
     co_mma0(acc, a, b.h[s][0], b.h[s][1]);
@@ -128,7 +161,7 @@ __device__ __forceinline__ void co_scale(float (&sum)[4], const float (&acc)[4],
 template <bool Q8>
 struct CoB32 {
     static constexpr int QB = Q8 ? 256 : 128, PITCH = QB + 16, SLOT = 16 * PITCH, SLOTS = Q8 ? 2 : 4, TABLE = 0;
-    static constexpr bool SUMS = false;
+    static constexpr bool SUMS = false, SCALED = true;
     static constexpr float COUNT = 1.0f;
     struct Cursor { const uint8_t * q; const uint8_t * d; };
     __device__ static __forceinline__ int k_of(int s) { return 16 * s; }
@@ -171,8 +204,7 @@ struct CoB32 {
                 const uint32_t k1152 = b.k1024 ^ 0x00800080u;
                 auto sb = [&](uint32_t q) { return co_less1152((q & 0x00ff00ffu) ^ k1152); };
                 const uint32_t a[4] = {sb(v[0]), sb(v[1]), sb(u[0]), sb(u[1])}, c[4] = {sb(v[2]), sb(v[3]), sb(u[2]), sb(u[3])};
-                co_mul0<P4>(acc, a, b, 2 * i);
-                co_mul<P4>(acc, c, b, 2 * i + 1);
+                co_block2<P4>(acc, a, c, b, 2 * i);
                 scale(acc, i);
             } else {              // two blocks of 16 bytes
 #pragma unroll
@@ -181,8 +213,7 @@ struct CoB32 {
                     auto hi = [&](uint32_t q) { return co_less1152(co_pick<0x00f000f0u>(q, b.k1024)); };
                     const uint32_t a[4] = {lo(v[2 * e]), lo(v[2 * e + 1]), lo(u[2 * e]), lo(u[2 * e + 1])};
                     const uint32_t c[4] = {hi(v[2 * e]), hi(v[2 * e + 1]), hi(u[2 * e]), hi(u[2 * e + 1])};
-                    co_mul0<P4>(acc, a, b, 4 * i + 2 * e);
-                    co_mul<P4>(acc, c, b, 4 * i + 2 * e + 1);
+                    co_block2<P4>(acc, a, c, b, 4 * i + 2 * e);
                     scale(acc, 2 * i + e);
                 }
             }
@@ -190,14 +221,15 @@ struct CoB32 {
     }
 };
 
-// Q4_K: four lane-ordered tiles of 512 bytes, then the rows' headers.  Table: d sc of [16 rows][8 sub-blocks], padded to 12.
+// Q4_K: four lane-ordered tiles of 512 bytes, then the rows' headers.  Table: d sc of [16 rows][8 sub-blocks], padded to 12; of the odd ones,
+// whose nibbles count 16, a 16th.
 struct CoQ4K {
     static constexpr int SLOT = 4 * 512 + 256, SLOTS = 4, TABLE = 16 * 12 * 4;
-    static constexpr bool SUMS = true;
+    static constexpr bool SUMS = true, SCALED = false;
     static constexpr float COUNT = CO_2_24;
     struct Cursor { const uint8_t * q; const uint8_t * h; };
     __device__ static __forceinline__ int k_of(int s) { return 16 * s; }
-    __device__ static __forceinline__ bool sixteenth(int s) { return s & 2; }
+    __device__ static __forceinline__ bool sixteenth(int) { return false; }
     __device__ static __forceinline__ void init(Cursor & c, const ColsArgs & g, int rt, int unit, int lane) {
         c.q = g.w + ((int64_t) rt * g.units + unit) * 2048 + lane * 16;
         c.h = g.w + g.off1 + (((int64_t) rt * 16 + (lane & 15)) * g.units + unit) * 16;
@@ -221,8 +253,8 @@ struct CoQ4K {
             const uint32_t h0 = slot + 2048 + gr * 16, h1 = h0 + 128, f0 = field(h0, t), f1 = field(h1, t), w0 = co_lds(h0), w1 = co_lds(h1);
             const float d0 = co_half(w0 & 0xffffu), d1 = co_half(w1 & 0xffffu), m0 = -32.0f * co_half(w0 >> 16), m1 = -32.0f * co_half(w1 >> 16);
             const uint32_t to = table + gr * 48 + t * 8;
-            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(d0 * (float) (f0 & 63u)), "f"(d0 * (float) ((f0 >> 12) & 63u)) : "memory");
-            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to + 8 * 48), "f"(d1 * (float) (f1 & 63u)), "f"(d1 * (float) ((f1 >> 12) & 63u)) : "memory");
+            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to), "f"(d0 * (float) (f0 & 63u)), "f"(d0 * 0.0625f * (float) ((f0 >> 12) & 63u)) : "memory");
+            asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to + 8 * 48), "f"(d1 * (float) (f1 & 63u)), "f"(d1 * 0.0625f * (float) ((f1 >> 12) & 63u)) : "memory");
             const uint32_t a[4] = {((f0 >> 6) & 63u) | ((f0 >> 2) & 0x003f0000u), ((f1 >> 6) & 63u) | ((f1 >> 2) & 0x003f0000u), 0u, 0u};
             float acc[4];
             co_mma0(acc, a, b.sum_h, 0u);
@@ -258,14 +290,14 @@ struct CoQ4K {
 };
 
 // Q6_K: per row 128 bytes of nibbles, 64 of bit pairs, 16 scales; then the words that hold the rows' d.  Table: d sc of
-// [16 rows][16 groups], padded to 20.
+// [16 rows][16 groups], padded to 20; of every third and fourth group, whose integers count 16, a 16th.
 struct CoQ6K {
     static constexpr int PITCH = 208, SLOT = 16 * PITCH + 64, SLOTS = 3, TABLE = 16 * 20 * 4;
-    static constexpr bool SUMS = false;
+    static constexpr bool SUMS = false, SCALED = true;
     static constexpr float COUNT = 1.0f;
     struct Cursor { const uint8_t * q; const uint8_t * x; const uint8_t * s; const uint8_t * d; };
     __device__ static __forceinline__ int k_of(int s) { return 128 * (s >> 3) + 16 * ((s >> 2) & 1) + 32 * (s & 3); }
-    __device__ static __forceinline__ bool sixteenth(int s) { return s & 2; }
+    __device__ static __forceinline__ bool sixteenth(int) { return false; }
     __device__ static __forceinline__ void init(Cursor & c, const ColsArgs & g, int rt, int unit, int lane) {
         const int64_t row0 = (int64_t) rt * 16, blk = (row0 + (lane & 15)) * g.units + unit;
         c.q = g.w + ((row0 + (lane >> 3)) * g.units + unit) * 128 + (lane & 7) * 16;
@@ -303,7 +335,8 @@ struct CoQ6K {
             for (int h = 0; h < 2; ++h) {
                 const float d = co_half(co_lds(slot + 16 * PITCH + (gr + 8 * h) * 4) >> ((odd >> gr & 1) * 16) & 0xffffu);   // `odd`: bit r = row r's block has an odd number (row r + 8 like row r)
                 const int w = (int) v[h];
-                co_sts4f(table + (gr + 8 * h) * 80 + t * 16, d * (float) (w << 24 >> 24), d * (float) (w << 16 >> 24), d * (float) (w << 8 >> 24), d * (float) (w >> 24));
+                const float d16 = d * 0.0625f;
+                co_sts4f(table + (gr + 8 * h) * 80 + t * 16, d * (float) (w << 24 >> 24), d * (float) (w << 16 >> 24), d16 * (float) (w << 8 >> 24), d16 * (float) (w >> 24));
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) sum[j] = 0.f;
@@ -336,7 +369,7 @@ struct CoQ6K {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 float acc[4];
-                co_mul0<P4>(acc, a[j], b, 4 * c + j);
+                co_block<P4>(acc, a[j], b, 4 * c + j);
                 co_scale(sum, acc, s0[j], s1[j]);
             }
         }
@@ -398,28 +431,37 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
         const float scale = __int_as_float((127 + sh) << 23), inv = __int_as_float((127 - sh) << 23);
         back[0] = __shfl_sync(0xffffffffu, inv, P4 ? (8 * t) & 15 : 8 * t);
         back[1] = __shfl_sync(0xffffffffu, inv, P4 ? (8 * t + 4) & 15 : 8 * t + 4);
-        const float less = lo_lane ? -1.0f : 0.0f;
-        const __half2 z = __float2half2_rn(0.0625f);
+        constexpr bool SCALED = P4 || F::SCALED;
+        // f, or what it is less its high part, scaled.  Two numbers an instruction (Q4_0 4096 x 12288, 4 columns: 10.5 us with one, 10.3)
+        const float2 up = lo_lane || !P4 ? make_float2(CO_LOW, CO_LOW) : make_float2(1.f, 1.f), less = lo_lane || !P4 ? make_float2(-CO_LOW, -CO_LOW) : make_float2(0.f, 0.f);
         float sums[8];
 #pragma unroll
         for (int s = 0; s < 16; ++s) {
-            const float f[4] = {v[s].x * scale, v[s].z * scale, v[s].y * scale, v[s].w * scale};
+            const float sc = F::sixteenth(s) ? scale * 0.0625f : scale;
+            const float2 f0 = __fmul2_rn(make_float2(v[s].x, v[s].y), make_float2(sc, sc)), f1 = __fmul2_rn(make_float2(v[s].z, v[s].w), make_float2(sc, sc));
             if constexpr (F::SUMS) {
-                const float q = (f[0] + f[1]) + (f[2] + f[3]);
+                const float q = (f0.x + f1.x) + (f0.y + f1.y);
                 sums[s / 2] = s % 2 ? sums[s / 2] + q : q;
             }
-            __half2 h[2] = {__floats2half2_rn(f[0], f[1]), __floats2half2_rn(f[2], f[3])};
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float2 r = __half22float2(h[i]);
-                if constexpr (P4) {   // f - 0 r or f - r
-                    __half2 u = __floats2half2_rn(fmaf(less, r.x, f[2 * i]), fmaf(less, r.y, f[2 * i + 1]));
-                    b.h[s][i] = h2(F::sixteenth(s) ? __hmul2(u, z) : u);
-                } else {
-                    const __half2 l = __floats2half2_rn(f[2 * i] - r.x, f[2 * i + 1] - r.y);
-                    b.h[s][i] = h2(F::sixteenth(s) ? __hmul2(h[i], z) : h[i]);
-                    b.l[s][i] = h2(F::sixteenth(s) ? __hmul2(l, z) : l);
-                }
+            const __half2 hx = __floats2half2_rn(f0.x, f1.x), hy = __floats2half2_rn(f0.y, f1.y);   // pairs (0, 2) and (1, 3)
+            const float2 rx = __half22float2(hx), ry = __half22float2(hy);
+            float2 u0, u1;
+            if constexpr (SCALED) {
+                u0 = __ffma2_rn(make_float2(rx.x, ry.x), less, __fmul2_rn(f0, up));
+                u1 = __ffma2_rn(make_float2(rx.y, ry.y), less, __fmul2_rn(f1, up));
+            } else {
+                u0 = __ffma2_rn(make_float2(rx.x, ry.x), make_float2(-1.f, -1.f), f0);
+                u1 = __ffma2_rn(make_float2(rx.y, ry.y), make_float2(-1.f, -1.f), f1);
+            }
+            const uint32_t ux = h2(__floats2half2_rn(u0.x, u1.x)), uy = h2(__floats2half2_rn(u0.y, u1.y));
+            if constexpr (P4) {
+                b.h[s][0] = ux;
+                b.h[s][1] = uy;
+            } else {
+                b.h[s][0] = h2(hx);
+                b.h[s][1] = h2(hy);
+                b.l[s][0] = ux;
+                b.l[s][1] = uy;
             }
         }
         if constexpr (F::SUMS) {   // over the lanes that share a block, a 32nd of them; lane t holds blocks 2 t and 2 t + 1
@@ -434,7 +476,7 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
             for (int j = 0; j < 2; ++j) a[j] = t == 0 ? sums[j] : t == 1 ? sums[2 + j] : t == 2 ? sums[4 + j] : sums[6 + j];
             const __half2 hh = __floats2half2_rn(a[0], a[1]);
             const float2 r = __half22float2(hh);
-            const __half2 ll = __floats2half2_rn(a[0] - r.x, a[1] - r.y);
+            const __half2 ll = __floats2half2_rn((a[0] - r.x) * (SCALED ? CO_LOW : 1.0f), (a[1] - r.y) * (SCALED ? CO_LOW : 1.0f));
             b.sum_h = h2(lo_lane ? ll : hh);
             if constexpr (!P4) b.sum_l = h2(ll);
         }
@@ -459,7 +501,7 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 const uint32_t at = red0 + parity * red_bytes + 4u * (uint32_t) ((((i - i0) << g.wr_log) + rg) * g.wk + kp) * TILE;
                 if constexpr (P4) {   // high and low parts' products: columns j and j + 4 (lanes t and t + 2)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], 2);
+                    for (int j = 0; j < 4; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], 2) * (1.0f / CO_LOW);
                 }
                 if (!P4 || t < 2) {
 #pragma unroll

@@ -107,12 +107,12 @@ def _zero_columns(dtype, k, n, large):
     return wq, np.ascontiguousarray(np.resize(wq, (n, wq.shape[1])))
 
 
-@pytest.mark.parametrize("ratio", [1e3], ids=lambda v: f"{v:.0e}")
+@pytest.mark.parametrize("ratio", [1e3, 1e5, 1e7], ids=lambda v: f"{v:.0e}")
 @pytest.mark.parametrize("dtype,k,n,m", [(U.Q4_0, 1024, 4096, 4), (U.Q4_0, 1024, 4096, 8), (U.Q8_0, 1024, 4096, 4), (U.Q8_0, 1024, 4096, 8),
                                          (U.Q6_K, 1024, 4096, 3), (U.Q6_K, 1024, 4096, 8), (U.Q4_0, 5120, 6144, 1)], ids=lambda v: str(v))
 def test_large_activations_at_zero_weights(sm100, stream, dtype, k, n, m, ratio):
-    """A weight of zero leaves nothing of its activation, however large that is beside the 255 others of its unit.  No offset is cancelled
-    afterwards: the bound of ordinary inputs."""
+    """A weight of zero leaves nothing of its activation, however large that is beside the 255 others of its unit.  The others then have 22 bits and
+    no cancelled offsets: the bound of ordinary inputs."""
     large = np.arange(7, k, 256)
     wq, full = _zero_columns(dtype, k, n, large)
     x = U.seeded_acts(m + k, m, k)
