@@ -12,7 +12,9 @@
 //
 // Activations: per column and unit one power of two brings the largest to [2^13, 2^14), then x = xh + 2^-11 xl, both f16: 22 bits, and because the low part is
 // scaled up they are there down to 2^-35 of the largest (2^-31 for half of Q4_0's).  Not with M > 4 of Q4_K, 2^-24 there: it replaces kernels of 16-bit
-// integers to the largest of 64 and would lose 0.4 us of 7.1 (4096 x 4096, 8 columns).
+// integers to the largest of 64 and would lose 0.4 us of 7.1 (4096 x 4096, 8 columns).  FINE: a third part likewise, which makes it the 24 bits of
+// an f32 number down to 2^-37 of the largest, for the single columns of Q6_K that f32 kernels would serve otherwise (7168 x 8192: 15.9 us with two parts, 16.8 with three).
+//   FINE    xh, xl and the third part of one token in three columns
 //   M <= 4: the eight columns of an MMA are xh and xl of four tokens; M <= 8: two MMAs, xh and xl of eight
 // Error against float64: 2e-7 to 1.3e-6 (the integer column kernels 2e-5 to 6e-5, the split GEMM 5e-6, the f32 matvec of the vocabulary head 9e-7).
 //
@@ -160,6 +162,7 @@ __device__ __forceinline__ void co_scale(float (&sum)[4], const float (&acc)[4],
 // Q4_0 and Q8_0: per row the unit's quants and its eight f16 scales
 template <bool Q8>
 struct CoB32 {
+    static constexpr bool FINE = false;
     static constexpr int QB = Q8 ? 256 : 128, PITCH = QB + 16, SLOT = 16 * PITCH, SLOTS = Q8 ? 2 : 4, TABLE = 0;
     static constexpr bool SUMS = false, SCALED = true;
     static constexpr float COUNT = 1.0f;
@@ -224,6 +227,7 @@ struct CoB32 {
 // Q4_K: four lane-ordered tiles of 512 bytes, then the rows' headers.  Table: d sc of [16 rows][8 sub-blocks], padded to 12; of the odd ones,
 // whose nibbles count 16, a 16th.
 struct CoQ4K {
+    static constexpr bool FINE = false;
     static constexpr int SLOT = 4 * 512 + 256, SLOTS = 4, TABLE = 16 * 12 * 4;
     static constexpr bool SUMS = true, SCALED = false;
     static constexpr float COUNT = CO_2_24;
@@ -291,7 +295,9 @@ struct CoQ4K {
 
 // Q6_K: per row 128 bytes of nibbles, 64 of bit pairs, 16 scales; then the words that hold the rows' d.  Table: d sc of
 // [16 rows][16 groups], padded to 20; of every third and fourth group, whose integers count 16, a 16th.
+template <bool F32>
 struct CoQ6K {
+    static constexpr bool FINE = F32;
     static constexpr int PITCH = 208, SLOT = 16 * PITCH + 64, SLOTS = 3, TABLE = 16 * 20 * 4;
     static constexpr bool SUMS = false, SCALED = true;
     static constexpr float COUNT = 1.0f;
@@ -428,12 +434,16 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
         const int e = __float_as_int(top) >> 23;
         int sh = e == 0 || e == 255 ? 0 : 13 + 127 - e;
         sh = sh > 126 ? 126 : sh;   // >= 13 - 127
-        const float scale = __int_as_float((127 + sh) << 23), inv = __int_as_float((127 - sh) << 23);
+        // FINE: the columns that nobody reads are zero, the fewer bits toggle
+        const float scale = F::FINE && ((lane >> 2) & 3) > (lo_lane ? 0 : 1) ? 0.f : __int_as_float((127 + sh) << 23), inv = __int_as_float((127 - sh) << 23);
         back[0] = __shfl_sync(0xffffffffu, inv, P4 ? (8 * t) & 15 : 8 * t);
         back[1] = __shfl_sync(0xffffffffu, inv, P4 ? (8 * t + 4) & 15 : 8 * t + 4);
         constexpr bool SCALED = P4 || F::SCALED;
         // f, or what it is less its high part, scaled.  Two numbers an instruction (Q4_0 4096 x 12288, 4 columns: 10.5 us with one, 10.3)
-        const float2 up = lo_lane || !P4 ? make_float2(CO_LOW, CO_LOW) : make_float2(1.f, 1.f), less = lo_lane || !P4 ? make_float2(-CO_LOW, -CO_LOW) : make_float2(0.f, 0.f);
+        // FINE: lanes 0..3 hold the first part, 16..19 the second, 4..7 the third, which takes another step.
+        const bool third = F::FINE && (lane >> 2) == 1, low = lo_lane || third || !P4;
+        const float2 up3 = third ? make_float2(CO_LOW, CO_LOW) : make_float2(1.f, 1.f), less3 = third ? make_float2(-CO_LOW, -CO_LOW) : make_float2(0.f, 0.f);
+        const float2 up = low ? make_float2(CO_LOW, CO_LOW) : make_float2(1.f, 1.f), less = low ? make_float2(-CO_LOW, -CO_LOW) : make_float2(0.f, 0.f);
         float sums[8];
 #pragma unroll
         for (int s = 0; s < 16; ++s) {
@@ -452,6 +462,11 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
             } else {
                 u0 = __ffma2_rn(make_float2(rx.x, ry.x), make_float2(-1.f, -1.f), f0);
                 u1 = __ffma2_rn(make_float2(rx.y, ry.y), make_float2(-1.f, -1.f), f1);
+            }
+            if constexpr (F::FINE) {
+                const float2 qx = __half22float2(__floats2half2_rn(u0.x, u1.x)), qy = __half22float2(__floats2half2_rn(u0.y, u1.y));
+                u0 = __ffma2_rn(make_float2(qx.x, qy.x), less3, __fmul2_rn(u0, up3));
+                u1 = __ffma2_rn(make_float2(qx.y, qy.y), less3, __fmul2_rn(u1, up3));
             }
             const uint32_t ux = h2(__floats2half2_rn(u0.x, u1.x)), uy = h2(__floats2half2_rn(u0.y, u1.y));
             if constexpr (P4) {
@@ -502,6 +517,10 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 if constexpr (P4) {   // high and low parts' products: columns j and j + 4 (lanes t and t + 2)
 #pragma unroll
                     for (int j = 0; j < 4; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], 2) * (1.0f / CO_LOW);
+                }
+                if constexpr (F::FINE) {   // the third part's products: column 1
+                    sum[0] = fmaf(sum[1], 1.0f / (CO_LOW * CO_LOW), sum[0]);
+                    sum[2] = fmaf(sum[3], 1.0f / (CO_LOW * CO_LOW), sum[2]);
                 }
                 if (!P4 || t < 2) {
 #pragma unroll
@@ -598,10 +617,10 @@ int launch_cols(cudaStream_t s, const ColsArgs & g) { return g.m <= 4 ? launch_c
 
 }  // namespace
 
-// The full 16-row tiles of a packed tensor, 1..8 columns.  *handled = false (and ST_OK) for
+// The full 16-row tiles of a packed tensor, 1..8 columns; `fine`: one column of Q6_K with the 24 bits of its activations.  *handled = false (and ST_OK) for
 // rows that are not whole units, or longer than four CTAs' units: larger clusters leave too many SMs idle (28672 x 8192, Q6_K, 1 column: 122 us with
 // clusters of 7, the f32 kernel 66).
-int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy, bool * handled) {
+int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy, bool fine, bool * handled) {
     *handled = false;
     if (k % CO_UNIT != 0 || k > CO_MOST_K || n < 16 || n > INT32_MAX - 16 || m < 1 || m > 8) return ST_OK;
     if ((((uintptr_t) x) & 15) != 0 || (m > 1 && ldx % 4 != 0) || (((uintptr_t) w) & 31) != 0) return ST_OK;
@@ -624,7 +643,7 @@ int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64
         case DT_Q4_0: return launch_cols<CoB32<false>>(s, g);
         case DT_Q8_0: return launch_cols<CoB32<true>>(s, g);
         case DT_Q4_K: return launch_cols<CoQ4K>(s, g);
-        case DT_Q6_K: return launch_cols<CoQ6K>(s, g);
+        case DT_Q6_K: return fine && m == 1 ? launch_cols<CoQ6K<true>, true>(s, g) : launch_cols<CoQ6K<false>>(s, g);
     }
     *handled = false;
     return ST_OK;

@@ -36,7 +36,7 @@ bool b32_imma_serves(int64_t k);
 bool q6k_imma_serves(int64_t k);
 int q4k_pass_width(int64_t k, int64_t m);
 int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
-                     bool * handled);
+                     bool fine, bool * handled);
 int gemm_split_mul_mat(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy,
                        bool * handled);
 int matvec_q4k_ring_multi(cudaStream_t s, int count, const void * const * ws, const int64_t * ns, int64_t k, const float * x,
@@ -634,8 +634,9 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
     // the batches that the split GEMM serves (further down)
     const bool split_wins = dtype == DT_Q6_K ? m == 3 || m >= 5 : (dtype == DT_Q4_0 || dtype == DT_Q8_0) && m >= 4;
     if (layout == LAYOUT_PACKED && x_aligned && cols_win(dtype, k, n, m, split_wins)) {
+        const bool fine = dtype == DT_Q6_K && m == 1 && n * k > q6k_imma_limit(k);   // f32 kernels' precision where they served
         bool handled = false;
-        const int st = quant_cols_tiles(s, dtype, w, k, n, x, ldx, m, y, ldy, &handled);
+        const int st = quant_cols_tiles(s, dtype, w, k, n, x, ldx, m, y, ldy, fine, &handled);
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = n / 16 * 16;

@@ -122,3 +122,17 @@ def test_large_activations_at_zero_weights(sm100, stream, dtype, k, n, m, ratio)
     assert _served(sm100).startswith("quant_cols")
     for t in range(m):
         assert sgref.nmse(got[t].astype(np.float64), want[t]) <= TOL, (t, sgref.nmse(got[t].astype(np.float64), want[t]))
+
+
+@pytest.mark.parametrize("ratio", [1e4, 1e6, 1e7, 1e9], ids=lambda v: f"{v:.0e}")
+@pytest.mark.parametrize("k,n", [(5120, 5120), (8192, 5120)])
+def test_one_column_keeps_24_bits_beside_large_activations(sm100, stream, k, n, ratio):
+    """f32 kernels served these rows: 24 bits of each activation whatever stands beside it, the bound of ordinary inputs."""
+    large = np.arange(7, k, 256)
+    wq, full = _zero_columns(U.Q6_K, k, n, large)
+    x = U.seeded_acts(3, 1, k)
+    x[:, large] = np.float32(ratio)
+    want = _want(U.Q6_K, wq, k, x)[:, np.arange(n) % 416]
+    got = U.device_mul_mat(sm100, stream, U.Q6_K, U.PACKED, full, k, x)
+    assert _served(sm100).startswith("quant_cols")
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-7
