@@ -430,6 +430,18 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
         for (int s = 0; s < 16; ++s) top = fmaxf(fmaxf(fmaxf(top, fabsf(v[s].x)), fmaxf(fabsf(v[s].y), fabsf(v[s].z))), fabsf(v[s].w));
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        bool infinite = false;
+        if constexpr (F::FINE) {   // as f32 gives it: an infinity times its weight.  It is left out of the scale and of the lower parts; every lane has the same column
+            infinite = top == INFINITY;
+            if (infinite) {
+                auto finite = [](float & f) { f = fabsf(f) == INFINITY ? 0.f : f; return fabsf(f); };
+                top = 0.f;
+#pragma unroll
+                for (int s = 0; s < 16; ++s) top = fmaxf(fmaxf(fmaxf(top, finite(v[s].x)), fmaxf(finite(v[s].y), finite(v[s].z))), finite(v[s].w));
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+            }
+        }
         // the largest to [2^13, 2^14); zeros and infinities as they are
         const int e = __float_as_int(top) >> 23;
         int sh = e == 0 || e == 255 ? 0 : 13 + 127 - e;
@@ -477,6 +489,20 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 b.h[s][1] = h2(hy);
                 b.l[s][0] = ux;
                 b.l[s][1] = uy;
+            }
+        }
+        if constexpr (F::FINE) {
+            if (infinite && lane < 4) {
+                auto put = [](uint32_t & h, float a, float c) {
+                    if (fabsf(a) == INFINITY) h = (h & 0xffff0000u) | (a > 0.f ? 0x7c00u : 0xfc00u);
+                    if (fabsf(c) == INFINITY) h = (h & 0x0000ffffu) | (c > 0.f ? 0x7c000000u : 0xfc000000u);
+                };
+#pragma unroll
+                for (int s = 0; s < 16; ++s) {
+                    const float4 f = __ldcg(reinterpret_cast<const float4 *>(src + F::k_of(s)));
+                    put(b.h[s][0], f.x, f.z);
+                    put(b.h[s][1], f.y, f.w);
+                }
             }
         }
         if constexpr (F::SUMS) {   // over the lanes that share a block, a 32nd of them; lane t holds blocks 2 t and 2 t + 1

@@ -136,3 +136,25 @@ def test_one_column_keeps_24_bits_beside_large_activations(sm100, stream, k, n, 
     got = U.device_mul_mat(sm100, stream, U.Q6_K, U.PACKED, full, k, x)
     assert _served(sm100).startswith("quant_cols")
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-7
+
+
+@pytest.mark.parametrize("k,n", [(5120, 5120), (8192, 5120)])
+@pytest.mark.parametrize("where", [[5], [5, 300], [4095, 4900]], ids=str)
+def test_one_column_infinities(sm100, stream, k, n, where):
+    """What f32 kernels make of an infinite activation: an infinity of the product's sign, NaN where the weight is zero or infinities cancel; finite
+    activations of any size beside it in the same unit do not show."""
+    large = np.array([64, 400])
+    wq, full = _zero_columns(U.Q6_K, k, n, large)
+    x = U.seeded_acts(4, 1, k)
+    x[0, 9], x[0, 310], x[0, 4097] = 1e30, -1e30, 1e-30
+    for i, j in enumerate(where):
+        x[0, j] = np.inf if i == 0 else -np.inf
+    with np.errstate(invalid="ignore"):
+        w = sgref.dequantize(U.Q6_K, wq, k).astype(np.float64)
+        want = np.zeros(len(w)) + sum(w[:, j] * float(x[0, j]) for j in where)   # finite terms do not change an infinity or a NaN
+    got = U.device_mul_mat(sm100, stream, U.Q6_K, U.PACKED, full, k, x)[0]
+    assert _served(sm100).startswith("quant_cols")
+    assert np.array_equal(got[:416], want.astype(np.float32), equal_nan=True)
+    assert np.array_equal(got, got[np.arange(n) % 416], equal_nan=True)
+    if len(where) == 1:
+        assert np.isinf(got).any()
