@@ -442,9 +442,9 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
             }
         }
-        // the largest to [2^13, 2^14); zeros and infinities as they are
+        // the largest to [2^13, 2^14), subnormal numbers as far as 2^126 brings them; infinities as they are
         const int e = __float_as_int(top) >> 23;
-        int sh = e == 0 || e == 255 ? 0 : 13 + 127 - e;
+        int sh = e == 255 ? 0 : 13 + 127 - e;
         sh = sh > 126 ? 126 : sh;   // >= 13 - 127
         // FINE: the columns that nobody reads are zero, the fewer bits toggle
         const float scale = F::FINE && ((lane >> 2) & 3) > (lo_lane ? 0 : 1) ? 0.f : __int_as_float((127 + sh) << 23), inv = __int_as_float((127 - sh) << 23);

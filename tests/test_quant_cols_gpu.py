@@ -158,3 +158,18 @@ def test_one_column_infinities(sm100, stream, k, n, where):
     assert np.array_equal(got, got[np.arange(n) % 416], equal_nan=True)
     if len(where) == 1:
         assert np.isinf(got).any()
+
+
+@pytest.mark.parametrize("exponent", [-120, -127, -135])
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q6_K, 5120, 5120, 1), (U.Q6_K, 1024, 4096, 3), (U.Q4_0, 1024, 4096, 8), (U.Q8_0, 1024, 4096, 2)], ids=lambda v: str(v))
+def test_columns_of_subnormal_numbers(sm100, stream, dtype, k, n, m, exponent):
+    """Activations that are subnormal numbers count like others; block scales of 2^10 keep the results normal, so the bound is that of their own bits: one
+    rounding of each input to 2^-149 is in the inputs already."""
+    wq = U.quantize(dtype, U.seeded_weights(8, 416, k) * np.float32(2.0 ** 14))
+    full = np.ascontiguousarray(np.resize(wq, (n, wq.shape[1])))
+    x = (U.seeded_acts(9, m, k).astype(np.float64) * 2.0 ** exponent).astype(np.float32)
+    want = _want(dtype, wq, k, x)[:, np.arange(n) % 416] * 2.0 ** -exponent
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, full, k, x).astype(np.float64) * 2.0 ** -exponent
+    assert _served(sm100).startswith("quant_cols")
+    for t in range(m):
+        assert sgref.nmse(got[t], want[t]) <= TOL, (t, sgref.nmse(got[t], want[t]))
