@@ -633,7 +633,10 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
     if (is_quant(dtype) && !x_aligned) return fail(ST_UNSUPPORTED, "mul_mat: activations must be 16-byte aligned (columns too)");
     // the batches that the split GEMM serves (further down)
     const bool split_wins = dtype == DT_Q6_K ? m == 3 || m >= 5 : (dtype == DT_Q4_0 || dtype == DT_Q8_0) && m >= 4;
-    if (layout == LAYOUT_PACKED && x_aligned && cols_win(dtype, k, n, m, split_wins)) {
+    static const int use_imma = env_int("SM100_Q4K_IMMA", 1), use_b32 = env_int("SM100_B32_IMMA", 1), use_q6k = env_int("SM100_Q6K_IMMA", 1), use_cols = env_int("SM100_QUANT_COLS", 1);
+    // the column kernel stands in for the format's tensor-core family and goes with its switch (2: that family wherever its shapes allow)
+    const int family = dtype == DT_Q4_K ? use_imma : dtype == DT_Q6_K ? use_q6k : use_b32;
+    if (use_cols && family && (family == 1 || m > 1) && layout == LAYOUT_PACKED && x_aligned && cols_win(dtype, k, n, m, split_wins)) {
         const bool fine = dtype == DT_Q6_K && m == 1 && n * k > q6k_imma_limit(k);   // f32 kernels' precision where they served
         bool handled = false;
         const int st = quant_cols_tiles(s, dtype, w, k, n, x, ldx, m, y, ldy, fine, &handled);
@@ -644,7 +647,6 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
             return took("quant_cols+rows", tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
-    static const int use_imma = env_int("SM100_Q4K_IMMA", 1);
     if (use_imma && layout == LAYOUT_PACKED && dtype == DT_Q4_K && x_aligned && m == 1) {
         // the ring kernel (consecutive launches overlap; it declines unless the stream's last launch was such a matvec);
         // leftover rows take the row kernel
@@ -669,7 +671,6 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
             return took("matvec_q4k_imma", ST_OK);
         }
     }
-    static const int use_b32 = env_int("SM100_B32_IMMA", 1);
     if (use_b32 && layout == LAYOUT_PACKED && (dtype == DT_Q4_0 || dtype == DT_Q8_0) && x_aligned && m == 1) {
         bool handled = false;
         const int st = matvec_b32_imma_tiles(s, dtype, w, k, n, x, y, &handled);
@@ -680,7 +681,6 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
             return took("matvec_b32_imma+rows", tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
-    static const int use_q6k = env_int("SM100_Q6K_IMMA", 1);
     if (use_q6k && layout == LAYOUT_PACKED && dtype == DT_Q6_K && x_aligned && m == 1 && (use_q6k > 1 || n * k <= q6k_imma_limit(k))) {
         bool handled = false;
         const int st = matvec_q6k_imma_tiles(s, w, k, n, x, y, &handled);

@@ -173,3 +173,48 @@ def test_columns_of_subnormal_numbers(sm100, stream, dtype, k, n, m, exponent):
     assert _served(sm100).startswith("quant_cols")
     for t in range(m):
         assert sgref.nmse(got[t], want[t]) <= TOL, (t, sgref.nmse(got[t], want[t]))
+
+
+def _child(args, env):
+    import os
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable] + args, capture_output=True, text=True, timeout=900, env=dict(os.environ, **env))
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    return r.stdout.strip().splitlines()[-1]
+
+
+@pytest.mark.parametrize("env,left", [({}, ["q4_0", "q4_k", "q6_k", "q8_0"]), ({"SM100_QUANT_COLS": "0"}, []), ({"SM100_Q6K_IMMA": "0"}, ["q4_0", "q4_k", "q8_0"]),
+                                      ({"SM100_B32_IMMA": "0"}, ["q4_k", "q6_k"]), ({"SM100_Q4K_IMMA": "0"}, ["q4_0", "q6_k", "q8_0"]),
+                                      ({"SM100_Q4K_IMMA": "0", "SM100_Q4K_MMA": "0", "SM100_Q6K_IMMA": "0", "SM100_B32_IMMA": "0", "SM100_MV_WIDE": "0"}, [])],
+                         ids=["default", "none", "no_q6k", "no_b32", "no_q4k", "cuda_core_only"])
+def test_switches(env, left):
+    """The family has a switch, and goes with those of the families whose calls it takes.  Every result against the oracle in the worker, bar of the matvec tests."""
+    import json
+    import os
+    out = json.loads(_child([os.path.join(os.path.dirname(os.path.abspath(__file__)), "matvec_branch_worker.py")], env))
+    assert out["worst"] <= 1e-6, out
+    assert sorted({name.split(":")[0] for name in out["kernels"] if "quant_cols" in name}) == left
+
+
+BATCHES = """
+import numpy as np
+from scrapgpulibrary_b200 import capi
+from tests import util as U
+s = capi.Stream(0)
+bad = []
+for dtype, k, n in [(U.Q4_0, 1024, 4112), (U.Q8_0, 2048, 6000), (U.Q6_K, 4096, 4096)]:
+    wq = U.quantize(dtype, np.resize(U.seeded_weights(dtype + k, 250, k), (n, k)))
+    x = U.seeded_acts(k, 32, k)
+    both = U.device_mul_mat(capi, s, dtype, U.PACKED, wq, k, x)
+    bad += [(dtype, m) for m in (24, 9, 8, 7, 5) if not np.array_equal(U.device_mul_mat(capi, s, dtype, U.PACKED, wq, k, x[:m]), both[:m])]
+print(bad)
+"""
+
+
+def test_without_it_columns_do_not_depend_on_their_batch():
+    """Bit for bit over 5 to 32 columns, from 4096 rows on too: for callers that want that rather than the faster and more accurate kernel."""
+    import os
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = {"SM100_QUANT_COLS": "0", "PYTHONPATH": root + os.pathsep + os.environ.get("PYTHONPATH", "")}
+    assert _child(["-c", BATCHES], env) == "[]"
