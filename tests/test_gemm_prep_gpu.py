@@ -39,3 +39,19 @@ def test_stage_images_of_q6_k_prompts(sm100, stream, k, m):
     got = U.device_mul_mat(sm100, stream, U.Q6_K, U.PACKED, wq, k, x)
     for t in range(m):
         assert sgref.nmse(got[t], want[t]) <= 1e-9, t
+
+
+# Row tiles of the GEMM: where it leaves few SMs, two, four and eight tokens a CTA, by the tokens; where it fills them (296) one; with 4 to 32 float4 a thread
+@pytest.mark.parametrize("k", [1024, 2048, 4096, 8192, 8224])
+@pytest.mark.parametrize("tiles,m", [(80, 37), (120, 100), (135, 64), (60, 250), (296, 45)])
+def test_tokens_per_cta_beside_a_gemm(sm100, stream, tiles, m, k):
+    """Every token on its own.  Rows repeat every 48, so that the oracle has few to multiply."""
+    n = tiles * 128
+    wq = U.quantize(U.Q4_0, U.seeded_weights(k, 48, k))
+    x = U.seeded_acts(k + m, m, k)
+    x *= np.float32(2.0) ** (np.arange(m, dtype=np.float32) % 7)[:, None]   # a factor taken from another token shows
+    want = sgref.mul_mat(U.Q4_0, wq, k, x)
+    got = U.device_mul_mat(sm100, stream, U.Q4_0, U.PACKED, np.ascontiguousarray(np.resize(wq, (n, wq.shape[1]))), k, x)
+    assert np.array_equal(got, got[:, np.arange(n) % 48])
+    for t in range(m):
+        assert sgref.nmse(got[t, :48], want[t]) <= 1e-6, t

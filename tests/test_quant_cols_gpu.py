@@ -35,7 +35,7 @@ def _check(sm100, stream, dtype, k, n, m, seed=0):
         assert sgref.nmse(got[:, r0:r0 + 16].astype(np.float64), want[:, r0:r0 + 16]) <= 4 * TOL, r0
 
 
-# one unit of K, an odd number of units, 17 (two CTAs, uneven), 48 (three); fewer and more row tiles than CTAs, rows behind the last
+# one unit of K, an odd number of units, 17 and 48 (clusters of three CTAs); fewer and more row tiles than CTAs, rows behind the last
 # whole tile; one window of row tiles and several
 SHAPES = [(256, 16384 + 16), (1280, 4096 + 5), (4352, 4096), (12288, 4096 + 48), (4096, 12288 + 16), (2048, 148 * 16 * 16)]
 
@@ -218,3 +218,10 @@ def test_without_it_columns_do_not_depend_on_their_batch():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     env = {"SM100_QUANT_COLS": "0", "PYTHONPATH": root + os.pathsep + os.environ.get("PYTHONPATH", "")}
     assert _child(["-c", BATCHES], env) == "[]"
+
+
+# what plan_cols deals to clusters of five (17 and 18 units) and six (53 and 54 units) CTAs, unevenly, four row tiles a CTA and one; with rows behind the last whole tile
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q6_K, 4352, 1456, 4), (U.Q4_0, 4352, 1461, 4), (U.Q8_0, 4608, 1472, 2), (U.Q4_K, 4352, 1456, 8), (U.Q4_K, 13568, 1696, 2),
+                                         (U.Q6_K, 13568, 1744, 4), (U.Q8_0, 13824, 1696, 3)], ids=lambda v: str(v))
+def test_clusters_of_five_and_six(sm100, stream, dtype, k, n, m):
+    _check(sm100, stream, dtype, k, n, m)
