@@ -595,9 +595,11 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
 // How K and the rows are dealt: a cluster of `cluster` CTAs (one per SM) shares K, wk units each; a CTA takes 2^wr_log row tiles at a time.
 struct ColsPlan { int cluster, wk, wr_log, at_once; };
 
-// The time of a plan goes with the row tiles that a warp walks down (`iters`) and with the warps that share an SM while it does so, plus
-// start and exchange.  12288 x 4096 (Q6_K, 4 columns), us: clusters of 3 with 16 warps a CTA 15.5, of 6 16.8, of 5 with 10 warps 18.6.  A CTA more
-// in the cluster counts 5 %: Q4_K, 2 columns, 3072 x 14336 with one CTA of 12 warps 9.6, three of 16 13.2; 5120 x 6144 two of 10 9.3, three of 14 10.6.
+// The time of a plan goes with the row tiles that a warp walks down (`iters`) and with the warps that share an SM while it does so (fewer than six are no faster each),
+// plus start, which goes with the warps too, and the exchange of a cluster; a CTA more in the cluster counts 5 %.  Over 3623 products (K 256 .. 14336, N 1024 .. 32768, the four
+// formats, 2, 4 and 8 columns) this choice is 1.3 % off the best plan on average, 133 of them by over 10 %.  A sum without start, and with little for a cluster, was 3.1 % off and
+// 432, up to 1.64 times the integer kernel's time with Q4_K.  8 columns of that, us, by that sum's plan / this one's / in the integer kernel: 768 x 11264 9.5 / 5.8 / 5.8;
+// 2048 x 2560 5.7 / 4.6 / 4.3; 4352 x 4096 10.3 / 8.4 / 7.3; 6144 x 4096 11.0 / 9.2 / 8.6.
 // at_once: clusters that run at a time where every CTA has an SM of its own; SMs lie in groups that a cluster does not cross, so it is
 // fewer than 148 / cluster (a 7 x 17 grid took twice as long as one of 15).
 inline bool plan_cols(int units, int tiles, ColsPlan & p) {
@@ -605,11 +607,14 @@ inline bool plan_cols(int units, int tiles, ColsPlan & p) {
     int64_t best = INT64_MAX;
     for (int c = 1; c <= 8 && c <= units; ++c) {
         const int wk = (units + c - 1) / c, at_once = most[c] * sm_count() / 148;
-        if (wk > CO_WARPS || at_once < 1) continue;
+        if (wk > CO_WARPS || at_once < 2) continue;
         for (int wl = 0; wk << wl <= CO_WARPS; ++wl) {
             const int64_t groups = (tiles + (1 << wl) - 1) >> wl, iters = (groups + at_once - 1) / at_once;
-            const int64_t cost = iters * ((wk << wl) + 4) * (19 + c) / 20 + (c > 1 ? 6 : 0);
-            if (cost < best) { best = cost; p = {c, wk, wl, at_once}; }
+            const int warps = wk << wl;
+            // a plan that needs every place for a cluster of three or more has to wait for one
+            const int64_t counted = c > 2 ? (groups + at_once - 2) / (at_once - 1) : iters;
+            const int64_t cost = counted * ((warps > 6 ? warps : 6) + 6) * (19 + c) + 40 * warps + (c > 1 ? 320 + 40 * c : 0);
+            if (cost < best || (cost == best && p.cluster == c)) { best = cost; p = {c, wk, wl, at_once}; }
         }
     }
     return best != INT64_MAX;

@@ -35,7 +35,7 @@ def _check(sm100, stream, dtype, k, n, m, seed=0):
         assert sgref.nmse(got[:, r0:r0 + 16].astype(np.float64), want[:, r0:r0 + 16]) <= 4 * TOL, r0
 
 
-# one unit of K, an odd number of units, 17 and 48 (clusters of three CTAs); fewer and more row tiles than CTAs, rows behind the last
+# one unit of K, an odd number of units, 17 and 48 (clusters of two and three CTAs, 17 unevenly); fewer and more row tiles than CTAs, rows behind the last
 # whole tile; one window of row tiles and several
 SHAPES = [(256, 16384 + 16), (1280, 4096 + 5), (4352, 4096), (12288, 4096 + 48), (4096, 12288 + 16), (2048, 148 * 16 * 16)]
 
@@ -220,8 +220,8 @@ def test_without_it_columns_do_not_depend_on_their_batch():
     assert _child(["-c", BATCHES], env) == "[]"
 
 
-# what plan_cols deals to clusters of five (17 and 18 units) and six (53 and 54 units) CTAs, unevenly, four row tiles a CTA and one; with rows behind the last whole tile
-@pytest.mark.parametrize("dtype,k,n,m", [(U.Q6_K, 4352, 1456, 4), (U.Q4_0, 4352, 1461, 4), (U.Q8_0, 4608, 1472, 2), (U.Q4_K, 4352, 1456, 8), (U.Q4_K, 13568, 1696, 2),
-                                         (U.Q6_K, 13568, 1744, 4), (U.Q8_0, 13824, 1696, 3)], ids=lambda v: str(v))
+# what plan_cols deals to clusters of five (35, 43 and 50 units; two row tiles a CTA and one) and six (53 and 54 units) CTAs, mostly unevenly; with rows behind the last whole tile
+@pytest.mark.parametrize("dtype,k,n,m", [(U.Q6_K, 11008, 1184, 4), (U.Q4_0, 12800, 1093, 4), (U.Q8_0, 8960, 1552, 2), (U.Q4_K, 11008, 1184, 8), (U.Q4_K, 13824, 1632, 2),
+                                         (U.Q6_K, 13568, 1648, 4), (U.Q4_K, 13568, 1616, 5), (U.Q8_0, 13824, 1653, 3)], ids=lambda v: str(v))
 def test_clusters_of_five_and_six(sm100, stream, dtype, k, n, m):
     _check(sm100, stream, dtype, k, n, m)
