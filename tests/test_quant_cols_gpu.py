@@ -225,3 +225,16 @@ def test_without_it_columns_do_not_depend_on_their_batch():
                                          (U.Q6_K, 13568, 1648, 4), (U.Q4_K, 13568, 1616, 5), (U.Q8_0, 13824, 1653, 3)], ids=lambda v: str(v))
 def test_clusters_of_five_and_six(sm100, stream, dtype, k, n, m):
     _check(sm100, stream, dtype, k, n, m)
+
+
+# one column where the kernel that served it before is the faster one, and its neighbours: rows of one to three units below 24576 rows; K = 8192 with few rows or rows left over
+@pytest.mark.parametrize("dtype,k,n,name", [(U.Q4_0, 512, 12288, "matvec_b32_imma"), (U.Q8_0, 1024, 16384, "matvec_b32_imma"), (U.Q4_0, 1280, 12288, "quant_cols"), (U.Q8_0, 512, 24576, "quant_cols"),
+                                            (U.Q6_K, 512, 12288, "matvec_q6k_imma"), (U.Q6_K, 768, 12288, "quant_cols"), (U.Q6_K, 8192, 4592, "matvec_wide"), (U.Q6_K, 8192, 4608, "quant_cols"),
+                                            (U.Q6_K, 8192, 5003, "matvec_wide")], ids=lambda v: str(v))
+def test_one_column_takes_the_faster_kernel(sm100, stream, dtype, k, n, name):
+    """Bound: 16-bit activations with a scale per 16 or 32 of them (1e-4), as in the matvec tests."""
+    wq = np.ascontiguousarray(np.resize(U.quantize(dtype, U.seeded_weights(k, 416, k)), (n, U.quantize(dtype, U.seeded_weights(1, 1, k)).shape[1])))
+    x = U.seeded_acts(n, 1, k)
+    got, want = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x), _want(dtype, wq[:416], k, x)[:, np.arange(n) % 416]
+    assert _served(sm100) == name
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 1e-4
