@@ -338,13 +338,13 @@ __global__ void __launch_bounds__(MAXT, MINB) matvec_wide(const uint8_t * __rest
 template <class U, int M, bool PACKED>
 __global__ void __launch_bounds__(256) matvec_rows(const uint8_t * __restrict__ w, Planes P, int64_t w_row_stride,
                                                    const float * x, int64_t ldx, float * y, int64_t ldy,
-                                                   int n_rows, int units_per_row) {
+                                                   int row_begin, int n_rows, int units_per_row) {
     pdl_wait();
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
     const int warps = blockDim.x >> 5;
     const int64_t bpr = units_per_row / U::UNITS_PER_BLOCK;
-    for (int r = blockIdx.x * warps + (threadIdx.x >> 5); r < n_rows; r += gridDim.x * warps) {
+    for (int r = row_begin + blockIdx.x * warps + (threadIdx.x >> 5); r < n_rows; r += gridDim.x * warps) {
         float acc[M];
 #pragma unroll
         for (int m = 0; m < M; ++m) acc[m] = 0.f;
@@ -518,18 +518,18 @@ static bool wide_ok(int64_t k, int64_t m) {
 
 template <class U, bool PACKED>
 static int launch_rows(cudaStream_t s, const void * w, int64_t w_row_stride, int64_t k, int64_t n, const float * x, int64_t ldx,
-                       int64_t m, float * y, int64_t ldy) {
+                       int64_t m, float * y, int64_t ldy, int64_t row_begin = 0) {
     const int upr = (int) (k / U::WEIGHTS);
     Planes P = {};
     if (PACKED) P = planes_for(U::DTYPE, n, k);
     const int threads = 256, warps = threads / 32;
-    int64_t grid = (n + warps - 1) / warps;
+    int64_t grid = (n - row_begin + warps - 1) / warps;
     const int64_t cap = (int64_t) sm_count() * 8;
     if (grid > cap) grid = cap;
     const dim3 g((unsigned) grid), b(threads);
     const uint8_t * wp = (const uint8_t *) w;
 #define SM100_ROWS_CASE(MM) \
-    case MM: return launch(matvec_rows<U, MM, PACKED>, g, b, 0, s, wp, P, w_row_stride, x, ldx, y, ldy, (int) n, upr);
+    case MM: return launch(matvec_rows<U, MM, PACKED>, g, b, 0, s, wp, P, w_row_stride, x, ldx, y, ldy, (int) row_begin, (int) n, upr);
     switch (m) {
         SM100_ROWS_CASE(1) SM100_ROWS_CASE(2) SM100_ROWS_CASE(3) SM100_ROWS_CASE(4)
         SM100_ROWS_CASE(5) SM100_ROWS_CASE(6) SM100_ROWS_CASE(7) SM100_ROWS_CASE(8)
@@ -555,8 +555,7 @@ template <class U>
 static int launch_tail(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
     return m <= 64 ? launch_tail_cols<U, 2>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy) : launch_tail_cols<U, 4>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
 }
-// Rows row_begin .. n - 1 of a packed tensor in f32, m columns, x 16-byte aligned.  Behind a single column too it takes half the time of matvec_rows, whose warps walk
-// along K alone (Q8_0 4096 x 5003, 11 rows: the whole product 17.0 -> 10.4 us).
+// Rows row_begin .. n - 1 of a packed tensor in f32, m columns, x 16-byte aligned.
 int tail_rows(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
     switch (dtype) {
         case DT_Q4_0: return launch_tail<UnitQ40>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
@@ -565,6 +564,22 @@ int tail_rows(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, i
         case DT_Q6_K: return launch_tail<UnitQ6K>(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
     }
     return fail(ST_UNSUPPORTED, "mul_mat: no packed rows of dtype %d", dtype);
+}
+
+// The rows behind whole tiles of a product of up to eight columns.  A CTA of matvec_tail shares four rows, at half the time of matvec_rows, whose warps walk along K
+// alone (Q8_0 4096 x 5003, 11 rows: the whole product 17.0 -> 10.4 us); but it adds its warps' sums up, goes two columns at a time, and short rows leave most of its
+// threads idle.  Longest rows that matvec_rows has the shorter time for, by the number of columns (whole products of 1001 to 3999 rows, matvec_rows / matvec_tail: Q6_K
+// 512 m = 1 1 / 1.19, m = 2 1 / 1.44, 2048 m = 2 1 / 1.11, 2560 m = 2 1 / 0.98; Q4_K 512 m = 2 1 / 1.34, 2048 m = 2 1 / 0.98; Q4_0 512 m = 2 1 / 1.06, 1024 1 / 0.92).
+static int leftover_rows(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, int64_t row_begin, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy) {
+    static const int q40[8] = {256, 512, 256, 256, 0, 0, 0, 0}, q80[8] = {256, 256, 0, 0, 0, 0, 0, 0};
+    static const int q4k[8] = {1024, 1536, 1024, 512, 512, 256, 0, 0}, q6k[8] = {2048, 2048, 1536, 1280, 1024, 768, 512, 256};
+    switch (dtype) {
+        case DT_Q4_0: if (k <= q40[m - 1]) return launch_rows<UnitQ40, true>(s, w, 0, k, n, x, ldx, m, y, ldy, row_begin); break;
+        case DT_Q8_0: if (k <= q80[m - 1]) return launch_rows<UnitQ80, true>(s, w, 0, k, n, x, ldx, m, y, ldy, row_begin); break;
+        case DT_Q4_K: if (k <= q4k[m - 1]) return launch_rows<UnitQ4K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, row_begin); break;
+        case DT_Q6_K: if (k <= q6k[m - 1]) return launch_rows<UnitQ6K, true>(s, w, 0, k, n, x, ldx, m, y, ldy, row_begin); break;
+    }
+    return tail_rows(s, dtype, w, k, n, row_begin, x, ldx, m, y, ldy);
 }
 
 template <class U>
@@ -647,7 +662,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (handled) {
             const int64_t full = n / 16 * 16;
             if (full == n) return took("quant_cols", ST_OK);
-            return took("quant_cols+rows", tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
+            return took("quant_cols+rows", leftover_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
     if (use_imma && layout == LAYOUT_PACKED && dtype == DT_Q4_K && x_aligned && m == 1) {
@@ -658,7 +673,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            if (full < n) return took("matvec_q4k_ring+rows", tail_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
+            if (full < n) return took("matvec_q4k_ring+rows", leftover_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
             return took("matvec_q4k_ring", ST_OK);
         }
     }
@@ -669,7 +684,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            if (full < n) return took("matvec_q4k_imma+rows", tail_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
+            if (full < n) return took("matvec_q4k_imma+rows", leftover_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
             if (m == 1) stream_tail_set(s, TAIL_Q4K_MATVEC);   // a second plain Q4_K matvec right behind this one starts a run of the ring kernel
             return took("matvec_q4k_imma", ST_OK);
         }
@@ -681,7 +696,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (handled) {
             const int64_t full = (n / 16) * 16;
             if (full == n) return took("matvec_b32_imma", ST_OK);
-            return took("matvec_b32_imma+rows", tail_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
+            return took("matvec_b32_imma+rows", leftover_rows(s, dtype, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
     if (use_q6k && layout == LAYOUT_PACKED && dtype == DT_Q6_K && x_aligned && m == 1 && (use_q6k > 1 || n * k <= q6k_imma_limit(k))) {
@@ -690,7 +705,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            return full == n ? took("matvec_q6k_imma", ST_OK) : took("matvec_q6k_imma+rows", tail_rows(s, DT_Q6_K, w, k, n, full, x, ldx, m, y, ldy));
+            return full == n ? took("matvec_q6k_imma", ST_OK) : took("matvec_q6k_imma+rows", leftover_rows(s, DT_Q6_K, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
     if (use_imma && layout == LAYOUT_PACKED && dtype == DT_Q4_K && x_aligned && m >= 3) {
@@ -712,7 +727,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         }
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            if (full < n) return took("matvec_q4k_imma_cols+rows", tail_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
+            if (full < n) return took("matvec_q4k_imma_cols+rows", leftover_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
             return took("matvec_q4k_imma_cols", ST_OK);
         }
     }
@@ -734,7 +749,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         }
         if (all) {
             const int64_t full = (n / 16) * 16;
-            if (full < n) return took("matvec_q4k_mma+rows", tail_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
+            if (full < n) return took("matvec_q4k_mma+rows", leftover_rows(s, DT_Q4_K, w, k, n, full, x, ldx, m, y, ldy));
             return took("matvec_q4k_mma", ST_OK);
         }
     }
@@ -758,7 +773,7 @@ int matvec(cudaStream_t s, int dtype, int layout, const void * w, int64_t w_row_
         if (st != ST_OK) return st;
         if (handled) {
             const int64_t full = (n / 16) * 16;
-            return full == n ? took("matvec_q6k_imma_cols", ST_OK) : took("matvec_q6k_imma_cols+rows", tail_rows(s, DT_Q6_K, w, k, n, full, x, ldx, m, y, ldy));
+            return full == n ? took("matvec_q6k_imma_cols", ST_OK) : took("matvec_q6k_imma_cols+rows", leftover_rows(s, DT_Q6_K, w, k, n, full, x, ldx, m, y, ldy));
         }
     }
     // Q6_K / Q4_0 / Q8_0 with few columns or rows: the single-column tensor-core and wide kernels have no multi-column form,

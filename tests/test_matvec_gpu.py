@@ -420,3 +420,17 @@ def test_hostpipe_mul_mat_matches_device_path(sm100, stream):
         lib.sm100_host_free(px)
         lib.sm100_host_free(py)
     wb.free()
+
+
+# the rows behind whole tiles: by the row kernel up to a length that falls with the columns, beyond by the tail kernel; one row, several, 15
+@pytest.mark.parametrize("dtype,k,m", [(U.Q4_0, 256, 1), (U.Q4_0, 512, 2), (U.Q4_0, 768, 2), (U.Q8_0, 256, 2), (U.Q8_0, 512, 2), (U.Q4_K, 1024, 1), (U.Q4_K, 1280, 1), (U.Q4_K, 1536, 2), (U.Q4_K, 1792, 2),
+                                       (U.Q4_K, 256, 6), (U.Q4_K, 512, 6), (U.Q6_K, 2048, 1), (U.Q6_K, 2304, 1), (U.Q6_K, 1280, 4), (U.Q6_K, 1536, 4), (U.Q6_K, 256, 8), (U.Q6_K, 512, 8)], ids=lambda v: str(v))
+@pytest.mark.parametrize("left", [1, 5, 15])
+def test_rows_behind_whole_tiles(sm100, stream, dtype, k, m, left):
+    """Both are f32 kernels: 2e-7 to 1.2e-6 against float64, bound 2e-6.  Nothing behind the last row is written (guarded output)."""
+    n = 64 + left
+    wq = U.quantize(dtype, U.seeded_weights(9000 + dtype + k, n, k))
+    x = U.seeded_acts(m + k, m, k)
+    want = (x.astype(np.float64) @ sgref.dequantize(dtype, wq, k).astype(np.float64).T)[:, 64:]
+    got = U.device_mul_mat(sm100, stream, dtype, U.PACKED, wq, k, x)[:, 64:]
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-6
