@@ -472,7 +472,15 @@ int gemm_passes(cudaStream_t s, int dtype, int layout, GemmArgs g, const float *
         int toks = 1;
         while (toks < 8 && (mpad / toks > most || g.nchunks * (KC / 4) * toks * 2 <= 4 * 256)) toks <<= 1;
         while (toks > 1 && (int64_t) g.nchunks * (KC / 4) * toks > (int64_t) PREP_MAX_V * 256) toks >>= 1;
-        const int per = (g.nchunks * (KC / 4) * toks + 255) / 256;
+        // Where many of them would meet on the SMs that the predecessor's last wave leaves free (behind one another such products are resident together),
+        // eight tokens a CTA and so many registers that an SM takes one.  us, 32 float4 a thread always / with the lines above alone / now: Q4_0 2048 x 4048, 512 tokens
+        // 18.9 / 21.6 / 18.8; 512 x 12288, 700 tokens 30.6 / 31.8 / 30.6; 2048 x 8192, 512 tokens 31.4 / 32.7 / 31.3.  Rows of 256 weights are over before that
+        // matters (256 x 4048, 512 tokens 12.3 / 11.4).
+        const int idle = sm_count() - 1 - (n_tiles * m_tiles - 1) % sm_count();
+        const bool crowd = toks > 1 && mpad / toks > 3 * idle && g.nchunks * KC > 256;
+        if (crowd)
+            while (toks < 8 && g.nchunks * (KC / 4) * toks * 2 <= PREP_MAX_V * 256) toks <<= 1;
+        const int per = crowd ? PREP_MAX_V : (g.nchunks * (KC / 4) * toks + 255) / 256;
         auto prep = per <= 4 ? gemm_prep_x<TN, 4> : per <= 8 ? gemm_prep_x<TN, 8> : per <= 16 ? gemm_prep_x<TN, 16> : gemm_prep_x<TN, PREP_MAX_V>;
         st = launch(prep, dim3((unsigned) (mpad / toks)), dim3(256), 0, s, x + c0 * ldx, ldx, (int) mm, (int) k, g.nchunks, toks,
                     dtype == DT_Q4_K ? 0 : dtype == DT_Q4_0 ? 2 : 1, tokscale, xh);

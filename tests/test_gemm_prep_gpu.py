@@ -55,3 +55,10 @@ def test_tokens_per_cta_beside_a_gemm(sm100, stream, tiles, m, k):
     assert np.array_equal(got, got[:, np.arange(n) % 48])
     for t in range(m):
         assert sgref.nmse(got[t, :48], want[t]) <= 1e-6, t
+
+
+# more CTAs of the preparation than there are free SMs in the last wave of the GEMM before it: eight tokens each with 32 float4 a thread, one wave of the GEMM and two
+@pytest.mark.parametrize("k", [544, 1024, 2048, 4128])
+@pytest.mark.parametrize("tiles,m", [(32, 500), (96, 700)])
+def test_crowded_preparation(sm100, stream, tiles, m, k):
+    test_tokens_per_cta_beside_a_gemm(sm100, stream, tiles, m, k)
