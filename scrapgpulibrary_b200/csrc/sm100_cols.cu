@@ -7,7 +7,7 @@
 // tiles of 16 rows, whose bytes it copies to a ring of its own in shared memory (cp.async: whole lines of the row-major planes, no registers
 // for what is in flight) and reads back as A fragments (ldmatrix: a matrix row is 16 bytes of a weight row).  The integers need no conversion:
 // a bit field under the exponent of 1024 is an f16 number, and one packed addition takes 1024 and the format's offset (8, 32, 128) off, exactly; the unsigned
-// ones of Q4_K stand under a zero exponent, subnormal numbers.  A block (32 weights, Q6_K 16) is multiplied into a fresh accumulator, which times the block's
+// ones of Q4_K (and OFFSET) stand under a zero exponent, subnormal numbers.  A block (32 weights, Q6_K 16) is multiplied into a fresh accumulator, which times the block's
 // scale goes to f32 sums: no weight is scaled or rounded, and the tensor core's truncation sees 32 products at most.
 //
 // Activations: per column and unit one power of two brings the largest to [2^13, 2^14), then x = xh + 2^-11 xl, both f16: 22 bits, and because the low part is
@@ -16,13 +16,14 @@
 // an f32 number down to 2^-37 of the largest, for the single columns of Q6_K that f32 kernels would serve otherwise (7168 x 8192: 15.9 us with two parts, 16.8 with three).
 //   FINE    xh, xl and the third part of one token in three columns
 //   M <= 4: the eight columns of an MMA are xh and xl of four tokens; M <= 8: two MMAs, xh and xl of eight
-// Error against float64: 2e-7 to 1.3e-6 (the integer column kernels 2e-5 to 6e-5, the split GEMM 5e-6, the f32 matvec of the vocabulary head 9e-7).
+// Error against float64: 8e-8 to 1.3e-7, Q4_K 6e-7 to 1.4e-6, OFFSET 3e-7 (the integer column kernels 2e-5 to 6e-5, the split GEMM 5e-6, the f32 matvec of the vocabulary head 1e-6).
 //
-// The partial tiles of a CTA's units meet in shared memory and are added in the order of K; where K is longer than a CTA's 16 units a cluster shares
-// it and its CTAs read each other's sums.  No memory of the call, one launch.
+// The partial tiles of a CTA's units meet in shared memory and are added in the order of K; where K is longer than a CTA's 16 units, or more
+// SMs have work that way, a cluster of two to six shares it and its CTAs read each other's sums.  No memory of the call, one launch.
 //
 // What bounds it: Q6_K the instructions that assemble 6 bits (the ALU pipe over 70 % busy in the loop), then 3 to 4 us of start (launch, activations from
-// L2, their conversion) that one CTA per SM does not hide; K = 4096, N = 12288, 4 columns without the products 9.3 us, without the weights 11.8, as it is 13.8.
+// L2, their conversion) that one CTA per SM does not hide; K = 4096, N = 12288, 4 columns 13.3 us (with the offsets taken off afterwards 13.8, of that
+// without the products 9.3, without the weights 11.8).
 #include "sm100_common.cuh"
 #include "sm100_layout.h"
 
@@ -106,8 +107,9 @@ __device__ __forceinline__ uint32_t co_pick(uint32_t a, uint32_t c) { uint32_t d
 __device__ __forceinline__ uint32_t co_less1032(uint32_t a) { return co_add2(a, 0xe408e408u); }
 __device__ __forceinline__ uint32_t co_less1152(uint32_t a) { return co_add2(a, 0xe480e480u); }
 
-// B: the activations, per step of 16 weights pairs (0, 2) and (1, 3) of the lane's four, and of Q4_K the sums over the blocks (2 t, 2 t + 1)
-template <bool P4> struct CoB { uint32_t h[16][2], l[P4 ? 1 : 16][P4 ? 1 : 2]; uint32_t sum_h, sum_l, k1024; };
+// B: the activations, per step of 16 weights pairs (0, 2) and (1, 3) of the lane's four, and where a format has them the sums over the blocks (2 t and 2 t + 1 of eight;
+// 4 t and 4 t + 2, 4 t + 1 and 4 t + 3 of sixteen)
+template <bool P4> struct CoB { uint32_t h[16][2], l[P4 ? 1 : 16][P4 ? 1 : 2]; uint32_t sum_h[2], sum_l, k1024; };
 
 // What the low parts are multiplied by: as they are, the low part of an activation 2^-14 of the largest would be a subnormal number, with fewer bits (an activation
 // 1e7 times the others left 2e-4 of them).  4096 x 12288, us before / now: Q8_0 4 columns 12.1 / 12.3, 8 columns 13.4 / 14.1; Q6_K 4 columns 12.9 / 13.4, 8 columns 17.1 / 17.7.
@@ -162,9 +164,10 @@ __device__ __forceinline__ void co_scale(float (&sum)[4], const float (&acc)[4],
 // Q4_0 and Q8_0: per row the unit's quants and its eight f16 scales
 template <bool Q8>
 struct CoB32 {
-    static constexpr bool FINE = false;
+    static constexpr bool FINE = false, OFFSET = false;
     static constexpr int QB = Q8 ? 256 : 128, PITCH = QB + 16, SLOT = 16 * PITCH, SLOTS = Q8 ? 2 : 4, TABLE = 0;
-    static constexpr bool SUMS = false, SCALED = true;
+    static constexpr int BLOCKS = 0;
+    static constexpr bool SCALED = true;
     static constexpr float COUNT = 1.0f;
     struct Cursor { const uint8_t * q; const uint8_t * d; };
     __device__ static __forceinline__ int k_of(int s) { return 16 * s; }
@@ -227,9 +230,10 @@ struct CoB32 {
 // Q4_K: four lane-ordered tiles of 512 bytes, then the rows' headers.  Table: d sc of [16 rows][8 sub-blocks], padded to 12; of the odd ones,
 // whose nibbles count 16, a 16th.
 struct CoQ4K {
-    static constexpr bool FINE = false;
+    static constexpr bool FINE = false, OFFSET = false;
     static constexpr int SLOT = 4 * 512 + 256, SLOTS = 4, TABLE = 16 * 12 * 4;
-    static constexpr bool SUMS = true, SCALED = false;
+    static constexpr int BLOCKS = 8;   // of a unit whose sums of x are wanted
+    static constexpr bool SCALED = false;
     static constexpr float COUNT = CO_2_24;
     struct Cursor { const uint8_t * q; const uint8_t * h; };
     __device__ static __forceinline__ int k_of(int s) { return 16 * s; }
@@ -261,7 +265,7 @@ struct CoQ4K {
             asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(to + 8 * 48), "f"(d1 * (float) (f1 & 63u)), "f"(d1 * 0.0625f * (float) ((f1 >> 12) & 63u)) : "memory");
             const uint32_t a[4] = {((f0 >> 6) & 63u) | ((f0 >> 2) & 0x003f0000u), ((f1 >> 6) & 63u) | ((f1 >> 2) & 0x003f0000u), 0u, 0u};
             float acc[4];
-            co_mma0(acc, a, b.sum_h, 0u);
+            co_mma0(acc, a, b.sum_h[0], 0u);
             if constexpr (!P4) co_mma(acc, a, b.sum_l, 0u);
             sum[0] = m0 * acc[0]; sum[1] = m0 * acc[1]; sum[2] = m1 * acc[2]; sum[3] = m1 * acc[3];
         }
@@ -295,12 +299,17 @@ struct CoQ4K {
 
 // Q6_K: per row 128 bytes of nibbles, 64 of bit pairs, 16 scales; then the words that hold the rows' d.  Table: d sc of
 // [16 rows][16 groups], padded to 20; of every third and fourth group, whose integers count 16, a 16th.
-template <bool F32>
+// OFFSET: the integers stay unsigned subnormal numbers, 32 times the sums of x comes off afterwards, and low parts are as they are: for the single columns that 16-bit integers
+// served before.  It is the more accurate of these two beside large activations (rows whose weights there are zero, at 1e3 / 1e5 times the others: 1e-4 / 0.02, the integers
+// 2e-3 / 0.2), and its bits stay, since a decode step makes 6e-5 of its logits of any other rounding here: every layer behind it rounds to 16 bits.
+enum { Q6K_TWO_PARTS, Q6K_FINE, Q6K_OFFSET };
+template <int FORM>
 struct CoQ6K {
-    static constexpr bool FINE = F32;
+    static constexpr bool FINE = FORM == Q6K_FINE, OFFSET = FORM == Q6K_OFFSET;
     static constexpr int PITCH = 208, SLOT = 16 * PITCH + 64, SLOTS = 3, TABLE = 16 * 20 * 4;
-    static constexpr bool SUMS = false, SCALED = true;
-    static constexpr float COUNT = 1.0f;
+    static constexpr int BLOCKS = OFFSET ? 16 : 0;
+    static constexpr bool SCALED = !OFFSET;
+    static constexpr float COUNT = OFFSET ? CO_2_24 : 1.0f;
     struct Cursor { const uint8_t * q; const uint8_t * x; const uint8_t * s; const uint8_t * d; };
     __device__ static __forceinline__ int k_of(int s) { return 128 * (s >> 3) + 16 * ((s >> 2) & 1) + 32 * (s & 3); }
     __device__ static __forceinline__ bool sixteenth(int) { return false; }
@@ -334,18 +343,24 @@ struct CoQ6K {
     __device__ static __forceinline__ void run(uint32_t slot, uint32_t table, int odd, int lane, const CoB<P4> & b, float (&sum)[4]) {
         const int gr = lane >> 2, t = lane & 3;
         const uint32_t at = slot + (lane & 15) * PITCH;   // matrices of rows 0-7 and 8-15
-        {   // lane (g, t): scales 4 t .. 4 t + 3 of rows g and g + 8
+        {   // lane (g, t): scales 4 t .. 4 t + 3 of rows g and g + 8, for the table and (OFFSET), as f16 integers, times the sums of x
             uint32_t v[2];
             co_ldsm2(v, at + 192);
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            if constexpr (OFFSET) {
+                const uint32_t a[4] = {co_less1152((v[0] & 0x00ff00ffu) ^ 0x64806480u), co_less1152((v[1] & 0x00ff00ffu) ^ 0x64806480u),
+                                       co_less1152(((v[0] >> 8) & 0x00ff00ffu) ^ 0x64806480u), co_less1152(((v[1] >> 8) & 0x00ff00ffu) ^ 0x64806480u)};
+                co_mma0(acc, a, b.sum_h[0], b.sum_h[1]);
+            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const float d = co_half(co_lds(slot + 16 * PITCH + (gr + 8 * h) * 4) >> ((odd >> gr & 1) * 16) & 0xffffu);   // `odd`: bit r = row r's block has an odd number (row r + 8 like row r)
                 const int w = (int) v[h];
-                const float d16 = d * 0.0625f;
+                const float d16 = OFFSET ? d : d * 0.0625f;
                 co_sts4f(table + (gr + 8 * h) * 80 + t * 16, d * (float) (w << 24 >> 24), d * (float) (w << 16 >> 24), d16 * (float) (w << 8 >> 24), d16 * (float) (w >> 24));
+                sum[2 * h] = OFFSET ? d * (-1024.0f / CO_2_24) * acc[2 * h] : 0.f;
+                sum[2 * h + 1] = OFFSET ? d * (-1024.0f / CO_2_24) * acc[2 * h + 1] : 0.f;
             }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) sum[j] = 0.f;
         }
         __syncwarp();
 #pragma unroll
@@ -353,24 +368,27 @@ struct CoQ6K {
             const float4 e0 = co_lds4f(table + gr * 80 + c * 16), e1 = co_lds4f(table + (gr + 8) * 80 + c * 16);
             uint32_t a[4][4];   // [group][fragment word]
             uint32_t n[4], x[2];
+            const uint32_t k1024 = OFFSET ? 0u : b.k1024;
             co_ldsm4(n, at + 32 * c + (lane >> 4) * 16);
             co_ldsm2(x, at + 128 + 16 * c);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t n0 = n[h], n1 = n[2 + h], m0 = n0 >> 8, m1 = n1 >> 8, y = x[h] >> 8, xa = x[h] << 4, xb = x[h] << 2, ya = y << 4, yb = y << 2;
-                a[0][h] = co_pick<0x000f000fu>(n0, co_pick<0x00300030u>(xa, b.k1024));
-                a[0][2 + h] = co_pick<0x000f000fu>(m0, co_pick<0x00300030u>(ya, b.k1024));
-                a[1][h] = co_pick<0x000f000fu>(n1, co_pick<0x00300030u>(xb, b.k1024));
-                a[1][2 + h] = co_pick<0x000f000fu>(m1, co_pick<0x00300030u>(yb, b.k1024));
-                a[2][h] = co_pick<0x00f000f0u>(n0, co_pick<0x03000300u>(xa, b.k1024));
-                a[2][2 + h] = co_pick<0x00f000f0u>(m0, co_pick<0x03000300u>(ya, b.k1024));
-                a[3][h] = co_pick<0x00f000f0u>(n1, co_pick<0x03000300u>(xb, b.k1024));
-                a[3][2 + h] = co_pick<0x00f000f0u>(m1, co_pick<0x03000300u>(yb, b.k1024));
+                a[0][h] = co_pick<0x000f000fu>(n0, co_pick<0x00300030u>(xa, k1024));
+                a[0][2 + h] = co_pick<0x000f000fu>(m0, co_pick<0x00300030u>(ya, k1024));
+                a[1][h] = co_pick<0x000f000fu>(n1, co_pick<0x00300030u>(xb, k1024));
+                a[1][2 + h] = co_pick<0x000f000fu>(m1, co_pick<0x00300030u>(yb, k1024));
+                a[2][h] = co_pick<0x00f000f0u>(n0, co_pick<0x03000300u>(xa, k1024));
+                a[2][2 + h] = co_pick<0x00f000f0u>(m0, co_pick<0x03000300u>(ya, k1024));
+                a[3][h] = co_pick<0x00f000f0u>(n1, co_pick<0x03000300u>(xb, k1024));
+                a[3][2 + h] = co_pick<0x00f000f0u>(m1, co_pick<0x03000300u>(yb, k1024));
             }
+            if constexpr (!OFFSET) {   // 1024 + q - 1056, 1024 + 16 q - 1536
 #pragma unroll
-            for (int j = 0; j < 4; ++j)   // 1024 + q - 1056, 1024 + 16 q - 1536
+                for (int j = 0; j < 4; ++j)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a[j][i] = co_add2(a[j][i], j < 2 ? 0xe420e420u : 0xe600e600u);
+                    for (int i = 0; i < 4; ++i) a[j][i] = co_add2(a[j][i], j < 2 ? 0xe420e420u : 0xe600e600u);
+            }
             const float s0[4] = {e0.x, e0.y, e0.z, e0.w}, s1[4] = {e1.x, e1.y, e1.z, e1.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -450,25 +468,28 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
         const float scale = F::FINE && ((lane >> 2) & 3) > (lo_lane ? 0 : 1) ? 0.f : __int_as_float((127 + sh) << 23), inv = __int_as_float((127 - sh) << 23);
         back[0] = __shfl_sync(0xffffffffu, inv, P4 ? (8 * t) & 15 : 8 * t);
         back[1] = __shfl_sync(0xffffffffu, inv, P4 ? (8 * t + 4) & 15 : 8 * t + 4);
-        constexpr bool SCALED = P4 || F::SCALED;
+        constexpr bool SCALED = (P4 && !F::OFFSET) || F::SCALED;
+        constexpr float LOW = SCALED ? CO_LOW : 1.0f;
         // f, or what it is less its high part, scaled.  Two numbers an instruction (Q4_0 4096 x 12288, 4 columns: 10.5 us with one, 10.3)
         // FINE: lanes 0..3 hold the first part, 16..19 the second, 4..7 the third, which takes another step.
         const bool third = F::FINE && (lane >> 2) == 1, low = lo_lane || third || !P4;
         const float2 up3 = third ? make_float2(CO_LOW, CO_LOW) : make_float2(1.f, 1.f), less3 = third ? make_float2(-CO_LOW, -CO_LOW) : make_float2(0.f, 0.f);
-        const float2 up = low ? make_float2(CO_LOW, CO_LOW) : make_float2(1.f, 1.f), less = low ? make_float2(-CO_LOW, -CO_LOW) : make_float2(0.f, 0.f);
-        float sums[8];
+        const float2 up = low ? make_float2(LOW, LOW) : make_float2(1.f, 1.f), less = low ? make_float2(-LOW, -LOW) : make_float2(0.f, 0.f);
+        const __half2 z = __float2half2_rn(0.0625f);
+        float sums[F::BLOCKS ? F::BLOCKS : 1];
 #pragma unroll
         for (int s = 0; s < 16; ++s) {
             const float sc = F::sixteenth(s) ? scale * 0.0625f : scale;
             const float2 f0 = __fmul2_rn(make_float2(v[s].x, v[s].y), make_float2(sc, sc)), f1 = __fmul2_rn(make_float2(v[s].z, v[s].w), make_float2(sc, sc));
-            if constexpr (F::SUMS) {
+            if constexpr (F::BLOCKS > 0) {
+                constexpr int PER = 16 / (F::BLOCKS ? F::BLOCKS : 16);
                 const float q = (f0.x + f1.x) + (f0.y + f1.y);
-                sums[s / 2] = s % 2 ? sums[s / 2] + q : q;
+                sums[s / PER] = s % PER ? sums[s / PER] + q : q;
             }
             const __half2 hx = __floats2half2_rn(f0.x, f1.x), hy = __floats2half2_rn(f0.y, f1.y);   // pairs (0, 2) and (1, 3)
             const float2 rx = __half22float2(hx), ry = __half22float2(hy);
             float2 u0, u1;
-            if constexpr (SCALED) {
+            if constexpr (SCALED || P4) {
                 u0 = __ffma2_rn(make_float2(rx.x, ry.x), less, __fmul2_rn(f0, up));
                 u1 = __ffma2_rn(make_float2(rx.y, ry.y), less, __fmul2_rn(f1, up));
             } else {
@@ -480,7 +501,11 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 u0 = __ffma2_rn(make_float2(qx.x, qy.x), less3, __fmul2_rn(u0, up3));
                 u1 = __ffma2_rn(make_float2(qx.y, qy.y), less3, __fmul2_rn(u1, up3));
             }
-            const uint32_t ux = h2(__floats2half2_rn(u0.x, u1.x)), uy = h2(__floats2half2_rn(u0.y, u1.y));
+            uint32_t ux = h2(__floats2half2_rn(u0.x, u1.x)), uy = h2(__floats2half2_rn(u0.y, u1.y));
+            if (F::OFFSET && (s & 2)) {
+                ux = h2(__hmul2(*reinterpret_cast<__half2 *>(&ux), z));
+                uy = h2(__hmul2(*reinterpret_cast<__half2 *>(&uy), z));
+            }
             if constexpr (P4) {
                 b.h[s][0] = ux;
                 b.h[s][1] = uy;
@@ -505,21 +530,28 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 }
             }
         }
-        if constexpr (F::SUMS) {   // over the lanes that share a block, a 32nd of them; lane t holds blocks 2 t and 2 t + 1
+        if constexpr (F::BLOCKS > 0) {   // over the lanes that share a block, a 32nd of them
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < F::BLOCKS; ++i) {
                 sums[i] += __shfl_xor_sync(0xffffffffu, sums[i], 1);
                 sums[i] += __shfl_xor_sync(0xffffffffu, sums[i], 2);
                 sums[i] *= 0.03125f;
             }
-            float a[2];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) a[j] = t == 0 ? sums[j] : t == 1 ? sums[2 + j] : t == 2 ? sums[4 + j] : sums[6 + j];
-            const __half2 hh = __floats2half2_rn(a[0], a[1]);
-            const float2 r = __half22float2(hh);
-            const __half2 ll = __floats2half2_rn((a[0] - r.x) * (SCALED ? CO_LOW : 1.0f), (a[1] - r.y) * (SCALED ? CO_LOW : 1.0f));
-            b.sum_h = h2(lo_lane ? ll : hh);
-            if constexpr (!P4) b.sum_l = h2(ll);
+            for (int i = 0; i < F::BLOCKS / 8; ++i) {
+                float a[2];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    constexpr int N = F::BLOCKS / 4;   // blocks of a lane
+                    const int o = F::BLOCKS == 8 ? j : 2 * j + i;
+                    a[j] = t == 0 ? sums[o] : t == 1 ? sums[N + o] : t == 2 ? sums[2 * N + o] : sums[3 * N + o];
+                }
+                const __half2 hh = __floats2half2_rn(a[0], a[1]);
+                const float2 r = __half22float2(hh);
+                const __half2 ll = __floats2half2_rn((a[0] - r.x) * LOW, (a[1] - r.y) * LOW);
+                b.sum_h[i] = h2(lo_lane ? ll : hh);
+                if constexpr (!P4) b.sum_l = h2(ll);
+            }
         }
     }
     pdl_launch_dependents();
@@ -542,7 +574,7 @@ __global__ void __launch_bounds__(32 * CO_WARPS, 1) quant_cols(const ColsArgs g)
                 const uint32_t at = red0 + parity * red_bytes + 4u * (uint32_t) ((((i - i0) << g.wr_log) + rg) * g.wk + kp) * TILE;
                 if constexpr (P4) {   // high and low parts' products: columns j and j + 4 (lanes t and t + 2)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], 2) * (1.0f / CO_LOW);
+                    for (int j = 0; j < 4; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], 2) * (F::OFFSET ? 1.0f : 1.0f / CO_LOW);
                 }
                 if constexpr (F::FINE) {   // the third part's products: column 1
                     sum[0] = fmaf(sum[1], 1.0f / (CO_LOW * CO_LOW), sum[0]);
@@ -648,7 +680,7 @@ int launch_cols(cudaStream_t s, const ColsArgs & g) { return g.m <= 4 ? launch_c
 
 }  // namespace
 
-// The full 16-row tiles of a packed tensor, 1..8 columns; `fine`: one column of Q6_K with the 24 bits of its activations.  *handled = false (and ST_OK) for
+// The full 16-row tiles of a packed tensor, 1..8 columns; `fine`: one column of Q6_K with the 24 bits of its activations, where f32 kernels would serve it.  *handled = false (and ST_OK) for
 // rows that are not whole units, or longer than four CTAs' units: larger clusters leave too many SMs idle (28672 x 8192, Q6_K, 1 column: 122 us with
 // clusters of 7, the f32 kernel 66).
 int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64_t n, const float * x, int64_t ldx, int64_t m, float * y, int64_t ldy, bool fine, bool * handled) {
@@ -674,7 +706,7 @@ int quant_cols_tiles(cudaStream_t s, int dtype, const void * w, int64_t k, int64
         case DT_Q4_0: return launch_cols<CoB32<false>>(s, g);
         case DT_Q8_0: return launch_cols<CoB32<true>>(s, g);
         case DT_Q4_K: return launch_cols<CoQ4K>(s, g);
-        case DT_Q6_K: return fine && m == 1 ? launch_cols<CoQ6K<true>, true>(s, g) : launch_cols<CoQ6K<false>>(s, g);
+        case DT_Q6_K: return m > 1 ? launch_cols<CoQ6K<Q6K_TWO_PARTS>>(s, g) : fine ? launch_cols<CoQ6K<Q6K_FINE>, true>(s, g) : launch_cols<CoQ6K<Q6K_OFFSET>, true>(s, g);
     }
     *handled = false;
     return ST_OK;
