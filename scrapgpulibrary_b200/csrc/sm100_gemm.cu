@@ -341,7 +341,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc(const GemmArgs g) {
 // (K > 32768) take the two-pass path: the same loop twice.
 // What bounds it is the number of CTAs and of bytes in flight: few float4 a thread (V = 4 up to K = 4096) and so many CTAs, of few registers each, rather than
 // eight tokens a CTA with 32 float4 a thread.  Products of 77 tokens (Q4_0, 4096 x 5003):
-// 23.2 -> 21.1 us, of 512 (Q8_0, 4096 x 12288) 74.0 -> 73.0; the preparation alone, cold, 6.5 -> 4.1 and 8.0 -> 6.0.
+// 23.2 -> 21.1 us behind one another (inputs that no cache holds: no gain), of 512 (Q8_0, 4096 x 12288) no more than repeated timing differs by; the preparation alone, cold,
+// 6.5 -> 4.1 and 8.0 -> 6.0.
 constexpr int PREP_MAX_V = 32;
 
 // `order`: places of the groups of four weights in a chunk (pos4 of the weight source): 0 = in order of K, 1 = as Q8_0 and F16

@@ -598,7 +598,7 @@ static int matvec_dispatch(cudaStream_t s, int layout, const void * w, int64_t w
 static int64_t q6k_imma_limit(int64_t k) { return k <= 4096 ? (int64_t) 64 << 20 : (int64_t) 20 << 20; }
 
 // Does the column kernel (sm100_cols.cu) take this product?  Where the integer kernels, the split GEMM, or with Q6_K and one column the f32
-// kernels were slower; not where f32 kernels serve a batch, whose error (2e-7) is below its own (up to 1.3e-6).  Measured over 250 shapes, K x N, us, before / after:
+// kernels were slower; not where f32 kernels serve a batch.  Measured over 7202 shapes, K x N, us, before / after:
 //   Q4_0  4 columns   4096 x 1024 9.0 / 5.5, 4096 x 12288 27.5 / 10.4, 12288 x 4096 24.5 / 12.5;  8 columns 9.1 / 5.7, 28.1 / 13.5, 25.1 / 15.1; Q8_0 alike
 //         1 column    the integer kernel is at its best where K is a multiple of 4096: 4096 x 4096 5.4 / 6.0, 8192 x 8192 11.5 / 12.3, 12288 x 4096 10.2 / 12.0, but
 //                     12288 x 1024 8.6 / 6.4; else 5120 x 6144 11.1 / 9.0, 7168 x 12288 21.2 / 15.2, 3072 x 6144 7.4 / 6.2, 6144 x 2048 7.2 / 6.2; 6144 x 4096 7.5 / 9.4,
@@ -606,12 +606,14 @@ static int64_t q6k_imma_limit(int64_t k) { return k <= 4096 ? (int64_t) 64 << 20
 //   Q4_K  2..4 columns  the integer kernels' launches overlap in a graph; three layers' projections, hidden / FFN, 4 columns 2048 / 6144 47.3 / 52.4, 4096 / 12288 86.1 / 87.8,
 //                     4864 / 12288 126 / 133, 5120 / 14336 146 / 117 (single launches 4096 x 4096 8.2 / 6.7, 6144 x 14336 20.1 / 15.5, 12288 x 14336 32.5 / 32.3)
 //         5..8 columns  the same graphs, 8 columns 57.4 / 57.8, 126 / 120, 5120 / 14336 224 / 147; single launches 4096 x 4096 8.0 / 7.6, 10240 x 6144 33.5 / 20.3,
-//                     12288 x 4096 21.8 / 15.1; the one loss seen is 5 columns at 3840 / 11264, 115 / 123 (8 columns 121 / 120)
+//                     12288 x 4096 21.8 / 15.1; slower with 2560 to 4608 rows, one round of the integer kernel (4864 x 4096 7.6 / 8.6, at most 15 %), and stays
+//                     for its accuracy (1e-6, the integer kernel 4e-5)
 //   Q6_K  1 column    4096 x 1024 7.0 / 5.9, 4096 x 12288 16.6 / 13.2, 2048 x 4096 5.1 / 5.8, 7168 x 8192 81.7 / 17.1 (an f32 kernel for rows of any length before);
 //                     in the streaming kernel 6144 x 4096 9.1 / 11.3, 8192 x 8192 20.6 / 17.0, 8192 x 4096 11.2 / 11.8, 8192 x 5003 13.1 / 18.6, 12288 x 4096 12.4 / 16.2,
 //                     4096 x 151936 123 / 124; 512 x 12288 4.7 / 5.5
 //         4 columns   4096 x 4096 13.2 / 8.2, 4096 x 12288 29.7 / 13.8, 12288 x 4096 31.6 / 17.2;  8 columns 15.4 / 9.3, 34.4 / 17.8, 32.1 / 21.2
-// Below 4096 rows five to eight columns stay with the split GEMM, where a column's result does not depend on its batch.
+// Below 4096 rows five to eight columns stay with the split GEMM although it is slower (4096 x 1024, 8 columns 9.1 / 5.7): a column there has the same bits in every batch of 5 to 32,
+// and a test holds them to that.  From 4096 rows on it has them with SM100_QUANT_COLS=0.
 static bool cols_win(int dtype, int64_t k, int64_t n, int64_t m, bool split_wins) {
     if (n < (split_wins && m >= 5 ? 4096 : 1024)) return false;
     switch (dtype) {

@@ -1,8 +1,8 @@
 """GPU parity of the column kernel (packed weights, up to 8 columns, integers times two f16 numbers on mma.sync) against float64.
 
 Tolerance: activations have 22 bits (2^-23), block scales and block sums are f32; the tensor core truncates its sums (2^-23 of the
-largest term, two to four MMAs a block), and the integers' offsets (8, 32, 128, the minima of Q4_K) make the terms up to three times as large as what is left of
-them: 3 (2^-23 + 4 2^-23) is 1.8e-6 at most per block, measured 2e-7 to 1.3e-6 over whole rows.  Bound: 4e-6, so NMSE 1.6e-11.
+largest term, two to four MMAs a block), and the minima of Q4_K (and the offset of 32 in the form of Q6_K that keeps it) make the terms up to three times as large as
+what is left of them: 3 (2^-23 + 4 2^-23) is 1.8e-6 at most per block, measured 8e-8 to 1.4e-6 over whole rows.  Bound: 4e-6, so NMSE 1.6e-11.
 """
 import numpy as np
 import pytest
